@@ -114,20 +114,19 @@ int svpf_clip_analyse_device(const svpf_analyser *a, const uint8_t *supers_dev, 
 /* Status of the last device launch that used `scratch_dev` (synchronises `stream`):
  * SVPF_OK, or SVPF_EPANIC when a pair hit an input the reference cannot process. */
 int svpf_device_status(const void *scratch_dev, void *stream);
-/* No counterpart in the reference (a tuning knob). Level 0 runs with look-ahead by default:
+/* No counterpart in the reference (a tuning knob). Levels run with look-ahead by default:
  * each warp of a search direction takes its own block in the reference's order, searches it
- * without the neighbour vectors not yet committed, then, in order, re-checks the reference's
- * selection with them and repeats the refinement when one wins; results are bit-identical
- * with it on or off. `levels` is a bit set: 1 level 0, 2 the coarser levels, 4 level 0 spread
- * over the GPU (with 1: a launch of its own with one CTA per warp, so every SM carries the same
- * share of the walking warps; the pair kernel and a finish kernel run before and after it).
- * 0 turns it off; the default is 5. Only the 128-thread launch shape with two CTAs per SM runs
- * it (the plain path's shape for launches of at most two frame pairs per SM); the others always
- * keep the serial order. Affects launches made after the call. */
+ * with the neighbour vectors published so far and repeats the refinement when a later one
+ * changes the reference's selection; results are bit-identical with it on or off. `levels` is
+ * a bit set: 1 level 0, 2 the coarser levels, 4 (with 1) every level but the smallest ones
+ * spread over the GPU in launches of their own, one CTA per warp, so every SM carries the same
+ * share of the warps and a single pair still fills many of them. 0 turns it off; the default
+ * is 5. Only the plain path and the server run it; batches always keep the serial order within
+ * a pair. Affects launches made after the call. */
 int svpf_analyser_set_lookahead(svpf_analyser *a, int32_t levels);
 /* The look-ahead counters of the last device launch on `scratch_dev` (synchronises `stream`):
- * out[0] level-0 blocks, out[1] blocks with deferred neighbour seeds, out[2] deferred seeds
- * evaluated, out[3] refinements run again. */
+ * out[0] level-0 blocks, out[1] blocks that started before all their neighbour seeds were final,
+ * out[2] seeds evaluated after the start, out[3] blocks whose refinement ran again. */
 int svpf_device_lookahead_stats(const void *scratch_dev, void *stream, int64_t out[4]);
 /* No counterpart in the reference. The same Analyse over a clip as
  * svpf_clip_analyse_device, for callers that cannot allocate device memory (a frame

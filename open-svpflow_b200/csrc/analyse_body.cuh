@@ -5,37 +5,37 @@
 // direction, SVPF_MINB = resident CTAs per SM the register budget is cut for (2, 4, 8: 128
 // registers per thread; 3, 6: 80), SVPF_VARIANT = the variant's namespace. Each variant
 // exports a plain launcher (one CTA per pair; in the look-ahead shapes, by default, the pair
-// kernel runs the coarser levels, a cooperative level-0 kernel with one CTA per warp walks
-// level 0 across the SMs and a finish kernel packs the payloads) and a persistent batch
+// kernel only makes the ground for each level, a cooperative walk kernel with one CTA per warp
+// searches it across the SMs, and a pack kernel writes the payloads) and a persistent batch
 // launcher (CTAs drain a device work queue of frame pairs from many clips).
 //
 // Restates crates/svpflow1/src/analyse_search.rs:68-2811 for the GPU:
-//   * one CTA per frame pair; its two halves (NT threads each) run the forward search
-//     (current -> reference) and the backward search (reference -> current). They meet
-//     at a CTA barrier once per level: the forward search of a level needs the
-//     backward field of the level above projected onto it, and vice versa (:128-191).
+//   * a frame pair has a forward search (current -> reference) and a backward search
+//     (reference -> current), which meet once per level: the forward search of a level
+//     needs the backward field of the level above projected onto it, and vice versa (:128-191).
 //   * inside a level the blocks run in the reference's serial order (serpentine at
 //     level 0, score-sorted at coarser levels, :302-419): each block takes already
-//     searched neighbours as candidates, so the order is a true dependency chain and
-//     its latency is what the design minimises. Every thread of a half holds the same
-//     block state and takes the same decisions, so a search step costs one barrier.
+//     searched neighbours as candidates, so the order is a true dependency chain. walk_level
+//     keeps many blocks of it in flight, one per warp, and is exact all the same; search_level
+//     takes them one by one, all warps of a direction on the same block (the batch kernel, the
+//     smallest levels, inputs on which the reference panics).
 //   * every step of a block's search is a batch of candidate vectors whose positions are
 //     known before any is evaluated (special candidates; the UMH cross + hexagons; an
-//     exhaustive square; a hexagon step; an expanding ring). A candidate is evaluated by
-//     a group of G lanes of one warp, one 4x4 tile per lane (SATD, SAD or pixel sums),
-//     reduced with shuffles; each warp keeps the first candidate of minimal cost and
-//     the half combines its warps after the step's barrier. First-minimum equals the
-//     reference's sequential `if cost < best.cost` scan (:1122-1155) whenever
-//     cost >= motion penalty, i.e. pnew >= -256; below that the step replays the
-//     sequential scan over each round's costs.
+//     exhaustive square; a hexagon step; an expanding ring), 32 at a time, one per lane. The
+//     lanes test their candidates and set them up side by side, the whole warp evaluates
+//     those that pass one after another (eval_cands), and the first of minimal cost is kept.
+//     First-minimum equals the reference's sequential `if cost < best.cost` scan (:1122-1155)
+//     whenever cost >= motion penalty, i.e. pnew >= -256; below that the step replays the
+//     sequential scan over the costs.
 //   * a candidate whose block and reference block lie inside their planes takes the fast
-//     path (word loads, packed byte ops); any other candidate takes the reference's own
-//     read path (edge-shifted, clamped, masked; :1638-2351) through cand_setup, which
-//     keeps the reference's wrapping index arithmetic.
+//     path, one whose reference block reaches out of a plane a clamped form of it
+//     (clamped_cands); any other candidate takes the reference's own read path (edge-shifted,
+//     clamped, masked; :1638-2351) through cand_setup, which keeps the reference's wrapping
+//     index arithmetic.
 //
-// Integer/indexing work: no tensor cores. 8-bit SATD runs in f16x2 on values that halves hold
-// exactly (see satd_rows_h); the two f64 formulas (adapt_lambda, exact_lambda) are IEEE-exact
-// (exact_lambda is host-precomputed).
+// SATD is a contraction with the 16x16 Sylvester matrix and runs on the tensor cores, exactly (see
+// the fast path); the two f64 formulas (adapt_lambda, exact_lambda) are IEEE-exact (exact_lambda is
+// host-precomputed).
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -46,11 +46,9 @@
 #if !defined(SVPF_NT) || !defined(SVPF_MINB) || !defined(SVPF_VARIANT)
 #error "define SVPF_NT, SVPF_MINB and SVPF_VARIANT before including analyse_body.cuh"
 #endif
-// SVPF_LOOKAHEAD: the shape runs the look-ahead (search_level_spec) when the parameter block asks
-// for it. Only the 128-thread shapes with two CTAs per SM (128 registers) do: there it measured
-// faster (the 1080p clip: 125.2 -> 134.3 pairs/s); with three CTAs per SM at 80 registers the
-// independent warps' instruction fetches cost more than the overlap gains (297 pairs at 960x540:
-// 593 -> 692 ms), so the other shapes keep the serial order.
+// SVPF_LOOKAHEAD: the shape's plain launcher walks the levels (walk_level) when the parameter block
+// asks for it. Only the 128-thread shapes with 128 registers do: the plain path and the server take
+// them; the others serve batches, whose queue keeps every CTA busy with pairs of its own.
 #ifndef SVPF_LOOKAHEAD
 #define SVPF_LOOKAHEAD 0
 #endif
@@ -72,10 +70,6 @@ constexpr unsigned DC_SHIFT = 0;
 constexpr int NT = SVPF_NT;        // threads per search direction
 static_assert(NT == 32 || NT == 64 || NT == 128, "threads per direction");
 constexpr int NW = NT / 32;
-static_assert(NW <= 4, "the look-ahead keeps at most NW - 1 = 3 deferred seeds per block");
-constexpr int NGMAX = NW * 32;     // candidate groups of a direction when a group is one lane
-constexpr int MAXSLOT = 16;        // special-candidate slots of a block
-constexpr int MW = 4;              // validity mask words per chunk of a search step: 128 candidates
 
 enum : uint8_t { LM_DIRECT = 1, LM_SATD_MASK = 2, LM_SAD_BREAK = 3, LM_EDGE = 4, LM_DC = 5 };
 enum : uint8_t { CM_NONE = 0, CM_DIRECT = 1, CM_SAD_BREAK = 3, CM_EDGE = 4 };
@@ -103,37 +97,24 @@ struct Cand {
 // entries are those of its first warp (Ctx::wbase). W: the warps it holds state for (the
 // direction's, or one for a CTA of the level-0 kernel).
 template <int W>
-struct DirShT {
-    // Groups that stage a block's source at once: one per warp with the look-ahead, else one per
-    // direction (shared memory not used for staging is L1 cache for the rest).
-    static constexpr int kSrc = (SVPF_LOOKAHEAD && W > 1) ? W : 1;
+struct alignas(16) DirShT {
     long long K[2][W];                    // per-warp best (cost, index, sad) of a step, double-buffered
     int I[2][W];
     unsigned S[2][W];
-    unsigned slotL[W][2][MAXSLOT];        // per group: special-candidate results (exact_sad values)
-    long long rk[2][W * 32], rm[2][W * 32];  // exact sequential scan: per-group cost, motion
-    unsigned rs[2][W * 32];
-    int ri[2][W * 32];
-    unsigned char rv[2][W * 32];
-    int committed;                        // look-ahead: blocks of the level committed so far (in order)
-    int late_;                            // look-ahead: a hand-over wait gave up
-    int unsafe_;                          // look-ahead: the level has an input the reference panics on
-    int bad_count;                        // look-ahead: bad-SAD blocks committed so far (:605)
+    unsigned slot[2][32];                 // special candidates' exact_sad, shared by a group's warps
+    unsigned dc[2][W], dcs[2], score[2];  // a block's luma sum (per warp; on the general path), its predictor's re-score
+    long long rk[2][32];                  // exact sequential scan: the costs of 32 candidates
+    unsigned rs[2][32];
+    int unsafe_;                          // the level has an input the reference panics on
     int gx, gy;           // global predictor (doubled) for the next level
     int order_len;
     int abort_;
-    // Per group: the block's source pixels, 4 per entry: luma (bw/4 x bh), then U and V
-    // (cw/4 x crows). A plane searched with SATD holds biased f16 pairs (8-bit samples; see
-    // satd_rows_h) or 16-bit pairs (x = pixels 0,1; y = pixels 2,3), a SAD plane the packed word in x.
-    uint2 srcp[kSrc][384];
-    int2 clist[W][32 * MW];  // per warp: the step's candidates passing the cuts, in order (mv, index)
-    int2 seedv[W][8];        // look-ahead, per group: the block's seeds evaluated at once (vector) ...
-    int seedq[W][8];         // ... and their places among the block's processed neighbours;
-    long long defc[W][3];    // the deferred seeds' cells (at most NW - 1 = 3) ...
-    int defq[W][3];          // ... and places
     long long r64[W][3];
     int r32[W][2];
 };
+// After the directions' DirShT, per warp of each: the block's staged source (512 bytes per group of
+// eight tiles) and the group's offsets (128 bytes), AnalyseParams::stage_groups of each.
+constexpr int kGroupBytes = 640;
 using DirSh = DirShT<NW>;  // a search direction of the pair kernels
 using WarpSh = DirShT<1>;  // a CTA (one warp) of the level-0 kernel
 
@@ -471,191 +452,88 @@ __device__ unsigned chroma_tile1(const Cand &c, const px_t *sp, const px_t *rp, 
 
 // -------------------------------------------------------------------------------------------
 // Fast path: candidates whose source and reference blocks lie inside their planes.
-// Samples are read as 32-bit words from 4-byte aligned addresses and funnel-shifted; the
-// caller guarantees 8 readable samples after the first sample of every row (see fast_setup).
 //
-// SATD runs in packed halfwords: a row's four sample differences are two halfword pairs
-// (samples 0,1 and 2,3); the horizontal 4-point transform runs inside the pairs, the vertical
-// one across the rows, and the last vertical stage with its absolute values is
-// |a+b| + |a-b| = 2 max(|a|, |b|), as in hadamard4. Every intermediate fits a signed halfword
-// (|value| <= 8 * max sample) and the four-row sum an unsigned one.
-__device__ __forceinline__ unsigned satd_rows(const uint32_t d01[4], const uint32_t d23[4]) {
-    uint32_t h0[4], h1[4];
-#pragma unroll
-    for (int r = 0; r < 4; r++) {
-        const uint32_t c = __vadd2(d01[r], d23[r]), e = __vsub2(d01[r], d23[r]);
-        const uint32_t p = __byte_perm(c, e, 0x5410), q = __byte_perm(c, e, 0x7632);
-        h0[r] = __vadd2(p, q);
-        h1[r] = __vsub2(p, q);
-    }
-    uint32_t acc = 0;
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-        const uint32_t *h = k ? h1 : h0;
-        const uint32_t a0 = __vadd2(h[0], h[1]), a1 = __vsub2(h[0], h[1]);
-        const uint32_t a2 = __vadd2(h[2], h[3]), a3 = __vsub2(h[2], h[3]);
-        acc = __vadd2(acc, __vmaxu2(__vabs2(a0), __vabs2(a2)));
-        acc = __vadd2(acc, __vmaxu2(__vabs2(a1), __vabs2(a3)));
-    }
-    return 2u * ((acc & 0xFFFFu) + (acc >> 16));
-}
-__device__ __forceinline__ uint32_t pairs_lo(uint32_t w) { return __byte_perm(w, 0u, 0x4140); }  // bytes 0, 1
-__device__ __forceinline__ uint32_t pairs_hi(uint32_t w) { return __byte_perm(w, 0u, 0x4342); }  // bytes 2, 3
+// One warp evaluates one candidate at a time. Its 4x4 tiles (luma, then U, then V) are taken in
+// groups of eight: lane 4 n + r loads the four samples of row r of the group's tile n as 32-bit
+// words from 4-byte aligned addresses, funnel-shifted (the caller guarantees 8 readable samples
+// after the first sample of every row, see fast_setup), so a load touches the eight rows of a
+// group once instead of one row of each of up to 32 candidates.
+//
+// SATD of a group is one tensor-core instruction: the 4x4 Hadamard transform of a tile is the
+// 16x16 Sylvester matrix times its 16 samples, so mma.m16n8k16 gives H ref for eight tiles, with
+// -H src (made once per block, stage_source) as its accumulator, and the warp sums the absolute
+// values of the 128 results. Exact: a sample s goes in as the half 1024 + s (one byte permute; the
+// bias is the same in src and ref and cancels), H holds +-1, products and sums are integers below
+// 2^15 and accumulate in f32. The coefficients' order and signs do not matter to the sum. SAD of a
+// group is a packed byte difference per lane.
+//
+// What it measured: see eval_cands.
+constexpr unsigned kFull = 0xFFFFFFFFu;
+constexpr float kIntBias = 8388608.f;  // 2^23: the low bits of such a float are the integer added to it
 
-#ifndef SVPF_PX16
-// 8-bit SATD runs in f16x2 instead: a sample s becomes the half 1024 + s (exponent of 1024,
-// s in the mantissa: one byte permute), so a difference of two samples is exact, and so is
-// every later value (integers of magnitude <= 8 * 255 = 2040 <= 2048, where halves are
-// exact). The four-row sums go to f32. Same arithmetic as satd_rows, fewer instructions
-// (the f16x2 add / sub / max are single instructions; |x| clears the sign bits).
-__device__ __forceinline__ uint32_t bias_lo(uint32_t w) { return __byte_perm(w, 0x64646464u, 0x4140); }
-__device__ __forceinline__ uint32_t bias_hi(uint32_t w) { return __byte_perm(w, 0x64646464u, 0x4342); }
-__device__ __forceinline__ uint32_t h2add(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-}
-__device__ __forceinline__ uint32_t h2sub(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-}
-__device__ __forceinline__ uint32_t h2max(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("max.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-}
-__device__ __forceinline__ uint32_t h2abs(uint32_t a) { return a & 0x7FFF7FFFu; }
-// acc + both halves of h, in f32 (sm_100 mixed-precision add)
-__device__ __forceinline__ float f32_add_h2(float acc, uint32_t h) {
-    asm("{.reg .b16 l, h; mov.b32 {l, h}, %1; add.rn.f32.f16 %0, l, %0; add.rn.f32.f16 %0, h, %0;}"
-        : "+f"(acc) : "r"(h));
-    return acc;
-}
-// d01 / d23: the rows' differences as f16 pairs (samples 0,1 and 2,3)
-__device__ __forceinline__ unsigned satd_rows_h(const uint32_t d01[4], const uint32_t d23[4]) {
-    uint32_t h0[4], h1[4];
-#pragma unroll
-    for (int r = 0; r < 4; r++) {
-        const uint32_t c = h2add(d01[r], d23[r]), e = h2sub(d01[r], d23[r]);
-        const uint32_t p = __byte_perm(c, e, 0x5410), q = __byte_perm(c, e, 0x7632);
-        h0[r] = h2add(p, q);
-        h1[r] = h2sub(p, q);
-    }
-    float acc = 0.f;
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-        const uint32_t *h = k ? h1 : h0;
-        const uint32_t a0 = h2add(h[0], h[1]), a1 = h2sub(h[0], h[1]);
-        const uint32_t a2 = h2add(h[2], h[3]), a3 = h2sub(h[2], h[3]);
-        acc = f32_add_h2(acc, h2max(h2abs(a0), h2abs(a2)));
-        acc = f32_add_h2(acc, h2max(h2abs(a1), h2abs(a3)));
-    }
-    return 2u * (unsigned)acc;
-}
-__device__ __forceinline__ uint32_t ld4u(const uint8_t *p) {
+struct Smp {  // four samples: 8-bit, the word in a; 16-bit, two halfword pairs
+    uint32_t a, b;
+};
+// A frame as the fast path reads it: its first sample's address rounded down to a word, and the bytes
+// that took off. Offsets are bytes from there, below 2^32 (planes are below 2^30 samples).
+struct Frame {
+    const char *p;
+    unsigned mis;
+};
+__device__ __forceinline__ Frame frame_of(const px_t *p) {
     const uintptr_t a = (uintptr_t)p;
-    const uint32_t *q = reinterpret_cast<const uint32_t *>(a & ~(uintptr_t)3);
-    return __funnelshift_r(__ldg(q), __ldg(q + 1), (unsigned)(a & 3) * 8u);
+    return Frame{(const char *)(a & ~(uintptr_t)3), (unsigned)(a & 3)};
 }
-// four samples as biased f16 pairs
-__device__ __forceinline__ uint2 ld4h(const px_t *p) {
-    const uint32_t w = ld4u(p);
-    return make_uint2(bias_lo(w), bias_hi(w));
+__device__ __forceinline__ const uint32_t *word_at(const Frame &f, unsigned o) {
+    return reinterpret_cast<const uint32_t *>(f.p + (size_t)(o & ~3u));
 }
-// The staged entry of 4 source samples for a plane searched with SATD (biased f16 pairs) or
-// SAD (the packed word).
-__device__ __forceinline__ uint2 stage4(const px_t *p, bool satd) {
-    const uint32_t w = ld4u(p);
-    return satd ? make_uint2(bias_lo(w), bias_hi(w)) : make_uint2(w, 0u);
+#ifndef SVPF_PX16
+__device__ __forceinline__ Smp ld4(const Frame &f, unsigned o) {
+    const uint32_t *q = word_at(f, o);
+    return Smp{__funnelshift_r(__ldg(q), __ldg(q + 1), o * 8u), 0u};  // the shift counts modulo 32
 }
-__device__ __forceinline__ unsigned sad4(uint2 staged, const px_t *rp) {
-    return __dp4a(__vabsdiffu4(staged.x, ld4u(rp)), 0x01010101u, 0u);
+// the samples as biased halves (samples 0,1 and 2,3)
+__device__ __forceinline__ void halves(const Smp &w, uint32_t &lo, uint32_t &hi) {
+    lo = __byte_perm(w.a, 0x64646464u, 0x4140);
+    hi = __byte_perm(w.a, 0x64646464u, 0x4342);
 }
-__device__ __forceinline__ unsigned sad4g(const px_t *sp, const px_t *rp) {
-    return __dp4a(__vabsdiffu4(ld4u(sp), ld4u(rp)), 0x01010101u, 0u);
+// acc + |s - r| summed where m is all ones (0: acc)
+__device__ __forceinline__ unsigned sad4(const Smp &s, const Smp &r, unsigned m, unsigned acc) {
+    return __dp4a(__vabsdiffu4(s.a, r.a), m & 0x01010101u, acc);
 }
-__device__ __forceinline__ unsigned sum4(const px_t *p) { return __dp4a(ld4u(p), 0x01010101u, 0u); }
+__device__ __forceinline__ unsigned sum4(const Smp &s) { return __dp4a(s.a, 0x01010101u, 0u); }
 #else
 // four 16-bit samples (2-byte aligned): three aligned words funnel-shifted into two pairs
-__device__ __forceinline__ uint2 ld4p(const px_t *p) {
-    const uintptr_t a = (uintptr_t)p;
-    const uint32_t *q = reinterpret_cast<const uint32_t *>(a & ~(uintptr_t)3);
-    const unsigned sh = (unsigned)(a & 3) * 8u;
+__device__ __forceinline__ Smp ld4(const Frame &f, unsigned o) {
+    const uint32_t *q = word_at(f, o);
     const uint32_t w0 = __ldg(q), w1 = __ldg(q + 1), w2 = __ldg(q + 2);
-    return make_uint2(__funnelshift_r(w0, w1, sh), __funnelshift_r(w1, w2, sh));
+    return Smp{__funnelshift_r(w0, w1, o * 8u), __funnelshift_r(w1, w2, o * 8u)};
 }
-__device__ __forceinline__ uint2 stage4(const px_t *p, bool) { return ld4p(p); }
-__device__ __forceinline__ unsigned sad4(uint2 staged, const px_t *rp) {
-    const uint2 r = ld4p(rp);
-    return __vsadu2(staged.x, r.x) + __vsadu2(staged.y, r.y);
+// samples 0..1023 fit the mantissa of 1024 + s too
+__device__ __forceinline__ void halves(const Smp &w, uint32_t &lo, uint32_t &hi) {
+    lo = w.a | 0x64006400u;
+    hi = w.b | 0x64006400u;
 }
-__device__ __forceinline__ unsigned sad4g(const px_t *sp, const px_t *rp) { return sad4(ld4p(sp), rp); }
-__device__ __forceinline__ unsigned sum4(const px_t *p) {
-    const uint2 w = ld4p(p);
-    return (w.x & 0xFFFFu) + (w.x >> 16) + (w.y & 0xFFFFu) + (w.y >> 16);
+__device__ __forceinline__ unsigned sad4(const Smp &s, const Smp &r, unsigned m, unsigned acc) {
+    return acc + ((__vsadu2(s.a, r.a) + __vsadu2(s.b, r.b)) & m);
 }
+__device__ __forceinline__ unsigned sum4(const Smp &s) { return (s.a & 0xFFFFu) + (s.a >> 16) + (s.b & 0xFFFFu) + (s.b >> 16); }
 #endif
 
-// tiles with both blocks in global memory (special candidates)
-__device__ __forceinline__ unsigned tile_satd(const px_t *sp, const px_t *rp, int st) {
-    uint32_t d01[4], d23[4];
-#ifndef SVPF_PX16
-#pragma unroll
-    for (int r = 0; r < 4; r++) {
-        const uint2 a = ld4h(sp + r * st), b = ld4h(rp + r * st);
-        d01[r] = h2sub(a.x, b.x);
-        d23[r] = h2sub(a.y, b.y);
-    }
-    return satd_rows_h(d01, d23);
-#else
-#pragma unroll
-    for (int r = 0; r < 4; r++) {
-        const uint2 a = ld4p(sp + r * st), b = ld4p(rp + r * st);
-        d01[r] = __vsub2(a.x, b.x);
-        d23[r] = __vsub2(a.y, b.y);
-    }
-    return satd_rows(d01, d23);
-#endif
+// This lane's part of the Sylvester matrix as the A operand of mma.m16n8k16: row m is coefficient
+// (m / 4, m % 4), column k < 8 is sample (k / 2, k % 2) of a tile and k >= 8 sample ((k - 8) / 2,
+// 2 + k % 2), the order in which a lane's two B registers hold its row.
+__device__ __forceinline__ uint32_t hadamard_pair(int m, int k) {  // columns k, k + 1 (k even)
+    const int r = (k & 7) >> 1, q = k >= 8 ? 2 : 0, mr = m >> 2, mq = m & 3;
+    const int s0 = __popc(mr & r) + __popc(mq & q), s1 = __popc(mr & r) + __popc(mq & (q + 1));
+    return ((s0 & 1) ? 0xBC00u : 0x3C00u) | (((s1 & 1) ? 0xBC00u : 0x3C00u) << 16);
 }
-__device__ __forceinline__ unsigned tile_sad(const px_t *sp, const px_t *rp, int st) {
-    unsigned s = 0;
-#pragma unroll
-    for (int r = 0; r < 4; r++) s += sad4g(sp + r * st, rp + r * st);
-    return s;
-}
-// tiles over the staged source (see DirSh::srcp)
-__device__ __forceinline__ unsigned tile_satd_p(const uint2 *sp, int spp, const px_t *rp, int st) {
-    uint32_t d01[4], d23[4];
-#ifndef SVPF_PX16
-#pragma unroll
-    for (int r = 0; r < 4; r++) {
-        const uint2 a = sp[r * spp], b = ld4h(rp + r * st);
-        d01[r] = h2sub(a.x, b.x);
-        d23[r] = h2sub(a.y, b.y);
-    }
-    return satd_rows_h(d01, d23);
-#else
-#pragma unroll
-    for (int r = 0; r < 4; r++) {
-        const uint2 a = sp[r * spp], b = ld4p(rp + r * st);
-        d01[r] = __vsub2(a.x, b.x);
-        d23[r] = __vsub2(a.y, b.y);
-    }
-    return satd_rows(d01, d23);
-#endif
-}
-__device__ __forceinline__ unsigned tile_sad_p(const uint2 *sp, int spp, const px_t *rp, int st) {
-    unsigned s = 0;
-#pragma unroll
-    for (int r = 0; r < 4; r++) s += sad4(sp[r * spp], rp + r * st);
-    return s;
-}
-__device__ __forceinline__ unsigned tile_sum(const px_t *sp, int st) {
-    unsigned s = 0;
-#pragma unroll
-    for (int r = 0; r < 4; r++) s += sum4(sp + r * st);
-    return s;
+__device__ __forceinline__ float4 mma_hadamard(const uint4 &h, uint32_t lo, uint32_t hi, const float4 &c) {
+    float4 d;
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
+        : "=f"(d.x), "=f"(d.y), "=f"(d.z), "=f"(d.w)
+        : "r"(h.x), "r"(h.y), "r"(h.z), "r"(h.w), "r"(lo), "r"(hi), "f"(c.x), "f"(c.y), "f"(c.z), "f"(c.w));
+    return d;
 }
 
 // -------------------------------------------------------------------------------------------
@@ -721,9 +599,17 @@ struct Ctx {
     int level, d, tid, satd, pel;
     int nw, wbase;   // warps of the group searching the block, and its first warp in the direction;
                      // tid is the thread's index in that group
-    int grp_lanes;   // G: lanes per candidate (power of two)
     int pnew;        // new-candidate penalty of the current search (opts.pnew; pnew / factor in the refine pass)
-    int tl, tcp;     // 4x4 luma tiles, 4x4 tiles per chroma plane of one candidate
+    // the fast path's groups of eight tiles (set_groups): per-lane masks, one bit per group
+    int ng;          // groups
+    unsigned lmask, cmask;  // the lane's tile is a luma one, a chroma one (neither: the place is empty)
+    unsigned dlmask, dcmask;  // the same of the tile pair whose SATD sums the lane holds
+    unsigned smask;  // the group is searched with SATD (the same in every lane)
+    unsigned lshift; // halvings of the luma sum
+    Frame fs, fr;
+    uint4 h;         // hadamard_pair's registers
+    unsigned *off;   // [ng][32] shared: byte offset of the lane's row from the candidate's luma / U block
+    float4 *src;     // [ng][32] shared: the block's staged source (-H src, or the samples)
 };
 
 // Barrier of the group searching a block: the direction's named barrier, or the warp.
@@ -732,16 +618,63 @@ __device__ __forceinline__ void gsync(const Ctx &x) {
     else dbar(x.d);
 }
 
+// Whether chroma takes part in a level's costs.
+__device__ __forceinline__ bool has_chroma(const LevelInfo &L) { return !L.smallest && (L.bw >> 1) >= 4 && (L.bh >> 1) >= 4; }
+
+// The groups of eight 4x4 tiles of a candidate of x.L. Luma and chroma share groups when both are
+// searched the same way; square blocks searched with SATD are, others (luma SAD, chroma SATD) start
+// chroma at a group of its own. x.off is written by every warp with the same values.
+__device__ __forceinline__ void set_groups(Ctx &x) {
+    const LevelInfo &L = *x.L;
+    const int lane = x.tid & 31;
+    const int bw = L.bw, bh = L.bh, cw = bw >> 1, ch = bh >> 1;
+    const bool lsatd = x.satd && is_blk(bw) && is_blk(bh) && bw == bh, chroma = has_chroma(L);
+    const int tx = imax(bw >> 2, 1), tl = tx * imax(bh >> 2, 1), lgtx = 31 - __clz(tx);
+    const int crows = x.satd ? cw : ch, ctx = imax(cw >> 2, 1), lgctx = 31 - __clz(ctx), tc = chroma ? ctx * (crows >> 2) : 0;
+    const int c0 = lsatd == (x.satd != 0) && tl > 1 ? tl : (tl + 7) & ~7;  // chroma's first tile place
+    x.ng = chroma ? (c0 + 2 * tc + 7) >> 3 : (tl + 7) >> 3;
+    x.lmask = x.cmask = x.dlmask = x.dcmask = x.smask = 0;
+    // a single tile (4x4 blocks) fills both places of its pair and counts twice
+    const int tl2 = tl == 1 && lsatd ? 2 : tl;
+    x.lshift = (lsatd ? 1 : 0) + (tl2 - tl);
+    const int row = lane & 3;
+    for (int g = 0; g < x.ng; g++) {
+        const int t = g * 8 + (lane >> 2), dt = g * 8 + (lane & 3) * 2;
+        unsigned o = 0;  // an empty place reads the block's first row
+        if (t < tl2) {
+            x.lmask |= 1u << g;
+            if (t < tl) o = (unsigned)(((t >> lgtx) * 4 + row) * x.G.ys32 + (t & (tx - 1)) * 4);
+            else o = (unsigned)(row * x.G.ys32);
+        } else if (t >= c0 && t < c0 + 2 * tc) {
+            const int pl = t - c0 >= tc, ct = t - c0 - pl * tc;
+            x.cmask |= 1u << g;
+            o = (unsigned)(pl ? (unsigned)x.G.clen : 0u) + (unsigned)(((ct >> lgctx) * 4 + row) * x.G.cs32 + (ct & (ctx - 1)) * 4);
+        }
+        x.off[g * 32 + lane] = o * (unsigned)sizeof(px_t);
+        if (dt < tl2) x.dlmask |= 1u << g;
+        else if (dt >= c0 && dt < c0 + 2 * tc) x.dcmask |= 1u << g;
+        if (g * 8 < c0 ? lsatd : x.satd != 0) x.smask |= 1u << g;
+    }
+    const int m = lane >> 2, k = (lane & 3) * 2;
+    x.h = make_uint4(hadamard_pair(m, k), hadamard_pair(m + 8, k), hadamard_pair(m, k + 8), hadamard_pair(m + 8, k + 8));
+    __syncwarp();
+}
+
+// The staging area of a warp (see kGroupBytes): x.src that of the group's first warp, x.off its own.
+__device__ __forceinline__ void set_stage(Ctx &x, unsigned char *area, int groups, int first, int warp) {
+    x.src = reinterpret_cast<float4 *>(area + (size_t)first * groups * kGroupBytes);
+    x.off = reinterpret_cast<unsigned *>(area + (size_t)warp * groups * kGroupBytes + (size_t)groups * 512);
+}
+
 // Per-block constants, identical in every thread of a direction.
 struct BlkC {
     int px, py, bw, bh, px2, py2;
-    int bnd0, bnd1, bnd2, bnd3, ubx, uby;  // mv_bounds; ub = bound above which the edge shift starts
-    int chroma, satd_mode, fastable, fast_src, cfast_src, dc_fast;
-    int cw, ch, crows, cpx, cpy, tilesx, ctilesx;
-    int lgtx, lgctx;                       // log2 of tilesx / ctilesx (block sizes are powers of two)
+    int bnd0, bnd1, bnd2, bnd3;            // mv_bounds
+    int chroma, fast_src;
     int fx0, fx1, fy0, fy1;                // vectors taking the fast path lie in this box (inclusive) ...
-    int lbase, llim, cbase, clim;          // ... and have lref <= llim, cref <= clim (offsets from these bases)
-    int64_t lsrc, csrc, dsrc;              // flat index of the source block (luma, chroma, luma at (px, py))
+    int lbase, llim, cbase, clim;          // ... and have lref <= llim, cref <= clim; the offsets (from the frame's
+                                           // first sample) of the reference blocks at vector 0
+    int64_t lsrc, csrc;                    // offset of the source block (luma, U)
 };
 
 __device__ __forceinline__ void make_blk(const Ctx &x, int px, int py, bool chroma, BlkC &b) {
@@ -753,309 +686,490 @@ __device__ __forceinline__ void make_blk(const Ctx &x, int px, int py, bool chro
     b.py2 = py - (x.level > 0 && py + bh >= G.lh);
     b.bnd0 = -pel * px; b.bnd1 = -pel * py;
     b.bnd2 = pel * (G.lw - px - bw) + 1; b.bnd3 = pel * (G.lh - py - bh) + 1;
-    b.ubx = b.bnd2 > b.bnd0 ? b.bnd2 : 0x7FFFFFFF;
-    b.uby = b.bnd3 > b.bnd1 ? b.bnd3 : 0x7FFFFFFF;
+    // bounds above which the edge shift starts
+    const int ubx = b.bnd2 > b.bnd0 ? b.bnd2 : 0x7FFFFFFF, uby = b.bnd3 > b.bnd1 ? b.bnd3 : 0x7FFFFFFF;
     b.chroma = chroma;
-    b.satd_mode = x.satd && is_blk(bw) && is_blk(bh) && bw == bh;
-    b.fastable = bw > 0 && bh > 0 && (bw & 3) == 0 && (bh & 3) == 0;
-    b.tilesx = bw >> 2;
-    b.lgtx = 31 - __clz(imax(b.tilesx, 1));
+    const bool fastable = bw > 0 && bh > 0 && (bw & 3) == 0 && (bh & 3) == 0;
     b.lsrc = ((int64_t)L.y_off + b.py2) * G.ys + b.px2;
-    b.fast_src = b.fastable && b.px2 >= 0 && b.py2 >= 0 && b.px2 + bw <= G.lw && b.py2 + bh <= G.lh &&
+    b.fast_src = fastable && b.px2 >= 0 && b.py2 >= 0 && b.px2 + bw <= G.lw && b.py2 + bh <= G.lh &&
                  b.lsrc + (int64_t)(bh - 1) * G.ys + bw + 8 <= G.ylen;
-    b.dsrc = ((int64_t)L.y_off + py) * G.ys + px;
-    b.dc_fast = b.fastable && px >= 0 && py >= 0 && px + bw <= G.lw && py + bh <= G.lh &&
-                b.dsrc + (int64_t)(bh - 1) * G.ys + bw + 8 <= G.ylen;
-    b.cw = bw / 2; b.ch = bh / 2;
-    b.crows = x.satd ? b.cw : b.ch;
-    b.ctilesx = (b.cw + 3) >> 2;
-    b.lgctx = 31 - __clz(imax(b.ctilesx, 1));
-    b.cpx = px / 2; b.cpy = py / 2;
-    b.csrc = ((int64_t)L.c_off + b.cpy) * G.cs + b.cpx;
-    b.cfast_src = (b.cw == 4 || b.cw == 8 || b.cw == 16) && b.ch >= 4 && (b.ch & 3) == 0 && px >= 0 && py >= 0 &&
-                  b.cpx + b.cw <= G.clw && b.cpy + b.ch <= G.clh &&
-                  b.csrc + (int64_t)(b.crows - 1) * G.cs + b.cw + 8 <= G.clen;
+    const int cw = bw / 2, ch = bh / 2, crows = x.satd ? cw : ch, cpx = px / 2, cpy = py / 2;
+    const int64_t csrc = ((int64_t)L.c_off + cpy) * G.cs + cpx;
+    b.csrc = G.ylen + csrc;
     // the fast-path box: no edge shift, reference block inside the level (luma, and chroma when
     // it is evaluated); with l0sub the luma offset is mv >> 1 and the chroma one mv >> 2
     const bool l0sub = x.level == 0 && pel >= 2;
     const int ls = l0sub ? 1 : 0, cshift = l0sub ? 2 : 1;
     b.fx0 = imax(b.bnd0, (-b.px2) * (1 << ls));
-    b.fx1 = imin(b.ubx - 1, (G.lw - bw - b.px2) * (1 << ls) + (1 << ls) - 1);
+    b.fx1 = imin(ubx - 1, (G.lw - bw - b.px2) * (1 << ls) + (1 << ls) - 1);
     b.fy0 = imax(b.bnd1, (-b.py2) * (1 << ls));
-    b.fy1 = imin(b.uby - 1, (G.lh - bh - b.py2) * (1 << ls) + (1 << ls) - 1);
-    if (b.chroma && b.cw >= 4 && b.ch >= 4) {
-        b.fx0 = imax(b.fx0, (-b.cpx) * (1 << cshift));
-        b.fx1 = imin(b.fx1, (G.clw - b.cw - b.cpx) * (1 << cshift) + (1 << cshift) - 1);
-        b.fy0 = imax(b.fy0, (-b.cpy) * (1 << cshift));
-        b.fy1 = imin(b.fy1, (G.clh - b.ch - b.cpy) * (1 << cshift) + (1 << cshift) - 1);
-        if (!b.cfast_src) b.fx1 = b.fx0 - 1;
+    b.fy1 = imin(uby - 1, (G.lh - bh - b.py2) * (1 << ls) + (1 << ls) - 1);
+    if (chroma && cw >= 4 && ch >= 4) {
+        const bool cfast_src = (cw == 4 || cw == 8 || cw == 16) && (ch & 3) == 0 && px >= 0 && py >= 0 &&
+                               cpx + cw <= G.clw && cpy + ch <= G.clh &&
+                               csrc + (int64_t)(crows - 1) * G.cs + cw + 8 <= G.clen;
+        b.fx0 = imax(b.fx0, (-cpx) * (1 << cshift));
+        b.fx1 = imin(b.fx1, (G.clw - cw - cpx) * (1 << cshift) + (1 << cshift) - 1);
+        b.fy0 = imax(b.fy0, (-cpy) * (1 << cshift));
+        b.fy1 = imin(b.fy1, (G.clh - ch - cpy) * (1 << cshift) + (1 << cshift) - 1);
+        if (!cfast_src) b.fast_src = 0;
     }
     if (!b.fast_src) b.fx1 = b.fx0 - 1;  // empty box
-    b.lbase = (int)L.y_off * G.ys32;
+    b.lbase = ((int)L.y_off + b.py2) * G.ys32 + b.px2;
     b.llim = (int)G.ylen - (bh - 1) * G.ys32 - bw - 8;
-    b.cbase = (int)L.c_off * G.cs32;
-    b.clim = (int)G.clen - (b.crows - 1) * G.cs32 - b.cw - 8;
+    b.cbase = (int)G.ylen + ((int)L.c_off + cpy) * G.cs32 + cpx;
+    b.clim = (int)(G.ylen + G.clen) - (crows - 1) * G.cs32 - cw - 8;
 }
 
-// Does (block, mv) take the fast path? If so, the flat indices of its reference blocks.
+// Does (block, mv) take the fast path? If so, the byte offsets of its reference blocks (see Frame).
 // It does when the reference takes its direct reads for both luma and chroma: no edge
 // shift, the luma block and the reference block inside the level, the chroma blocks too.
-__device__ __forceinline__ bool fast_setup(const Ctx &x, const BlkC &b, int mvx, int mvy, int &lref, int &cref) {
+__device__ __forceinline__ bool fast_setup(const Ctx &x, const BlkC &b, int mvx, int mvy, unsigned &lref, unsigned &cref) {
     if (mvx < b.fx0 || mvx > b.fx1 || mvy < b.fy0 || mvy > b.fy1) return false;
     const int pel = imax(x.pel, 1);
     const bool l0sub = x.level == 0 && pel >= 2;
     const int sub = l0sub ? (mvy & 1) * pel + (mvx & 1) : 0;
     const int mx = l0sub ? mvx >> 1 : mvx, my = l0sub ? mvy >> 1 : mvy;
-    lref = b.lbase + (sub * x.G.lh + b.py2 + my) * x.G.ys32 + b.px2 + mx;
-    if (lref > b.llim) return false;
+    const int lr = b.lbase + (sub * x.G.lh + my) * x.G.ys32 + mx;
+    if (lr > b.llim) return false;
+    lref = (unsigned)lr * (unsigned)sizeof(px_t) + x.fr.mis;
     cref = 0;
-    if (b.chroma && b.cw >= 4 && b.ch >= 4) {
+    if (b.chroma && b.bw >= 8 && b.bh >= 8) {
         const int mcx = l0sub ? mvx >> 2 : mvx >> 1, mcy = l0sub ? mvy >> 2 : mvy >> 1;
-        cref = b.cbase + ((l0sub ? sub * x.G.clh : 0) + b.cpy + mcy) * x.G.cs32 + b.cpx + mcx;
-        if (cref > b.clim) return false;
+        const int cr = b.cbase + ((l0sub ? sub * x.G.clh : 0) + mcy) * x.G.cs32 + mcx;
+        if (cr > b.clim) return false;
+        cref = (unsigned)cr * (unsigned)sizeof(px_t) + x.fr.mis;
     }
     return true;
 }
 
-struct Res {
-    unsigned L, U, V;
-    int lsatd, cmode, csatd;
-};
+__device__ __forceinline__ void set_geo(Geo &G, const AnalyseParams &P, const LevelInfo &L) {
+    G.lw = L.lw; G.lh = L.lh; G.clw = L.lw / 2; G.clh = L.lh / 2;
+    G.ys = P.y_stride; G.cs = P.c_stride; G.ylen = P.y_len; G.clen = P.c_len;
+    G.ys32 = (int)P.y_stride; G.cs32 = (int)P.c_stride;
+}
+__device__ __forceinline__ Planes planes_of(const px_t *frame, const AnalyseParams &P) {
+    return Planes{frame, frame + P.y_len, frame + P.y_len + P.c_len};
+}
 
-// The general path for one lane: the reference's own read path through cand_setup.
-// Arguments by value only, so nothing of the caller's state lives in local memory.
-__device__ __noinline__ Res slow_lane(const AnalyseParams *P, const LevelInfo *L, Geo G, Planes S, Planes R, int level,
-                                      int px, int py, int bw, int bh, int mvx, int mvy, bool chroma, int satd, int pel,
-                                      bool dc, int sub, int Gl, int TL, int TCp) {
-    Res r{0, 0, 0, 0, 0, 0};
+__device__ __forceinline__ void set_frames(Ctx &x, const AnalyseParams &P, const px_t *src, const px_t *ref) {
+    x.S = planes_of(src, P);
+    x.R = planes_of(ref, P);
+    x.fs = frame_of(src);
+    x.fr = frame_of(ref);
+}
+
+// One candidate on the general path, the reference's own read path through cand_setup, by the whole
+// warp: exact_sad's luma (x) and chroma (y) parts. SLOW_DC: the sum of the block's luma samples
+// (block_luma_dc). Out of line, with few arguments, so that the callers keep their registers.
+enum { SLOW_CHROMA = 1, SLOW_DC = 2, SLOW_STAGED = 4 };
+__device__ __noinline__ uint2 slow_warp(const AnalyseParams *Pp, const LevelInfo *Lp, const px_t *src, const px_t *ref,
+                                        int level, int px, int py, int mvx, int mvy, int what) {
+    const AnalyseParams &P = *Pp;
+    const LevelInfo &L = *Lp;
+    Geo G;
+    set_geo(G, P, L);
+    const Planes S = planes_of(src, P), R = planes_of(ref, P);
+    const bool chroma = (what & SLOW_CHROMA) != 0;
     Cand c;
-    cand_setup(c, *P, *L, G, level, px, py, bw, bh, mvx, mvy, chroma, satd, pel, dc);
-    r.lsatd = c.lsatd; r.cmode = c.cmode; r.csatd = c.csatd;
-    const int T = TL + (chroma ? 2 * TCp : 0);
-    for (int t = sub; t < T; t += Gl) {
-        if (t < TL) r.L += luma_tile(c, S, R, G, bw, bh, t);
+    cand_setup(c, P, L, G, level, px, py, L.bw, L.bh, mvx, mvy, chroma, L.satd, L.pel, (what & SLOW_DC) != 0);
+    unsigned rl = 0, ru = 0, rv = 0;
+    const int T = L.tl + (chroma ? 2 * L.tc : 0);
+    for (int t = (int)(threadIdx.x & 31); t < T; t += 32) {
+        if (t < L.tl) rl += luma_tile(c, S, R, G, L.bw, L.bh, t);
         else if (c.cmode != CM_NONE) {
-            int ct = t - TL;
-            const int pl = ct >= TCp;
-            ct -= pl * TCp;
-            const unsigned v = chroma_tile1(c, pl ? S.v : S.u, pl ? R.v : R.u, G, bw / 2, ct);
-            if (pl) r.V += v; else r.U += v;
+            int ct = t - L.tl;
+            const int pl = ct >= L.tc;
+            ct -= pl * L.tc;
+            const unsigned v = chroma_tile1(c, pl ? S.v : S.u, pl ? R.v : R.u, G, L.bw / 2, ct);
+            if (pl) rv += v; else ru += v;
         }
     }
-    return r;
+    rl = __reduce_add_sync(kFull, rl);
+    ru = __reduce_add_sync(kFull, ru);
+    rv = __reduce_add_sync(kFull, rv);
+    unsigned C = 0;
+    if (c.cmode != CM_NONE && chroma) C = c.csatd ? sat_mul(sat_add(ru >> 1, rv >> 1), 4) : sat_mul(ru + rv, 4);
+    return make_uint2(c.lsatd ? (rl >> 1) : rl, C);
 }
-
-
-// Lanes per candidate for a step of n candidates: the widest power-of-two group (at most a
-// warp, at least the level's G) that still puts every candidate in one round. Small steps
-// (a hexagon, a ring, the special candidates) then finish in fewer tiles per lane.
-__device__ __forceinline__ int step_lanes(int G, int n, int nw) {
-    while (G < 32 && nw * (16 / G) >= n) G <<= 1;
-    return G;
+__device__ __forceinline__ uint2 eval_slow(const Ctx &x, int px, int py, int mvx, int mvy, int what) {
+    return slow_warp(x.P, x.L, x.S.y, x.R.y, x.level, px, py, mvx, mvy, what);
 }
+__device__ __forceinline__ unsigned sad_of(uint2 lc) { return sat_add(lc.x, lc.y); }
 
-// Work of one lane (`sub` of G) on one candidate: its share of the 4x4 tiles.
-// kind 0: block at (b.px, b.py); 1: the same mv on the block at (px, py) (general path);
-// 2: the block's luma pixel sum (block_luma_dc).
-__device__ __forceinline__ Res eval_lane(const Ctx &x, const BlkC &b, int kind, int px, int py, int mvx, int mvy,
-                                         bool chroma, int sub, int G) {
-    const int TL = x.tl, TCp = x.tcp;
-    int lref = 0, cref = 0;
-    bool fast = false;
-    if (kind == 0) fast = fast_setup(x, b, mvx, mvy, lref, cref);
-    else if (kind == 2) fast = b.dc_fast;
-    if (!fast)
-        return slow_lane(x.P, x.L, x.G, x.S, x.R, x.level, kind == 1 ? px : b.px, kind == 1 ? py : b.py, b.bw, b.bh,
-                         mvx, mvy, chroma, x.satd, x.pel, kind == 2, sub, G, TL, TCp);
-    Res r{0, 0, 0, 0, 0, 0};
-    const int T = TL + (chroma ? 2 * TCp : 0);
-    const int ys = x.G.ys32, cs = x.G.cs32;
-    r.lsatd = kind == 2 ? 0 : b.satd_mode;
-    r.cmode = (chroma && b.cw >= 4 && b.ch >= 4) ? CM_DIRECT : CM_NONE;
-    r.csatd = x.satd;
-    const px_t *sl = x.S.y + (kind == 2 ? b.dsrc : b.lsrc);
-#pragma unroll 1
-    for (int t = sub; t < T; t += G) {
-        if (t < TL) {
-            const int ty = t >> b.lgtx, tx = t & (b.tilesx - 1);
-            const int o = ty * 4 * ys + tx * 4;
-            if (kind == 2) r.L += tile_sum(sl + o, ys);
-            else if (r.lsatd) r.L += tile_satd(sl + o, x.R.y + lref + o, ys);
-            else r.L += tile_sad(sl + o, x.R.y + lref + o, ys);
-        } else if (r.cmode != CM_NONE) {
-            int ct = t - TL;
-            const int pl = ct >= TCp;
-            ct -= pl * TCp;
-            const int ty = ct >> b.lgctx, tx = ct & (b.ctilesx - 1);
-            if (ty * 4 >= b.crows) continue;
-            const int o = ty * 4 * cs + tx * 4;
-            const px_t *sp = (pl ? x.S.v : x.S.u) + b.csrc + o, *rp = (pl ? x.R.v : x.R.u) + cref + o;
-            const unsigned v = r.csatd ? tile_satd(sp, rp, cs) : tile_sad(sp, rp, cs);
-            if (pl) r.V += v; else r.U += v;
-        }
-    }
-    return r;
-}
-
-// the three sums of a group of G lanes (independent shuffles, so they overlap)
-__device__ __forceinline__ void group_sum3(Res &r, int G) {
+// U groups of NB candidates: every load is in flight before the first is used, and a group's staged
+// source, offset and masks are read once for all of them.
+template <int U, int NB, bool SATD>
+__device__ __forceinline__ void eval_groups(const Ctx &x, int g0, const unsigned (&lr)[NB], const unsigned (&cr)[NB],
+                                            float (&fl)[NB], float (&fc)[NB], unsigned (&il)[NB], unsigned (&ic)[NB]) {
+    const int lane = x.tid & 31;
+    Smp w[U][NB];
+    float4 c[U];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        if (o < G) {
-            r.L += __shfl_xor_sync(0xFFFFFFFFu, r.L, o);
-            r.U += __shfl_xor_sync(0xFFFFFFFFu, r.U, o);
-            r.V += __shfl_xor_sync(0xFFFFFFFFu, r.V, o);
+    for (int u = 0; u < U; u++) {
+        const int g = g0 + u;
+        const unsigned o = x.off[g * 32 + lane];
+        const bool chroma = (x.cmask >> g) & 1u;
+        c[u] = x.src[g * 32 + lane];
+#pragma unroll
+        for (int q = 0; q < NB; q++) w[u][q] = ld4(x.fr, (chroma ? cr[q] : lr[q]) + o);
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const int g = g0 + u;
+        if (SATD) {
+            const float wl = (x.dlmask >> g) & 1u ? 1.f : 0.f, wc = (x.dcmask >> g) & 1u ? 1.f : 0.f;
+#pragma unroll
+            for (int q = 0; q < NB; q++) {
+                uint32_t lo, hi;
+                halves(w[u][q], lo, hi);
+                const float4 d = mma_hadamard(x.h, lo, hi, c[u]);
+                const float v = (fabsf(d.x) + fabsf(d.y)) + (fabsf(d.z) + fabsf(d.w));
+                fl[q] = fmaf(v, wl, fl[q]);
+                fc[q] = fmaf(v, wc, fc[q]);
+            }
+        } else {
+            const unsigned ml = 0u - ((x.lmask >> g) & 1u), mc = 0u - ((x.cmask >> g) & 1u);
+            const Smp sm{__float_as_uint(c[u].x), __float_as_uint(c[u].y)};
+#pragma unroll
+            for (int q = 0; q < NB; q++) {
+                il[q] = sad4(sm, w[u][q], ml, il[q]);
+                ic[q] = sad4(sm, w[u][q], mc, ic[q]);
+            }
         }
     }
 }
-__device__ __forceinline__ void finalize(const Res &r, unsigned &L, unsigned &C) {
-    L = r.lsatd ? (r.L >> 1) : r.L;
-    if (r.cmode == CM_NONE) C = 0;
-    else if (r.csatd) C = sat_mul(sat_add(r.U >> 1, r.V >> 1), 4);
-    else C = sat_mul(r.U + r.V, 4);
+
+// NB candidates on the fast path by the whole warp. lref, cref: the lanes' set-ups; m: the lanes
+// still to take, of which the lowest NB go (fewer left: the last one again, unused). Three groups,
+// all SATD (16x16 blocks with chroma, TRI): in one go; else group by group. A 4x4 tile's SATD is even
+// (its coefficients share their parity), so halving the sum of tiles is halving each plane's.
+template <int NB, bool TRI>
+__device__ __forceinline__ void eval_fast(const Ctx &x, unsigned lref, unsigned cref, unsigned &m, unsigned &L, unsigned &C) {
+    const int lane = x.tid & 31;
+    unsigned lr[NB], cr[NB], il[NB], ic[NB];
+    float fl[NB], fc[NB];
+    int who[NB];
+#pragma unroll
+    for (int q = 0; q < NB; q++) {
+        who[q] = m ? __ffs(m) - 1 : who[q > 0 ? q - 1 : 0];
+        m &= m - 1;
+        lr[q] = __shfl_sync(kFull, lref, who[q]);
+        cr[q] = __shfl_sync(kFull, cref, who[q]);
+        fl[q] = fc[q] = kIntBias;
+        il[q] = ic[q] = 0;
+    }
+    if (TRI) {
+        eval_groups<3, NB, true>(x, 0, lr, cr, fl, fc, il, ic);
+    } else {
+#pragma unroll 1
+        for (int g = 0; g < x.ng; g++) {
+            if ((x.smask >> g) & 1u) eval_groups<1, NB, true>(x, g, lr, cr, fl, fc, il, ic);
+            else eval_groups<1, NB, false>(x, g, lr, cr, fl, fc, il, ic);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < NB; q++) {
+        const unsigned sl = __reduce_add_sync(kFull, il[q] + (__float_as_uint(fl[q]) - __float_as_uint(kIntBias)));
+        const unsigned sc = __reduce_add_sync(kFull, ic[q] + (__float_as_uint(fc[q]) - __float_as_uint(kIntBias)));
+        if (lane == who[q]) {
+            L = sl >> x.lshift;
+            C = x.satd ? (sc >> 1) * 4u : sc * 4u;
+        }
+    }
 }
 
-// One search step: candidates g over the block against the running best `best_cost`.
-// Every warp computes which candidates pass exact_ok and the motion-penalty cut (a
-// ballot bitmask, identical in every warp), then groups take the passing candidates
-// in order. On return, identically in every thread: win = accepted candidate or -1,
-// and the new best cost / sad when accepted.
+// The block's source for the fast path (Ctx::src) and the sum of its luma samples, each warp of
+// the group taking every nw-th group of tiles: the sum is the warp's part.
+__device__ __forceinline__ unsigned stage_source(const Ctx &x, const BlkC &b) {
+    unsigned s = 0;
+    const int lane = x.tid & 31;
+    const unsigned lo_ = (unsigned)b.lsrc * (unsigned)sizeof(px_t) + x.fs.mis, co = (unsigned)b.csrc * (unsigned)sizeof(px_t) + x.fs.mis;
+#pragma unroll 1
+    for (int g = x.tid >> 5; g < x.ng; g += x.nw) {
+        const bool chroma = (x.cmask >> g) & 1u;
+        const Smp w = ld4(x.fs, (chroma ? co : lo_) + x.off[g * 32 + lane]);
+        if (((x.lmask >> g) & 1u) && !(x.lshift == 2 && lane >= 4)) s += sum4(w);
+        float4 c = make_float4(__uint_as_float(w.a), __uint_as_float(w.b), 0.f, 0.f);
+        if ((x.smask >> g) & 1u) {
+            uint32_t lo, hi;
+            halves(w, lo, hi);
+            c = mma_hadamard(x.h, lo, hi, make_float4(0.f, 0.f, 0.f, 0.f));
+            c = make_float4(-c.x, -c.y, -c.z, -c.w);
+        }
+        x.src[g * 32 + lane] = c;
+    }
+    return __reduce_add_sync(kFull, s);
+}
+
+// Four samples whose first would be at x of a row of n >= 4 samples, places outside the row taking
+// the row's end sample (w: the samples loaded at x clamped to 0 .. n - 4): e = x - that place.
+__device__ __forceinline__ Smp spread_ends(const Smp &w, int e) {
+    e = iclamp(e, -3, 3);
+    const unsigned sel = __funnelshift_r(0x33210000u, 0x33u, (unsigned)(12 + 4 * e)) & 0xFFFFu;  // sample i + e, clamped
+#ifndef SVPF_PX16
+    return Smp{__byte_perm(w.a, 0u, sel), 0u};
+#else
+    const unsigned j0 = sel & 3u, j1 = (sel >> 4) & 3u, j2 = (sel >> 8) & 3u, j3 = (sel >> 12) & 3u;
+    const unsigned s01 = (j0 * 0x22u + 0x10u) | (j1 * 0x2200u + 0x1000u), s23 = (j2 * 0x22u + 0x10u) | (j3 * 0x2200u + 0x1000u);
+    return Smp{__byte_perm(w.a, w.b, s01), __byte_perm(w.a, w.b, s23)};
+#endif
+}
+
+// The candidates that do not take the fast path, lanes `mask`, for a block at (px, py). Most of them
+// (a quarter-pel field, whose vectors the reference reads as half-pel ones, has them everywhere) lie
+// inside mv_bounds with the block's source inside its planes and only the reference block reaching
+// out: then every read is the staged source against samples clamped to the plane (:1719-1852,
+// :2353-2436), and chroma is compared by SATD where its block lies inside and by SAD where it does
+// not (:2169-2303). They go through the groups of eight tiles as on the fast path, NB at a time; the
+// others one by one through slow_warp. Out of line: called once for all of a step's such candidates.
+__device__ __noinline__ uint2 clamped_cands(const AnalyseParams *Pp, const LevelInfo *Lp, const px_t *src, const px_t *ref,
+                                            const float4 *stage, int level, int px, int py, unsigned mask, int mvx, int mvy,
+                                            int what) {
+    constexpr int NB = 4;
+    const AnalyseParams &P = *Pp;
+    const LevelInfo &L = *Lp;
+    Ctx x;  // the fields the group tables need
+    x.L = Lp;
+    x.satd = L.satd;
+    x.tid = (int)(threadIdx.x & 31);
+    set_geo(x.G, P, L);
+    const int lane = x.tid;
+    const Geo &G = x.G;
+    const int bw = L.bw, bh = L.bh, cw = bw >> 1, ch = bh >> 1, pel = imax(L.pel, 1);
+    const bool chroma = (what & SLOW_CHROMA) != 0 && cw >= 4 && ch >= 4;
+    const int px2 = px - (level > 0 && px + bw >= G.lw), py2 = py - (level > 0 && py + bh >= G.lh);
+    const int cpx = px / 2, cpy = py / 2;
+    const bool l0sub = level == 0 && pel >= 2;
+    const Frame fs = frame_of(src), fr = frame_of(ref);
+    // this lane's candidate: may it go through the groups?
+    const int sub = l0sub ? (mvy & 1) * pel + (mvx & 1) : 0;
+    const int lrow0 = (int)L.y_off + sub * G.lh, crow0 = (int)L.c_off + sub * G.clh;
+    const int rx = px2 + (l0sub ? mvx >> 1 : mvx), ry = py2 + (l0sub ? mvy >> 1 : mvy);
+    const int crx = cpx + (l0sub ? mvx >> 2 : mvx >> 1), cry = cpy + (l0sub ? mvy >> 2 : mvy >> 1);
+    const int b0 = -pel * px, b1 = -pel * py, b2 = pel * (G.lw - px - bw) + 1, b3 = pel * (G.lh - py - bh) + 1;
+    bool ok = (what & SLOW_STAGED) != 0 && (bw == bh || !L.satd) && mvx >= b0 && mvy >= b1 && !(b2 > b0 && mvx >= b2) &&
+              !(b3 > b1 && mvy >= b3);
+    ok = ok && (int64_t)(lrow0 + iclamp(ry + bh - 1, 0, G.lh - 1)) * G.ys + iclamp(rx + bw - 4, 0, G.lw - 4) + 8 <= G.ylen;
+    if (chroma)
+        ok = ok && (int64_t)(crow0 + iclamp(cry + ch - 1, 0, G.clh - 1)) * G.cs + iclamp(crx + cw - 4, 0, G.clw - 4) + 8 <= G.clen;
+    const bool cdirect = crx >= 0 && cry >= 0 && crx + cw <= G.clw && cry + ch <= G.clh;
+    unsigned mm = __ballot_sync(kFull, ok) & mask, ms = mask & ~mm;
+    const unsigned cdm = __ballot_sync(kFull, cdirect);
+    uint2 out = make_uint2(0u, 0u);
+    if (mm) {
+        // the group tables (as set_groups), without offsets
+        const bool lsatd = L.satd && bw == bh;  // ok implies the same kind for both
+        const int tx = imax(bw >> 2, 1), tl = tx * imax(bh >> 2, 1), lgtx = 31 - __clz(tx);
+        const int ctx = imax(cw >> 2, 1), lgctx = 31 - __clz(ctx), tc = chroma ? ctx * (ch >> 2) : 0;
+        const int c0 = lsatd == (L.satd != 0) && tl > 1 ? tl : (tl + 7) & ~7;
+        const int tl2 = tl == 1 && lsatd ? 2 : tl, ng = chroma ? (c0 + 2 * tc + 7) >> 3 : (tl + 7) >> 3;
+        const int lshift = (lsatd ? 1 : 0) + (tl2 - tl);
+        const int m = lane >> 2, k = (lane & 3) * 2;
+        const uint4 h = make_uint4(hadamard_pair(m, k), hadamard_pair(m + 8, k), hadamard_pair(m, k + 8), hadamard_pair(m + 8, k + 8));
+#pragma unroll 1
+        while (mm) {
+            int who[NB], qx[NB], qy[NB], ql[NB], cx[NB], cy[NB], ql2[NB];
+            float fl[NB], fc[NB];
+            unsigned il[NB], ic[NB];
+#pragma unroll
+            for (int q = 0; q < NB; q++) {
+                who[q] = mm ? __ffs(mm) - 1 : who[q > 0 ? q - 1 : 0];
+                mm &= mm - 1;
+                qx[q] = __shfl_sync(kFull, rx, who[q]);
+                qy[q] = __shfl_sync(kFull, ry, who[q]);
+                ql[q] = __shfl_sync(kFull, lrow0, who[q]);
+                cx[q] = __shfl_sync(kFull, crx, who[q]);
+                cy[q] = __shfl_sync(kFull, cry, who[q]);
+                ql2[q] = __shfl_sync(kFull, crow0, who[q]);
+                fl[q] = fc[q] = kIntBias;
+                il[q] = ic[q] = 0;
+            }
+#pragma unroll 1
+            for (int g = 0; g < ng; g++) {
+                const int t = g * 8 + (lane >> 2), dt = g * 8 + (lane & 3) * 2;
+                const bool isl = t < tl2, isc = t >= c0 && t < c0 + 2 * tc;
+                const int pl = t - c0 >= tc, ct = t - c0 - pl * tc, tt = t < tl ? t : 0;
+                const int ox = isc ? (ct & (ctx - 1)) * 4 : (tt & (tx - 1)) * 4;
+                const int oy = (isc ? (ct >> lgctx) * 4 : (tt >> lgtx) * 4) + (lane & 3);
+                const int w_ = isc ? G.clw : G.lw, h_ = isc ? G.clh : G.lh, st = isc ? G.cs32 : G.ys32;
+                const unsigned plane = isc ? (unsigned)G.ylen + (pl ? (unsigned)G.clen : 0u) : 0u;
+                const float4 c = stage[g * 32 + lane];
+                Smp w[NB];
+#pragma unroll
+                for (int q = 0; q < NB; q++) {
+                    const int xx = (isc ? cx[q] : qx[q]) + ox, yy = iclamp((isc ? cy[q] : qy[q]) + oy, 0, h_ - 1);
+                    const int xa = iclamp(xx, 0, w_ - 4);
+                    const unsigned o = plane + (unsigned)(((isc ? ql2[q] : ql[q]) + yy) * st + xa);
+                    w[q] = spread_ends(ld4(fr, o * (unsigned)sizeof(px_t) + fr.mis), xx - xa);
+                }
+                const bool satd = g * 8 < c0 ? lsatd : L.satd != 0;
+                const unsigned ml = 0u - (unsigned)isl, mc = 0u - (unsigned)isc;
+                if (satd) {
+                    const float wl = dt < tl2 ? 1.f : 0.f, wc = dt >= c0 && dt < c0 + 2 * tc ? 1.f : 0.f;
+                    Smp s0{0u, 0u};
+                    if (isc)
+                        s0 = ld4(fs, (plane + (unsigned)(((int)L.c_off + cpy + oy) * st + cpx + ox)) * (unsigned)sizeof(px_t) + fs.mis);
+#pragma unroll
+                    for (int q = 0; q < NB; q++) {
+                        uint32_t lo, hi;
+                        halves(w[q], lo, hi);
+                        const float4 d = mma_hadamard(h, lo, hi, c);
+                        const float v = (fabsf(d.x) + fabsf(d.y)) + (fabsf(d.z) + fabsf(d.w));
+                        fl[q] = fmaf(v, wl, fl[q]);
+                        fc[q] = fmaf(v, wc, fc[q]);
+                        ic[q] = sad4(s0, w[q], mc, ic[q]);
+                    }
+                } else {
+                    const Smp sm{__float_as_uint(c.x), __float_as_uint(c.y)};
+#pragma unroll
+                    for (int q = 0; q < NB; q++) {
+                        il[q] = sad4(sm, w[q], ml, il[q]);
+                        ic[q] = sad4(sm, w[q], mc, ic[q]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < NB; q++) {
+                const unsigned sl = __reduce_add_sync(kFull, il[q] + (__float_as_uint(fl[q]) - __float_as_uint(kIntBias)));
+                const unsigned st_ = __reduce_add_sync(kFull, __float_as_uint(fc[q]) - __float_as_uint(kIntBias));
+                const unsigned sa = __reduce_add_sync(kFull, ic[q]);
+                if (lane == who[q])
+                    out = make_uint2(sl >> lshift, L.satd && ((cdm >> who[q]) & 1u) ? (st_ >> 1) * 4u : sa * 4u);
+            }
+        }
+    }
+#pragma unroll 1
+    while (ms) {
+        const int j = __ffs(ms) - 1;
+        ms &= ms - 1;
+        const uint2 r = slow_warp(Pp, Lp, src, ref, level, px, py, __shfl_sync(kFull, mvx, j), __shfl_sync(kFull, mvy, j), what);
+        if (lane == j) out = r;
+    }
+    return out;
+}
+
+// Evaluates every lane's candidate (lanes with `ok`): L and C of exact_sad in the lane that holds
+// it. The lanes set their candidates up side by side, then the warp evaluates one after another.
+// Bound: the latency of the loads, which the candidates evaluated together overlap, then instruction
+// issue. Per 16x16 candidate with chroma this is about 120 warp instructions with all that surrounds
+// it, against 167 when groups of lanes each transformed whole tiles in f16x2 (13.7 k against 19.2 k
+// per level-0 block of the 1080p configuration).
+__device__ __forceinline__ void eval_cands(const Ctx &x, const BlkC &b, bool ok, int mvx, int mvy, unsigned &L, unsigned &C) {
+    const int lane = x.tid & 31;
+    unsigned lref = 0, cref = 0;
+    const bool fast = ok && fast_setup(x, b, mvx, mvy, lref, cref);
+    unsigned mf = __ballot_sync(kFull, fast), ms = __ballot_sync(kFull, ok && !fast);
+    L = C = 0;
+#pragma unroll 1
+    while (mf) {
+        if (x.ng == 3 && x.smask == 7u) eval_fast<4, true>(x, lref, cref, mf, L, C);
+        else if (__popc(mf) > 4) eval_fast<8, false>(x, lref, cref, mf, L, C);
+        else eval_fast<4, false>(x, lref, cref, mf, L, C);
+    }
+    if (ms) {
+        const uint2 r = clamped_cands(x.P, x.L, x.S.y, x.R.y, x.src, x.level, b.px, b.py, ms, mvx, mvy,
+                                      (b.chroma ? SLOW_CHROMA : 0) | (b.fast_src ? SLOW_STAGED : 0));
+        if ((ms >> lane) & 1u) { L = r.x; C = r.y; }
+    }
+    if (!b.chroma) C = 0;
+}
+
+// The lane holding the least (cost, place) among those with `act`, or -1. Costs of a word or less
+// take two redux; the others a shuffle tree.
+__device__ __forceinline__ int first_min(bool act, long long cost, int place) {
+    if (!__any_sync(kFull, act)) return -1;
+    bool e;
+    if (!__any_sync(kFull, act && (unsigned long long)cost >= 0xFFFFFFFFull)) {
+        const unsigned u = act ? (unsigned)cost : 0xFFFFFFFFu;
+        const unsigned least = __reduce_min_sync(kFull, u);
+        e = act && u == least;
+    } else {
+        long long m = act ? cost : 0x7FFFFFFFFFFFFFFFLL;
+#pragma unroll 1
+        for (int o = 16; o > 0; o >>= 1) {
+            const long long v = __shfl_xor_sync(kFull, m, o);
+            m = v < m ? v : m;
+        }
+        e = act && cost == m;
+    }
+    const int pm = __reduce_min_sync(kFull, e ? place : 0x7FFFFFFF);
+    return __ffs(__ballot_sync(kFull, e && place == pm)) - 1;
+}
+
+// One search step: candidates g over the block against the running best `best_cost`, 32 at a time,
+// one per lane. The group's warps share the candidates that pass exact_ok and the motion-penalty
+// cut, every nw-th of them, and combine their winners. A candidate whose motion penalty reaches the
+// best cost cannot win (cost >= penalty for pnew >= -256), so the reference's skip and a skip
+// against an earlier, larger best decide alike. On return, identically in every thread: win =
+// accepted candidate or -1, and the new best cost / sad when accepted.
 template <class SH>
 __device__ __forceinline__ void eval_step(const Ctx &x, const BlkC &b, SH &s, int &ph, const Gen &g, int lambda,
                                           int predx, int predy, long long &best_cost, unsigned &best_sad, int &win) {
     const int lane = x.tid & 31, warp = x.tid >> 5, wi = x.wbase + warp;  // wi: the warp's place in the direction
     const bool serial = x.pnew < -256;
     const int pnew = x.pnew;
-    long long bk = 0x7FFFFFFFFFFFFFFFLL;
-    int bi = 0x7FFFFFFF;
+    long long bk = best_cost;  // the warp's own best
+    int bi = -1;
     unsigned bs = 0;
     win = -1;
-    const unsigned lt_mask = (1u << lane) - 1u;
-    for (int base = 0; base < g.n; base += 32 * MW) {
-        int total = 0;
-        const long long cut = best_cost;
-        // this warp's copy of the passing candidates, in candidate order (every warp
-        // computes the same list, so no barrier is needed)
 #pragma unroll 1
-        for (int w = 0; w < MW; w++) {
-            if (base + w * 32 >= g.n) break;  // uniform
-            const int i = base + w * 32 + lane;
-            bool ok = i < g.n;
-            int2 mv = make_int2(0, 0);
-            if (ok) {
-                mv = gen_mv(g, i);
-                ok = mv.x >= b.bnd0 && mv.y >= b.bnd1 && mv.x < b.bnd2 && mv.y < b.bnd3;  // exact_ok
-                if (ok) ok = motion_penalty(lambda, predx, predy, mv.x, mv.y) < cut;  // a later candidate faces a lower best
-            }
-            const unsigned m = __ballot_sync(0xFFFFFFFFu, ok);
-            if (ok)  // |mv| <= pel * plane size, so each component fits a halfword
-                s.clist[wi][total + __popc(m & lt_mask)] =
-                    make_int2((int)(((unsigned)mv.x & 0xFFFFu) | ((unsigned)mv.y << 16)), i);
-            total += __popc(m);
+    for (int base = 0; base < g.n; base += 32) {
+        const int i = base + lane;
+        bool ok = i < g.n;
+        int2 mv = make_int2(0, 0);
+        long long motion = 0;
+        if (ok) {
+            mv = gen_mv(g, i);
+            ok = mv.x >= b.bnd0 && mv.y >= b.bnd1 && mv.x < b.bnd2 && mv.y < b.bnd3;  // exact_ok
+            motion = motion_penalty(lambda, predx, predy, mv.x, mv.y);
+            if (ok) ok = motion < best_cost;  // a later candidate faces a lower best
         }
-        __syncwarp();
-        const int G = step_lanes(x.grp_lanes, total, x.nw);
-        const int grp = warp * (32 / G) + lane / G, sub = lane & (G - 1), NG = x.nw * (32 / G);
-        const int rb = x.wbase * 32;  // the group's entries of the sequential-scan arrays
-        for (int r0 = 0; r0 < total; r0 += NG) {
-            const int rk = r0 + grp;
-            const bool act = rk < total;
-            int i = 0;
-            int2 mv = make_int2(0, 0);
-            if (act) {  // the rk-th passing candidate
-                const int2 e = s.clist[wi][rk];
-                i = e.y;
-                mv = make_int2((int)(short)(e.x & 0xFFFF), e.x >> 16);
-            }
-            int lref = 0, cref = 0;
-            bool fast = false;
-            Res r{0, 0, 0, 0, 0, 0};
-            long long motion = 0;
-            if (act) {
-                motion = motion_penalty(lambda, predx, predy, mv.x, mv.y);
-                fast = fast_setup(x, b, mv.x, mv.y, lref, cref);
-                if (!fast)
-                    r = slow_lane(x.P, x.L, x.G, x.S, x.R, x.level, b.px, b.py, b.bw, b.bh, mv.x, mv.y, b.chroma != 0,
-                                  x.satd, x.pel, false, sub, G, x.tl, x.tcp);
-            }
-            // this lane's 4x4 tiles: luma, then U, then V (the source block is staged in shared memory)
-            if (act && fast) {
-                r.lsatd = b.satd_mode;
-                r.cmode = (b.chroma && b.cw >= 4 && b.ch >= 4) ? CM_DIRECT : CM_NONE;
-                r.csatd = x.satd;
-                const int T = x.tl + (r.cmode != CM_NONE ? 2 * x.tcp : 0);
-                const int ys = x.G.ys32, cs = x.G.cs32, nlw = b.tilesx * b.bh;
-                const px_t *rl = x.R.y + lref;
-                int t = sub;  // luma tiles, then chroma: two loops, no per-tile branch on the plane
-#pragma unroll 1
-                for (; t < x.tl; t += G) {
-                    const int ty = t >> b.lgtx, tx = t & (b.tilesx - 1);
-                    const px_t *rp = rl + (ty * 4 * ys + tx * 4);
-                    const uint2 *sp = s.srcp[SH::kSrc > 1 ? x.wbase : 0] + ((ty * 4) << b.lgtx) + tx;
-                    r.L += b.satd_mode ? tile_satd_p(sp, b.tilesx, rp, ys) : tile_sad_p(sp, b.tilesx, rp, ys);
-                }
-#pragma unroll 1
-                for (; t < T; t += G) {
-                    const int ct0 = t - x.tl;
-                    const int pl = ct0 >= x.tcp;
-                    const int ct = ct0 - pl * x.tcp;
-                    const int ty = ct >> b.lgctx, tx = ct & (b.ctilesx - 1);
-                    if (ty * 4 >= b.crows) continue;
-                    const px_t *rp = (pl ? x.R.v : x.R.u) + cref + (ty * 4 * cs + tx * 4);
-                    const uint2 *sp = s.srcp[SH::kSrc > 1 ? x.wbase : 0] + nlw + pl * b.ctilesx * b.crows +
-                                      ((ty * 4) << b.lgctx) + tx;
-                    const unsigned v = x.satd ? tile_satd_p(sp, b.ctilesx, rp, cs) : tile_sad_p(sp, b.ctilesx, rp, cs);
-                    if (pl) r.V += v; else r.U += v;
-                }
-            }
-            group_sum3(r, G);
-            long long K = 0x7FFFFFFFFFFFFFFFLL;
-            unsigned sad = 0;
-            if (act) {
-                unsigned L, C;
-                finalize(r, L, C);
-                if (!b.chroma) C = 0;
-                K = motion + pen(pnew, L) + (b.chroma ? pen(pnew, C) : 0LL);  // :1158-1221
-                sad = sat_add(L, C);
-            }
-            if (serial) {  // exact sequential semantics for penalties that can be negative
-                if (sub == 0) {
-                    s.rk[ph][rb + grp] = K; s.rm[ph][rb + grp] = motion; s.rs[ph][rb + grp] = sad;
-                    s.rv[ph][rb + grp] = act; s.ri[ph][rb + grp] = i;
-                }
+        bool mine = ok;
+        const int rank = __popc(__ballot_sync(kFull, ok) & ((1u << lane) - 1u));
+        if (x.nw > 1) mine = ok && rank % x.nw == warp;
+        if (!serial) mine = mine && motion < bk;
+        unsigned L, C;
+        eval_cands(x, b, mine, mv.x, mv.y, L, C);
+        const long long K = motion + pen(pnew, L) + (b.chroma ? pen(pnew, C) : 0LL);  // :1158-1221
+        const unsigned sad = sat_add(L, C);
+        if (serial) {  // exact sequential semantics for penalties that can be negative
+            long long kk = K;
+            unsigned ss = sad;
+            if (x.nw > 1) {  // every warp sees every cost
+                if (mine) { s.rk[ph][lane] = K; s.rs[ph][lane] = sad; }
                 gsync(x);
-                const int m = imin(NG, total - r0);
-                for (int j = rb; j < rb + m; j++) {
-                    if (s.rm[ph][j] >= best_cost) continue;
-                    if (s.rk[ph][j] < best_cost) { best_cost = s.rk[ph][j]; best_sad = s.rs[ph][j]; win = s.ri[ph][j]; }
-                }
+                kk = s.rk[ph][lane];
+                ss = s.rs[ph][lane];
                 ph ^= 1;
-            } else if (act && sub == 0 && (K < bk || (K == bk && i < bi))) {
-                bk = K; bi = i; bs = sad;
+            }
+            for (unsigned m = __ballot_sync(kFull, ok); m; m &= m - 1) {
+                const int j = __ffs(m) - 1;
+                const long long mj = __shfl_sync(kFull, motion, j), kj = __shfl_sync(kFull, kk, j);
+                const unsigned sj = __shfl_sync(kFull, ss, j);
+                if (mj < best_cost && kj < best_cost) { best_cost = kj; best_sad = sj; win = base + j; }
+            }
+        } else {
+            const int j = first_min(mine && K < bk, K, lane);
+            if (j >= 0) {
+                bk = __shfl_sync(kFull, K, j);
+                bs = __shfl_sync(kFull, sad, j);
+                bi = base + j;
+                if (x.nw == 1) { best_cost = bk; best_sad = bs; win = bi; }
             }
         }
-        __syncwarp();  // the next chunk rewrites this warp's list
     }
-    if (serial) return;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const long long ok_ = __shfl_xor_sync(0xFFFFFFFFu, bk, o);
-        const int oi = __shfl_xor_sync(0xFFFFFFFFu, bi, o);
-        const unsigned os = __shfl_xor_sync(0xFFFFFFFFu, bs, o);
-        if (ok_ < bk || (ok_ == bk && oi < bi)) { bk = ok_; bi = oi; bs = os; }
-    }
-    if (x.nw > 1) {  // combine the group's warps (one warp already holds its result in every lane)
-        if (lane == 0) { s.K[ph][wi] = bk; s.I[ph][wi] = bi; s.S[ph][wi] = bs; }
-        gsync(x);
-        bk = s.K[ph][x.wbase]; bi = s.I[ph][x.wbase]; bs = s.S[ph][x.wbase];
-        for (int w = x.wbase + 1; w < x.wbase + x.nw; w++) {
-            const long long k = s.K[ph][w];
-            const int ii = s.I[ph][w];
-            if (k < bk || (k == bk && ii < bi)) { bk = k; bi = ii; bs = s.S[ph][w]; }
-        }
+    if (serial || x.nw == 1) return;
+    // combine the group's warps
+    if (lane == 0) { s.K[ph][wi] = bk; s.I[ph][wi] = bi; s.S[ph][wi] = bs; }
+    gsync(x);
+    for (int w = x.wbase; w < x.wbase + x.nw; w++) {
+        const int ii = s.I[ph][w];
+        if (ii < 0) continue;
+        const long long k = s.K[ph][w];
+        if (k < best_cost || (k == best_cost && win >= 0 && ii < win)) { best_cost = k; best_sad = s.S[ph][w]; win = ii; }
     }
     ph ^= 1;
-    if (bi != 0x7FFFFFFF && bk < best_cost) { best_cost = bk; best_sad = bs; win = bi; }
 }
 
 // adapt_lambda, :1555-1564 (f64, IEEE-exact: one add, one division, two products)
@@ -1097,6 +1211,18 @@ __device__ __noinline__ unsigned plane_activity(const px_t *data, int64_t len, i
             total += hadamard4(dd);
         }
     return area ? (total >> 1) / area : 0;
+}
+
+// The three planes' activity of a block (its luma at (lx, ly), which the level's last column and row shift).
+__device__ __noinline__ unsigned block_activity(const AnalyseParams *Pp, const LevelInfo *Lp, const px_t *src, int lx, int ly,
+                                                int px, int py) {
+    const AnalyseParams &P = *Pp;
+    const LevelInfo &L = *Lp;
+    const Planes S = planes_of(src, P);
+    const bool satd = L.satd != 0;
+    return plane_activity(S.y, P.y_len, P.y_stride, L.y_off + ly, lx, L.bw, L.bh, satd) +
+           plane_activity(S.u, P.c_len, P.c_stride, L.c_off + py / 2, px / 2, L.bw / 2, L.bh / 2, satd) +
+           plane_activity(S.v, P.c_len, P.c_stride, L.c_off + py / 2, px / 2, L.bw / 2, L.bh / 2, satd);
 }
 
 __device__ __forceinline__ int adaptive_radius(int radius, unsigned act) {
@@ -1166,31 +1292,21 @@ __device__ __forceinline__ uint2 mkvec(int dx, int dy, unsigned score) {
     return make_uint2((uint32_t)(uint16_t)(short)dx | ((uint32_t)(uint16_t)(short)dy << 16), score);
 }
 
+// A direction's words in the pair's scratch (AnalyseParams::off_ctl, 64 bytes) from one launch to the
+// next, and of a walked level. GO: the next walk has this direction's level to do; LATE: a bounded
+// wait gave up; BAD: bad-SAD blocks of the level so far; GX, GY, ORDER: global predictor and length of
+// the order; PREV: the other direction's projection exists; ABORT: the direction stopped (the status
+// word says why), its payload stays unwritten.
+enum { CTL_GO, CTL_LATE, CTL_BAD, CTL_GX, CTL_GY, CTL_ORDER, CTL_PREV, CTL_ABORT };
+
+// The bad-SAD threshold after `count` bad blocks (:605-616).
+__device__ __forceinline__ int bad_limit(const AnalyseParams &P, int count) {
+    return sat_i32((long long)P.coarse_bad_sad + (long long)(sat_i32((long long)P.coarse_bad_sad * count) / 16));
+}
+
 // search states of one block (exact_search_block :684-768, exact_refine_search :771-826,
 // exact_hex2 :942-1033, exact_umh :1036-1119, bad-SAD expansion :611-672)
 enum { S_REFINE, S_HEX_START, S_HEX_ITER, S_HEX_EXIT, S_BAD, S_BAD_RING, S_FINAL_RING, S_STORE };
-
-// The block's source pixels into shared memory (DirSh::srcp) for the fast path.
-template <class SH>
-__device__ __forceinline__ void stage_source(const Ctx &x, SH &s, const BlkC &b) {
-    if (b.fast_src) {
-        const int nlw = b.tilesx * b.bh;
-        const int nth = x.nw * 32;
-        uint2 *sp = s.srcp[SH::kSrc > 1 ? x.wbase : 0];
-        for (int t = x.tid; t < nlw; t += nth) {
-            const int row = t >> b.lgtx, col = t & (b.tilesx - 1);
-            sp[t] = stage4(x.S.y + b.lsrc + row * x.G.ys32 + col * 4, b.satd_mode != 0);
-        }
-        if (b.chroma && b.cfast_src) {
-            const int nc = b.ctilesx * b.crows;
-            for (int t = x.tid; t < 2 * nc; t += nth) {
-                const int pl = t >= nc, u = t - pl * nc;
-                const int row = u >> b.lgctx, col = u & (b.ctilesx - 1);
-                sp[nlw + t] = stage4((pl ? x.S.v : x.S.u) + b.csrc + row * x.G.cs32 + col * 4, x.satd != 0);
-            }
-        }
-    }
-}
 
 // The refinement and bad-SAD expansion of one block (exact_refine_search :771-826,
 // exact_hex2 :942-1033, exact_umh :1036-1119, the expansion :611-672): a state machine
@@ -1198,76 +1314,95 @@ __device__ __forceinline__ void stage_source(const Ctx &x, SH &s, const BlkC &b)
 // (ppx, ppy): predictor of the motion penalty; (own_x, own_y): the block's own predictor,
 // which the bad-SAD expansion switches to. `stage`: RS_ALL runs the refinement and the
 // expansion, RS_REFINE_ONLY stops where the expansion's test begins, RS_BAD_ONLY starts
-// there (the look-ahead runs the two apart: the test reads the bad count of the blocks
-// committed before), RS_NONE runs nothing.
+// there (a walk runs the two apart: the test reads the bad count of the blocks before),
+// RS_NONE runs nothing.
 enum { RS_NONE, RS_ALL, RS_REFINE_ONLY, RS_BAD_ONLY };
-template <class SH>
-__device__ __forceinline__ void run_search_steps(const Ctx &x, const BlkC &b, SH &s, int &ph, int stage, int stype,
-                                                 int radius, int lambda, int ppx, int ppy, int own_x, int own_y,
-                                                 int64_t idx, int &bad_count, int &bmx, int &bmy, unsigned &bsad,
-                                                 long long &bcost) {
-    const AnalyseParams &P = *x.P;
-    const LevelInfo &L = *x.L;
-    const int level = x.level;
-    int predx = ppx, predy = ppy;
-    int state = stage == RS_NONE ? S_STORE : (stage == RS_BAD_ONLY ? S_BAD : S_REFINE);
-    int hbx = 0, hby = 0, hdir = -2, hi = 0, hrad = 0, hret = 0, bad_r = 0, bad_max = 0;
-    unsigned found = 0;
-    for (;;) {
-        Gen g{0, 0, 0, 0, 0, 0, 0};
-        bool sets_mv = true, issue = false;
-        while (!issue && state != S_STORE) {
+struct Search {
+    int state, stage, stype, radius;
+    int predx, predy;                       // predictor of the motion penalty
+    int bmx, bmy;                           // the best so far
+    unsigned bsad;
+    long long bcost;
+    int hbx, hby, hdir, hi, hrad, hret, bad_r, bad_max;
+    unsigned found;
+    bool sets_mv;
+
+    __device__ __forceinline__ void begin(int stage_, int stype_, int radius_, int ppx, int ppy) {
+        stage = stage_; stype = stype_; radius = radius_;
+        predx = ppx; predy = ppy;
+        state = stage == RS_NONE ? S_STORE : (stage == RS_BAD_ONLY ? S_BAD : S_REFINE);
+        hdir = -2; hi = hrad = hret = 0;
+    }
+    // The next step's candidates; false when there is none.
+    __device__ __forceinline__ bool next(const Ctx &x, const BlkC &b, int own_x, int own_y, int64_t idx, int &bad_count, Gen &g) {
+        const AnalyseParams &P = *x.P;
+        const LevelInfo &L = *x.L;
+        sets_mv = true;
+        while (state != S_STORE) {
             if (state == S_BAD && stage == RS_REFINE_ONLY) {
                 state = S_STORE;
                 break;
             }
             if (state == S_REFINE) {
-                if (stype == 4) { g = make_gen(BK_EXH, bmx, bmy, radius, 0, 0); issue = true; state = S_BAD; }
-                else if (stype == 3) {
-                    g = make_gen(BK_UMH, bmx, bmy, radius, 0, 0); issue = true;
+                if (stype == 4) { state = S_BAD; g = make_gen(BK_EXH, bmx, bmy, radius, 0, 0); return true; }
+                if (stype == 3) {
                     state = S_HEX_START; hrad = radius; hret = 0;
-                } else if (stype == 2) { state = S_HEX_START; hrad = radius; hret = 0; }
+                    g = make_gen(BK_UMH, bmx, bmy, radius, 0, 0);
+                    return true;
+                }
+                if (stype == 2) { state = S_HEX_START; hrad = radius; hret = 0; }
                 else state = S_BAD;
             } else if (state == S_HEX_START) {
                 hbx = bmx; hby = bmy;
-                if (hrad > 1) { g = make_gen(BK_HEX6, hbx, hby, 0, 0, 0); sets_mv = false; issue = true; state = S_HEX_ITER; }
-                else { g = make_gen(BK_RING, hbx, hby, 1, 1, 0); issue = true; state = hret ? S_FINAL_RING : S_BAD; }
+                if (hrad > 1) { sets_mv = false; state = S_HEX_ITER; g = make_gen(BK_HEX6, hbx, hby, 0, 0, 0); return true; }
+                state = hret ? S_FINAL_RING : S_BAD;
+                g = make_gen(BK_RING, hbx, hby, 1, 1, 0);
+                return true;
             } else if (state == S_HEX_ITER) {
                 if (hi < hrad / 2 && hbx >= b.bnd0 && hby >= b.bnd1 && hbx < b.bnd2 && hby < b.bnd3) {
-                    g = make_gen(BK_HEX3, hbx, hby, 0, 0, c_mod6m1[hdir + 1]); sets_mv = false; issue = true;
-                } else state = S_HEX_EXIT;
+                    sets_mv = false;
+                    g = make_gen(BK_HEX3, hbx, hby, 0, 0, c_mod6m1[hdir + 1]);
+                    return true;
+                }
+                state = S_HEX_EXIT;
             } else if (state == S_HEX_EXIT) {
                 bmx = hbx; bmy = hby;
-                g = make_gen(BK_RING, hbx, hby, 1, 1, 0); issue = true; state = hret ? S_FINAL_RING : S_BAD;
+                state = hret ? S_FINAL_RING : S_BAD;
+                g = make_gen(BK_RING, hbx, hby, 1, 1, 0);
+                return true;
             } else if (state == S_BAD) {
                 found = bsad;
-                const int bl = sat_i32((long long)P.coarse_bad_sad + (long long)(sat_i32((long long)P.coarse_bad_sad * bad_count) / 16));
-                if (level > 0 && idx > 1 && P.coarse_bad_sad > 0 && (int)bsad > bl) {
+                if (x.level > 0 && idx > 1 && P.coarse_bad_sad > 0 && (int)bsad > bad_limit(P, bad_count)) {
                     bad_count++;
                     predx = own_x; predy = own_y;  // the block's own predictor
                     if (P.coarse_bad_range < 0) {
                         bad_max = -P.coarse_bad_range * L.pel; bad_r = L.pel;
-                        if (bad_r < bad_max) { g = make_gen(BK_RING, 0, 0, bad_r, L.pel, 0); issue = true; state = S_BAD_RING; }
-                        else state = S_FINAL_RING;
+                        if (bad_r < bad_max) { state = S_BAD_RING; g = make_gen(BK_RING, 0, 0, bad_r, L.pel, 0); return true; }
+                        state = S_FINAL_RING;
                     } else if (P.coarse_bad_range > 0) {
                         hrad = P.coarse_bad_range * L.pel; hret = 1;
-                        g = make_gen(BK_UMH, 0, 0, hrad, 0, 0); issue = true; state = S_HEX_START;
+                        state = S_HEX_START;
+                        g = make_gen(BK_UMH, 0, 0, hrad, 0, 0);
+                        return true;
                     } else state = S_FINAL_RING;
                 } else state = S_STORE;
             } else if (state == S_BAD_RING) {
                 if (bsad < found / 4) state = S_FINAL_RING;
                 else {
                     bad_r += L.pel;
-                    if (bad_r < bad_max) { g = make_gen(BK_RING, 0, 0, bad_r, L.pel, 0); issue = true; }
-                    else state = S_FINAL_RING;
+                    if (bad_r < bad_max) { g = make_gen(BK_RING, 0, 0, bad_r, L.pel, 0); return true; }
+                    state = S_FINAL_RING;
                 }
             } else {  // S_FINAL_RING
-                g = make_gen(BK_RING, bmx, bmy, 1, 1, 0); issue = true; state = S_STORE;
+                state = S_STORE;
+                g = make_gen(BK_RING, bmx, bmy, 1, 1, 0);
+                return true;
             }
         }
-        if (!issue) break;
-        int w;
-        eval_step(x, b, s, ph, g, lambda, predx, predy, bcost, bsad, w);
+        return false;
+    }
+    // The step's outcome: candidate w of g was accepted (its cost and sad are in bcost, bsad), or none (-1).
+    __device__ __forceinline__ void took(const Gen &g, int w) {
         if (g.kind == BK_HEX6 || g.kind == BK_HEX3) {  // exact_check_dir: a label, best.mv set at exit
             if (w >= 0) {
                 hdir = g.kind == BK_HEX6 ? w : g.odir + w - 1;
@@ -1280,6 +1415,56 @@ __device__ __forceinline__ void run_search_steps(const Ctx &x, const BlkC &b, SH
             bmx = m.x; bmy = m.y;
         }
     }
+};
+
+// Runs q (begun) to its end, one step after another.
+template <class SH>
+__device__ __forceinline__ void run_search(const Ctx &x, const BlkC &b, SH &s, int &ph, Search &q, int lambda, int own_x,
+                                           int own_y, int64_t idx, int &bad_count) {
+    Gen g{0, 0, 0, 0, 0, 0, 0};
+    while (q.next(x, b, own_x, own_y, idx, bad_count, g)) {
+        int w;
+        eval_step(x, b, s, ph, g, lambda, q.predx, q.predy, q.bcost, q.bsad, w);
+        q.took(g, w);
+    }
+}
+
+// The payload's luma byte: the mean of the block's samples inside the level (:673-679).
+__device__ __forceinline__ uint8_t block_mean(const BlkC &b, const LevelInfo &L, unsigned sum) {
+    const int rows = b.py >= 0 ? imax(0, imin(b.bh, L.lh - b.py)) : 0;
+    const int cols = b.px >= 0 ? imax(0, imin(b.bw, L.lw - b.px)) : 0;
+    const unsigned cnt = (unsigned)(rows * cols);
+    const unsigned dc = (cnt ? sum / cnt : 0) >> DC_SHIFT;
+    return (uint8_t)(dc > 255 ? 255 : dc);
+}
+
+// The special candidates of a block (exact_search_block, :708-746), one per lane: lanes 0..8 the
+// 3x3 neighbours in the reference's order, then the field's vector, the previous one, the global
+// predictor and zero. The reference scans field, previous, global, zero, then the neighbours that
+// are already processed, keeping the first of minimal cost, i.e. the least (cost, place).
+constexpr int kField = 9, kPrev = 10, kGlobal = 11, kZero = 12;
+
+// exact_sad of the lanes' candidates (lanes with `act`); equal vectors are evaluated once. With
+// several warps in the group they share the candidates and meet at a barrier.
+template <class SH>
+__device__ __forceinline__ unsigned special_sads(const Ctx &x, const BlkC &b, SH &s, int &ph, bool act, int mx, int my) {
+    const int lane = x.tid & 31;
+    const unsigned long long key = ((unsigned long long)(unsigned)mx << 32) | (unsigned)my;
+    const unsigned peers = __match_any_sync(kFull, key) & __ballot_sync(kFull, act);
+    const int leader = act ? __ffs(peers) - 1 : lane;
+    bool eval = act && leader == lane;
+    const int rank = __popc(__ballot_sync(kFull, eval) & ((1u << lane) - 1u));
+    if (x.nw > 1) eval = eval && rank % x.nw == (x.tid >> 5);
+    unsigned L, C;
+    eval_cands(x, b, eval, mx, my, L, C);
+    unsigned sad = sat_add(L, C);
+    if (x.nw > 1) {
+        if (eval) s.slot[ph][lane] = sad;
+        gsync(x);
+        sad = s.slot[ph][lane];  // of the leaders; the others' entries are not used
+        ph ^= 1;
+    }
+    return __shfl_sync(kFull, sad, leader);
 }
 
 // The per-direction search of one level (exact_search_level, :480-681). Every thread
@@ -1320,519 +1505,472 @@ __device__ __forceinline__ void search_level(const Ctx &x, DirSh &s, DirScratch 
         const int2 imv = vmv(interp);
         BlkC b;
         make_blk(x, px, py, !smallest, b);
-        stage_source(x, s, b);  // read by the refinement steps, after the next barrier
-        // ---- special candidates (exact_search_block, :708-746): slot list in the
-        // reference's evaluation roles; slot j is evaluated by group j
-        int n = 0, rs_slot = -1, prev_slot = -1, nseeds = 0;
-        int m0x = imv.x, m0y = imv.y;                    // slot 0: the interpolated predictor
-        n = 1;
-        if (edge && !smallest) rs_slot = n++;            // re-score the predictor at its source block (:536-549)
-        int pmx = 0, pmy = 0;
-        if (prevp) {
-            const uint2 pv = prevp[idx];
-            if (pv.y != 0xFFFFFFFFu && pv.y > 0) {
-                const int2 pm = vmv(pv);
-                pmx = pm.x; pmy = pm.y;
-                prev_slot = n++;
+        const int phb = ph;  // this block's entries of dc and score; the specials' barrier below publishes them
+        {
+            unsigned part = 0;
+            if (b.fast_src) part = stage_source(x, b);  // read by the evaluation, after the barrier below
+            if (lane == 0) s.dc[phb][warp] = part;
+        }
+        const bool dc_fast = b.fast_src && b.px2 == px && b.py2 == py;
+        if (!dc_fast && warp == x.nw - 1) {  // block_luma_dc on the reference's read path
+            const uint2 r = eval_slow(x, px, py, 0, 0, SLOW_DC);
+            if (lane == 0) s.dcs[phb] = r.x;
+        }
+        if (edge && !smallest && warp == 0) {  // re-score the predictor at its source block (:536-549)
+            const uint2 r = eval_slow(x, sxi * P.step_x, syi * P.step_y, imv.x, imv.y, SLOW_CHROMA);
+            if (lane == 0) s.score[phb] = sad_of(r);
+        }
+        gsync(x);
+        const unsigned pred_score = edge && !smallest ? s.score[phb] : interp.y;
+        const bool field_valid = pred_score != 0xFFFFFFFFu;
+        // ---- the special candidates, one per lane
+        bool act = false;
+        int mx = 0, my = 0;
+        if (lane < 9) {
+            const int ny = by - 1 + lane / 3, nx = bx - 1 + lane % 3;
+            if (ny >= 0 && ny < gh && nx >= 0 && nx < gw) {
+                const int64_t ci = (int64_t)ny * gw + nx;
+                const int64_t p = level == 0 ? initial_order_pos(gw, gh, nx, ny) : (int64_t)ds.pos[ci];
+                act = p < k;
+                if (act) { const int2 m = vmv(ci == last_idx ? last_val : field[ci]); mx = m.x; my = m.y; }
             }
-        }
-        const int zslot = n++, gslot = n++, nslot0 = n;
-        const int gxv = s.gx, gyv = s.gy;
-        int sdx[8], sdy[8];
-        bool panic = false;
-        // the 3x3 neighbourhood: positions in the order and current vectors, loaded together
-        int64_t npos[9];
-        uint2 nval[9];
-#pragma unroll
-        for (int q = 0; q < 9; q++) {
-            const int ny = by - 1 + q / 3, nx = bx - 1 + q % 3;
-            npos[q] = 0x7FFFFFFFFFFFFFFFLL;
-            nval[q] = make_uint2(0, 0);
-            if (ny < 0 || ny >= gh || nx < 0 || nx >= gw) continue;
-            const int64_t ci = (int64_t)ny * gw + nx;
-            npos[q] = level == 0 ? initial_order_pos(gw, gh, nx, ny) : (int64_t)ds.pos[ci];
-            nval[q] = ci == last_idx ? last_val : field[ci];
-        }
-#pragma unroll
-        for (int q = 0; q < 9; q++) {
-            const int64_t p = npos[q];
-            if (p < k) {
-                if (nseeds >= 8) { panic = true; continue; }  // seeds[8] overflows: the reference panics
-                const int2 nm = vmv(nval[q]);
-#pragma unroll
-                for (int t = 0; t < 8; t++)
-                    if (t == nseeds) { sdx[t] = nm.x; sdy[t] = nm.y; }
-                nseeds++;
+        } else if (lane == kField) {
+            act = field_valid; mx = imv.x; my = imv.y;
+        } else if (lane == kPrev) {
+            if (prevp) {
+                const uint2 pv = prevp[idx];
+                act = pv.y != 0xFFFFFFFFu && pv.y > 0;
+                const int2 m = vmv(pv);
+                mx = m.x; my = m.y;
             }
+        } else if (lane == kGlobal) {
+            act = true; mx = s.gx; my = s.gy;
+        } else if (lane == kZero) {
+            act = true;
         }
-        if (panic) {
+        const unsigned seeds = __ballot_sync(kFull, act) & 0x1FFu;
+        if (__popc(seeds) > 8) {  // seeds[8] overflows: the reference panics
             if (x.tid == 0) { atomicOr(status, ST_PANIC); s.abort_ = 1; }
             break;
         }
-        n += nseeds;
-        const int dcslot = n++;
-        // ---- evaluate the special slots
-        const int G = step_lanes(x.grp_lanes, n, x.nw);
-        const int grp = warp * (32 / G) + lane / G, sub = lane & (G - 1), NG = x.nw * (32 / G);
-        unsigned (*slotL)[MAXSLOT] = s.slotL[x.wbase];
-        for (int j0 = 0; j0 < n; j0 += NG) {
-            const int j = j0 + grp;
-            const bool act = j < n;
-            int kind = 0, mx = 0, my = 0;
-            bool ch = !smallest;
-            if (j == 0) { mx = m0x; my = m0y; }
-            else if (j == rs_slot) { mx = m0x; my = m0y; kind = 1; ch = true; }
-            else if (j == prev_slot) { mx = pmx; my = pmy; }
-            else if (j == zslot) { mx = 0; my = 0; }
-            else if (j == gslot) { mx = gxv; my = gyv; }
-            else if (j == dcslot) { kind = 2; ch = false; }
-            else if (j >= nslot0 && j < nslot0 + nseeds) {
-#pragma unroll
-                for (int t = 0; t < 8; t++)
-                    if (t == j - nslot0) { mx = sdx[t]; my = sdy[t]; }
-            }
-            Res r{0, 0, 0, 0, 0, 0};
-            if (act) r = eval_lane(x, b, kind, sxi * P.step_x, syi * P.step_y, mx, my, ch, sub, G);
-            group_sum3(r, G);
-            if (act && sub == 0) {
-                unsigned Lv, Cv;
-                if (kind == 2) { Lv = r.L; Cv = 0; }
-                else finalize(r, Lv, Cv);
-                slotL[ph][j] = ch ? sat_add(Lv, Cv) : Lv;  // exact_sad: luma (+ chroma)
-            }
-        }
-        gsync(x);
-        const int phs = ph;
-        ph ^= 1;
-        // ---- selection among the special candidates (:716-747)
-        const unsigned pred_score = rs_slot >= 0 ? slotL[phs][rs_slot] : interp.y;
-        const bool field_valid = pred_score != 0xFFFFFFFFu;
-        int bmx = 0, bmy = 0;
-        unsigned bsad;
-        long long bcost;
-        bool refine = false;
+        const bool search = !(level == 0 && P.distance == 0);
+        if (!search) act = lane == (field_valid ? kField : kZero);
+        const unsigned sd = special_sads(x, b, s, ph, act, mx, my);
+        const int pp = lane < 9 ? P.pnbour : lane == kPrev ? P.prev : lane == kGlobal ? P.pglobal : lane == kZero ? P.pzero : 0;
+        const int place = lane < 9 ? 4 + __popc(seeds & ((1u << lane) - 1u)) : lane - kField;
+        const long long cost = (long long)sd + (((long long)pp * sd) >> 8);
+        const int wl = first_min(act, cost, place);
+        Search q;
+        q.bmx = __shfl_sync(kFull, mx, wl); q.bmy = __shfl_sync(kFull, my, wl);
+        q.bsad = __shfl_sync(kFull, sd, wl);
+        q.bcost = (long long)q.bsad;
         int lambda = 0, radius = 0, stype = 0, ppx = imv.x, ppy = imv.y;
-        if (level == 0 && P.distance == 0) {
-            if (field_valid) { bmx = imv.x; bmy = imv.y; bsad = slotL[phs][0]; }
-            else bsad = slotL[phs][zslot];
-            bcost = (long long)bsad;
-        } else {
-            if (field_valid) { bmx = imv.x; bmy = imv.y; bsad = slotL[phs][0]; bcost = (long long)bsad; }
-            else { bsad = 0xFFFFFFFFu; bcost = 0x7FFFFFFFFFFFFFFFLL; }
-            if (prev_slot >= 0) {
-                const unsigned sd = slotL[phs][prev_slot];
-                const long long cst = (long long)sd + (((long long)P.prev * sd) >> 8);
-                if (cst < bcost) { bmx = pmx; bmy = pmy; bsad = sd; bcost = cst; ppx = pmx; ppy = pmy; }
-            }
-            {
-                const unsigned sd = slotL[phs][gslot];
-                const long long cst = (long long)sd + (((long long)P.pglobal * sd) >> 8);
-                if (cst < bcost) { bmx = gxv; bmy = gyv; bsad = sd; bcost = cst; }
-            }
-            {
-                const unsigned sd = slotL[phs][zslot];
-                const long long cst = (long long)sd + (((long long)P.pzero * sd) >> 8);
-                if (cst < bcost) { bmx = 0; bmy = 0; bsad = sd; bcost = cst; }
-            }
-#pragma unroll
-            for (int q = 0; q < 8; q++) {
-                if (q >= nseeds) break;
-                const unsigned sd = slotL[phs][nslot0 + q];
-                const long long cst = (long long)sd + (((long long)P.pnbour * sd) >> 8);
-                if (cst < bcost) { bmx = sdx[q]; bmy = sdy[q]; bsad = sd; bcost = cst; }
-            }
-            bcost = (long long)bsad;
+        if (search) {
+            const long long cf = __shfl_sync(kFull, cost, kField), cp = __shfl_sync(kFull, cost, kPrev);
+            const bool prev = __shfl_sync(kFull, act, kPrev);
+            const int pmx = __shfl_sync(kFull, mx, kPrev), pmy = __shfl_sync(kFull, my, kPrev);
+            if (prev && (!field_valid || cp < cf)) { ppx = pmx; ppy = pmy; }
             lambda = adapt_lambda(L.lambda_base, L.lsad, pred_score);
             radius = L.base_radius;
             if (level > 0 && P.coarse_distance < 0) {
-                const unsigned act = plane_activity(x.S.y, x.G.ylen, x.G.ys, L.y_off + b.py2, b.px2, b.bw, b.bh, x.satd) +
-                                     plane_activity(x.S.u, x.G.clen, x.G.cs, L.c_off + py / 2, px / 2, b.bw / 2, b.bh / 2, x.satd) +
-                                     plane_activity(x.S.v, x.G.clen, x.G.cs, L.c_off + py / 2, px / 2, b.bw / 2, b.bh / 2, x.satd);
-                radius = adaptive_radius(radius, act);
+                radius = adaptive_radius(radius, block_activity(x.P, x.L, x.S.y, b.px2, b.py2, px, py));
             }
             stype = (edge && level == 1) ? 0 : L.search_type;
-            refine = true;
         }
-        const unsigned dcsum = slotL[phs][dcslot];
-        run_search_steps(x, b, s, ph, refine ? RS_ALL : RS_NONE, stype, radius, lambda, ppx, ppy, imv.x, imv.y, idx,
-                         bad_count, bmx, bmy, bsad, bcost);
+        unsigned dcsum = 0;
+        if (dc_fast)
+            for (int w = 0; w < x.nw; w++) dcsum += s.dc[phb][w];
+        else dcsum = s.dcs[phb];
+        q.begin(search ? RS_ALL : RS_NONE, stype, radius, ppx, ppy);
+        run_search(x, b, s, ph, q, lambda, imv.x, imv.y, idx, bad_count);
         // ---- store (:673-679)
-        const int rows = b.py >= 0 ? imax(0, imin(b.bh, L.lh - b.py)) : 0;
-        const int cols = b.px >= 0 ? imax(0, imin(b.bw, L.lw - b.px)) : 0;
-        const unsigned cnt = (unsigned)(rows * cols);
-        unsigned dc = (cnt ? dcsum / cnt : 0) >> DC_SHIFT;
-        if (dc > 255) dc = 255;
-        const uint2 v = mkvec(bmx, bmy, smallest ? sat_mul(bsad, 3) : bsad);
+        const uint2 v = mkvec(q.bmx, q.bmy, smallest ? sat_mul(q.bsad, 3) : q.bsad);
         if (x.tid == 0) {
             field[idx] = v;
-            lumaf[idx] = (uint8_t)dc;
+            lumaf[idx] = block_mean(b, L, dcsum);
         }
         last_idx = idx;
         last_val = v;
+        if (ph == phb) ph ^= 1;  // the next block writes other entries of dc and score
     }
 }
 
-// ---- level 0 with look-ahead (speculative and exact) ------------------------------------
-// The calling warp waits until blocks 0 .. k-1 of the level are committed (*committed counts
-// them; the committing warp stores its results, fences, then bumps the count). Bounded: false once
-// kWaitCycles have passed or another warp of the direction has given up (the caller flags
-// ST_TIMEOUT and carries on, so every warp still reaches its barriers). The fence after the wait
-// makes the committed blocks' stores visible to every lane. XSM: the count and the stores it
-// publishes are in global memory, written by warps on other SMs.
-template <bool XSM>
-__device__ __forceinline__ bool wait_commits(volatile int *committed, int64_t k, volatile int *late) {
-    const long long t0 = clock64();
-    for (;;) {
-        const int seen = (int64_t)*committed >= k;
-        if (__all_sync(0xFFFFFFFFu, seen)) break;
-        const int give_up = *late || clock64() - t0 > kWaitCycles;
-        if (__shfl_sync(0xFFFFFFFFu, give_up, 0)) {
-            if ((threadIdx.x & 31) == 0) *late = 1;
-            return false;
-        }
-        __nanosleep(32);
-    }
-    if (XSM) __threadfence();
-    else __threadfence_block();
-    return true;
-}
-
-// exact_search_level (:480-681) with D = NW blocks in flight per direction, one per warp
-// ("look-ahead"). Warp w searches blocks w, w + D, w + 2D, ... of the level's order. Of what a
-// block reads, only these can come from the blocks searched just before it: the vectors of its
-// processed neighbours, taken as seeds (:570-585); at level > 0 an edge block's predictor, the
-// current vector of an inner cell (:520-549); the bad-SAD count (:605-616). Everything else
-// (the interpolated predictor of an inner block, lambda, radius, search type, the
-// previous-frame, zero and global candidates) comes from the coarser level, the other direction
-// and the block itself. A warp starts block k once it has committed block k - D, so cells
-// processed at order positions <= k - D hold their final vectors; seeds from the at most D - 1
-// cells processed at positions in (k - D, k) are "deferred": the block's special candidates and
-// its refinement run without them. The warp then waits for block k - 1's commit (a count of
-// committed blocks in shared memory: blocks commit in the reference's order) and replays the
-// reference's selection
-// with the deferred seeds at their places in the scan: :740-746 keep the first candidate of
-// minimal cost, i.e. the least (cost, place), so the speculative best stands unless a deferred
-// seed costs less, or the same at an earlier place. If one wins with another vector, the
-// refinement runs again from it; with the same vector (hence the same SAD) the refinement
-// already run is the reference's. The bad-SAD test and expansion run after the hand-over, with
-// the count of the blocks before. An edge block whose predictor cell is among the deferred ones
-// waits for block k - 1 first and runs without look-ahead. Stored vectors are the reference's in
-// every case; on the 1080p workload fewer than 1 % of level-0 blocks run their refinement twice.
-// A level with an input on which the reference would panic takes search_level instead.
-// stats (nullable): [0] blocks, [1] blocks with deferred seeds, [2] deferred seeds evaluated
-// (the others had the vector of a candidate already evaluated), [3] refinements run again.
+// ---- a level walked by several warps (look-ahead: speculative and exact) -------------------
+// exact_search_level (:480-681) with D blocks of a direction in flight, one per warp. Warp g
+// searches blocks g, g + D, g + 2D, ... of the level's order. Of what a block reads, only these come
+// from blocks searched before it: the vectors of its processed neighbours, taken as seeds
+// (:570-585); at level > 0 an edge block's predictor, the vector of an inner cell (:520-549); the
+// bad-SAD count (:605-616). Everything else (the interpolated predictor, lambda, radius, search
+// type, the previous-frame, zero and global candidates) comes from the coarser level, the other
+// direction and the block itself.
 //
-// spec_walk is one warp's part: blocks g, g + D, ... of the level (x: a one-warp group; x.tid
-// the lane). The count of committed blocks, the flag of a wait that gave up and the
-// direction's abort flag are passed in: in shared memory when the direction's warps share a CTA
-// (XSM false), in the pair's scratch when they are CTAs on different SMs (XSM true, the level-0
-// kernel), where the field's cells written during the level are read from L2 (__ldcg: the SM's
-// L1 is not coherent with the other SMs' stores) and commits fence device-wide.
-template <bool XSM>
-__device__ __forceinline__ uint2 ld_cell(const uint2 *p) {
-    if (XSM) return __ldcg(p);
-    return *p;
+// A block publishes its vector in one 64-bit word per cell (AnalyseParams::off_keys, cleared before
+// the level): the vector and a tag, stored and read in one piece, so the word itself says what it is
+// and no fence or count is needed. The tag says whether the vector is the final one or a tentative
+// one: a block searches with the vectors that its processed neighbours have published when it starts,
+// tentative ones included (one that has published nothing is left out), publishes the result as
+// tentative, and then watches the words of the neighbours that were not final. When one changes, the
+// selection among the special candidates is made anew (:740-746 keep the first candidate of minimal
+// cost, i.e. the least (cost, place)), and if that selects another vector the refinement runs again
+// from it and the result is published anew; with the same vector (hence the same SAD) the refinement
+// already run is the reference's. Once all of them are final and were the ones used, the block's own
+// vector is final. So every stored vector is the reference's, whatever D and however the warps run,
+// a block depends on its neighbours alone, not on the whole order before it, and a repeated refinement
+// holds up the blocks after it only if its outcome differs from what they used: where a fifth of the
+// blocks repeat it (noisy fields), waiting for each in turn was the larger part of the walk.
+//
+// The bad-SAD test needs the number of bad blocks before this one. Its threshold only grows with
+// that number, so a block at or below the first threshold is not bad whatever the number; any other
+// waits until every earlier block has passed its test (each warp publishes the next block it has not
+// tested, in the histogram's words, which are free while a level is searched) and then reads the
+// number. The lowest block that is not finished waits for nothing, and every warp takes its blocks in
+// order, so the warps, all resident, always make progress; the waits are bounded all the same.
+// A level with an input on which the reference would panic takes search_level instead.
+// stats (nullable): [0] blocks, [1] blocks that started before all their processed neighbours were
+// final, [2] seeds evaluated after the start (the others had the vector of a candidate already
+// evaluated), [3] blocks that ran their refinement again.
+__device__ __forceinline__ unsigned long long ld_tag(const unsigned long long *p) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
 }
-template <bool XSM, class SH>
-__device__ __forceinline__ void spec_walk(const Ctx &x, SH &s, DirScratch &ds, const uint2 *prevp, int g, int64_t order_len,
-                                          int gxv, int gyv, volatile int *committed, volatile int *late_flag,
-                                          int *abort_flag, int *status, unsigned long long *stats) {
+__device__ __forceinline__ void st_tag(unsigned long long *p, unsigned long long v) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ int ld_word(const int *p) {
+    int v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_word(int *p, int v) {
+    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+// The warp waits until done() holds in every lane. Bounded: false once kWaitCycles have passed or
+// another warp of the direction has given up (the caller flags ST_TIMEOUT and carries on).
+template <class F>
+__device__ __forceinline__ bool spin(F done, int *late) {
+    const long long t0 = clock64();
+    for (int it = 1;; it++) {
+        if (__all_sync(kFull, done())) return true;
+        if ((it & 127) == 0) {
+            const int give_up = ld_word(late) || clock64() - t0 > kWaitCycles;
+            if (__shfl_sync(kFull, give_up, 0)) {
+                if ((threadIdx.x & 31) == 0) st_word(late, 1);
+                return false;
+            }
+        }
+    }
+}
+
+enum { TAG_NONE, TAG_TENTATIVE, TAG_FINAL };
+__device__ __forceinline__ unsigned long long tag_word(int tag, int mx, int my) {
+    return ((unsigned long long)tag << 32) | mkvec(mx, my, 0).x;
+}
+
+constexpr int kMaxWalkers = 64;  // warps of a direction that may walk a level
+template <class SH>
+__device__ __forceinline__ void walk_level(const Ctx &x, SH &s, const DirScratch &ds, const uint2 *prevp, int g, int D,
+                                           int order_len, int gxv, int gyv, int *ctl, int *status, unsigned long long *stats) {
     const AnalyseParams &P = *x.P;
     const LevelInfo &L = *x.L;
     const int level = x.level, gw = L.gw, gh = L.gh;
     uint2 *field = ds.vec[level & 1];
     uint8_t *lumaf = ds.luma[level & 1];
     const bool smallest = L.smallest != 0;
-    constexpr int D = NW;
+    int *progress = (int *)ds.hist;
     const int lane = x.tid;
     int ph = 0;
-    unsigned long long n_blk = 0, n_def = 0, n_eval = 0, n_rerun = 0;
+    int n_blk = 0, n_def = 0, n_eval = 0, n_rerun = 0;
     bool late = false;
-    unsigned (*slotL)[MAXSLOT] = s.slotL[x.wbase];
-    auto wait_prev = [&](int64_t k) {  // block k - 1 is committed (and its stores visible) after this
-        if (k > 0 && !wait_commits<XSM>(committed, k, late_flag)) late = true;
-    };
-    auto pos_of = [&](int nx, int ny) -> int64_t {
-        return level == 0 ? initial_order_pos(gw, gh, nx, ny) : (int64_t)ds.pos[(int64_t)ny * gw + nx];
-    };
-    for (int64_t k = g; k < order_len; k += D) {
+    for (int k = g; k < order_len; k += D) {
         const int2 bxy = level == 0 ? initial_order_at(gw, gh, k) : unpack_xy(ds.order[k]);
         const int bx = bxy.x, by = bxy.y;
-        const int64_t idx = (int64_t)by * gw + bx;
+        const int idx = by * gw + bx;
         int px = (level > 0 && bx == gw - 1) ? L.lw - P.block_w : bx * P.step_x;
         int py = (level > 0 && by == gh - 1) ? L.lh - P.block_h : by * P.step_y;
         px += L.pxoff;
         py += L.pyoff;
         const bool edge = level > 0 && (bx == gw - 1 || by == gh - 1);
         const int sxi = imin(bx, gw - 2), syi = imin(by, gh - 2);
-        const int64_t sidx = (int64_t)syi * gw + sxi;
-        // an edge block's predictor is its inner cell's current vector: when another warp may not
-        // have committed that cell yet, take the hand-over first (the block runs without look-ahead)
-        bool waited = false;
-        if (edge) {
-            const int64_t p = pos_of(sxi, syi);
-            if (p < k && p > k - D) { wait_prev(k); waited = true; }
+        // ---- the special candidates, one per lane (see special_sads)
+        bool act = false, seed = false, open = false;  // open: a seed that is not final yet
+        int mx = 0, my = 0;
+        int ncell = 0;
+        if (lane < 9) {
+            const int ny = by - 1 + lane / 3, nx = bx - 1 + lane % 3;
+            if (ny >= 0 && ny < gh && nx >= 0 && nx < gw) {
+                ncell = ny * gw + nx;
+                act = (level == 0 ? (int)initial_order_pos(gw, gh, nx, ny) : ds.pos[ncell]) < k;
+                seed = act;
+                if (act) {
+                    const unsigned long long v = ld_tag(ds.keys + ncell);
+                    const int2 m = vmv(make_uint2((unsigned)v, 0));
+                    mx = m.x; my = m.y;
+                    act = (int)(v >> 32) != TAG_NONE;
+                    open = (int)(v >> 32) != TAG_FINAL;
+                }
+            }
+        } else if (lane == kPrev) {
+            if (prevp) {
+                const uint2 pv = prevp[idx];
+                act = pv.y != 0xFFFFFFFFu && pv.y > 0;
+                const int2 m = vmv(pv);
+                mx = m.x; my = m.y;
+            }
+        } else if (lane == kGlobal) {
+            act = true; mx = gxv; my = gyv;
+        } else if (lane == kZero) {
+            act = true;
         }
-        const uint2 interp = ld_cell<XSM>(field + (edge ? sidx : idx));
+        uint2 interp;
+        if (edge) {  // its inner cell comes earlier in the order (level_spec_ok): that cell's final vector
+            unsigned long long v = 0;
+            if (!spin([&] { v = ld_tag(ds.keys + syi * gw + sxi); return (int)(v >> 32) == TAG_FINAL; }, ctl + CTL_LATE)) late = true;
+            interp = make_uint2((unsigned)v, 0);  // the score is taken anew below
+        } else {
+            interp = field[idx];
+        }
         const int2 imv = vmv(interp);
+        if (lane == kField) { mx = imv.x; my = imv.y; }
+        const unsigned seeds = __ballot_sync(kFull, seed);  // at most 8 (level_spec_ok)
         BlkC b;
         make_blk(x, px, py, !smallest, b);
-        stage_source(x, s, b);
-        // ---- special candidates (exact_search_block, :708-746), as in search_level, without
-        // the deferred seeds
-        int n = 1, rs_slot = -1, prev_slot = -1;
-        if (edge && !smallest) rs_slot = n++;  // re-score the predictor at its source block (:536-549)
-        int pmx = 0, pmy = 0;
-        if (prevp) {
-            const uint2 pv = prevp[idx];
-            if (pv.y != 0xFFFFFFFFu && pv.y > 0) {
-                const int2 pm = vmv(pv);
-                pmx = pm.x; pmy = pm.y;
-                prev_slot = n++;
-            }
-        }
-        const int zslot = n++, gslot = n++, nslot0 = n;
-        // seeds evaluated now and deferred seeds, in shared memory (written by lane 0; the values are
-        // the same in every lane)
-        int2 *sv = s.seedv[x.wbase];
-        int *sq = s.seedq[x.wbase], *dq = s.defq[x.wbase];
-        long long *dcell = s.defc[x.wbase];
-        int nseeds = 0, nall = 0, ndef = 0;
-#pragma unroll 1
-        for (int q = 0; q < 9; q++) {
-            const int ny = by - 1 + q / 3, nx = bx - 1 + q % 3;
-            if (ny < 0 || ny >= gh || nx < 0 || nx >= gw) continue;
-            const int64_t p = pos_of(nx, ny);
-            if (p >= k) continue;
-            const int64_t ci = (int64_t)ny * gw + nx;
-            if (!waited && p > k - D) {  // searched by another warp, maybe not yet committed
-                if (lane == 0) { dq[ndef] = nall; dcell[ndef] = ci; }
-                ndef++;
-            } else {
-                const int2 nm = vmv(ld_cell<XSM>(field + ci));
-                if (lane == 0) { sv[nseeds] = nm; sq[nseeds] = nall; }
-                nseeds++;
-            }
-            nall++;  // at most 8: levels with more processed neighbours take search_level
-        }
+        unsigned dcsum = 0;
+        if (b.fast_src) dcsum = stage_source(x, b);
+        if (!(b.fast_src && b.px2 == px && b.py2 == py))  // block_luma_dc on the reference's read path
+            dcsum = eval_slow(x, px, py, 0, 0, SLOW_DC).x;
+        unsigned pred_score = interp.y;
+        if (edge)  // re-score the predictor at its source block (:536-549)
+            pred_score = sad_of(eval_slow(x, sxi * P.step_x, syi * P.step_y, imv.x, imv.y, SLOW_CHROMA));
         __syncwarp();
-        n += nseeds;
-        const int dcslot = n++;
-        {
-            const int G = step_lanes(x.grp_lanes, n, 1);
-            const int grp = lane / G, sub = lane & (G - 1), NG = 32 / G;
-            for (int j0 = 0; j0 < n; j0 += NG) {
-                const int j = j0 + grp;
-                const bool act = j < n;
-                int kind = 0, mx = 0, my = 0;
-                bool ch = !smallest;
-                if (j == 0) { mx = imv.x; my = imv.y; }
-                else if (j == rs_slot) { mx = imv.x; my = imv.y; kind = 1; ch = true; }
-                else if (j == prev_slot) { mx = pmx; my = pmy; }
-                else if (j == zslot) { mx = 0; my = 0; }
-                else if (j == gslot) { mx = gxv; my = gyv; }
-                else if (j == dcslot) { kind = 2; ch = false; }
-                else if (j >= nslot0 && j < nslot0 + nseeds) { mx = sv[j - nslot0].x; my = sv[j - nslot0].y; }
-                Res r{0, 0, 0, 0, 0, 0};
-                if (act) r = eval_lane(x, b, kind, sxi * P.step_x, syi * P.step_y, mx, my, ch, sub, G);
-                group_sum3(r, G);
-                if (act && sub == 0) {
-                    unsigned Lv, Cv;
-                    if (kind == 2) { Lv = r.L; Cv = 0; }
-                    else finalize(r, Lv, Cv);
-                    slotL[ph][j] = ch ? sat_add(Lv, Cv) : Lv;
-                }
-            }
-        }
-        __syncwarp();
-        const int phs = ph;
-        ph ^= 1;
-        // ---- selection (:716-747); places in the reference's scan: field 0, previous 1,
-        // global 2, zero 3, the neighbour seeds 4 + their place among the seeds
-        const unsigned pred_score = rs_slot >= 0 ? slotL[phs][rs_slot] : interp.y;
         const bool field_valid = pred_score != 0xFFFFFFFFu;
-        int bmx = 0, bmy = 0, bpos = -1;
-        unsigned bsad;
-        long long bcost;
-        bool refine = false;
+        if (lane == kField) act = field_valid;
+        const bool search = !(level == 0 && P.distance == 0);
+        if (!search) act = lane == (field_valid ? kField : kZero);
+        // ---- selection (:716-747)
+        const int pp = lane < 9 ? P.pnbour : lane == kPrev ? P.prev : lane == kGlobal ? P.pglobal : lane == kZero ? P.pzero : 0;
+        const int place = lane < 9 ? 4 + __popc(seeds & ((1u << lane) - 1u)) : lane - kField;
+        unsigned sd = 0;
+        bool fresh = act;  // lanes whose candidate is to be evaluated
+        bool started = false, reran = false, published = false;
+        int selx = 0, sely = 0;
         int lambda = 0, radius = 0, stype = 0, ppx = imv.x, ppy = imv.y;
-        if (level == 0 && P.distance == 0) {  // level 0 without a search: the field's vector or zero
-            if (field_valid) { bmx = imv.x; bmy = imv.y; bsad = slotL[phs][0]; }
-            else bsad = slotL[phs][zslot];
-            bcost = (long long)bsad;
-        } else {
-            if (field_valid) { bmx = imv.x; bmy = imv.y; bsad = slotL[phs][0]; bcost = (long long)bsad; bpos = 0; }
-            else { bsad = 0xFFFFFFFFu; bcost = 0x7FFFFFFFFFFFFFFFLL; }
-            if (prev_slot >= 0) {
-                const unsigned sd = slotL[phs][prev_slot];
-                const long long cst = (long long)sd + (((long long)P.prev * sd) >> 8);
-                if (cst < bcost) { bmx = pmx; bmy = pmy; bsad = sd; bcost = cst; ppx = pmx; ppy = pmy; bpos = 1; }
-            }
-            {
-                const unsigned sd = slotL[phs][gslot];
-                const long long cst = (long long)sd + (((long long)P.pglobal * sd) >> 8);
-                if (cst < bcost) { bmx = gxv; bmy = gyv; bsad = sd; bcost = cst; bpos = 2; }
-            }
-            {
-                const unsigned sd = slotL[phs][zslot];
-                const long long cst = (long long)sd + (((long long)P.pzero * sd) >> 8);
-                if (cst < bcost) { bmx = 0; bmy = 0; bsad = sd; bcost = cst; bpos = 3; }
-            }
-#pragma unroll 1
-            for (int q = 0; q < nseeds; q++) {
-                const unsigned sd = slotL[phs][nslot0 + q];
-                const long long cst = (long long)sd + (((long long)P.pnbour * sd) >> 8);
-                if (cst < bcost) { bmx = sv[q].x; bmy = sv[q].y; bsad = sd; bcost = cst; bpos = 4 + sq[q]; }
-            }
-            lambda = adapt_lambda(L.lambda_base, L.lsad, pred_score);
-            radius = L.base_radius;
-            if (level > 0 && P.coarse_distance < 0) {
-                const unsigned act = plane_activity(x.S.y, x.G.ylen, x.G.ys, L.y_off + b.py2, b.px2, b.bw, b.bh, x.satd) +
-                                     plane_activity(x.S.u, x.G.clen, x.G.cs, L.c_off + py / 2, px / 2, b.bw / 2, b.bh / 2, x.satd) +
-                                     plane_activity(x.S.v, x.G.clen, x.G.cs, L.c_off + py / 2, px / 2, b.bw / 2, b.bh / 2, x.satd);
-                radius = adaptive_radius(radius, act);
-            }
-            stype = (edge && level == 1) ? 0 : L.search_type;
-            refine = true;
-        }
-        const long long sel_cost = bcost;
-        const int sel_x = bmx, sel_y = bmy;
-        bcost = (long long)bsad;
-        const unsigned dcsum = slotL[phs][dcslot];
-        // One call site of the search state machine (it is inlined, so each site is a copy of the
-        // evaluation code): pass 0 the refinement with the seeds known at the start; pass 1 the
-        // refinement again from a deferred seed that wins; pass 2 the bad-SAD test and expansion
-        // (:604-672) with the count of the blocks committed before.
-        int stage = refine ? RS_REFINE_ONLY : RS_NONE, pass = 0, bad_count = 0;
+        Search q;
+        q.begin(RS_NONE, 0, 0, 0, 0);
+        Gen g_{0, 0, 0, 0, 0, 0, 0};  // the step in work, its next 32 candidates, and the one accepted so far
+        int base = 0, win = -1;
+        bool stepping = false;
+        int bad_count = 0;
+        bool final = false;
+        // Each turn evaluates up to 32 candidates, one per lane: special ones that are new, else the next
+        // of the search step in work (one call site of the evaluation, which is inlined). While a search
+        // runs, seeds that have become final are looked at between its turns; tentative ones only when
+        // there is nothing else to do, since the work they cause may be in vain.
         for (;;) {
-            run_search_steps(x, b, s, ph, stage, stype, radius, lambda, ppx, ppy, imv.x, imv.y, idx, bad_count, bmx,
-                             bmy, bsad, bcost);
-            if (pass == 0) {
-                if (!waited) wait_prev(k);
-                n_blk++;
-                if (refine && ndef > 0) {
-                    n_def++;
-                    long long cb = sel_cost;
-                    int cpos = bpos, cx = sel_x, cy = sel_y;
-                    unsigned csad = 0;
-                    bool dwin = false;
-#pragma unroll 1
-                    for (int j = 0; j < ndef; j++) {
-                        const int64_t ci = dcell[j];
-                        const int pos = 4 + dq[j];
-                        const int2 m = vmv(ld_cell<XSM>(field + ci));
-                        // its exact_sad: from an evaluated candidate with the same vector (same block,
-                        // same reads), else evaluated now
-                        unsigned sd = 0;
-                        bool have = true;
-                        if (m.x == imv.x && m.y == imv.y) sd = slotL[phs][0];
-                        else if (prev_slot >= 0 && m.x == pmx && m.y == pmy) sd = slotL[phs][prev_slot];
-                        else if (m.x == 0 && m.y == 0) sd = slotL[phs][zslot];
-                        else if (m.x == gxv && m.y == gyv) sd = slotL[phs][gslot];
-                        else {
-                            have = false;
-                            for (int t = 0; t < nseeds && !have; t++)
-                                if (sv[t].x == m.x && sv[t].y == m.y) {
-                                    sd = slotL[phs][nslot0 + t];
-                                    have = true;
-                                }
+            bool special = __any_sync(kFull, fresh);
+            if (!special && !stepping) {
+                if (q.next(x, b, imv.x, imv.y, idx, bad_count, g_)) { stepping = true; base = 0; win = -1; }
+                else {
+                    if (final) break;
+                    if (__any_sync(kFull, open)) {  // publish, then wait for news
+                        if (!published && lane == 0) st_tag(ds.keys + idx, tag_word(TAG_TENTATIVE, q.bmx, q.bmy));
+                        published = true;
+                        unsigned long long v = 0;
+                        if (!spin([&] {
+                                if (open) v = ld_tag(ds.keys + ncell);
+                                const int2 m = vmv(make_uint2((unsigned)v, 0));
+                                fresh = open && (int)(v >> 32) != TAG_NONE && (!act || m.x != mx || m.y != my);
+                                return __any_sync(kFull, fresh) || !(open && (int)(v >> 32) != TAG_FINAL);
+                            }, ctl + CTL_LATE)) {
+                            late = true;
+                            open = false;
                         }
-                        if (!have) {
-                            Res r = eval_lane(x, b, 0, 0, 0, m.x, m.y, !smallest, lane, 32);
-                            group_sum3(r, 32);
-                            unsigned Lv, Cv;
-                            finalize(r, Lv, Cv);
-                            sd = !smallest ? sat_add(Lv, Cv) : Lv;
-                            n_eval++;
-                        }
-                        const long long cst = (long long)sd + (((long long)P.pnbour * sd) >> 8);
-                        if (cst < cb || (cst == cb && pos < cpos)) {
-                            cb = cst; cpos = pos; cx = m.x; cy = m.y; csad = sd; dwin = true;
-                        }
-                    }
-                    if (dwin && (cx != sel_x || cy != sel_y)) {  // a deferred seed with another vector wins
-                        n_rerun++;
-                        bmx = cx; bmy = cy; bsad = csad; bcost = (long long)csad;
-                        pass = 1;
+                        if ((int)(v >> 32) == TAG_FINAL) open = false;
+                        if (fresh) { const int2 m = vmv(make_uint2((unsigned)v, 0)); mx = m.x; my = m.y; act = true; }
                         continue;
                     }
+                    final = true;  // every seed is final and is the one used
+                    if (search && level > 0 && P.coarse_bad_sad > 0) {
+                        bool bad = false;
+                        if (idx > 1 && (int)q.bsad > P.coarse_bad_sad) {  // above the threshold of a count of 0
+                            if (!spin([&] {
+                                    bool ok = true;
+                                    for (int h = lane; h < D; h += 32) ok = ok && (h == g || ld_word(progress + h) >= k);
+                                    return ok;
+                                }, ctl + CTL_LATE))
+                                late = true;
+                            __threadfence();
+                            bad_count = ld_word(ctl + CTL_BAD);
+                            bad = (int)q.bsad > bad_limit(P, bad_count);
+                            if (bad && lane == 0) { st_word(ctl + CTL_BAD, bad_count + 1); __threadfence(); }
+                            __syncwarp();
+                        }
+                        if (lane == 0) st_word(progress + g, k + D);
+                        if (bad) { q.begin(RS_BAD_ONLY, stype, radius, ppx, ppy); continue; }
+                    }
+                    break;
                 }
             }
-            if (pass < 2 && refine && level > 0) {
-                bad_count = s.bad_count;
-                stage = RS_BAD_ONLY;
-                pass = 2;
-                continue;
+            // ---- what to evaluate: exact_sad of the new special candidates (an equal vector's that is
+            // known, else one for all that are equal), or the step's candidates inside the bounds whose
+            // motion penalty does not reach the best cost (see eval_step)
+            bool eval;
+            int vx, vy, from = lane;
+            long long motion = 0;
+            if (special) {
+                const unsigned peers = __match_any_sync(kFull, ((unsigned long long)(unsigned)mx << 32) | (unsigned)my);
+                const unsigned known = peers & __ballot_sync(kFull, act && !fresh), asked = peers & __ballot_sync(kFull, fresh);
+                if (fresh) from = __ffs(known ? known : asked) - 1;
+                eval = fresh && !known && from == lane;
+                vx = mx; vy = my;
+                if (started) n_eval += __popc(__ballot_sync(kFull, eval));
+            } else {
+                const int2 m = gen_mv(g_, imin(base + lane, g_.n - 1));
+                vx = m.x; vy = m.y;
+                motion = motion_penalty(lambda, q.predx, q.predy, vx, vy);
+                eval = base + lane < g_.n && vx >= b.bnd0 && vy >= b.bnd1 && vx < b.bnd2 && vy < b.bnd3 && motion < q.bcost;
             }
-            break;
+            unsigned long long news = 0;
+            const bool look = open && started;
+            if (look) news = ld_tag(ds.keys + ncell);  // in flight during the evaluation
+            unsigned l, c;
+            eval_cands(x, b, eval, vx, vy, l, c);
+            if (special) {
+                if (eval) sd = sat_add(l, c);
+                sd = __shfl_sync(kFull, sd, from);
+                fresh = false;
+                const long long cost = (long long)sd + (((long long)pp * sd) >> 8);
+                const int wl = first_min(act, cost, place);
+                const int nx = __shfl_sync(kFull, mx, wl), ny = __shfl_sync(kFull, my, wl);
+                const unsigned nsad = __shfl_sync(kFull, sd, wl);
+                if (!started) {
+                    if (search) {
+                        const long long cf = __shfl_sync(kFull, cost, kField), cp = __shfl_sync(kFull, cost, kPrev);
+                        const bool prev = __shfl_sync(kFull, act, kPrev);
+                        const int pmx = __shfl_sync(kFull, mx, kPrev), pmy = __shfl_sync(kFull, my, kPrev);
+                        if (prev && (!field_valid || cp < cf)) { ppx = pmx; ppy = pmy; }
+                        lambda = adapt_lambda(L.lambda_base, L.lsad, pred_score);
+                        radius = L.base_radius;
+                        if (level > 0 && P.coarse_distance < 0)
+                            radius = adaptive_radius(radius, block_activity(x.P, x.L, x.S.y, b.px2, b.py2, px, py));
+                        stype = (edge && level == 1) ? 0 : L.search_type;
+                    }
+                    if (!search) open = false;  // no seed takes part
+                    n_def += __any_sync(kFull, open);
+                }
+                if (!started || nx != selx || ny != sely) {  // the refinement, from this vector
+                    reran = started;
+                    selx = nx; sely = ny;
+                    q.bmx = nx; q.bmy = ny; q.bsad = nsad; q.bcost = (long long)nsad;
+                    q.begin(search ? RS_REFINE_ONLY : RS_NONE, stype, radius, ppx, ppy);
+                    stepping = false;
+                    published = false;
+                }
+                started = true;
+            } else {
+                const long long K = motion + pen(x.pnew, l) + (b.chroma ? pen(x.pnew, c) : 0LL);  // :1158-1221
+                const unsigned sad = sat_add(l, c);
+                if (x.pnew < -256) {  // exact sequential semantics for penalties that can be negative
+                    for (unsigned m = __ballot_sync(kFull, eval); m; m &= m - 1) {
+                        const int j = __ffs(m) - 1;
+                        const long long mj = __shfl_sync(kFull, motion, j), kj = __shfl_sync(kFull, K, j);
+                        const unsigned sj = __shfl_sync(kFull, sad, j);
+                        if (mj < q.bcost && kj < q.bcost) { q.bcost = kj; q.bsad = sj; win = base + j; }
+                    }
+                } else {
+                    const int j = first_min(eval && K < q.bcost, K, lane);
+                    if (j >= 0) {
+                        q.bcost = __shfl_sync(kFull, K, j);
+                        q.bsad = __shfl_sync(kFull, sad, j);
+                        win = base + j;
+                    }
+                }
+                base += 32;
+                if (base >= g_.n) { q.took(g_, win); stepping = false; }
+            }
+            if (look && (int)(news >> 32) == TAG_FINAL) {  // a seed has become final
+                const int2 m = vmv(make_uint2((unsigned)news, 0));
+                fresh = !act || m.x != mx || m.y != my;
+                mx = m.x; my = m.y;
+                act = true;
+                open = false;
+            }
         }
-        if (pass == 2 && lane == 0) s.bad_count = bad_count;
-        // ---- store (:673-679) and hand the order on to the next block's warp
-        const int rows = b.py >= 0 ? imax(0, imin(b.bh, L.lh - b.py)) : 0;
-        const int cols = b.px >= 0 ? imax(0, imin(b.bw, L.lw - b.px)) : 0;
-        const unsigned cnt = (unsigned)(rows * cols);
-        unsigned dc = (cnt ? dcsum / cnt : 0) >> DC_SHIFT;
-        if (dc > 255) dc = 255;
+        n_blk++;
+        n_rerun += reran;
+        const int bmx = q.bmx, bmy = q.bmy;
+        const unsigned bsad = q.bsad;
+        // ---- store (:673-679)
         if (lane == 0) {
-            field[idx] = mkvec(bmx, bmy, smallest ? sat_mul(bsad, 3) : bsad);
-            lumaf[idx] = (uint8_t)dc;
-            // the block's stores (and bad_count) before the count that publishes them
-            if (XSM) __threadfence();
-            else __threadfence_block();
-            *committed = (int)(k + 1);
+            const uint2 v = mkvec(bmx, bmy, smallest ? sat_mul(bsad, 3) : bsad);
+            st_tag(ds.keys + idx, tag_word(TAG_FINAL, bmx, bmy));
+            field[idx] = v;
+            lumaf[idx] = block_mean(b, L, dcsum);
         }
         __syncwarp();
     }
     if (lane == 0) {
-        if (late) { atomicOr(status, ST_TIMEOUT); *abort_flag = 1; }
+        if (late) { atomicOr(status, ST_TIMEOUT); ctl[CTL_ABORT] = 1; }
         if (stats && level == 0) {
-            atomicAdd(stats + 0, n_blk);
-            atomicAdd(stats + 1, n_def);
-            atomicAdd(stats + 2, n_eval);
-            atomicAdd(stats + 3, n_rerun);
+            atomicAdd(stats + 0, (unsigned long long)n_blk);
+            atomicAdd(stats + 1, (unsigned long long)n_def);
+            atomicAdd(stats + 2, (unsigned long long)n_eval);
+            atomicAdd(stats + 3, (unsigned long long)n_rerun);
         }
     }
 }
-// The direction's warps of one CTA walk the level together (the count in shared memory).
-__device__ __forceinline__ void search_level_spec(const Ctx &xd, DirSh &s, DirScratch &ds, const uint2 *prevp, int *status,
-                                                  unsigned long long *stats) {
-    if (xd.tid == 0) { s.committed = 0; s.late_ = 0; s.bad_count = 0; }
+// What a walk starts from: no cell published, no block tested. Every thread of the direction.
+__device__ __forceinline__ void start_walk(const Ctx &x, const DirScratch &ds, int *ctl, int ncell) {
+    for (int i = x.tid; i < ncell; i += NT) ds.keys[i] = 0;
+    for (int h = x.tid; h < kMaxWalkers; h += NT) ((int *)ds.hist)[h] = h;
+    if (x.tid == 0) { ctl[CTL_LATE] = 0; ctl[CTL_BAD] = 0; }
+}
+// The direction's warps of one CTA walk the level together.
+__device__ __forceinline__ void walk_in_cta(const Ctx &xd, DirSh &s, const DirScratch &ds, const uint2 *prevp, int *ctl,
+                                            int *status, unsigned long long *stats, unsigned char *area, int groups) {
+    start_walk(xd, ds, ctl, xd.L->gw * xd.L->gh);
+    __threadfence();
     dbar(xd.d);
     const int g = xd.tid >> 5;
     Ctx x = xd;
     x.nw = 1;
     x.wbase = g;
     x.tid = xd.tid & 31;
-    spec_walk<false>(x, s, ds, prevp, g, s.order_len, s.gx, s.gy, &s.committed, &s.late_, &s.abort_, status, stats);
+    set_stage(x, area, groups, g, g);
+    walk_level(x, s, ds, prevp, g, NW, s.order_len, s.gx, s.gy, ctl, status, stats);
+    __threadfence();
+    dbar(xd.d);
+    if (xd.tid == 0 && ctl[CTL_ABORT]) s.abort_ = 1;
     dbar(xd.d);
 }
 
-// Whether search_level_spec may run this level: it takes neither the reference's panics
-// (search_level reports them at the block where the reference stops) nor grids below 3 x 3.
+// Whether walk_level may run this level: it takes neither the reference's panics (search_level
+// reports them at the block where the reference stops) nor grids below 3 x 3, nor an order that
+// visits a cell twice, leaves one out or puts an edge block before its inner cell.
 // Called by every thread of the direction; the answer is the same in all of them.
-__device__ __forceinline__ bool level_spec_ok(const Ctx &x, DirSh &s, DirScratch &ds) {
+__device__ __forceinline__ bool level_spec_ok(const Ctx &x, DirSh &s, const DirScratch &ds) {
     const LevelInfo &L = *x.L;
     const int level = x.level, gw = L.gw, gh = L.gh;
     const int64_t ncell = (int64_t)gw * gh, order_len = s.order_len;
-    if (gw < 3 || gh < 3) return false;
+    if (gw < 3 || gh < 3 || order_len != ncell || (level > 0 && L.smallest)) return false;
     if (x.tid == 0) s.unsafe_ = 0;
     dbar(x.d);
     int bad = 0;
+    auto pos_of = [&](int cx, int cy) { return level == 0 ? initial_order_pos(gw, gh, cx, cy) : (int64_t)ds.pos[(int64_t)cy * gw + cx]; };
     for (int64_t k = x.tid; k < order_len && !bad; k += NT) {
         const int2 bxy = level == 0 ? initial_order_at(gw, gh, k) : unpack_xy(ds.order[k]);
         const int bx = bxy.x, by = bxy.y;
-        const int64_t idx = (int64_t)by * gw + bx;
-        const int64_t sidx = (int64_t)imin(by, gh - 2) * gw + imin(bx, gw - 2);
-        if (sidx < 0 || sidx >= ncell || idx < 0 || idx >= ncell || bx < 0 || by < 0 || bx >= gw || by >= gh) {
+        if (bx < 0 || by < 0 || bx >= gw || by >= gh || pos_of(bx, by) != k) {
             bad = 1;
             break;
         }
+        if (level > 0 && (bx == gw - 1 || by == gh - 1) && pos_of(imin(bx, gw - 2), imin(by, gh - 2)) >= k) bad = 1;
         int nproc = 0;
         for (int q = 0; q < 9; q++) {
             const int ny = by - 1 + q / 3, nx = bx - 1 + q % 3;
             if (ny < 0 || ny >= gh || nx < 0 || nx >= gw) continue;
-            const int64_t p = level == 0 ? initial_order_pos(gw, gh, nx, ny) : (int64_t)ds.pos[(int64_t)ny * gw + nx];
-            nproc += p < k;
+            nproc += pos_of(nx, ny) < k;
         }
         if (nproc > 8) bad = 1;
     }
@@ -1851,106 +1989,78 @@ __device__ __forceinline__ long long floor_div(long long a, long long b) {  // i
 // exact_recalculate (:1326-1451): when refine[0].thsad is set, the level-0 field is
 // interpolated onto the half-size output blocks and each block whose interpolated score is
 // above the threshold is searched again. Blocks do not read each other's results, so the
-// visiting order does not matter; the direction's threads take them one after another with
-// the same evaluation machinery as the hierarchy. Output: ds.vec[1] / ds.luma[1].
-__device__ __forceinline__ void refine_pass(Ctx &x, DirSh &s, DirScratch &ds) {
+// visiting order does not matter: one warp takes one block, with the same evaluation machinery as
+// the hierarchy. x: a one-warp group; `border`: the block shape x is set to, -1 before the first
+// block. Output: ds.vec[1] / ds.luma[1].
+template <class SH>
+__device__ __forceinline__ void refine_block(Ctx &x, SH &s, DirScratch &ds, int bx, int by, int &shape) {
     const AnalyseParams &P = *x.P;
     const uint2 *field = ds.vec[0];
-    uint2 *out = ds.vec[1];
-    uint8_t *outl = ds.luma[1];
     const int ogw = P.lv[0].gw, ogh = P.lv[0].gh;
     const int obw = P.block_w, obh = P.block_h, osx = P.step_x, osy = P.step_y;
     const int bw = P.out_bw, bh = P.out_bh;
     const int sx = imax(bw - P.out_ox, 1), sy = imax(bh - P.out_oy, 1);
     const int gw = P.out_gw, gh = P.out_gh;
-    const int lw = P.lv[0].lw, lh = P.lv[0].lh;
-    x.level = 0;
-    x.pel = P.lv[0].pel;
-    x.satd = P.refine_satd;
     int ph = 0;
-    for (int by = 0; by < gh; by++) {
-        for (int bx = 0; bx < gw; bx++) {
-            const int cx = bw / 2 + sx * bx, cy = bh / 2 + sy * by;
-            const int ox_ = (cx - obw / 2) / osx, oy_ = (cy - obh / 2) / osy;
-            const long long dx_ = imax(cx - (obw / 2 + osx * ox_), 0), dy_ = imax(cy - (obh / 2 + osy * oy_), 0);
-            const uint2 p00 = field[(int64_t)iclamp(oy_, 0, ogh - 1) * ogw + iclamp(ox_, 0, ogw - 1)];
-            const uint2 p10 = field[(int64_t)iclamp(oy_, 0, ogh - 1) * ogw + iclamp(ox_ + 1, 0, ogw - 1)];
-            const uint2 p01 = field[(int64_t)iclamp(oy_ + 1, 0, ogh - 1) * ogw + iclamp(ox_, 0, ogw - 1)];
-            const uint2 p11 = field[(int64_t)iclamp(oy_ + 1, 0, ogh - 1) * ogw + iclamp(ox_ + 1, 0, ogw - 1)];
-            auto interp = [&](long long a, long long b_, long long c, long long d) {
-                const long long top = a * osx + dx_ * (b_ - a);
-                const long long bottom = c * osx + dx_ * (d - c);
-                return floor_div(top + floor_div(dy_ * (bottom - top), osy), osx);
-            };
-            const int2 m00 = vmv(p00), m10 = vmv(p10), m01 = vmv(p01), m11 = vmv(p11);
-            const int mvx = (int)interp(m00.x, m10.x, m01.x, m11.x);
-            const int mvy = (int)interp(m00.y, m10.y, m01.y, m11.y);
-            const long long parent = interp(p00.y, p10.y, p01.y, p11.y) * (long long)(bw * bh) / (long long)(obw * obh);
-            const int px = bx * sx, py = by * sy;
-            const bool border = bx == 0 || by == 0 || bx == gw - 1 || by == gh - 1;
-            const int factor = (border && bw > 4) ? 3 : 1;
-            const int epx = px + (factor == 3 ? bw / 4 : 0), epy = py + (factor == 3 ? bh / 4 : 0);
-            x.L = &P.rlv[factor == 3 ? 1 : 0];
-            const LevelInfo &L = *x.L;
-            x.tl = L.tl;
-            x.tcp = L.tc;
-            {
-                const int T = L.tl + 2 * L.tc;
-                const int tpl = iclamp(P.tiles_per_lane, 1, 8);
-                const int want = (T + tpl - 1) / tpl;
-                int g = 1;
-                while (g < want && g < 32) g <<= 1;
-                x.grp_lanes = g;
-            }
-            x.pnew = P.pnew / factor;
-            BlkC b;
-            make_blk(x, epx, epy, true, b);
-            // exact_clip (:1269-1273) of the interpolated vector into mv_bounds
-            const int pmx = iclamp(mvx, b.bnd0, imax(b.bnd2 - 1, b.bnd0)), pmy = iclamp(mvy, b.bnd1, imax(b.bnd3 - 1, b.bnd1));
-            const int threshold = P.refine_thsad / factor;
-            const bool search = parent > (long long)threshold;
-            stage_source(x, s, b);
-            {  // slot 0: exact_sad at the clipped predictor (when searching); slot 1: block_luma_dc
-                const int Gl = step_lanes(x.grp_lanes, 2, x.nw), lane = x.tid & 31, grp = (x.tid >> 5) * (32 / Gl) + lane / Gl;
-                const int sub = lane & (Gl - 1);
-                const bool act = (grp == 0 && search) || grp == 1;
-                Res r{0, 0, 0, 0, 0, 0};
-                if (act) r = eval_lane(x, b, grp == 1 ? 2 : 0, 0, 0, pmx, pmy, grp == 0, sub, Gl);
-                group_sum3(r, Gl);
-                if (act && sub == 0) {
-                    unsigned Lv, Cv;
-                    if (grp == 1) { Lv = r.L; Cv = 0; }
-                    else finalize(r, Lv, Cv);
-                    s.slotL[x.wbase][ph][grp] = grp == 0 ? sat_add(Lv, Cv) : Lv;
-                }
-            }
-            dbar(x.d);
-            const int phs = ph;
-            ph ^= 1;
-            int bmx = pmx, bmy = pmy;
-            unsigned bsad = parent < 0 ? 0u : (parent > 0xFFFFFFFFLL ? 0xFFFFFFFFu : (unsigned)parent);
-            long long bcost = parent < 0 ? 0 : parent;
-            if (search) {
-                bsad = s.slotL[x.wbase][phs][0];
-                bcost = (long long)bsad;
-                const int lambda = by == 0 ? 0 : (P.lambda >> 2) / factor;
-                int bad = 0;
-                run_search_steps(x, b, s, ph, RS_ALL, P.refine_search_type, abs(P.refine_distance), lambda, pmx, pmy, pmx,
-                                 pmy, 0, bad, bmx, bmy, bsad, bcost);
-            }
-            const unsigned dcsum = s.slotL[x.wbase][phs][1];
-            const int rows = b.py >= 0 ? imax(0, imin(b.bh, lh - b.py)) : 0;
-            const int cols = b.px >= 0 ? imax(0, imin(b.bw, lw - b.px)) : 0;
-            const unsigned cnt = (unsigned)(rows * cols);
-            unsigned dc = (cnt ? dcsum / cnt : 0) >> DC_SHIFT;
-            if (dc > 255) dc = 255;
-            if (x.tid == 0) {
-                out[(int64_t)by * gw + bx] = mkvec(bmx, bmy, sat_mul(bsad, (unsigned)factor));
-                outl[(int64_t)by * gw + bx] = (uint8_t)dc;
-            }
-        }
+    const int cx = bw / 2 + sx * bx, cy = bh / 2 + sy * by;
+    const int ox_ = (cx - obw / 2) / osx, oy_ = (cy - obh / 2) / osy;
+    const long long dx_ = imax(cx - (obw / 2 + osx * ox_), 0), dy_ = imax(cy - (obh / 2 + osy * oy_), 0);
+    const uint2 p00 = field[(int64_t)iclamp(oy_, 0, ogh - 1) * ogw + iclamp(ox_, 0, ogw - 1)];
+    const uint2 p10 = field[(int64_t)iclamp(oy_, 0, ogh - 1) * ogw + iclamp(ox_ + 1, 0, ogw - 1)];
+    const uint2 p01 = field[(int64_t)iclamp(oy_ + 1, 0, ogh - 1) * ogw + iclamp(ox_, 0, ogw - 1)];
+    const uint2 p11 = field[(int64_t)iclamp(oy_ + 1, 0, ogh - 1) * ogw + iclamp(ox_ + 1, 0, ogw - 1)];
+    auto interp = [&](long long a, long long b_, long long c, long long d) {
+        const long long top = a * osx + dx_ * (b_ - a);
+        const long long bottom = c * osx + dx_ * (d - c);
+        return floor_div(top + floor_div(dy_ * (bottom - top), osy), osx);
+    };
+    const int2 m00 = vmv(p00), m10 = vmv(p10), m01 = vmv(p01), m11 = vmv(p11);
+    const int mvx = (int)interp(m00.x, m10.x, m01.x, m11.x);
+    const int mvy = (int)interp(m00.y, m10.y, m01.y, m11.y);
+    const long long parent = interp(p00.y, p10.y, p01.y, p11.y) * (long long)(bw * bh) / (long long)(obw * obh);
+    const int px = bx * sx, py = by * sy;
+    const bool border = bx == 0 || by == 0 || bx == gw - 1 || by == gh - 1;
+    const int factor = (border && bw > 4) ? 3 : 1;
+    const int epx = px + (factor == 3 ? bw / 4 : 0), epy = py + (factor == 3 ? bh / 4 : 0);
+    x.L = &P.rlv[factor == 3 ? 1 : 0];
+    const LevelInfo &L = *x.L;
+    if (shape != factor) {
+        shape = factor;
+        __syncwarp();
+        set_groups(x);
     }
-    dbar(x.d);
+    x.pnew = P.pnew / factor;
+    BlkC b;
+    make_blk(x, epx, epy, true, b);
+    // exact_clip (:1269-1273) of the interpolated vector into mv_bounds
+    const int pmx = iclamp(mvx, b.bnd0, imax(b.bnd2 - 1, b.bnd0)), pmy = iclamp(mvy, b.bnd1, imax(b.bnd3 - 1, b.bnd1));
+    const int threshold = P.refine_thsad / factor;
+    const bool search = parent > (long long)threshold;
+    unsigned dcsum = 0;
+    if (b.fast_src) dcsum = stage_source(x, b);
+    __syncwarp();
+    if (!b.fast_src) {
+        dcsum = eval_slow(x, b.px, b.py, 0, 0, SLOW_DC).x;
+    }
+    Search q;
+    q.bmx = pmx; q.bmy = pmy;
+    q.bsad = parent < 0 ? 0u : (parent > 0xFFFFFFFFLL ? 0xFFFFFFFFu : (unsigned)parent);
+    q.bcost = parent < 0 ? 0 : parent;
+    if (search) {
+        unsigned l, c;
+        eval_cands(x, b, (x.tid & 31) == 0, pmx, pmy, l, c);
+        q.bsad = __shfl_sync(kFull, sat_add(l, c), 0);  // exact_sad at the clipped predictor
+        q.bcost = (long long)q.bsad;
+    }
+    const int lambda = by == 0 ? 0 : (P.lambda >> 2) / factor;
+    int bad = 0;
+    q.begin(search ? RS_ALL : RS_NONE, P.refine_search_type, abs(P.refine_distance), pmx, pmy);
+    run_search(x, b, s, ph, q, lambda, pmx, pmy, 0, bad);
+    if ((x.tid & 31) == 0) {
+        ds.vec[1][(int64_t)by * gw + bx] = mkvec(q.bmx, q.bmy, sat_mul(q.bsad, (unsigned)factor));
+        ds.luma[1][(int64_t)by * gw + bx] = block_mean(b, L, dcsum);
+    }
+    __syncwarp();  // the next block stages over this one's source
 }
 
 // exact_global_doubled (:1285-1324) over the dir's threads
@@ -2068,13 +2178,6 @@ __device__ void reorder(const Ctx &x, DirSh &s, const uint2 *field, int gw, int 
     dbar(x.d);
 }
 
-// The hand-over words of one direction (AnalyseParams::off_ctl) when level 0 runs in the
-// level-0 kernel: the pair kernel leaves the level with GO set (and the count, the global
-// predictor and whether the other direction's projection exists); the level-0 kernel's warps
-// count their commits in COMMITTED and flag a wait that gave up in LATE; ABORT, set by either,
-// tells the finish kernel to leave the pair's payload unwritten (the status word says why).
-enum { CTL_GO, CTL_COMMITTED, CTL_LATE, CTL_GX, CTL_GY, CTL_ABORT, CTL_PREV };
-
 __device__ __forceinline__ DirScratch dir_scratch(const AnalyseParams &P, uint8_t *scr, int d) {
     DirScratch ds;
     ds.vec[0] = (uint2 *)(scr + P.off_field[d]);
@@ -2092,30 +2195,16 @@ __device__ __forceinline__ DirScratch dir_scratch(const AnalyseParams &P, uint8_
     return ds;
 }
 
-// The per-level fields of the search context. tpl_scale multiplies the 4x4 tiles a lane takes
-// per candidate: the level-0 kernel's warps each search a block alone, where fewer, longer lane
-// groups measured faster (two lanes per 16x16 SATD + chroma candidate: 209.4 -> 213.1 pairs/s;
-// eight lanes: 186.4).
-__device__ __forceinline__ void set_level(Ctx &x, const AnalyseParams &P, int level, int tpl_scale = 1) {
+// The per-level fields of the search context, and the warp's group tables.
+__device__ __forceinline__ void set_level(Ctx &x, const AnalyseParams &P, int level) {
     const LevelInfo &L = P.lv[level];
     x.L = &L;
     x.level = level;
     x.satd = L.satd;
     x.pel = L.pel;
-    x.G.lw = L.lw; x.G.lh = L.lh; x.G.clw = L.lw / 2; x.G.clh = L.lh / 2;
-    x.G.ys = P.y_stride; x.G.cs = P.c_stride; x.G.ylen = P.y_len; x.G.clen = P.c_len;
-    x.G.ys32 = (int)P.y_stride; x.G.cs32 = (int)P.c_stride;
+    set_geo(x.G, P, L);
     x.pnew = P.pnew;
-    x.tl = L.tl;
-    x.tcp = L.tc;
-    {  // lanes per candidate: about `tiles_per_lane` 4x4 tiles per lane
-        const int T = L.tl + (L.smallest ? 0 : 2 * L.tc);
-        const int tpl = iclamp(P.tiles_per_lane, 1, 8) * tpl_scale;
-        const int want = (T + tpl - 1) / tpl;
-        int g = 1;
-        while (g < want && g < 32) g <<= 1;
-        x.grp_lanes = g;
-    }
+    set_groups(x);
 }
 
 // Pair b of a launch (analyse_filter.rs:277-282: frame n pairs with min(n + delta, num_frames - 1)).
@@ -2133,12 +2222,14 @@ __device__ __forceinline__ PairRef pair_at(const PairSrc &psrc, int64_t pair) {
 // One frame pair, both directions: the whole of analyse_pair (:68-226) plus the payload
 // (:2740-2811). Called by every thread of the CTA; threads of a direction the
 // configuration does not search (vectors 1 or 2 under a 2-direction batch CTA) only
-// take part in the CTA-wide barriers. Status bits go to *status. split: a direction whose
-// level 0 takes the look-ahead leaves it to the level-0 kernel (see CTL_GO) and the finish
-// kernel packs the payload.
+// take part in the CTA-wide barriers. Status bits go to *status.
+// Levels hi .. lo: the whole hierarchy in one call (split false), or the part between two walks:
+// what follows the search of level hi + 1 (global predictor, order) unless hi is the first level, the
+// levels above lo whole, and level lo up to its search, which the walk kernel does (see CTL_GO);
+// a level that the walk may not take is searched here.
 __device__ __forceinline__ void analyse_pair_dev(const AnalyseParams &P, const PairRef pr, uint8_t *__restrict__ pay,
                                                  uint8_t *__restrict__ scr, int *status, int &cta_abort,
-                                                 unsigned long long *spec_stats, bool split) {
+                                                 unsigned long long *spec_stats, bool split, int hi, int lo, int groups) {
     extern __shared__ __align__(16) unsigned char smem[];
     const bool bidir = P.vectors == 3;
     const int half = (int)(threadIdx.x / NT);
@@ -2156,11 +2247,19 @@ __device__ __forceinline__ void analyse_pair_dev(const AnalyseParams &P, const P
     x.tid = tid;
     x.nw = NW;
     x.wbase = 0;
-    x.S = Planes{src, src + P.y_len, src + P.y_len + P.c_len};
-    x.R = Planes{ref, ref + P.y_len, ref + P.y_len + P.c_len};
+    unsigned char *area = smem + sizeof(DirSh) * (blockDim.x / NT) + (size_t)half * NW * groups * kGroupBytes;
+    set_stage(x, area, groups, 0, tid >> 5);
+    set_frames(x, P, src, ref);
     if (threadIdx.x == 0) cta_abort = 0;
-    if (tid == 0) { s.abort_ = idle ? 2 : 0; s.gx = 0; s.gy = 0; s.order_len = 0; }
-    if (split && tid == 0 && !idle) { ctl[CTL_GO] = 0; ctl[CTL_ABORT] = 0; }
+    const bool resume = hi < P.nlevels - 1;
+    if (tid == 0) {
+        s.abort_ = 0; s.gx = 0; s.gy = 0; s.order_len = 0;
+        if (idle) s.abort_ = 2;
+        else if (resume) {
+            s.abort_ = ctl[CTL_ABORT]; s.gx = ctl[CTL_GX]; s.gy = ctl[CTL_GY]; s.order_len = ctl[CTL_ORDER];
+            ctl[CTL_GO] = 0;
+        } else { ctl[CTL_GO] = 0; ctl[CTL_ABORT] = 0; }
+    }
     __syncthreads();
     const uint2 *other_proj[2] = {nullptr, nullptr};
     {
@@ -2169,10 +2268,19 @@ __device__ __forceinline__ void analyse_pair_dev(const AnalyseParams &P, const P
         other_proj[1] = (const uint2 *)(scr + P.off_proj[od][1]);
     }
     int pgw = 0, pgh = 0;  // grid of the previous (coarser) level
-    for (int level = P.nlevels - 1; level >= 0; level--) {
+    auto after_search = [&](int level) {
         const LevelInfo &L = P.lv[level];
-        // the coarser levels of a split launch: twice the tiles per lane (217.0 against 215.2 pairs/s)
-        set_level(x, P, level, split && level > 0 ? 2 : 1);
+        const uint2 *f = ds.vec[level & 1];
+        global_doubled(x, s, f, (int64_t)L.gw * L.gh, ds.hist);
+        reorder(x, s, f, L.gw, L.gh, ds, status);
+    };
+    if (resume) {
+        pgw = P.lv[hi + 1].gw; pgh = P.lv[hi + 1].gh;
+        if (!s.abort_) after_search(hi + 1);
+    }
+    for (int level = hi; level >= lo; level--) {
+        const LevelInfo &L = P.lv[level];
+        set_level(x, P, level);
         const int gw = L.gw, gh = L.gh;
         const int64_t ncell = (int64_t)gw * gh;
         const bool first = level == P.nlevels - 1;
@@ -2290,72 +2398,46 @@ __device__ __forceinline__ void analyse_pair_dev(const AnalyseParams &P, const P
         __syncthreads();  // both directions' projections of this level are ready
         if (!s.abort_) {
             const uint2 *prevp = (first) ? nullptr : other_proj[level & 1];
-            if (SVPF_LOOKAHEAD && NW > 1 && (P.lookahead & (level == 0 ? 1 : 2)) && level_spec_ok(x, s, ds)) {
-                if (split && level == 0) {  // the level-0 kernel walks it
-                    if (tid == 0) {
-                        ctl[CTL_COMMITTED] = 0; ctl[CTL_LATE] = 0; ctl[CTL_GX] = s.gx; ctl[CTL_GY] = s.gy;
-                        ctl[CTL_PREV] = prevp != nullptr; ctl[CTL_GO] = 1;
-                    }
+            const bool leave = split && level == lo;
+            const bool walk = SVPF_LOOKAHEAD && NW > 1 && (leave || (!split && (P.lookahead & (level == 0 ? 1 : 2))));
+            if (walk && level_spec_ok(x, s, ds)) {
+                if (leave) {  // the walk kernel's
+                    start_walk(x, ds, ctl, (int)ncell);
+                    if (tid == 0) { ctl[CTL_PREV] = prevp != nullptr; ctl[CTL_GO] = 1; }
                 } else {
-                    search_level_spec(x, s, ds, prevp, status, spec_stats);
+                    walk_in_cta(x, s, ds, prevp, ctl, status, spec_stats, area, groups);
                 }
             } else {
                 search_level(x, s, ds, prevp, status);
             }
         }
         dbar(half);
-        if (!s.abort_ && level > 0) {
-            const uint2 *f = ds.vec[level & 1];
-            global_doubled(x, s, f, ncell, ds.hist);
-            reorder(x, s, f, gw, gh, ds, status);
-        }
+        if (!s.abort_ && level > 0 && !(split && level == lo)) after_search(level);
         pgw = gw; pgh = gh;
         if (tid == 0 && s.abort_ == 1) cta_abort = 1;
         __syncthreads();
     }
-    if (split && tid == 0 && !idle && s.abort_ == 1) ctl[CTL_ABORT] = 1;
+    if (split && tid == 0 && !idle) {
+        ctl[CTL_GX] = s.gx; ctl[CTL_GY] = s.gy; ctl[CTL_ORDER] = s.order_len;
+        if (s.abort_ == 1) ctl[CTL_ABORT] = 1;
+    }
 }
 
-// After the hierarchy: the refine pass when configured, then rescale_scores (:2716-2738)
-// and pack_vector_frame (:2740-2811). Out of line, called where little else is live, so
-// neither adds to the hierarchy's register pressure. Every thread of the CTA calls it.
-__device__ __noinline__ void finish_pair(const AnalyseParams *Pp, const PairRef pr, uint8_t *pay, uint8_t *scr) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    const AnalyseParams &P = *Pp;
+// rescale_scores (:2716-2738) + pack_vector_frame (:2740-2811) of one direction's cells first, first +
+// step, ...; the thread with `head` also writes the payload's header and the direction's.
+__device__ __forceinline__ void pack_cells(const AnalyseParams &P, const DirScratch &ds, int d, uint8_t *pay, int64_t first,
+                                           int64_t step, bool head) {
     const bool bidir = P.vectors == 3;
-    const int half = (int)(threadIdx.x / NT);
-    if (!bidir && half == 1) return;
-    const int d = bidir ? half : ((P.vectors & 2) ? 0 : 1);
-    const int tid = threadIdx.x % NT;
-    DirSh &s = reinterpret_cast<DirSh *>(smem)[half];
-    DirScratch ds = dir_scratch(P, scr, d);
-    if (P.has_refine) {
-        const px_t *src = (const px_t *)(d == 0 ? pr.cur : pr.ref);
-        const px_t *ref = (const px_t *)(d == 0 ? pr.ref : pr.cur);
-        Ctx x;
-        x.P = &P;
-        x.d = half;
-        x.tid = tid;
-        x.nw = NW;
-        x.wbase = 0;
-        x.S = Planes{src, src + P.y_len, src + P.y_len + P.c_len};
-        x.R = Planes{ref, ref + P.y_len, ref + P.y_len + P.c_len};
-        const LevelInfo &L0 = P.lv[0];
-        x.G.lw = L0.lw; x.G.lh = L0.lh; x.G.clw = L0.lw / 2; x.G.clh = L0.lh / 2;
-        x.G.ys = P.y_stride; x.G.cs = P.c_stride; x.G.ylen = P.y_len; x.G.clen = P.c_len;
-        x.G.ys32 = (int)P.y_stride; x.G.cs32 = (int)P.c_stride;
-        refine_pass(x, s, ds);
-    }
-    // ---- rescale_scores (:2716-2738) + pack_vector_frame (:2740-2811)
     const uint2 *f = ds.vec[P.has_refine ? 1 : 0];
     const uint8_t *fl = ds.luma[P.has_refine ? 1 : 0];
     const int64_t count = (int64_t)P.out_gw * P.out_gh;
     const int64_t region = bidir ? (d == 1 ? 0x40 : 0x40 + 4 + count * 8) : 0x40;
-    if (threadIdx.x == 0) {
-        for (int i = 0; i < 16; i++) reinterpret_cast<int *>(pay)[i] = P.header[i];
+    if (head) {
+        if (!bidir || d == 0)
+            for (int i = 0; i < 16; i++) reinterpret_cast<int *>(pay)[i] = P.header[i];
+        *reinterpret_cast<int *>(pay + region) = (int)(2 * count + 1);
     }
-    if (tid == 0) *reinterpret_cast<int *>(pay + region) = (int)(2 * count + 1);
-    for (int64_t i = tid; i < count; i += NT) {
+    for (int64_t i = first; i < count; i += step) {
         const uint2 v = f[i];
         const int2 m = vmv(v);
         const int mag = abs(m.x) + abs(m.y);
@@ -2376,73 +2458,135 @@ __device__ __noinline__ void finish_pair(const AnalyseParams *Pp, const PairRef 
     }
 }
 
-// One CTA per frame pair. split: level 0 (where it takes the look-ahead) and the payload are
-// left to analyse_level0_kernel and analyse_finish_kernel.
+// A one-warp context at the refine pass's level.
+__device__ __forceinline__ void refine_ctx(Ctx &x, const AnalyseParams &P, const PairRef pr, int d) {
+    const px_t *src = (const px_t *)(d == 0 ? pr.cur : pr.ref);
+    const px_t *ref = (const px_t *)(d == 0 ? pr.ref : pr.cur);
+    x.P = &P;
+    x.tid = (int)(threadIdx.x & 31);
+    x.nw = 1;
+    set_frames(x, P, src, ref);
+    x.level = 0;
+    x.pel = P.lv[0].pel;
+    x.satd = P.refine_satd;
+    set_geo(x.G, P, P.lv[0]);
+}
+
+// After the hierarchy in one CTA: the refine pass when configured, then the payload. Out of line,
+// called where little else is live, so neither adds to the hierarchy's register pressure. Every
+// thread of the CTA calls it.
+__device__ __noinline__ void finish_pair(const AnalyseParams *Pp, const PairRef pr, uint8_t *pay, uint8_t *scr, int groups) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const AnalyseParams &P = *Pp;
+    const bool bidir = P.vectors == 3;
+    const int half = (int)(threadIdx.x / NT);
+    if (!bidir && half == 1) return;
+    const int d = bidir ? half : ((P.vectors & 2) ? 0 : 1);
+    const int tid = threadIdx.x % NT;
+    DirSh &s = reinterpret_cast<DirSh *>(smem)[half];
+    DirScratch ds = dir_scratch(P, scr, d);
+    if (P.has_refine) {
+        Ctx x;
+        refine_ctx(x, P, pr, d);
+        x.d = half;
+        x.wbase = tid >> 5;
+        set_stage(x, smem + sizeof(DirSh) * (blockDim.x / NT) + (size_t)half * NW * groups * kGroupBytes, groups, x.wbase,
+                  x.wbase);
+        int shape = -1;
+        const int n = P.out_gw * P.out_gh;
+        for (int i = x.wbase; i < n; i += NW) refine_block(x, s, ds, i % P.out_gw, i / P.out_gw, shape);
+        dbar(half);
+    }
+    pack_cells(P, ds, d, pay, tid, NT, tid == 0);
+}
+
+// One CTA per frame pair: the whole pair, or (split) the levels hi .. lo between two walks.
 __global__ void __launch_bounds__(2 * NT, SVPF_MINB)
     analyse_kernel(const __grid_constant__ AnalyseParams P, const PairSrc psrc, uint8_t *__restrict__ payloads,
-                   uint8_t *__restrict__ scratch, int *status, int split) {
+                   uint8_t *__restrict__ scratch, int *status, int split, int hi, int lo) {
     __shared__ int cta_abort;
     const int64_t pair = blockIdx.x;
     const PairRef pr = pair_at(psrc, pair);
     uint8_t *scr = scratch + pair * P.scratch_per_pair;
-    analyse_pair_dev(P, pr, payloads + pair * P.payload_len, scr, status, cta_abort, psrc.stats, split != 0);
+    analyse_pair_dev(P, pr, payloads + pair * P.payload_len, scr, status, cta_abort, psrc.stats, split != 0, hi, lo,
+                     P.stage_groups);
     __syncthreads();
-    if (!split && !cta_abort) finish_pair(&P, pr, payloads + pair * P.payload_len, scr);
+    if (!split && !cta_abort) finish_pair(&P, pr, payloads + pair * P.payload_len, scr, P.stage_groups);
 }
 
-// Level 0 spread over the GPU: one CTA per warp of a search direction, (pair, direction, g) for
-// the pairs first .. of the launch; warp g walks blocks g, g + NW, ... of the level exactly as
-// the pair kernel's look-ahead does, but its partners run on other SMs, so every SM holds about
-// the same number of walking warps whatever the pair count (one CTA per pair leaves some SMs
-// with two pairs and others with one). The warps of a direction wait on one another, so the
-// launch is cooperative: all its CTAs are resident at once, or it does not start.
-constexpr int kLevel0Warps = 1;    // warps per CTA (of one direction)
-constexpr int kLevel0TileScale = 2;  // see set_level
-constexpr int kLevel0PerSM = 16;   // warps per SM: 128 registers per thread
-__global__ void __launch_bounds__(32 * kLevel0Warps, kLevel0PerSM / kLevel0Warps)
-    analyse_level0_kernel(const __grid_constant__ AnalyseParams P, const PairSrc psrc, int64_t first,
-                          uint8_t *__restrict__ scratch, int *status) {
-    __shared__ WarpSh sh[kLevel0Warps];
-    constexpr int per_dir = NW / kLevel0Warps;  // CTAs per direction
+// One level spread over the GPU: a CTA per warp, D of them per search direction of the pairs first ..
+// of the launch. The warps of a direction wait on one another, so the launch is cooperative: all its
+// CTAs are resident at once, or it does not start.
+constexpr int kWalkPerSM = 16;  // CTAs per SM: 128 registers per thread
+__global__ void __launch_bounds__(32, kWalkPerSM)
+    analyse_walk_kernel(const __grid_constant__ AnalyseParams P, const PairSrc psrc, int64_t first, int level, int D,
+                        uint8_t *__restrict__ scratch, int *status) {
+    __shared__ WarpSh s;
+    extern __shared__ __align__(16) unsigned char stage[];
     const int ndir = P.vectors == 3 ? 2 : 1;
-    const int64_t pair = first + blockIdx.x / (ndir * per_dir);
-    const int rem = (int)(blockIdx.x % (ndir * per_dir)), half = rem / per_dir;
-    const int w = (int)(threadIdx.x >> 5), g = (rem % per_dir) * kLevel0Warps + w;
-    WarpSh &s = sh[w];
-    const int d = ndir == 2 ? half : ((P.vectors & 2) ? 0 : 1);
+    const int64_t pair = first + blockIdx.x / (ndir * D);
+    const int rem = (int)(blockIdx.x % (ndir * D)), g = rem % D;
+    const int d = ndir == 2 ? rem / D : ((P.vectors & 2) ? 0 : 1);
     uint8_t *scr = scratch + pair * P.scratch_per_pair;
     int *ctl = (int *)(scr + P.off_ctl[d]);
-    if (!ctl[CTL_GO]) return;  // the pair kernel ran this level itself, or the direction stopped
+    if (!ctl[CTL_GO]) return;  // the pair kernel searched the level itself, or the direction stopped
     const PairRef pr = pair_at(psrc, pair);
-    const px_t *src = (const px_t *)(d == 0 ? pr.cur : pr.ref);
-    const px_t *ref = (const px_t *)(d == 0 ? pr.ref : pr.cur);
-    DirScratch ds = dir_scratch(P, scr, d);
+    const DirScratch ds = dir_scratch(P, scr, d);
     Ctx x;
     x.P = &P;
     x.d = 0;
-    x.tid = (int)(threadIdx.x & 31);
+    x.tid = (int)threadIdx.x;
     x.nw = 1;
     x.wbase = 0;
-    x.S = Planes{src, src + P.y_len, src + P.y_len + P.c_len};
-    x.R = Planes{ref, ref + P.y_len, ref + P.y_len + P.c_len};
-    set_level(x, P, 0, kLevel0TileScale);
+    set_frames(x, P, (const px_t *)(d == 0 ? pr.cur : pr.ref), (const px_t *)(d == 0 ? pr.ref : pr.cur));
+    set_stage(x, stage, P.stage_groups, 0, 0);
+    set_level(x, P, level);
     const int od = ndir == 2 ? 1 - d : d;
-    const uint2 *prevp = ctl[CTL_PREV] ? (const uint2 *)(scr + P.off_proj[od][0]) : nullptr;
-    spec_walk<true>(x, s, ds, prevp, g, initial_order_len(P.lv[0].gw, P.lv[0].gh), ctl[CTL_GX], ctl[CTL_GY],
-                    ctl + CTL_COMMITTED, ctl + CTL_LATE, ctl + CTL_ABORT, status, psrc.stats);
+    const uint2 *prevp = ctl[CTL_PREV] ? (const uint2 *)(scr + P.off_proj[od][level & 1]) : nullptr;
+    walk_level(x, s, ds, prevp, g, D, ctl[CTL_ORDER], ctl[CTL_GX], ctl[CTL_GY], ctl, status, psrc.stats);
 }
 
-// After the level-0 kernel: the refine pass, rescale and packing of every pair not stopped.
-__global__ void __launch_bounds__(2 * NT, SVPF_MINB)
-    analyse_finish_kernel(const __grid_constant__ AnalyseParams P, const PairSrc psrc, uint8_t *__restrict__ payloads,
-                          uint8_t *__restrict__ scratch) {
-    const int64_t pair = blockIdx.x;
-    uint8_t *scr = scratch + pair * P.scratch_per_pair;
+// Neither direction of a pair stopped.
+__device__ __forceinline__ bool pair_whole(const AnalyseParams &P, const uint8_t *scr) {
     const bool bidir = P.vectors == 3;
     const int d0 = bidir ? 0 : ((P.vectors & 2) ? 0 : 1);
-    if (((const int *)(scr + P.off_ctl[d0]))[CTL_ABORT] || (bidir && ((const int *)(scr + P.off_ctl[1]))[CTL_ABORT]))
-        return;
-    finish_pair(&P, pair_at(psrc, pair), payloads + pair * P.payload_len, scr);
+    return !((const int *)(scr + P.off_ctl[d0]))[CTL_ABORT] && !(bidir && ((const int *)(scr + P.off_ctl[1]))[CTL_ABORT]);
+}
+
+// The refine pass of a split launch: its blocks are independent, so they go to `per_dir` one-warp
+// CTAs per direction, every per_dir-th block to each.
+__global__ void __launch_bounds__(32, kWalkPerSM)
+    analyse_refine_kernel(const __grid_constant__ AnalyseParams P, const PairSrc psrc, int per_dir, uint8_t *__restrict__ scratch) {
+    __shared__ WarpSh s;
+    extern __shared__ __align__(16) unsigned char stage[];
+    const int ndir = P.vectors == 3 ? 2 : 1;
+    const int64_t pair = blockIdx.x / (ndir * per_dir);
+    const int rem = (int)(blockIdx.x % (ndir * per_dir));
+    const int d = ndir == 2 ? rem / per_dir : ((P.vectors & 2) ? 0 : 1);
+    uint8_t *scr = scratch + pair * P.scratch_per_pair;
+    if (!pair_whole(P, scr)) return;
+    DirScratch ds = dir_scratch(P, scr, d);
+    Ctx x;
+    refine_ctx(x, P, pair_at(psrc, pair), d);
+    x.d = 0;
+    x.wbase = 0;
+    set_stage(x, stage, P.stage_groups, 0, 0);
+    int shape = -1;
+    const int n = P.out_gw * P.out_gh;
+    for (int i = rem % per_dir; i < n; i += per_dir) refine_block(x, s, ds, i % P.out_gw, i / P.out_gw, shape);
+}
+
+// The payloads of a split launch: kPackThreads cells of one direction per CTA.
+constexpr int kPackThreads = 256;
+__global__ void __launch_bounds__(kPackThreads)
+    analyse_pack_kernel(const __grid_constant__ AnalyseParams P, uint8_t *__restrict__ payloads, uint8_t *__restrict__ scratch) {
+    const int64_t pair = blockIdx.y;
+    const int d = P.vectors == 3 ? (int)blockIdx.z : ((P.vectors & 2) ? 0 : 1);
+    uint8_t *scr = scratch + pair * P.scratch_per_pair;
+    if (!pair_whole(P, scr)) return;
+    const DirScratch ds = dir_scratch(P, scr, d);
+    const int64_t i = (int64_t)blockIdx.x * kPackThreads + threadIdx.x;
+    pack_cells(P, ds, d, payloads + pair * P.payload_len, i, (int64_t)gridDim.x * kPackThreads, i == 0);
 }
 
 // Persistent form: a grid sized to the resident CTAs drains the item list in order (the
@@ -2451,7 +2595,7 @@ __global__ void __launch_bounds__(2 * NT, SVPF_MINB)
 __global__ void __launch_bounds__(2 * NT, SVPF_MINB)
     analyse_batch_kernel(const AnalyseParams *__restrict__ clips, const BatchItem *__restrict__ items, int nitems,
                          unsigned *__restrict__ next_item, uint8_t *__restrict__ scratch, int64_t scratch_per_cta,
-                         int *__restrict__ clip_status) {
+                         int *__restrict__ clip_status, int groups) {
     __shared__ int cta_abort;
     __shared__ int item_sh;
     __shared__ __align__(16) AnalyseParams P;
@@ -2468,29 +2612,33 @@ __global__ void __launch_bounds__(2 * NT, SVPF_MINB)
             for (int i = threadIdx.x; i < (int)(sizeof(AnalyseParams) / 16); i += blockDim.x) dst[i] = src[i];
         }
         __syncthreads();
-        analyse_pair_dev(P, bi.pair, bi.payload, scr, clip_status + bi.clip, cta_abort, nullptr, false);
+        analyse_pair_dev(P, bi.pair, bi.payload, scr, clip_status + bi.clip, cta_abort, nullptr, false, P.nlevels - 1, 0, groups);
         __syncthreads();
-        if (!cta_abort) finish_pair(&P, bi.pair, bi.payload, scr);
+        if (!cta_abort) finish_pair(&P, bi.pair, bi.payload, scr, groups);
         __syncthreads();  // P, item_sh and the shared search state are reused by the next item
     }
 }
 
 }  // namespace
 
-size_t dir_shared_bytes() { return sizeof(DirSh); }
+// Dynamic shared memory of a pair CTA of `ndir` directions.
+size_t pair_shared(int ndir, int groups) { return (size_t)ndir * (sizeof(DirSh) + (size_t)NW * groups * kGroupBytes); }
 
+// The kernels' shared-memory limits. They are raised once, to the most groups a supported block
+// can have; each launch asks for its own configuration's bytes.
 cudaError_t prepare() {
     static cudaError_t once = [] {
-        const int smem = (int)(2 * sizeof(DirSh));
+        const int smem = (int)pair_shared(2, kMaxStageGroups);
         cudaError_t e = cudaFuncSetAttribute(analyse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(analyse_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(analyse_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         return e;
     }();
     return once;
 }
+
+// Levels of fewer blocks than this are searched by the pair's CTA, without a launch of their own.
+constexpr int kWalkCells = 160;
 
 cudaError_t launch_plain(const AnalyseParams &P, const PairSrc &psrc, int npairs, uint8_t *payloads, uint8_t *scratch,
                          int *status_dev, cudaStream_t stream, int *launches) {
@@ -2498,58 +2646,78 @@ cudaError_t launch_plain(const AnalyseParams &P, const PairSrc &psrc, int npairs
     if (cudaError_t e = prepare()) return e;
     const int ndir = P.vectors == 3 ? 2 : 1;
     const bool split = SVPF_LOOKAHEAD && NW > 1 && (P.lookahead & 5) == 5;
-    analyse_kernel<<<npairs, NT * ndir, sizeof(DirSh) * ndir, stream>>>(P, psrc, payloads, scratch, status_dev,
-                                                                       split ? 1 : 0);
-    if (launches) *launches += 1;
-    if (!split) return cudaGetLastError();
-    if (cudaError_t e = cudaGetLastError()) return e;
-    // level 0: the CTAs of one launch wait on one another, so each launch takes the pairs whose
-    // CTAs are all resident at once (one launch for up to 296 bidirectional pairs on 148 SMs)
-    static const int resident = [] {
-        int dev = 0, sms = 0, per_sm = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, analyse_level0_kernel, 32 * kLevel0Warps, 0) !=
-                cudaSuccess)
-            return 0;
-        return sms * per_sm * kLevel0Warps;  // warps
-    }();
-    const int64_t most = resident / (ndir * NW);
-    if (most < 1) return cudaErrorCooperativeLaunchTooLarge;
-    const int64_t launches_needed = (npairs + most - 1) / most;
-    const int64_t group = (npairs + launches_needed - 1) / launches_needed;  // even groups
-    for (int64_t f = 0; f < npairs; f += group) {
-        const int64_t n = npairs - f < group ? npairs - f : group;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)(n * ndir * NW / kLevel0Warps));
-        cfg.blockDim = dim3(32 * kLevel0Warps);
-        cfg.dynamicSmemBytes = 0;
-        cfg.stream = stream;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeCooperative;
-        attr[0].val.cooperative = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        if (cudaError_t e = cudaLaunchKernelEx(&cfg, analyse_level0_kernel, P, psrc, f, scratch, status_dev)) return e;
-        if (launches) *launches += 1;
+    const size_t pair_smem = pair_shared(ndir, P.stage_groups);
+    auto count = [&] { if (launches) *launches += 1; return cudaGetLastError(); };
+    if (!split) {
+        analyse_kernel<<<npairs, NT * ndir, pair_smem, stream>>>(P, psrc, payloads, scratch, status_dev, 0, P.nlevels - 1, 0);
+        return count();
     }
-    analyse_finish_kernel<<<npairs, NT * ndir, sizeof(DirSh) * ndir, stream>>>(P, psrc, payloads, scratch);
-    if (launches) *launches += 1;
-    return cudaGetLastError();
+    // The CTAs of a walk wait on one another, so a launch takes the pairs whose CTAs are all resident at
+    // once: D warps per direction, as many as fit (at least kMinWalkers, with the pairs in several
+    // launches when they would not)
+    const size_t stage = (size_t)P.stage_groups * kGroupBytes;
+    int dev = 0, sms = 0, per_sm = 0;
+    if (cudaError_t e = cudaGetDevice(&dev)) return e;
+    if (cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) return e;
+    if (cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, analyse_walk_kernel, 32, stage)) return e;
+    const int64_t resident = (int64_t)sms * per_sm;
+    constexpr int kMinWalkers = 4;
+    const int64_t most = resident / (ndir * kMinWalkers);
+    if (most < 1) return cudaErrorCooperativeLaunchTooLarge;
+    const int64_t walks = (npairs + most - 1) / most;
+    const int64_t group = (npairs + walks - 1) / walks;  // even groups
+    int64_t D = resident / (ndir * group);
+    D = D < kMinWalkers ? kMinWalkers : D > kMaxWalkers ? kMaxWalkers : D;
+    int hi = P.nlevels - 1, lo = hi;
+    while (lo > 0 && P.lv[lo].gw * P.lv[lo].gh < kWalkCells) lo--;
+    for (; lo >= 0; hi = lo - 1, lo = hi) {
+        analyse_kernel<<<npairs, NT * ndir, pair_smem, stream>>>(P, psrc, payloads, scratch, status_dev, 1, hi, lo);
+        if (cudaError_t e = count()) return e;
+        for (int64_t f = 0; f < npairs; f += group) {
+            const int64_t n = npairs - f < group ? npairs - f : group;
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3((unsigned)(n * ndir * D));
+            cfg.blockDim = dim3(32);
+            cfg.dynamicSmemBytes = stage;
+            cfg.stream = stream;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeCooperative;
+            attr[0].val.cooperative = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            if (cudaError_t e = cudaLaunchKernelEx(&cfg, analyse_walk_kernel, P, psrc, f, lo, (int)D, scratch, status_dev)) return e;
+            if (launches) *launches += 1;
+        }
+    }
+    const int cells = P.out_gw * P.out_gh;
+    if (P.has_refine) {
+        int64_t per_dir = (2 * resident + npairs * ndir - 1) / (npairs * ndir);  // about two waves
+        if (per_dir > cells) per_dir = cells;
+        analyse_refine_kernel<<<(unsigned)(npairs * ndir * per_dir), 32, stage, stream>>>(P, psrc, (int)per_dir, scratch);
+        if (cudaError_t e = count()) return e;
+    }
+    for (int f = 0; f < npairs; f += 65535) {  // grid rows
+        const int n = npairs - f < 65535 ? npairs - f : 65535;
+        analyse_pack_kernel<<<dim3((cells + kPackThreads - 1) / kPackThreads, n, ndir), kPackThreads, 0, stream>>>(
+            P, payloads + (int64_t)f * P.payload_len, scratch + (int64_t)f * P.scratch_per_pair);
+        if (cudaError_t e = count()) return e;
+    }
+    return cudaSuccess;
 }
 
-cudaError_t batch_blocks_per_sm(int *blocks) {
+cudaError_t batch_blocks_per_sm(int groups, int *blocks) {
     if (cudaError_t e = prepare()) return e;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, analyse_batch_kernel, 2 * NT, 2 * sizeof(DirSh));
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, analyse_batch_kernel, 2 * NT, pair_shared(2, groups));
 }
 
 cudaError_t launch_batch(const AnalyseParams *clips_dev, const BatchItem *items_dev, int nitems, unsigned *next_item_dev,
-                         uint8_t *scratch, int64_t scratch_per_cta, int *clip_status_dev, int grid, cudaStream_t stream,
-                         int *launches) {
+                         uint8_t *scratch, int64_t scratch_per_cta, int *clip_status_dev, int groups, int grid,
+                         cudaStream_t stream, int *launches) {
     if (nitems <= 0 || grid <= 0) return cudaSuccess;
     if (cudaError_t e = prepare()) return e;
-    analyse_batch_kernel<<<grid, 2 * NT, 2 * sizeof(DirSh), stream>>>(clips_dev, items_dev, nitems, next_item_dev,
-                                                                      scratch, scratch_per_cta, clip_status_dev);
+    analyse_batch_kernel<<<grid, 2 * NT, pair_shared(2, groups), stream>>>(clips_dev, items_dev, nitems, next_item_dev,
+                                                                           scratch, scratch_per_cta, clip_status_dev,
+                                                                           groups);
     if (launches) *launches += 1;
     return cudaGetLastError();
 }

@@ -98,6 +98,7 @@ struct svpf_batch {
     int64_t off_params = 0, off_items = 0, off_counter = 0, off_status = 0, off_scratch = 0;
     int64_t scratch_per_cta = 0;
     int max_ctas = 0;          // scratch slots allocated
+    int groups = 1;            // the most AnalyseParams::stage_groups of the clips
     int sms = 0;
     int variant = 3, tiles_per_lane = 8, grid = 0;  // nt128_b3 until tuned
     std::string signature;
@@ -134,7 +135,7 @@ int upload_params(svpf_batch *b) {
 
 int grid_for(svpf_batch *b, int variant, int nitems, int *grid) {
     int per_sm = 0;
-    BCU(analyse_variant(variant).batch_blocks_per_sm(&per_sm));
+    BCU(analyse_variant(variant).batch_blocks_per_sm(b->groups, &per_sm));
     if (per_sm <= 0) return bfail(SVPF_ECUDA, "batch kernel does not fit on an SM");
     int g = per_sm * b->sms;
     if (g > b->max_ctas) g = b->max_ctas;
@@ -154,8 +155,8 @@ int record_run(svpf_batch *b, cudaStream_t st, int nitems, int grid, int *launch
     BCU(cudaMemsetAsync(b->counter_dev(), 0, 256, st));
     BCU(cudaMemsetAsync(b->status_dev(), 0, sizeof(int) * b->clips.size(), st));
     cudaError_t e = analyse_variant(b->variant).launch_batch(b->params_dev(), b->items_dev(), nitems, b->counter_dev(),
-                                                             b->scratch_dev(), b->scratch_per_cta, b->status_dev(), grid,
-                                                             st, &nl);
+                                                             b->scratch_dev(), b->scratch_per_cta, b->status_dev(),
+                                                             b->groups, grid, st, &nl);
     if (e != cudaSuccess) return bcuda(e, "batch analyse launch");
     *launches = nl;
     return SVPF_OK;
@@ -243,6 +244,7 @@ int svpf_batch_create(int32_t nclips, const svpf_super *const *supers, const svp
         c.supers_off = off; off += al256(c.super_frame_bytes * c.nframes);
         c.payloads_off = off; off += al256(c.P.payload_len * c.nframes);
         max_scratch = std::max(max_scratch, al256(c.P.scratch_per_pair));
+        b->groups = std::max(b->groups, (int)c.P.stage_groups);
         b->clips.push_back(c);
         snprintf(sig, sizeof(sig), "%dx%d/b%d/v%d/l%d", c.P.luma_w, c.P.luma_h, c.P.block_w, c.P.vectors, c.P.nlevels);
         mix[sig]++;
@@ -282,7 +284,7 @@ int svpf_batch_create(int32_t nclips, const svpf_super *const *supers, const svp
     int most = 0;
     for (int v = 0; v < analyse_variant_count(); v++) {
         int per_sm = 0;
-        if (analyse_variant(v).batch_blocks_per_sm(&per_sm) != cudaSuccess) {
+        if (analyse_variant(v).batch_blocks_per_sm(b->groups, &per_sm) != cudaSuccess) {
             delete b;
             return bfail(SVPF_ECUDA, "occupancy query failed");
         }
@@ -417,8 +419,8 @@ int svpf_batch_autotune(svpf_batch *b, int32_t *variant, int32_t *tiles_per_lane
         BCU(cudaMemsetAsync(b->status_dev(), 0, sizeof(int) * b->clips.size(), b->stream));
         BCU(cudaEventRecord(e0, b->stream));
         cudaError_t e = analyse_variant(v).launch_batch(b->params_dev(), b->items_dev(), n, b->counter_dev(),
-                                                        b->scratch_dev(), b->scratch_per_cta, b->status_dev(), grid,
-                                                        b->stream, &nl);
+                                                        b->scratch_dev(), b->scratch_per_cta, b->status_dev(),
+                                                        b->groups, grid, b->stream, &nl);
         if (e != cudaSuccess) return bcuda(e, "batch analyse launch");
         BCU(cudaEventRecord(e1, b->stream));
         add_launches(nl);

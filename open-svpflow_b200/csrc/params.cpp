@@ -35,6 +35,12 @@ bool build_analyse_params(const AnalyseOpts &o, const SuperLayout &Lay, AnalyseP
     P.lambda = o.lambda;
     P.tiles_per_lane = 8;
     P.lookahead = 5;
+    // groups of eight 4x4 tiles of a candidate (luma, then both chroma planes, which may start a
+    // group of their own): what a warp stages per block
+    auto groups = [&](const LevelInfo &L) {
+        const int tl = L.tl, tc = L.smallest ? 0 : L.tc;
+        return ((tl + 7) / 8 * 8 + 2 * tc + 7) / 8;
+    };
     // per level
     int64_t max_cells = 1, max_order = 1;
     for (int lv = 0; lv < o.levels; lv++) {
@@ -91,6 +97,7 @@ bool build_analyse_params(const AnalyseOpts &o, const SuperLayout &Lay, AnalyseP
         if (cells > max_cells) max_cells = cells;
         const int64_t ol = cells + L.gw + L.gh + 8;
         if (ol > max_order) max_order = ol;
+        if (groups(L) > P.stage_groups) P.stage_groups = groups(L);
         if (L.tl + L.tc > 96 || L.gw > 65535 || L.gh > 65535) { err = "unsupported block / grid size"; return false; }
     }
     {  // level-0 grid must be at least 2x2: below that the reference indexes field[-1]
@@ -118,6 +125,7 @@ bool build_analyse_params(const AnalyseOpts &o, const SuperLayout &Lay, AnalyseP
             R.tl = ((R.bw + 3) / 4) * ((R.bh + 3) / 4);
             const int cw = R.bw / 2, ch = R.bh / 2;
             R.tc = cw > 0 ? ((cw + 3) / 4) * (((cw > ch ? cw : ch) + 3) / 4) : 0;
+            if (groups(R) > P.stage_groups) P.stage_groups = groups(R);
             if (R.tl + R.tc > 96) { err = "unsupported block / grid size"; return false; }
         }
         if ((int64_t)gw * gh > max_cells) max_cells = (int64_t)gw * gh;

@@ -53,13 +53,12 @@ struct BatchItem {
 // The launchers every Analyse variant TU exports (analyse_body.cuh).
 #define SVPF_DECLARE_ANALYSE_VARIANT(ns)                                                                          \
     namespace ns {                                                                                                \
-    size_t dir_shared_bytes();                                                                                    \
     cudaError_t launch_plain(const AnalyseParams &P, const PairSrc &src, int npairs, uint8_t *payloads,           \
                              uint8_t *scratch, int *status_dev, cudaStream_t stream, int *launches);              \
-    cudaError_t batch_blocks_per_sm(int *blocks);                                                                 \
+    cudaError_t batch_blocks_per_sm(int groups, int *blocks);                                                     \
     cudaError_t launch_batch(const AnalyseParams *clips_dev, const BatchItem *items_dev, int nitems,              \
                              unsigned *next_item_dev, uint8_t *scratch, int64_t scratch_per_cta,                  \
-                             int *clip_status_dev, int grid, cudaStream_t stream, int *launches);                 \
+                             int *clip_status_dev, int groups, int grid, cudaStream_t stream, int *launches);     \
     }
 SVPF_DECLARE_ANALYSE_VARIANT(nt128)
 SVPF_DECLARE_ANALYSE_VARIANT(nt64)
@@ -76,9 +75,10 @@ struct AnalyseVariant {
     int threads_per_dir, min_blocks;
     cudaError_t (*launch_plain)(const AnalyseParams &, const PairSrc &, int, uint8_t *, uint8_t *, int *,
                                 cudaStream_t, int *);
-    cudaError_t (*batch_blocks_per_sm)(int *);
+    // groups: the most AnalyseParams::stage_groups of the batch's clips
+    cudaError_t (*batch_blocks_per_sm)(int groups, int *);
     cudaError_t (*launch_batch)(const AnalyseParams *, const BatchItem *, int, unsigned *, uint8_t *, int64_t, int *,
-                                int, cudaStream_t, int *);
+                                int groups, int grid, cudaStream_t, int *);
 };
 int analyse_variant_count();
 const AnalyseVariant &analyse_variant(int i);  // 0 = the plain path's default (nt128)

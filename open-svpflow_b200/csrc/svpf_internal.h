@@ -13,6 +13,7 @@
 namespace svpf {
 
 constexpr int kMaxLevels = 16;
+constexpr int kMaxStageGroups = 17;  // groups of eight 4x4 tiles: luma tiles + 2 x chroma tiles <= 128, chroma maybe apart
 
 struct SuperOpts {
     int32_t pel = 2, gpu = 1, scale_down = 4, scale_up = 0;
@@ -104,19 +105,21 @@ struct alignas(16) AnalyseParams {
     int32_t has_refine, refine_thsad, refine_search_type, refine_distance, refine_satd, lambda;
     LevelInfo rlv[2];         // refine pass block shapes: output block, half of it (border blocks)
     int32_t rescale_denom;
-    int32_t tiles_per_lane;   // 4x4 tiles one lane evaluates per candidate (2, 4 or 8): a launch tuning knob
+    int32_t tiles_per_lane;   // accepted (2, 4 or 8) and kept; the evaluation no longer splits a candidate over lanes
     int32_t px_bytes;         // 1: 8-bit samples; 2: uint16 samples (the 10-bit extension)
     int32_t lookahead;        // look-ahead (one block per warp in flight, exact either way): bit 0 level 0,
-                              // bit 1 the coarser levels (slower: measured), bit 2 level 0 spread over
-                              // the GPU (its own launch, one CTA per warp); a tuning knob, default 5
-    int32_t pad0_, pad1_, pad2_;
+                              // bit 1 the coarser levels, both in the pair's CTA; bits 0 and 2: every level
+                              // but the smallest spread over the GPU (launches of their own, one CTA per
+                              // warp); a tuning knob, default 5
+    int32_t stage_groups;     // the most groups of eight 4x4 tiles a candidate of any level has (shared staging)
+    int32_t pad0_, pad1_;
     int64_t payload_len;
     int32_t header[16];       // payload words 0x00..0x3C
     // per-pair scratch layout (bytes)
     int64_t max_cells, max_order;
     int64_t off_field[2], off_next[2], off_proj[2][2], off_order[2], off_order2[2], off_pos[2];
     int64_t off_keys[2], off_hist[2], off_seen[2], off_out[2];
-    int64_t off_ctl[2];       // per direction: the hand-over words of the level-0 kernel (CTL_*)
+    int64_t off_ctl[2];       // per direction: the words that go from launch to launch (CTL_*)
     int64_t scratch_per_pair;
 };
 
