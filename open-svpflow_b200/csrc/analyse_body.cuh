@@ -91,6 +91,31 @@ struct Cand {
     uint8_t lmode, cmode, lsatd, csatd;
 };
 
+// Per-block constants, identical in every thread of a direction. In shared memory, one copy per warp, like
+// Search: they are read once per 32 candidates, and registers are what bounds the warps in flight.
+struct BlkC {
+    int px, py, bw, bh, px2, py2;
+    int bnd0, bnd1, bnd2, bnd3;            // mv_bounds
+    int chroma, fast_src;
+    int fx0, fx1, fy0, fy1;                // vectors taking the fast path lie in this box (inclusive) ...
+    int lbase, llim, cbase, clim;          // ... and have lref <= llim, cref <= clim; the offsets (from the frame's
+                                           // first sample) of the reference blocks at vector 0
+    int64_t lsrc, csrc;                    // offset of the source block (luma, U)
+};
+
+// What a block's search keeps from turn to turn, identical in every lane of the warp (see Search_next).
+struct Search {
+    int state, stage, stype, radius;
+    int predx, predy;                       // predictor of the motion penalty
+    int lambda, own_x, own_y, ppx, ppy;     // the block's penalty factor, its own predictor and the refinement's
+    int bmx, bmy;                           // the best so far
+    unsigned bsad;
+    long long bcost;
+    int hbx, hby, hdir, hi, hrad, hret, bad_r, bad_max;
+    unsigned found;
+    int sets_mv;
+};
+
 // Shared state of one search direction. A block is searched by a group of warps: the whole
 // direction (coarser levels), or one warp (level 0 with look-ahead, one block per warp in
 // flight). Per-warp entries are indexed by the warp's place in the direction; a group's
@@ -98,6 +123,10 @@ struct Cand {
 // direction's, or one for a CTA of the level-0 kernel).
 template <int W>
 struct alignas(16) DirShT {
+    Search q[W];                          // per warp: its block's search ...
+    BlkC blk[W];                          // ... and constants
+    int lmx[W][32], lmy[W][32];           // per warp: the special candidates, one per lane, ...
+    unsigned lsd[W][32];                  // ... and their exact_sad
     long long K[2][W];                    // per-warp best (cost, index, sad) of a step, double-buffered
     int I[2][W];
     unsigned S[2][W];
@@ -665,17 +694,6 @@ __device__ __forceinline__ void set_stage(Ctx &x, unsigned char *area, int group
     x.src = reinterpret_cast<float4 *>(area + (size_t)first * groups * kGroupBytes);
     x.off = reinterpret_cast<unsigned *>(area + (size_t)warp * groups * kGroupBytes + (size_t)groups * 512);
 }
-
-// Per-block constants, identical in every thread of a direction.
-struct BlkC {
-    int px, py, bw, bh, px2, py2;
-    int bnd0, bnd1, bnd2, bnd3;            // mv_bounds
-    int chroma, fast_src;
-    int fx0, fx1, fy0, fy1;                // vectors taking the fast path lie in this box (inclusive) ...
-    int lbase, llim, cbase, clim;          // ... and have lref <= llim, cref <= clim; the offsets (from the frame's
-                                           // first sample) of the reference blocks at vector 0
-    int64_t lsrc, csrc;                    // offset of the source block (luma, U)
-};
 
 __device__ __forceinline__ void make_blk(const Ctx &x, int px, int py, bool chroma, BlkC &b) {
     const LevelInfo &L = *x.L;
@@ -1317,115 +1335,107 @@ enum { S_REFINE, S_HEX_START, S_HEX_ITER, S_HEX_EXIT, S_BAD, S_BAD_RING, S_FINAL
 // there (a walk runs the two apart: the test reads the bad count of the blocks before),
 // RS_NONE runs nothing.
 enum { RS_NONE, RS_ALL, RS_REFINE_ONLY, RS_BAD_ONLY };
-struct Search {
-    int state, stage, stype, radius;
-    int predx, predy;                       // predictor of the motion penalty
-    int bmx, bmy;                           // the best so far
-    unsigned bsad;
-    long long bcost;
-    int hbx, hby, hdir, hi, hrad, hret, bad_r, bad_max;
-    unsigned found;
-    bool sets_mv;
-
-    __device__ __forceinline__ void begin(int stage_, int stype_, int radius_, int ppx, int ppy) {
-        stage = stage_; stype = stype_; radius = radius_;
-        predx = ppx; predy = ppy;
-        state = stage == RS_NONE ? S_STORE : (stage == RS_BAD_ONLY ? S_BAD : S_REFINE);
-        hdir = -2; hi = hrad = hret = 0;
-    }
-    // The next step's candidates; false when there is none.
-    __device__ __forceinline__ bool next(const Ctx &x, const BlkC &b, int own_x, int own_y, int64_t idx, int &bad_count, Gen &g) {
-        const AnalyseParams &P = *x.P;
-        const LevelInfo &L = *x.L;
-        sets_mv = true;
-        while (state != S_STORE) {
-            if (state == S_BAD && stage == RS_REFINE_ONLY) {
-                state = S_STORE;
-                break;
-            }
-            if (state == S_REFINE) {
-                if (stype == 4) { state = S_BAD; g = make_gen(BK_EXH, bmx, bmy, radius, 0, 0); return true; }
-                if (stype == 3) {
-                    state = S_HEX_START; hrad = radius; hret = 0;
-                    g = make_gen(BK_UMH, bmx, bmy, radius, 0, 0);
-                    return true;
-                }
-                if (stype == 2) { state = S_HEX_START; hrad = radius; hret = 0; }
-                else state = S_BAD;
-            } else if (state == S_HEX_START) {
-                hbx = bmx; hby = bmy;
-                if (hrad > 1) { sets_mv = false; state = S_HEX_ITER; g = make_gen(BK_HEX6, hbx, hby, 0, 0, 0); return true; }
-                state = hret ? S_FINAL_RING : S_BAD;
-                g = make_gen(BK_RING, hbx, hby, 1, 1, 0);
-                return true;
-            } else if (state == S_HEX_ITER) {
-                if (hi < hrad / 2 && hbx >= b.bnd0 && hby >= b.bnd1 && hbx < b.bnd2 && hby < b.bnd3) {
-                    sets_mv = false;
-                    g = make_gen(BK_HEX3, hbx, hby, 0, 0, c_mod6m1[hdir + 1]);
-                    return true;
-                }
-                state = S_HEX_EXIT;
-            } else if (state == S_HEX_EXIT) {
-                bmx = hbx; bmy = hby;
-                state = hret ? S_FINAL_RING : S_BAD;
-                g = make_gen(BK_RING, hbx, hby, 1, 1, 0);
-                return true;
-            } else if (state == S_BAD) {
-                found = bsad;
-                if (x.level > 0 && idx > 1 && P.coarse_bad_sad > 0 && (int)bsad > bad_limit(P, bad_count)) {
-                    bad_count++;
-                    predx = own_x; predy = own_y;  // the block's own predictor
-                    if (P.coarse_bad_range < 0) {
-                        bad_max = -P.coarse_bad_range * L.pel; bad_r = L.pel;
-                        if (bad_r < bad_max) { state = S_BAD_RING; g = make_gen(BK_RING, 0, 0, bad_r, L.pel, 0); return true; }
-                        state = S_FINAL_RING;
-                    } else if (P.coarse_bad_range > 0) {
-                        hrad = P.coarse_bad_range * L.pel; hret = 1;
-                        state = S_HEX_START;
-                        g = make_gen(BK_UMH, 0, 0, hrad, 0, 0);
-                        return true;
-                    } else state = S_FINAL_RING;
-                } else state = S_STORE;
-            } else if (state == S_BAD_RING) {
-                if (bsad < found / 4) state = S_FINAL_RING;
-                else {
-                    bad_r += L.pel;
-                    if (bad_r < bad_max) { g = make_gen(BK_RING, 0, 0, bad_r, L.pel, 0); return true; }
-                    state = S_FINAL_RING;
-                }
-            } else {  // S_FINAL_RING
-                state = S_STORE;
-                g = make_gen(BK_RING, bmx, bmy, 1, 1, 0);
+__device__ __forceinline__ void search_begin(Search &q, int stage) {
+    q.stage = stage;
+    q.predx = q.ppx; q.predy = q.ppy;
+    q.state = stage == RS_NONE ? S_STORE : (stage == RS_BAD_ONLY ? S_BAD : S_REFINE);
+    q.hdir = -2; q.hi = q.hrad = q.hret = 0;
+}
+// The next step's candidates; false when there is none.
+__device__ __forceinline__ bool search_next(Search &q, const Ctx &x, const BlkC &b, int64_t idx, int &bad_count, Gen &g) {
+    const AnalyseParams &P = *x.P;
+    const LevelInfo &L = *x.L;
+    q.sets_mv = 1;
+    while (q.state != S_STORE) {
+        if (q.state == S_BAD && q.stage == RS_REFINE_ONLY) {
+            q.state = S_STORE;
+            break;
+        }
+        if (q.state == S_REFINE) {
+            if (q.stype == 4) { q.state = S_BAD; g = make_gen(BK_EXH, q.bmx, q.bmy, q.radius, 0, 0); return true; }
+            if (q.stype == 3) {
+                q.state = S_HEX_START; q.hrad = q.radius; q.hret = 0;
+                g = make_gen(BK_UMH, q.bmx, q.bmy, q.radius, 0, 0);
                 return true;
             }
+            if (q.stype == 2) { q.state = S_HEX_START; q.hrad = q.radius; q.hret = 0; }
+            else q.state = S_BAD;
+        } else if (q.state == S_HEX_START) {
+            q.hbx = q.bmx; q.hby = q.bmy;
+            if (q.hrad > 1) { q.sets_mv = 0; q.state = S_HEX_ITER; g = make_gen(BK_HEX6, q.hbx, q.hby, 0, 0, 0); return true; }
+            q.state = q.hret ? S_FINAL_RING : S_BAD;
+            g = make_gen(BK_RING, q.hbx, q.hby, 1, 1, 0);
+            return true;
+        } else if (q.state == S_HEX_ITER) {
+            if (q.hi < q.hrad / 2 && q.hbx >= b.bnd0 && q.hby >= b.bnd1 && q.hbx < b.bnd2 && q.hby < b.bnd3) {
+                q.sets_mv = 0;
+                g = make_gen(BK_HEX3, q.hbx, q.hby, 0, 0, c_mod6m1[q.hdir + 1]);
+                return true;
+            }
+            q.state = S_HEX_EXIT;
+        } else if (q.state == S_HEX_EXIT) {
+            q.bmx = q.hbx; q.bmy = q.hby;
+            q.state = q.hret ? S_FINAL_RING : S_BAD;
+            g = make_gen(BK_RING, q.hbx, q.hby, 1, 1, 0);
+            return true;
+        } else if (q.state == S_BAD) {
+            q.found = q.bsad;
+            if (x.level > 0 && idx > 1 && P.coarse_bad_sad > 0 && (int)q.bsad > bad_limit(P, bad_count)) {
+                bad_count++;
+                q.predx = q.own_x; q.predy = q.own_y;  // the block's own predictor
+                if (P.coarse_bad_range < 0) {
+                    q.bad_max = -P.coarse_bad_range * L.pel; q.bad_r = L.pel;
+                    if (q.bad_r < q.bad_max) { q.state = S_BAD_RING; g = make_gen(BK_RING, 0, 0, q.bad_r, L.pel, 0); return true; }
+                    q.state = S_FINAL_RING;
+                } else if (P.coarse_bad_range > 0) {
+                    q.hrad = P.coarse_bad_range * L.pel; q.hret = 1;
+                    q.state = S_HEX_START;
+                    g = make_gen(BK_UMH, 0, 0, q.hrad, 0, 0);
+                    return true;
+                } else q.state = S_FINAL_RING;
+            } else q.state = S_STORE;
+        } else if (q.state == S_BAD_RING) {
+            if (q.bsad < q.found / 4) q.state = S_FINAL_RING;
+            else {
+                q.bad_r += L.pel;
+                if (q.bad_r < q.bad_max) { g = make_gen(BK_RING, 0, 0, q.bad_r, L.pel, 0); return true; }
+                q.state = S_FINAL_RING;
+            }
+        } else {  // S_FINAL_RING
+            q.state = S_STORE;
+            g = make_gen(BK_RING, q.bmx, q.bmy, 1, 1, 0);
+            return true;
         }
-        return false;
     }
-    // The step's outcome: candidate w of g was accepted (its cost and sad are in bcost, bsad), or none (-1).
-    __device__ __forceinline__ void took(const Gen &g, int w) {
-        if (g.kind == BK_HEX6 || g.kind == BK_HEX3) {  // exact_check_dir: a label, best.mv set at exit
-            if (w >= 0) {
-                hdir = g.kind == BK_HEX6 ? w : g.odir + w - 1;
-                hbx += c_hex2[hdir + 1].x; hby += c_hex2[hdir + 1].y;
-                hi = g.kind == BK_HEX6 ? 1 : hi + 1;
-                state = S_HEX_ITER;
-            } else state = S_HEX_EXIT;
-        } else if (w >= 0 && sets_mv) {
-            const int2 m = gen_mv(g, w);
-            bmx = m.x; bmy = m.y;
-        }
+    return false;
+}
+// The step's outcome: candidate w of g was accepted (its cost and sad are in bcost, q.bsad), or none (-1).
+__device__ __forceinline__ void search_took(Search &q, const Gen &g, int w) {
+    if (g.kind == BK_HEX6 || g.kind == BK_HEX3) {  // exact_check_dir: a label, best.mv set at exit
+        if (w >= 0) {
+            q.hdir = g.kind == BK_HEX6 ? w : g.odir + w - 1;
+            q.hbx += c_hex2[q.hdir + 1].x; q.hby += c_hex2[q.hdir + 1].y;
+            q.hi = g.kind == BK_HEX6 ? 1 : q.hi + 1;
+            q.state = S_HEX_ITER;
+        } else q.state = S_HEX_EXIT;
+    } else if (w >= 0 && q.sets_mv) {
+        const int2 m = gen_mv(g, w);
+        q.bmx = m.x; q.bmy = m.y;
     }
-};
+}
 
 // Runs q (begun) to its end, one step after another.
 template <class SH>
-__device__ __forceinline__ void run_search(const Ctx &x, const BlkC &b, SH &s, int &ph, Search &q, int lambda, int own_x,
-                                           int own_y, int64_t idx, int &bad_count) {
+__device__ __forceinline__ void run_search(const Ctx &x, const BlkC &b, SH &s, int &ph, Search &q, int64_t idx, int &bad_count) {
     Gen g{0, 0, 0, 0, 0, 0, 0};
-    while (q.next(x, b, own_x, own_y, idx, bad_count, g)) {
+    while (search_next(q, x, b, idx, bad_count, g)) {
         int w;
-        eval_step(x, b, s, ph, g, lambda, q.predx, q.predy, q.bcost, q.bsad, w);
-        q.took(g, w);
+        long long cost = q.bcost;
+        unsigned sad = q.bsad;
+        eval_step(x, b, s, ph, g, q.lambda, q.predx, q.predy, cost, sad, w);
+        q.bcost = cost;
+        q.bsad = sad;
+        search_took(q, g, w);
     }
 }
 
@@ -1503,7 +1513,8 @@ __device__ __forceinline__ void search_level(const Ctx &x, DirSh &s, DirScratch 
         const int64_t fi = edge ? sidx : idx;
         const uint2 interp = fi == last_idx ? last_val : field[fi];
         const int2 imv = vmv(interp);
-        BlkC b;
+        BlkC &b = s.blk[warp];
+        Search &q = s.q[warp];
         make_blk(x, px, py, !smallest, b);
         const int phb = ph;  // this block's entries of dc and score; the specials' barrier below publishes them
         {
@@ -1560,10 +1571,10 @@ __device__ __forceinline__ void search_level(const Ctx &x, DirSh &s, DirScratch 
         const int place = lane < 9 ? 4 + __popc(seeds & ((1u << lane) - 1u)) : lane - kField;
         const long long cost = (long long)sd + (((long long)pp * sd) >> 8);
         const int wl = first_min(act, cost, place);
-        Search q;
+        const unsigned wsad = __shfl_sync(kFull, sd, wl);
         q.bmx = __shfl_sync(kFull, mx, wl); q.bmy = __shfl_sync(kFull, my, wl);
-        q.bsad = __shfl_sync(kFull, sd, wl);
-        q.bcost = (long long)q.bsad;
+        q.bsad = wsad;
+        q.bcost = (long long)wsad;
         int lambda = 0, radius = 0, stype = 0, ppx = imv.x, ppy = imv.y;
         if (search) {
             const long long cf = __shfl_sync(kFull, cost, kField), cp = __shfl_sync(kFull, cost, kPrev);
@@ -1581,8 +1592,10 @@ __device__ __forceinline__ void search_level(const Ctx &x, DirSh &s, DirScratch 
         if (dc_fast)
             for (int w = 0; w < x.nw; w++) dcsum += s.dc[phb][w];
         else dcsum = s.dcs[phb];
-        q.begin(search ? RS_ALL : RS_NONE, stype, radius, ppx, ppy);
-        run_search(x, b, s, ph, q, lambda, imv.x, imv.y, idx, bad_count);
+        q.stype = stype; q.radius = radius; q.lambda = lambda;
+        q.ppx = ppx; q.ppy = ppy; q.own_x = imv.x; q.own_y = imv.y;
+        search_begin(q, search ? RS_ALL : RS_NONE);
+        run_search(x, b, s, ph, q, idx, bad_count);
         // ---- store (:673-679)
         const uint2 v = mkvec(q.bmx, q.bmy, smallest ? sat_mul(q.bsad, 3) : q.bsad);
         if (x.tid == 0) {
@@ -1679,85 +1692,88 @@ __device__ __forceinline__ void walk_level(const Ctx &x, SH &s, const DirScratch
     uint8_t *lumaf = ds.luma[level & 1];
     const bool smallest = L.smallest != 0;
     int *progress = (int *)ds.hist;
-    const int lane = x.tid;
-    int ph = 0;
+    const int lane = x.tid, wi = x.wbase;
+    BlkC &b = s.blk[wi];
+    Search &q = s.q[wi];
     int n_blk = 0, n_def = 0, n_eval = 0, n_rerun = 0;
     bool late = false;
     for (int k = g; k < order_len; k += D) {
         const int2 bxy = level == 0 ? initial_order_at(gw, gh, k) : unpack_xy(ds.order[k]);
         const int bx = bxy.x, by = bxy.y;
         const int idx = by * gw + bx;
-        int px = (level > 0 && bx == gw - 1) ? L.lw - P.block_w : bx * P.step_x;
-        int py = (level > 0 && by == gh - 1) ? L.lh - P.block_h : by * P.step_y;
-        px += L.pxoff;
-        py += L.pyoff;
         const bool edge = level > 0 && (bx == gw - 1 || by == gh - 1);
-        const int sxi = imin(bx, gw - 2), syi = imin(by, gh - 2);
         // ---- the special candidates, one per lane (see special_sads)
-        bool act = false, seed = false, open = false;  // open: a seed that is not final yet
-        int mx = 0, my = 0;
-        int ncell = 0;
-        if (lane < 9) {
-            const int ny = by - 1 + lane / 3, nx = bx - 1 + lane % 3;
-            if (ny >= 0 && ny < gh && nx >= 0 && nx < gw) {
-                ncell = ny * gw + nx;
-                act = (level == 0 ? (int)initial_order_pos(gw, gh, nx, ny) : ds.pos[ncell]) < k;
-                seed = act;
-                if (act) {
-                    const unsigned long long v = ld_tag(ds.keys + ncell);
-                    const int2 m = vmv(make_uint2((unsigned)v, 0));
-                    mx = m.x; my = m.y;
-                    act = (int)(v >> 32) != TAG_NONE;
-                    open = (int)(v >> 32) != TAG_FINAL;
+        const int ncell = idx + (lane < 9 ? (lane / 3 - 1) * gw + lane % 3 - 1 : 0);
+        unsigned seeds, openm, actm;  // lanes holding a seed, one that is not final yet, a candidate
+        unsigned pred_score;
+        {
+            int px = (level > 0 && bx == gw - 1) ? L.lw - P.block_w : bx * P.step_x;
+            int py = (level > 0 && by == gh - 1) ? L.lh - P.block_h : by * P.step_y;
+            px += L.pxoff;
+            py += L.pyoff;
+            const int sxi = imin(bx, gw - 2), syi = imin(by, gh - 2);
+            bool act = false, seed = false, open = false;
+            int mx = 0, my = 0;
+            if (lane < 9) {
+                const int ny = by - 1 + lane / 3, nx = bx - 1 + lane % 3;
+                if (ny >= 0 && ny < gh && nx >= 0 && nx < gw) {
+                    seed = (level == 0 ? (int)initial_order_pos(gw, gh, nx, ny) : ds.pos[ncell]) < k;
+                    if (seed) {
+                        const unsigned long long v = ld_tag(ds.keys + ncell);
+                        const int2 m = vmv(make_uint2((unsigned)v, 0));
+                        mx = m.x; my = m.y;
+                        act = (int)(v >> 32) != TAG_NONE;
+                        open = (int)(v >> 32) != TAG_FINAL;
+                    }
                 }
+            } else if (lane == kPrev) {
+                if (prevp) {
+                    const uint2 pv = prevp[idx];
+                    act = pv.y != 0xFFFFFFFFu && pv.y > 0;
+                    const int2 m = vmv(pv);
+                    mx = m.x; my = m.y;
+                }
+            } else if (lane == kGlobal) {
+                act = true; mx = gxv; my = gyv;
+            } else if (lane == kZero) {
+                act = true;
             }
-        } else if (lane == kPrev) {
-            if (prevp) {
-                const uint2 pv = prevp[idx];
-                act = pv.y != 0xFFFFFFFFu && pv.y > 0;
-                const int2 m = vmv(pv);
-                mx = m.x; my = m.y;
+            uint2 interp;
+            if (edge) {  // its inner cell comes earlier in the order (level_spec_ok): that cell's final vector
+                unsigned long long v = 0;
+                if (!spin([&] { v = ld_tag(ds.keys + syi * gw + sxi); return (int)(v >> 32) == TAG_FINAL; }, ctl + CTL_LATE)) late = true;
+                interp = make_uint2((unsigned)v, 0);  // the score is taken anew below
+            } else {
+                interp = field[idx];
             }
-        } else if (lane == kGlobal) {
-            act = true; mx = gxv; my = gyv;
-        } else if (lane == kZero) {
-            act = true;
+            const int2 imv = vmv(interp);
+            if (lane == kField) { mx = imv.x; my = imv.y; }
+            make_blk(x, px, py, !smallest, b);
+            q.own_x = q.ppx = imv.x; q.own_y = q.ppy = imv.y;
+            __syncwarp();
+            unsigned dcsum = 0;
+            if (b.fast_src) dcsum = stage_source(x, b);
+            if (!(b.fast_src && b.px2 == px && b.py2 == py))  // block_luma_dc on the reference's read path
+                dcsum = eval_slow(x, px, py, 0, 0, SLOW_DC).x;
+            if (lane == 0) lumaf[idx] = block_mean(b, L, dcsum);
+            pred_score = interp.y;
+            if (edge)  // re-score the predictor at its source block (:536-549)
+                pred_score = sad_of(eval_slow(x, sxi * P.step_x, syi * P.step_y, imv.x, imv.y, SLOW_CHROMA));
+            const bool field_valid = pred_score != 0xFFFFFFFFu;
+            if (lane == kField) act = field_valid;
+            const bool search = !(level == 0 && P.distance == 0);
+            if (!search) act = lane == (field_valid ? kField : kZero);
+            seeds = __ballot_sync(kFull, seed);  // at most 8 (level_spec_ok)
+            openm = __ballot_sync(kFull, open);
+            actm = __ballot_sync(kFull, act);
+            s.lmx[wi][lane] = mx;
+            s.lmy[wi][lane] = my;
+            __syncwarp();
         }
-        uint2 interp;
-        if (edge) {  // its inner cell comes earlier in the order (level_spec_ok): that cell's final vector
-            unsigned long long v = 0;
-            if (!spin([&] { v = ld_tag(ds.keys + syi * gw + sxi); return (int)(v >> 32) == TAG_FINAL; }, ctl + CTL_LATE)) late = true;
-            interp = make_uint2((unsigned)v, 0);  // the score is taken anew below
-        } else {
-            interp = field[idx];
-        }
-        const int2 imv = vmv(interp);
-        if (lane == kField) { mx = imv.x; my = imv.y; }
-        const unsigned seeds = __ballot_sync(kFull, seed);  // at most 8 (level_spec_ok)
-        BlkC b;
-        make_blk(x, px, py, !smallest, b);
-        unsigned dcsum = 0;
-        if (b.fast_src) dcsum = stage_source(x, b);
-        if (!(b.fast_src && b.px2 == px && b.py2 == py))  // block_luma_dc on the reference's read path
-            dcsum = eval_slow(x, px, py, 0, 0, SLOW_DC).x;
-        unsigned pred_score = interp.y;
-        if (edge)  // re-score the predictor at its source block (:536-549)
-            pred_score = sad_of(eval_slow(x, sxi * P.step_x, syi * P.step_y, imv.x, imv.y, SLOW_CHROMA));
-        __syncwarp();
-        const bool field_valid = pred_score != 0xFFFFFFFFu;
-        if (lane == kField) act = field_valid;
-        const bool search = !(level == 0 && P.distance == 0);
-        if (!search) act = lane == (field_valid ? kField : kZero);
-        // ---- selection (:716-747)
-        const int pp = lane < 9 ? P.pnbour : lane == kPrev ? P.prev : lane == kGlobal ? P.pglobal : lane == kZero ? P.pzero : 0;
-        const int place = lane < 9 ? 4 + __popc(seeds & ((1u << lane) - 1u)) : lane - kField;
-        unsigned sd = 0;
-        bool fresh = act;  // lanes whose candidate is to be evaluated
+        unsigned freshm = actm;  // lanes whose candidate is to be evaluated
         bool started = false, reran = false, published = false;
         int selx = 0, sely = 0;
-        int lambda = 0, radius = 0, stype = 0, ppx = imv.x, ppy = imv.y;
-        Search q;
-        q.begin(RS_NONE, 0, 0, 0, 0);
+        q.state = S_STORE;
         Gen g_{0, 0, 0, 0, 0, 0, 0};  // the step in work, its next 32 candidates, and the one accepted so far
         int base = 0, win = -1;
         bool stepping = false;
@@ -1768,30 +1784,33 @@ __device__ __forceinline__ void walk_level(const Ctx &x, SH &s, const DirScratch
         // runs, seeds that have become final are looked at between its turns; tentative ones only when
         // there is nothing else to do, since the work they cause may be in vain.
         for (;;) {
-            bool special = __any_sync(kFull, fresh);
-            if (!special && !stepping) {
-                if (q.next(x, b, imv.x, imv.y, idx, bad_count, g_)) { stepping = true; base = 0; win = -1; }
+            if (!freshm && !stepping) {
+                if (search_next(q, x, b, idx, bad_count, g_)) { stepping = true; base = 0; win = -1; }
                 else {
                     if (final) break;
-                    if (__any_sync(kFull, open)) {  // publish, then wait for news
+                    if (openm) {  // publish, then wait for news
                         if (!published && lane == 0) st_tag(ds.keys + idx, tag_word(TAG_TENTATIVE, q.bmx, q.bmy));
                         published = true;
+                        const bool open = (openm >> lane) & 1u, act = (actm >> lane) & 1u;
+                        const int mx = s.lmx[wi][lane], my = s.lmy[wi][lane];
                         unsigned long long v = 0;
                         if (!spin([&] {
                                 if (open) v = ld_tag(ds.keys + ncell);
                                 const int2 m = vmv(make_uint2((unsigned)v, 0));
-                                fresh = open && (int)(v >> 32) != TAG_NONE && (!act || m.x != mx || m.y != my);
-                                return __any_sync(kFull, fresh) || !(open && (int)(v >> 32) != TAG_FINAL);
+                                freshm = __ballot_sync(kFull, open && (int)(v >> 32) != TAG_NONE && (!act || m.x != mx || m.y != my));
+                                return freshm || !(open && (int)(v >> 32) != TAG_FINAL);
                             }, ctl + CTL_LATE)) {
                             late = true;
-                            open = false;
+                            openm = 0;
                         }
-                        if ((int)(v >> 32) == TAG_FINAL) open = false;
-                        if (fresh) { const int2 m = vmv(make_uint2((unsigned)v, 0)); mx = m.x; my = m.y; act = true; }
+                        openm &= ~__ballot_sync(kFull, (int)(v >> 32) == TAG_FINAL);
+                        actm |= freshm;
+                        if ((freshm >> lane) & 1u) { const int2 m = vmv(make_uint2((unsigned)v, 0)); s.lmx[wi][lane] = m.x; s.lmy[wi][lane] = m.y; }
+                        __syncwarp();
                         continue;
                     }
                     final = true;  // every seed is final and is the one used
-                    if (search && level > 0 && P.coarse_bad_sad > 0) {
+                    if (!(level == 0 && P.distance == 0) && level > 0 && P.coarse_bad_sad > 0) {
                         bool bad = false;
                         if (idx > 1 && (int)q.bsad > P.coarse_bad_sad) {  // above the threshold of a count of 0
                             if (!spin([&] {
@@ -1807,7 +1826,7 @@ __device__ __forceinline__ void walk_level(const Ctx &x, SH &s, const DirScratch
                             __syncwarp();
                         }
                         if (lane == 0) st_word(progress + g, k + D);
-                        if (bad) { q.begin(RS_BAD_ONLY, stype, radius, ppx, ppy); continue; }
+                        if (bad) { search_begin(q, RS_BAD_ONLY); continue; }
                     }
                     break;
                 }
@@ -1815,55 +1834,63 @@ __device__ __forceinline__ void walk_level(const Ctx &x, SH &s, const DirScratch
             // ---- what to evaluate: exact_sad of the new special candidates (an equal vector's that is
             // known, else one for all that are equal), or the step's candidates inside the bounds whose
             // motion penalty does not reach the best cost (see eval_step)
+            const bool special = freshm != 0;
             bool eval;
             int vx, vy, from = lane;
             long long motion = 0;
             if (special) {
-                const unsigned peers = __match_any_sync(kFull, ((unsigned long long)(unsigned)mx << 32) | (unsigned)my);
-                const unsigned known = peers & __ballot_sync(kFull, act && !fresh), asked = peers & __ballot_sync(kFull, fresh);
+                vx = s.lmx[wi][lane]; vy = s.lmy[wi][lane];
+                const unsigned peers = __match_any_sync(kFull, ((unsigned long long)(unsigned)vx << 32) | (unsigned)vy);
+                const unsigned known = peers & actm & ~freshm, asked = peers & freshm;
+                const bool fresh = (freshm >> lane) & 1u;
                 if (fresh) from = __ffs(known ? known : asked) - 1;
                 eval = fresh && !known && from == lane;
-                vx = mx; vy = my;
                 if (started) n_eval += __popc(__ballot_sync(kFull, eval));
             } else {
                 const int2 m = gen_mv(g_, imin(base + lane, g_.n - 1));
                 vx = m.x; vy = m.y;
-                motion = motion_penalty(lambda, q.predx, q.predy, vx, vy);
+                motion = motion_penalty(q.lambda, q.predx, q.predy, vx, vy);
                 eval = base + lane < g_.n && vx >= b.bnd0 && vy >= b.bnd1 && vx < b.bnd2 && vy < b.bnd3 && motion < q.bcost;
             }
             unsigned long long news = 0;
-            const bool look = open && started;
-            if (look) news = ld_tag(ds.keys + ncell);  // in flight during the evaluation
+            const unsigned lookm = started ? openm : 0;
+            if ((lookm >> lane) & 1u) news = ld_tag(ds.keys + ncell);  // in flight during the evaluation
             unsigned l, c;
             eval_cands(x, b, eval, vx, vy, l, c);
             if (special) {
-                if (eval) sd = sat_add(l, c);
-                sd = __shfl_sync(kFull, sd, from);
-                fresh = false;
+                if (eval) s.lsd[wi][lane] = sat_add(l, c);
+                __syncwarp();
+                const unsigned sd = s.lsd[wi][from];
+                __syncwarp();
+                s.lsd[wi][lane] = sd;
+                freshm = 0;
+                const int pp = lane < 9 ? P.pnbour : lane == kPrev ? P.prev : lane == kGlobal ? P.pglobal : lane == kZero ? P.pzero : 0;
+                const int place = lane < 9 ? 4 + __popc(seeds & ((1u << lane) - 1u)) : lane - kField;
                 const long long cost = (long long)sd + (((long long)pp * sd) >> 8);
-                const int wl = first_min(act, cost, place);
-                const int nx = __shfl_sync(kFull, mx, wl), ny = __shfl_sync(kFull, my, wl);
+                const int wl = first_min((actm >> lane) & 1u, cost, place);
+                const int nx = s.lmx[wi][wl], ny = s.lmy[wi][wl];
                 const unsigned nsad = __shfl_sync(kFull, sd, wl);
+                const bool search = !(level == 0 && P.distance == 0);
                 if (!started) {
                     if (search) {
                         const long long cf = __shfl_sync(kFull, cost, kField), cp = __shfl_sync(kFull, cost, kPrev);
-                        const bool prev = __shfl_sync(kFull, act, kPrev);
-                        const int pmx = __shfl_sync(kFull, mx, kPrev), pmy = __shfl_sync(kFull, my, kPrev);
-                        if (prev && (!field_valid || cp < cf)) { ppx = pmx; ppy = pmy; }
-                        lambda = adapt_lambda(L.lambda_base, L.lsad, pred_score);
-                        radius = L.base_radius;
+                        if (((actm >> kPrev) & 1u) && (!((actm >> kField) & 1u) || cp < cf)) { q.ppx = s.lmx[wi][kPrev]; q.ppy = s.lmy[wi][kPrev]; }
+                        q.lambda = adapt_lambda(L.lambda_base, L.lsad, pred_score);
+                        int radius = L.base_radius;
                         if (level > 0 && P.coarse_distance < 0)
-                            radius = adaptive_radius(radius, block_activity(x.P, x.L, x.S.y, b.px2, b.py2, px, py));
-                        stype = (edge && level == 1) ? 0 : L.search_type;
+                            radius = adaptive_radius(radius, block_activity(x.P, x.L, x.S.y, b.px2, b.py2, b.px, b.py));
+                        q.radius = radius;
+                        q.stype = (edge && level == 1) ? 0 : L.search_type;
+                    } else {
+                        openm = 0;  // no seed takes part
                     }
-                    if (!search) open = false;  // no seed takes part
-                    n_def += __any_sync(kFull, open);
+                    n_def += openm != 0;
                 }
                 if (!started || nx != selx || ny != sely) {  // the refinement, from this vector
                     reran = started;
                     selx = nx; sely = ny;
                     q.bmx = nx; q.bmy = ny; q.bsad = nsad; q.bcost = (long long)nsad;
-                    q.begin(search ? RS_REFINE_ONLY : RS_NONE, stype, radius, ppx, ppy);
+                    search_begin(q, search ? RS_REFINE_ONLY : RS_NONE);
                     stepping = false;
                     published = false;
                 }
@@ -1871,15 +1898,16 @@ __device__ __forceinline__ void walk_level(const Ctx &x, SH &s, const DirScratch
             } else {
                 const long long K = motion + pen(x.pnew, l) + (b.chroma ? pen(x.pnew, c) : 0LL);  // :1158-1221
                 const unsigned sad = sat_add(l, c);
+                long long best = q.bcost;
                 if (x.pnew < -256) {  // exact sequential semantics for penalties that can be negative
                     for (unsigned m = __ballot_sync(kFull, eval); m; m &= m - 1) {
                         const int j = __ffs(m) - 1;
                         const long long mj = __shfl_sync(kFull, motion, j), kj = __shfl_sync(kFull, K, j);
                         const unsigned sj = __shfl_sync(kFull, sad, j);
-                        if (mj < q.bcost && kj < q.bcost) { q.bcost = kj; q.bsad = sj; win = base + j; }
+                        if (mj < best && kj < best) { best = kj; q.bcost = kj; q.bsad = sj; win = base + j; }
                     }
                 } else {
-                    const int j = first_min(eval && K < q.bcost, K, lane);
+                    const int j = first_min(eval && K < best, K, lane);
                     if (j >= 0) {
                         q.bcost = __shfl_sync(kFull, K, j);
                         q.bsad = __shfl_sync(kFull, sad, j);
@@ -1887,26 +1915,30 @@ __device__ __forceinline__ void walk_level(const Ctx &x, SH &s, const DirScratch
                     }
                 }
                 base += 32;
-                if (base >= g_.n) { q.took(g_, win); stepping = false; }
+                if (base >= g_.n) { search_took(q, g_, win); stepping = false; }
             }
-            if (look && (int)(news >> 32) == TAG_FINAL) {  // a seed has become final
-                const int2 m = vmv(make_uint2((unsigned)news, 0));
-                fresh = !act || m.x != mx || m.y != my;
-                mx = m.x; my = m.y;
-                act = true;
-                open = false;
+            if (lookm) {  // seeds that have become final
+                const bool fin = (int)(news >> 32) == TAG_FINAL;
+                const unsigned finm = __ballot_sync(kFull, fin);
+                if (finm) {
+                    const int2 m = vmv(make_uint2((unsigned)news, 0));
+                    const bool fresh = fin && (!((actm >> lane) & 1u) || m.x != s.lmx[wi][lane] || m.y != s.lmy[wi][lane]);
+                    freshm = __ballot_sync(kFull, fresh);
+                    if (fresh) { s.lmx[wi][lane] = m.x; s.lmy[wi][lane] = m.y; }
+                    actm |= finm;
+                    openm &= ~finm;
+                    __syncwarp();
+                }
             }
         }
         n_blk++;
         n_rerun += reran;
-        const int bmx = q.bmx, bmy = q.bmy;
-        const unsigned bsad = q.bsad;
         // ---- store (:673-679)
         if (lane == 0) {
-            const uint2 v = mkvec(bmx, bmy, smallest ? sat_mul(bsad, 3) : bsad);
-            st_tag(ds.keys + idx, tag_word(TAG_FINAL, bmx, bmy));
+            const unsigned bsad = q.bsad;
+            const uint2 v = mkvec(q.bmx, q.bmy, smallest ? sat_mul(bsad, 3) : bsad);
+            st_tag(ds.keys + idx, tag_word(TAG_FINAL, q.bmx, q.bmy));
             field[idx] = v;
-            lumaf[idx] = block_mean(b, L, dcsum);
         }
         __syncwarp();
     }
@@ -2030,7 +2062,8 @@ __device__ __forceinline__ void refine_block(Ctx &x, SH &s, DirScratch &ds, int 
         set_groups(x);
     }
     x.pnew = P.pnew / factor;
-    BlkC b;
+    BlkC &b = s.blk[x.wbase];
+    Search &q = s.q[x.wbase];
     make_blk(x, epx, epy, true, b);
     // exact_clip (:1269-1273) of the interpolated vector into mv_bounds
     const int pmx = iclamp(mvx, b.bnd0, imax(b.bnd2 - 1, b.bnd0)), pmy = iclamp(mvy, b.bnd1, imax(b.bnd3 - 1, b.bnd1));
@@ -2042,20 +2075,22 @@ __device__ __forceinline__ void refine_block(Ctx &x, SH &s, DirScratch &ds, int 
     if (!b.fast_src) {
         dcsum = eval_slow(x, b.px, b.py, 0, 0, SLOW_DC).x;
     }
-    Search q;
     q.bmx = pmx; q.bmy = pmy;
     q.bsad = parent < 0 ? 0u : (parent > 0xFFFFFFFFLL ? 0xFFFFFFFFu : (unsigned)parent);
     q.bcost = parent < 0 ? 0 : parent;
     if (search) {
         unsigned l, c;
         eval_cands(x, b, (x.tid & 31) == 0, pmx, pmy, l, c);
-        q.bsad = __shfl_sync(kFull, sat_add(l, c), 0);  // exact_sad at the clipped predictor
-        q.bcost = (long long)q.bsad;
+        const unsigned sad = __shfl_sync(kFull, sat_add(l, c), 0);  // exact_sad at the clipped predictor
+        q.bsad = sad;
+        q.bcost = (long long)sad;
     }
     const int lambda = by == 0 ? 0 : (P.lambda >> 2) / factor;
     int bad = 0;
-    q.begin(search ? RS_ALL : RS_NONE, P.refine_search_type, abs(P.refine_distance), pmx, pmy);
-    run_search(x, b, s, ph, q, lambda, pmx, pmy, 0, bad);
+    q.stype = P.refine_search_type; q.radius = abs(P.refine_distance); q.lambda = lambda;
+    q.ppx = q.own_x = pmx; q.ppy = q.own_y = pmy;
+    search_begin(q, search ? RS_ALL : RS_NONE);
+    run_search(x, b, s, ph, q, 0, bad);
     if ((x.tid & 31) == 0) {
         ds.vec[1][(int64_t)by * gw + bx] = mkvec(q.bmx, q.bmy, sat_mul(q.bsad, (unsigned)factor));
         ds.luma[1][(int64_t)by * gw + bx] = block_mean(b, L, dcsum);
@@ -2517,8 +2552,14 @@ __global__ void __launch_bounds__(2 * NT, SVPF_MINB)
 // One level spread over the GPU: a CTA per warp, D of them per search direction of the pairs first ..
 // of the launch. The warps of a direction wait on one another, so the launch is cooperative: all its
 // CTAs are resident at once, or it does not start.
-constexpr int kWalkPerSM = 16;  // CTAs per SM: 128 registers per thread
-__global__ void __launch_bounds__(32, kWalkPerSM)
+// PER_SM: CTAs per SM the registers are cut for, 16 (128 per thread) or 20 (96; more spills, but a quarter
+// more warps). Few pairs leave the chain of blocks as the bound, where the first is faster (one 1080p pair
+// 35.7 against 37.9 ms, 16 frames 640x360 10-bit 190 against 212), many pairs the latency of the loads, which
+// more warps hide (240 frames 1080p 786 against 742 ms; 24 CTAs, 80 registers: 762): the line is where the
+// first could give a direction kDenseWalkers warps.
+constexpr int kWalkPerSM = 16, kDensePerSM = 20, kDenseWalkers = 8;
+template <int PER_SM>
+__global__ void __launch_bounds__(32, PER_SM)
     analyse_walk_kernel(const __grid_constant__ AnalyseParams P, const PairSrc psrc, int64_t first, int level, int D,
                         uint8_t *__restrict__ scratch, int *status) {
     __shared__ WarpSh s;
@@ -2659,7 +2700,10 @@ cudaError_t launch_plain(const AnalyseParams &P, const PairSrc &psrc, int npairs
     int dev = 0, sms = 0, per_sm = 0;
     if (cudaError_t e = cudaGetDevice(&dev)) return e;
     if (cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) return e;
-    if (cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, analyse_walk_kernel, 32, stage)) return e;
+    if (cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, analyse_walk_kernel<kWalkPerSM>, 32, stage)) return e;
+    const bool dense = (int64_t)sms * per_sm < (int64_t)npairs * ndir * kDenseWalkers;
+    if (dense)
+        if (cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, analyse_walk_kernel<kDensePerSM>, 32, stage)) return e;
     const int64_t resident = (int64_t)sms * per_sm;
     constexpr int kMinWalkers = 4;
     const int64_t most = resident / (ndir * kMinWalkers);
@@ -2685,7 +2729,9 @@ cudaError_t launch_plain(const AnalyseParams &P, const PairSrc &psrc, int npairs
             attr[0].val.cooperative = 1;
             cfg.attrs = attr;
             cfg.numAttrs = 1;
-            if (cudaError_t e = cudaLaunchKernelEx(&cfg, analyse_walk_kernel, P, psrc, f, lo, (int)D, scratch, status_dev)) return e;
+            if (cudaError_t e = cudaLaunchKernelEx(&cfg, dense ? analyse_walk_kernel<kDensePerSM> : analyse_walk_kernel<kWalkPerSM>, P,
+                                                   psrc, f, lo, (int)D, scratch, status_dev))
+                return e;
             if (launches) *launches += 1;
         }
     }
