@@ -2558,20 +2558,15 @@ __global__ void __launch_bounds__(2 * NT, SVPF_MINB)
 // more warps hide (240 frames 1080p 786 against 742 ms; 24 CTAs, 80 registers: 762): the line is where the
 // first could give a direction kDenseWalkers warps.
 constexpr int kWalkPerSM = 16, kDensePerSM = 20, kDenseWalkers = 8;
-template <int PER_SM>
-__global__ void __launch_bounds__(32, PER_SM)
-    analyse_walk_kernel(const __grid_constant__ AnalyseParams P, const PairSrc psrc, int64_t first, int level, int D,
-                        uint8_t *__restrict__ scratch, int *status) {
+__device__ __forceinline__ void walk_cta(const AnalyseParams &P, const PairRef pr, uint8_t *scr, int dir, int g, int D, int level,
+                                         int groups, int *status, unsigned long long *stats) {
     __shared__ WarpSh s;
     extern __shared__ __align__(16) unsigned char stage[];
     const int ndir = P.vectors == 3 ? 2 : 1;
-    const int64_t pair = first + blockIdx.x / (ndir * D);
-    const int rem = (int)(blockIdx.x % (ndir * D)), g = rem % D;
-    const int d = ndir == 2 ? rem / D : ((P.vectors & 2) ? 0 : 1);
-    uint8_t *scr = scratch + pair * P.scratch_per_pair;
+    if (dir >= ndir) return;
+    const int d = ndir == 2 ? dir : ((P.vectors & 2) ? 0 : 1);
     int *ctl = (int *)(scr + P.off_ctl[d]);
     if (!ctl[CTL_GO]) return;  // the pair kernel searched the level itself, or the direction stopped
-    const PairRef pr = pair_at(psrc, pair);
     const DirScratch ds = dir_scratch(P, scr, d);
     Ctx x;
     x.P = &P;
@@ -2580,11 +2575,21 @@ __global__ void __launch_bounds__(32, PER_SM)
     x.nw = 1;
     x.wbase = 0;
     set_frames(x, P, (const px_t *)(d == 0 ? pr.cur : pr.ref), (const px_t *)(d == 0 ? pr.ref : pr.cur));
-    set_stage(x, stage, P.stage_groups, 0, 0);
+    set_stage(x, stage, groups, 0, 0);
     set_level(x, P, level);
     const int od = ndir == 2 ? 1 - d : d;
     const uint2 *prevp = ctl[CTL_PREV] ? (const uint2 *)(scr + P.off_proj[od][level & 1]) : nullptr;
-    walk_level(x, s, ds, prevp, g, D, ctl[CTL_ORDER], ctl[CTL_GX], ctl[CTL_GY], ctl, status, psrc.stats);
+    walk_level(x, s, ds, prevp, g, D, ctl[CTL_ORDER], ctl[CTL_GX], ctl[CTL_GY], ctl, status, stats);
+}
+template <int PER_SM>
+__global__ void __launch_bounds__(32, PER_SM)
+    analyse_walk_kernel(const __grid_constant__ AnalyseParams P, const PairSrc psrc, int64_t first, int level, int D,
+                        uint8_t *__restrict__ scratch, int *status) {
+    const int ndir = P.vectors == 3 ? 2 : 1;
+    const int64_t pair = first + blockIdx.x / (ndir * D);
+    const int rem = (int)(blockIdx.x % (ndir * D));
+    walk_cta(P, pair_at(psrc, pair), scratch + pair * P.scratch_per_pair, rem / D, rem % D, D, level, P.stage_groups, status,
+             psrc.stats);
 }
 
 // Neither direction of a pair stopped.
@@ -2596,25 +2601,29 @@ __device__ __forceinline__ bool pair_whole(const AnalyseParams &P, const uint8_t
 
 // The refine pass of a split launch: its blocks are independent, so they go to `per_dir` one-warp
 // CTAs per direction, every per_dir-th block to each.
-__global__ void __launch_bounds__(32, kWalkPerSM)
-    analyse_refine_kernel(const __grid_constant__ AnalyseParams P, const PairSrc psrc, int per_dir, uint8_t *__restrict__ scratch) {
+__device__ __forceinline__ void refine_cta(const AnalyseParams &P, const PairRef pr, uint8_t *scr, int dir, int g, int per_dir,
+                                           int groups) {
     __shared__ WarpSh s;
     extern __shared__ __align__(16) unsigned char stage[];
     const int ndir = P.vectors == 3 ? 2 : 1;
-    const int64_t pair = blockIdx.x / (ndir * per_dir);
-    const int rem = (int)(blockIdx.x % (ndir * per_dir));
-    const int d = ndir == 2 ? rem / per_dir : ((P.vectors & 2) ? 0 : 1);
-    uint8_t *scr = scratch + pair * P.scratch_per_pair;
-    if (!pair_whole(P, scr)) return;
+    if (dir >= ndir || !pair_whole(P, scr)) return;
+    const int d = ndir == 2 ? dir : ((P.vectors & 2) ? 0 : 1);
     DirScratch ds = dir_scratch(P, scr, d);
     Ctx x;
-    refine_ctx(x, P, pair_at(psrc, pair), d);
+    refine_ctx(x, P, pr, d);
     x.d = 0;
     x.wbase = 0;
-    set_stage(x, stage, P.stage_groups, 0, 0);
+    set_stage(x, stage, groups, 0, 0);
     int shape = -1;
     const int n = P.out_gw * P.out_gh;
-    for (int i = rem % per_dir; i < n; i += per_dir) refine_block(x, s, ds, i % P.out_gw, i / P.out_gw, shape);
+    for (int i = g; i < n; i += per_dir) refine_block(x, s, ds, i % P.out_gw, i / P.out_gw, shape);
+}
+__global__ void __launch_bounds__(32, kWalkPerSM)
+    analyse_refine_kernel(const __grid_constant__ AnalyseParams P, const PairSrc psrc, int per_dir, uint8_t *__restrict__ scratch) {
+    const int ndir = P.vectors == 3 ? 2 : 1;
+    const int64_t pair = blockIdx.x / (ndir * per_dir);
+    const int rem = (int)(blockIdx.x % (ndir * per_dir));
+    refine_cta(P, pair_at(psrc, pair), scratch + pair * P.scratch_per_pair, rem / per_dir, rem % per_dir, per_dir, P.stage_groups);
 }
 
 // The payloads of a split launch: kPackThreads cells of one direction per CTA.
@@ -2629,6 +2638,9 @@ __global__ void __launch_bounds__(kPackThreads)
     const int64_t i = (int64_t)blockIdx.x * kPackThreads + threadIdx.x;
     pack_cells(P, ds, d, payloads + pair * P.payload_len, i, (int64_t)gridDim.x * kPackThreads, i == 0);
 }
+
+// Levels of fewer blocks than this are searched by the pair's CTA, without a launch of their own.
+constexpr int kWalkCells = 160;
 
 // Persistent form: a grid sized to the resident CTAs drains the item list in order (the
 // host sorts it largest-first); each CTA pulls the next item with one atomic, copies the
@@ -2660,6 +2672,68 @@ __global__ void __launch_bounds__(2 * NT, SVPF_MINB)
     }
 }
 
+// The coarsest level of P that a walk takes; the levels above it are the pair kernel's.
+__host__ __device__ inline int first_walk(const AnalyseParams &P) {
+    int lo = P.nlevels - 1;
+    while (lo > 0 && P.lv[lo].gw * P.lv[lo].gh < kWalkCells) lo--;
+    return lo;
+}
+
+#if SVPF_LOOKAHEAD && !defined(SVPF_PX16)
+// The batch form of the split launch: every item of a group of items (one scratch slot each) goes level
+// by level, the clips' finest levels aligned: `lo` is the level of this round, and an item whose clip has
+// its first walk at a finer level waits. Between two walks:
+__global__ void __launch_bounds__(2 * NT, SVPF_MINB)
+    batch_ground_kernel(const AnalyseParams *__restrict__ clips, const BatchItem *__restrict__ items, int lo,
+                        uint8_t *__restrict__ scratch, int64_t scratch_per_slot, int *__restrict__ clip_status, int groups) {
+    __shared__ int cta_abort;
+    __shared__ __align__(16) AnalyseParams P;
+    const BatchItem bi = items[blockIdx.x];
+    {
+        const int4 *src = reinterpret_cast<const int4 *>(clips + bi.clip);
+        int4 *dst = reinterpret_cast<int4 *>(&P);
+        for (int i = threadIdx.x; i < (int)(sizeof(AnalyseParams) / 16); i += blockDim.x) dst[i] = src[i];
+    }
+    __syncthreads();
+    const int start = first_walk(P);
+    if (lo > start) return;
+    analyse_pair_dev(P, bi.pair, bi.payload, scratch + (int64_t)blockIdx.x * scratch_per_slot, clip_status + bi.clip, cta_abort,
+                     nullptr, true, lo == start ? P.nlevels - 1 : lo, lo, groups);
+}
+// The walks of a round: 2 D one-warp CTAs per item (see analyse_walk_kernel).
+template <int PER_SM>
+__global__ void __launch_bounds__(32, PER_SM)
+    batch_walk_kernel(const AnalyseParams *__restrict__ clips, const BatchItem *__restrict__ items, int lo, int D,
+                      uint8_t *__restrict__ scratch, int64_t scratch_per_slot, int *__restrict__ clip_status, int groups) {
+    const int slot = blockIdx.x / (2 * D), rem = blockIdx.x % (2 * D);
+    const BatchItem bi = items[slot];
+    const AnalyseParams &P = clips[bi.clip];
+    if (lo > first_walk(P)) return;
+    walk_cta(P, bi.pair, scratch + (int64_t)slot * scratch_per_slot, rem / D, rem % D, D, lo, groups, clip_status + bi.clip, nullptr);
+}
+__global__ void __launch_bounds__(32, kWalkPerSM)
+    batch_refine_kernel(const AnalyseParams *__restrict__ clips, const BatchItem *__restrict__ items, int per_dir,
+                        uint8_t *__restrict__ scratch, int64_t scratch_per_slot, int groups) {
+    const int slot = blockIdx.x / (2 * per_dir), rem = blockIdx.x % (2 * per_dir);
+    const BatchItem bi = items[slot];
+    const AnalyseParams &P = clips[bi.clip];
+    if (P.has_refine) refine_cta(P, bi.pair, scratch + (int64_t)slot * scratch_per_slot, rem / per_dir, rem % per_dir, per_dir, groups);
+}
+__global__ void __launch_bounds__(kPackThreads)
+    batch_pack_kernel(const AnalyseParams *__restrict__ clips, const BatchItem *__restrict__ items, uint8_t *__restrict__ scratch,
+                      int64_t scratch_per_slot) {
+    const int slot = blockIdx.y;
+    const BatchItem bi = items[slot];
+    const AnalyseParams &P = clips[bi.clip];
+    if ((int)blockIdx.z >= (P.vectors == 3 ? 2 : 1)) return;
+    const int d = P.vectors == 3 ? (int)blockIdx.z : ((P.vectors & 2) ? 0 : 1);
+    uint8_t *scr = scratch + (int64_t)slot * scratch_per_slot;
+    if (!pair_whole(P, scr)) return;
+    const int64_t i = (int64_t)blockIdx.x * kPackThreads + threadIdx.x;
+    pack_cells(P, dir_scratch(P, scr, d), d, bi.payload, i, (int64_t)gridDim.x * kPackThreads, i == 0);
+}
+#endif
+
 }  // namespace
 
 // Dynamic shared memory of a pair CTA of `ndir` directions.
@@ -2678,8 +2752,43 @@ cudaError_t prepare() {
     return once;
 }
 
-// Levels of fewer blocks than this are searched by the pair's CTA, without a launch of their own.
-constexpr int kWalkCells = 160;
+namespace {
+constexpr int kMinWalkers = 4;  // warps per direction of a walk, at least
+// The build and the resident CTAs of a walk over `ndirs` search directions.
+struct WalkShape {
+    bool dense;
+    size_t smem;
+    int64_t resident;
+};
+cudaError_t walk_shape(int groups, int64_t ndirs, WalkShape &w) {
+    w.smem = (size_t)groups * kGroupBytes;
+    int dev = 0, sms = 0, per_sm = 0;
+    if (cudaError_t e = cudaGetDevice(&dev)) return e;
+    if (cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) return e;
+    if (cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, analyse_walk_kernel<kWalkPerSM>, 32, w.smem)) return e;
+    w.dense = (int64_t)sms * per_sm < ndirs * kDenseWalkers;
+    if (w.dense)
+        if (cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, analyse_walk_kernel<kDensePerSM>, 32, w.smem)) return e;
+    w.resident = (int64_t)sms * per_sm;
+    return cudaSuccess;
+}
+// The CTAs of a walk wait on one another, so the launch is cooperative and takes the directions whose
+// CTAs are all resident at once.
+template <class... P, class... A>
+cudaError_t launch_walk(void (*kernel)(P...), int64_t ctas, size_t smem, cudaStream_t stream, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)ctas);
+    cfg.blockDim = dim3(32);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+}  // namespace
 
 cudaError_t launch_plain(const AnalyseParams &P, const PairSrc &psrc, int npairs, uint8_t *payloads, uint8_t *scratch,
                          int *status_dev, cudaStream_t stream, int *launches) {
@@ -2693,44 +2802,26 @@ cudaError_t launch_plain(const AnalyseParams &P, const PairSrc &psrc, int npairs
         analyse_kernel<<<npairs, NT * ndir, pair_smem, stream>>>(P, psrc, payloads, scratch, status_dev, 0, P.nlevels - 1, 0);
         return count();
     }
-    // The CTAs of a walk wait on one another, so a launch takes the pairs whose CTAs are all resident at
-    // once: D warps per direction, as many as fit (at least kMinWalkers, with the pairs in several
-    // launches when they would not)
-    const size_t stage = (size_t)P.stage_groups * kGroupBytes;
-    int dev = 0, sms = 0, per_sm = 0;
-    if (cudaError_t e = cudaGetDevice(&dev)) return e;
-    if (cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) return e;
-    if (cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, analyse_walk_kernel<kWalkPerSM>, 32, stage)) return e;
-    const bool dense = (int64_t)sms * per_sm < (int64_t)npairs * ndir * kDenseWalkers;
-    if (dense)
-        if (cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, analyse_walk_kernel<kDensePerSM>, 32, stage)) return e;
-    const int64_t resident = (int64_t)sms * per_sm;
-    constexpr int kMinWalkers = 4;
+    // D warps per direction, as many as are resident at once (at least kMinWalkers, with the pairs in
+    // several launches when they would not be)
+    WalkShape w;
+    if (cudaError_t e = walk_shape(P.stage_groups, (int64_t)npairs * ndir, w)) return e;
+    const size_t stage = w.smem;
+    const int64_t resident = w.resident;
     const int64_t most = resident / (ndir * kMinWalkers);
     if (most < 1) return cudaErrorCooperativeLaunchTooLarge;
     const int64_t walks = (npairs + most - 1) / most;
     const int64_t group = (npairs + walks - 1) / walks;  // even groups
     int64_t D = resident / (ndir * group);
     D = D < kMinWalkers ? kMinWalkers : D > kMaxWalkers ? kMaxWalkers : D;
-    int hi = P.nlevels - 1, lo = hi;
-    while (lo > 0 && P.lv[lo].gw * P.lv[lo].gh < kWalkCells) lo--;
+    int hi = P.nlevels - 1, lo = first_walk(P);
     for (; lo >= 0; hi = lo - 1, lo = hi) {
         analyse_kernel<<<npairs, NT * ndir, pair_smem, stream>>>(P, psrc, payloads, scratch, status_dev, 1, hi, lo);
         if (cudaError_t e = count()) return e;
         for (int64_t f = 0; f < npairs; f += group) {
             const int64_t n = npairs - f < group ? npairs - f : group;
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3((unsigned)(n * ndir * D));
-            cfg.blockDim = dim3(32);
-            cfg.dynamicSmemBytes = stage;
-            cfg.stream = stream;
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeCooperative;
-            attr[0].val.cooperative = 1;
-            cfg.attrs = attr;
-            cfg.numAttrs = 1;
-            if (cudaError_t e = cudaLaunchKernelEx(&cfg, dense ? analyse_walk_kernel<kDensePerSM> : analyse_walk_kernel<kWalkPerSM>, P,
-                                                   psrc, f, lo, (int)D, scratch, status_dev))
+            if (cudaError_t e = launch_walk(w.dense ? analyse_walk_kernel<kDensePerSM> : analyse_walk_kernel<kWalkPerSM>,
+                                            n * ndir * D, stage, stream, P, psrc, f, lo, (int)D, scratch, status_dev))
                 return e;
             if (launches) *launches += 1;
         }
@@ -2751,22 +2842,79 @@ cudaError_t launch_plain(const AnalyseParams &P, const PairSrc &psrc, int npairs
     return cudaSuccess;
 }
 
-cudaError_t batch_blocks_per_sm(int groups, int *blocks) {
+cudaError_t batch_blocks_per_sm(const BatchInfo &info, int *blocks) {
     if (cudaError_t e = prepare()) return e;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, analyse_batch_kernel, 2 * NT, pair_shared(2, groups));
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, analyse_batch_kernel, 2 * NT, pair_shared(2, info.groups));
 }
 
 cudaError_t launch_batch(const AnalyseParams *clips_dev, const BatchItem *items_dev, int nitems, unsigned *next_item_dev,
-                         uint8_t *scratch, int64_t scratch_per_cta, int *clip_status_dev, int groups, int grid,
+                         uint8_t *scratch, int64_t scratch_per_cta, int *clip_status_dev, const BatchInfo &info, int grid,
                          cudaStream_t stream, int *launches) {
     if (nitems <= 0 || grid <= 0) return cudaSuccess;
     if (cudaError_t e = prepare()) return e;
-    analyse_batch_kernel<<<grid, 2 * NT, pair_shared(2, groups), stream>>>(clips_dev, items_dev, nitems, next_item_dev,
-                                                                           scratch, scratch_per_cta, clip_status_dev,
-                                                                           groups);
+    analyse_batch_kernel<<<grid, 2 * NT, pair_shared(2, info.groups), stream>>>(clips_dev, items_dev, nitems, next_item_dev,
+                                                                                scratch, scratch_per_cta, clip_status_dev,
+                                                                                info.groups);
     if (launches) *launches += 1;
     return cudaGetLastError();
 }
+
+#if SVPF_LOOKAHEAD && !defined(SVPF_PX16)
+// The batch walked level by level (batch_ground_kernel): `grid` pairs at a time.
+int first_walk_level(const AnalyseParams &P) { return first_walk(P); }
+
+// Pairs of a group per SM: enough to fill the SMs with at least kMinWalkers warps per direction.
+cudaError_t batch_walk_pairs_per_sm(const BatchInfo &info, int *pairs) {
+    WalkShape w;
+    if (cudaError_t e = prepare()) return e;
+    if (cudaError_t e = walk_shape(info.groups, (int64_t)1 << 30, w)) return e;
+    int dev = 0, sms = 0;
+    if (cudaError_t e = cudaGetDevice(&dev)) return e;
+    if (cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) return e;
+    *pairs = (int)(w.resident / sms / (2 * kMinWalkers));
+    return cudaSuccess;
+}
+
+cudaError_t launch_batch_walk(const AnalyseParams *clips_dev, const BatchItem *items_dev, int nitems, unsigned *,
+                              uint8_t *scratch, int64_t scratch_per_slot, int *clip_status_dev, const BatchInfo &info,
+                              int grid, cudaStream_t stream, int *launches) {
+    if (nitems <= 0 || grid <= 0) return cudaSuccess;
+    if (cudaError_t e = prepare()) return e;
+    static const cudaError_t ground = cudaFuncSetAttribute(batch_ground_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                           (int)pair_shared(2, kMaxStageGroups));
+    if (ground != cudaSuccess) return ground;
+    auto count = [&] { if (launches) *launches += 1; return cudaGetLastError(); };
+    const int ngroups = (nitems + grid - 1) / grid, group = (nitems + ngroups - 1) / ngroups;  // even groups
+    WalkShape w;
+    if (cudaError_t e = walk_shape(info.groups, (int64_t)group * 2, w)) return e;
+    int64_t D = w.resident / (group * 2);
+    if (D < 1) return cudaErrorCooperativeLaunchTooLarge;
+    if (D > kMaxWalkers) D = kMaxWalkers;
+    for (int f = 0; f < nitems; f += group) {
+        const int n = nitems - f < group ? nitems - f : group;
+        const BatchItem *it = items_dev + f;
+        for (int lo = info.rounds - 1; lo >= 0; lo--) {
+            batch_ground_kernel<<<n, 2 * NT, pair_shared(2, info.groups), stream>>>(clips_dev, it, lo, scratch, scratch_per_slot,
+                                                                                    clip_status_dev, info.groups);
+            if (cudaError_t e = count()) return e;
+            if (cudaError_t e = launch_walk(w.dense ? batch_walk_kernel<kDensePerSM> : batch_walk_kernel<kWalkPerSM>, n * 2 * D,
+                                            w.smem, stream, clips_dev, it, lo, (int)D, scratch, scratch_per_slot,
+                                            clip_status_dev, info.groups))
+                return e;
+            if (launches) *launches += 1;
+        }
+        if (info.refine) {
+            const int per_dir = (int)((2 * w.resident + 2 * n - 1) / (2 * n));
+            batch_refine_kernel<<<n * 2 * per_dir, 32, w.smem, stream>>>(clips_dev, it, per_dir, scratch, scratch_per_slot, info.groups);
+            if (cudaError_t e = count()) return e;
+        }
+        batch_pack_kernel<<<dim3((info.cells + kPackThreads - 1) / kPackThreads, n, 2), kPackThreads, 0, stream>>>(
+            clips_dev, it, scratch, scratch_per_slot);
+        if (cudaError_t e = count()) return e;
+    }
+    return cudaSuccess;
+}
+#endif
 
 }  // namespace SVPF_VARIANT
 }  // namespace svpf

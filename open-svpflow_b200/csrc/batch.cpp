@@ -4,16 +4,19 @@
 // The reference analyses one clip at a time, one output frame per getFrame call
 // (crates/svpflow1/src/analyse_filter.rs:229-334); every frame pair is independent of
 // every other (analyse_search.rs:68-92 reads only its two super frames). A batch therefore
-// flattens the frame pairs of all its clips into one item list and lets a grid of
-// resident CTAs drain it through a device-side counter (analyse_batch_kernel). The item
-// list is sorted largest-first (longest-processing-time order) so that the small pairs
-// fill the tail of the launch.
+// flattens the frame pairs of all its clips into one item list, sorted largest-first, and runs
+// it in one of two ways. The shape "walk" (the default) takes groups of items of about the same
+// size, as many as give every search direction four warps or more on the whole GPU, level by
+// level, the clips' finest levels aligned (batch_ground_kernel, batch_walk_kernel). The other
+// shapes let a grid of resident CTAs drain the list through a device-side counter, a pair per
+// CTA (analyse_batch_kernel): 12 clips of 320x240 to 854x480 take 134 ms walked and 320 ms
+// drained by the fastest of them, since a drained pair runs at one CTA's speed.
 //
 // Device memory of a batch is one allocation made at creation: every clip's source
 // frames, super frames and payloads, the per-clip parameter blocks, the item list, a
-// status word per clip and one search scratch slot per resident CTA. A run is one CUDA
+// status word per clip and one search scratch slot per item in work. A run is one CUDA
 // graph (the Super launches of every clip, the reset of the queue counter and the status
-// words, the persistent Analyse launch) captured once per launch shape and replayed.
+// words, the Analyse launches) captured once per launch shape and replayed.
 //
 // The launch shape (threads per search direction, 4x4 tiles per lane) does not change
 // any result; svpf_batch_autotune times the compiled shapes on the batch's largest items
@@ -98,9 +101,9 @@ struct svpf_batch {
     int64_t off_params = 0, off_items = 0, off_counter = 0, off_status = 0, off_scratch = 0;
     int64_t scratch_per_cta = 0;
     int max_ctas = 0;          // scratch slots allocated
-    int groups = 1;            // the most AnalyseParams::stage_groups of the clips
+    BatchInfo info;
     int sms = 0;
-    int variant = 3, tiles_per_lane = 8, grid = 0;  // nt128_b3 until tuned
+    int variant = 5, tiles_per_lane = 8, grid = 0;  // "walk" until tuned
     std::string signature;
     cudaStream_t stream = nullptr;
     cudaGraphExec_t graph = nullptr;
@@ -135,7 +138,7 @@ int upload_params(svpf_batch *b) {
 
 int grid_for(svpf_batch *b, int variant, int nitems, int *grid) {
     int per_sm = 0;
-    BCU(analyse_variant(variant).batch_blocks_per_sm(b->groups, &per_sm));
+    BCU(analyse_variant(variant).batch_blocks_per_sm(b->info, &per_sm));
     if (per_sm <= 0) return bfail(SVPF_ECUDA, "batch kernel does not fit on an SM");
     int g = per_sm * b->sms;
     if (g > b->max_ctas) g = b->max_ctas;
@@ -156,7 +159,7 @@ int record_run(svpf_batch *b, cudaStream_t st, int nitems, int grid, int *launch
     BCU(cudaMemsetAsync(b->status_dev(), 0, sizeof(int) * b->clips.size(), st));
     cudaError_t e = analyse_variant(b->variant).launch_batch(b->params_dev(), b->items_dev(), nitems, b->counter_dev(),
                                                              b->scratch_dev(), b->scratch_per_cta, b->status_dev(),
-                                                             b->groups, grid, st, &nl);
+                                                             b->info, grid, st, &nl);
     if (e != cudaSuccess) return bcuda(e, "batch analyse launch");
     *launches = nl;
     return SVPF_OK;
@@ -244,7 +247,10 @@ int svpf_batch_create(int32_t nclips, const svpf_super *const *supers, const svp
         c.supers_off = off; off += al256(c.super_frame_bytes * c.nframes);
         c.payloads_off = off; off += al256(c.P.payload_len * c.nframes);
         max_scratch = std::max(max_scratch, al256(c.P.scratch_per_pair));
-        b->groups = std::max(b->groups, (int)c.P.stage_groups);
+        b->info.groups = std::max(b->info.groups, (int)c.P.stage_groups);
+        b->info.rounds = std::max(b->info.rounds, nt128::first_walk_level(c.P) + 1);
+        b->info.cells = std::max(b->info.cells, c.P.out_gw * c.P.out_gh);
+        b->info.refine = b->info.refine || c.P.has_refine;
         b->clips.push_back(c);
         snprintf(sig, sizeof(sig), "%dx%d/b%d/v%d/l%d", c.P.luma_w, c.P.luma_h, c.P.block_w, c.P.vectors, c.P.nlevels);
         mix[sig]++;
@@ -284,7 +290,7 @@ int svpf_batch_create(int32_t nclips, const svpf_super *const *supers, const svp
     int most = 0;
     for (int v = 0; v < analyse_variant_count(); v++) {
         int per_sm = 0;
-        if (analyse_variant(v).batch_blocks_per_sm(b->groups, &per_sm) != cudaSuccess) {
+        if (analyse_variant(v).batch_blocks_per_sm(b->info, &per_sm) != cudaSuccess) {
             delete b;
             return bfail(SVPF_ECUDA, "occupancy query failed");
         }
@@ -420,7 +426,7 @@ int svpf_batch_autotune(svpf_batch *b, int32_t *variant, int32_t *tiles_per_lane
         BCU(cudaEventRecord(e0, b->stream));
         cudaError_t e = analyse_variant(v).launch_batch(b->params_dev(), b->items_dev(), n, b->counter_dev(),
                                                         b->scratch_dev(), b->scratch_per_cta, b->status_dev(),
-                                                        b->groups, grid, b->stream, &nl);
+                                                        b->info, grid, b->stream, &nl);
         if (e != cudaSuccess) return bcuda(e, "batch analyse launch");
         BCU(cudaEventRecord(e1, b->stream));
         add_launches(nl);

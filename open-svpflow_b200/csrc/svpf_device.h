@@ -50,15 +50,24 @@ struct BatchItem {
     int32_t pad_;
 };
 
+// What a batch launch needs to know of all its clips.
+struct BatchInfo {
+    int groups = 1;     // the most AnalyseParams::stage_groups
+    int rounds = 1;     // the most levels a clip has walked (first_walk_level + 1)
+    int cells = 1;      // the most cells of an output grid
+    bool refine = false;  // a clip has the refine pass
+};
+
 // The launchers every Analyse variant TU exports (analyse_body.cuh).
 #define SVPF_DECLARE_ANALYSE_VARIANT(ns)                                                                          \
     namespace ns {                                                                                                \
     cudaError_t launch_plain(const AnalyseParams &P, const PairSrc &src, int npairs, uint8_t *payloads,           \
                              uint8_t *scratch, int *status_dev, cudaStream_t stream, int *launches);              \
-    cudaError_t batch_blocks_per_sm(int groups, int *blocks);                                                     \
+    cudaError_t batch_blocks_per_sm(const BatchInfo &info, int *blocks);                                          \
     cudaError_t launch_batch(const AnalyseParams *clips_dev, const BatchItem *items_dev, int nitems,              \
                              unsigned *next_item_dev, uint8_t *scratch, int64_t scratch_per_cta,                  \
-                             int *clip_status_dev, int groups, int grid, cudaStream_t stream, int *launches);     \
+                             int *clip_status_dev, const BatchInfo &info, int grid, cudaStream_t stream,          \
+                             int *launches);                                                                      \
     }
 SVPF_DECLARE_ANALYSE_VARIANT(nt128)
 SVPF_DECLARE_ANALYSE_VARIANT(nt64)
@@ -66,6 +75,14 @@ SVPF_DECLARE_ANALYSE_VARIANT(nt32)
 SVPF_DECLARE_ANALYSE_VARIANT(nt128b3)
 SVPF_DECLARE_ANALYSE_VARIANT(nt64b6)
 SVPF_DECLARE_ANALYSE_VARIANT(nt128p16)  // uint16 samples (AnalyseParams::px_bytes == 2)
+// The batch walked level by level over the GPU, as the plain path walks a clip's pairs.
+namespace nt128 {
+int first_walk_level(const AnalyseParams &P);
+cudaError_t batch_walk_pairs_per_sm(const BatchInfo &info, int *pairs);
+cudaError_t launch_batch_walk(const AnalyseParams *clips_dev, const BatchItem *items_dev, int nitems, unsigned *next_item_dev,
+                              uint8_t *scratch, int64_t scratch_per_slot, int *clip_status_dev, const BatchInfo &info, int grid,
+                              cudaStream_t stream, int *launches);
+}
 
 
 // A compiled launch shape of the Analyse kernels: threads per search direction and the
@@ -75,10 +92,9 @@ struct AnalyseVariant {
     int threads_per_dir, min_blocks;
     cudaError_t (*launch_plain)(const AnalyseParams &, const PairSrc &, int, uint8_t *, uint8_t *, int *,
                                 cudaStream_t, int *);
-    // groups: the most AnalyseParams::stage_groups of the batch's clips
-    cudaError_t (*batch_blocks_per_sm)(int groups, int *);
+    cudaError_t (*batch_blocks_per_sm)(const BatchInfo &, int *);
     cudaError_t (*launch_batch)(const AnalyseParams *, const BatchItem *, int, unsigned *, uint8_t *, int64_t, int *,
-                                int groups, int grid, cudaStream_t, int *);
+                                const BatchInfo &, int grid, cudaStream_t, int *);
 };
 int analyse_variant_count();
 const AnalyseVariant &analyse_variant(int i);  // 0 = the plain path's default (nt128)

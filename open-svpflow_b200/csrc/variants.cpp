@@ -10,7 +10,7 @@ const AnalyseVariant kVariants[] = {
     {"nt32_b8", 32, 8, nt32::launch_plain, nt32::batch_blocks_per_sm, nt32::launch_batch},
     {"nt128_b3", 128, 3, nt128b3::launch_plain, nt128b3::batch_blocks_per_sm, nt128b3::launch_batch},
     {"nt64_b6", 64, 6, nt64b6::launch_plain, nt64b6::batch_blocks_per_sm, nt64b6::launch_batch},
-
+    {"walk", 128, 2, nt128::launch_plain, nt128::batch_walk_pairs_per_sm, nt128::launch_batch_walk},
 };
 }  // namespace
 
