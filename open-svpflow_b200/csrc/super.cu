@@ -554,6 +554,659 @@ __global__ void __launch_bounds__(256, 4) super_level01_kernel(SuperDev D, const
     }
 }
 
+// ---- packed frames (row pitch = width for the source and the super frame, as in the portable
+// layout): any width, any alignment, both sample types. Level 0 is then one flat stream per plane
+// (its sub-planes follow one another without a gap), and the pyramid is reduced by warps that walk
+// down the rows.
+
+// Sample arithmetic in 32-bit words: 4 bytes or 2 halfwords.
+template <typename T>
+__device__ __forceinline__ uint32_t avg_word(uint32_t a, uint32_t b) {  // rounded up, per sample
+    return (a | b) - (((a ^ b) >> 1) & (sizeof(T) == 1 ? 0x7F7F7F7Fu : 0x7FFF7FFFu));
+}
+// Loads of global memory that a kernel may itself have written: through L1 where its own CTA wrote it
+// (before a barrier), from L2 (CG) where another SM did.
+template <bool CG>
+__device__ __forceinline__ uint32_t ld_word(const void *p) {
+    uint32_t v;
+    if (CG) asm volatile("ld.global.cg.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    else asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+// `N` words from byte address p on, whatever its alignment; reads whole 4-byte words that hold a byte of it.
+template <int N, bool CG>
+__device__ __forceinline__ void load_words(const uint8_t *p, uint32_t (&w)[N]) {
+    const uintptr_t a = (uintptr_t)p;
+    const uint32_t *q = reinterpret_cast<const uint32_t *>(a & ~(uintptr_t)3);
+    const unsigned sh = (unsigned)(a & 3) * 8u;
+    if (sh == 0) {
+#pragma unroll
+        for (int i = 0; i < N; i++) w[i] = ld_word<CG>(q + i);
+    } else {
+        uint32_t v[N + 1];
+#pragma unroll
+        for (int i = 0; i <= N; i++) v[i] = ld_word<CG>(q + i);
+#pragma unroll
+        for (int i = 0; i < N; i++) w[i] = __funnelshift_r(v[i], v[i + 1], sh);
+    }
+}
+// 16 bytes at p and the sample after them (in nxt's low bits)
+__device__ __forceinline__ uint4 load_chunk(const uint8_t *p, uint32_t &nxt) {
+    const uintptr_t a = (uintptr_t)p;
+    if ((a & 15) == 0) {
+        const uint4 v = __ldg(reinterpret_cast<const uint4 *>(p));
+        nxt = __ldg(reinterpret_cast<const uint32_t *>(p + 16));
+        return v;
+    }
+    const uint32_t *q = reinterpret_cast<const uint32_t *>(a & ~(uintptr_t)3);
+    const unsigned sh = (unsigned)(a & 3) * 8u;
+    uint32_t w[6];
+#pragma unroll
+    for (int i = 0; i < 5; i++) w[i] = __ldg(q + i);
+    w[5] = sh ? __ldg(q + 5) : 0u;
+    nxt = __funnelshift_r(w[4], w[5], sh);
+    return make_uint4(__funnelshift_r(w[0], w[1], sh), __funnelshift_r(w[1], w[2], sh), __funnelshift_r(w[2], w[3], sh),
+                      __funnelshift_r(w[3], w[4], sh));
+}
+template <typename T>
+__device__ __forceinline__ uint4 avg_chunk(uint4 a, uint4 b) {
+    return make_uint4(avg_word<T>(a.x, b.x), avg_word<T>(a.y, b.y), avg_word<T>(a.z, b.z), avg_word<T>(a.w, b.w));
+}
+template <typename T>
+__device__ __forceinline__ uint4 next_chunk(uint4 a, uint32_t nxt) {  // one sample further on
+    constexpr int sh = 8 * (int)sizeof(T);
+    return make_uint4(__funnelshift_r(a.x, a.y, sh), __funnelshift_r(a.y, a.z, sh), __funnelshift_r(a.z, a.w, sh),
+                      __funnelshift_r(a.w, nxt, sh));
+}
+
+struct FlatPlane {
+    const uint8_t *src;  // the frame's plane
+    uint8_t *out;        // its level-0 region
+    uint32_t S, hs;      // row length and plane size, in samples
+};
+// Sub-plane p of the level-0 region at offset o (fill_bilinear_pel2, super_build.rs:179-224, in closed
+// form): the copied plane, of which reads go on into the h plane behind it.
+template <typename T>
+__device__ __forceinline__ unsigned flat_sample(const FlatPlane &P, uint32_t o) {
+    const T *s = reinterpret_cast<const T *>(P.src);
+    if (o < P.hs) return s[o];
+    const uint32_t c = o - P.hs;
+    return avg8(s[c], c + 1 < P.hs ? s[c + 1] : avg8(s[0], s[1]));
+}
+template <typename T>
+__device__ __forceinline__ unsigned flat_value(const FlatPlane P, bool subpel, uint32_t p, uint32_t o) {
+    const unsigned v = flat_sample<T>(P, o);
+    if (p == 0) return v;
+    if (!subpel || p > 3) return 0;
+    if (p == 1) return avg8(v, flat_sample<T>(P, o + 1));
+    if (o < P.S) return p == 2 ? v : flat_sample<T>(P, o + 1);  // the v and hv planes' first rows are copies
+    return avg8(v, flat_sample<T>(P, o + P.S + (p == 3 ? 1 : 0)));
+}
+// The aligned 16 bytes of the level-0 region that hold its byte position `at` (a multiple of 16 from
+// the region's start rounded down). The chunks inside one sub-plane and away from the plane's first and
+// last rows go in words; the source is read at whatever alignment its rows have. read_end: bytes of the
+// source plane that may be read (whole words included).
+template <typename T>
+__device__ __forceinline__ void flat_chunk(const FlatPlane &P, bool subpel, uint32_t nsub, int64_t at, int64_t region,
+                                           const uint8_t *read_end) {
+    constexpr uint32_t n = 16 / sizeof(T);
+    const uint32_t S = P.S, hs = P.hs;
+    if (at >= 0 && at + 16 <= region && (at & (int64_t)(sizeof(T) - 1)) == 0) {
+        const uint32_t i = (uint32_t)(at / (int64_t)sizeof(T)), p = i / hs, o = i - p * hs;
+        if (o + n <= hs) {
+            uint4 *out = reinterpret_cast<uint4 *>(P.out + at);
+            const uint8_t *s = P.src + (size_t)o * sizeof(T);
+            const uint32_t y2 = o + n + S + 1;  // past the last sample a v / hv chunk reads
+            if (p > 3 || (p > 0 && !subpel)) {
+                *out = make_uint4(0, 0, 0, 0);
+                return;
+            }
+            uint32_t nx, nb;
+            if (s + 24 <= read_end && (p == 0 || o + n < hs)) {
+                if (p < 2) {
+                    const uint4 A = load_chunk(s, nx);
+                    *out = p == 0 ? A : avg_chunk<T>(A, next_chunk<T>(A, nx));
+                    return;
+                }
+                if (o + n <= S) {
+                    const uint4 A = load_chunk(s, nx);
+                    *out = p == 2 ? A : next_chunk<T>(A, nx);
+                    return;
+                }
+                const uint8_t *t = s + (size_t)S * sizeof(T);
+                if (o >= S && y2 <= hs && t + 24 <= read_end) {
+                    const uint4 A = load_chunk(s, nx), B = load_chunk(t, nb);
+                    *out = avg_chunk<T>(A, p == 2 ? B : next_chunk<T>(B, nb));
+                    return;
+                }
+                if (o >= hs - S && o + n + S + 2 <= 2 * hs) {  // the last row: the h plane's first row stands below it
+                    const uint8_t *c = P.src + (size_t)(o - (hs - S) + (p == 3 ? 1 : 0)) * sizeof(T);
+                    const uint4 A = load_chunk(s, nx), C = load_chunk(c, nb);
+                    *out = avg_chunk<T>(A, avg_chunk<T>(C, next_chunk<T>(C, nb)));
+                    return;
+                }
+            }
+        }
+    }
+    for (int64_t b = at < 0 ? 0 : at; b < at + 16 && b < region; b += (int64_t)sizeof(T)) {
+        const uint32_t i = (uint32_t)(b / (int64_t)sizeof(T)), p = i / hs;
+        reinterpret_cast<T *>(P.out)[i] = (T)flat_value<T>(P, subpel, p, i - p * hs);
+    }
+}
+
+// The same of every sub-plane at once where their sizes are multiples of 16 bytes, so that the chunk at
+// byte position `at` of each is aligned alike: the source is read once for all of them. at >= 0, inside
+// the sub-plane.
+template <typename T>
+__device__ __forceinline__ void flat_chunk_all(const FlatPlane &P, bool subpel, uint32_t nsub, uint32_t at, const uint8_t *read_end) {
+    constexpr uint32_t n = 16 / sizeof(T);
+    const uint32_t S = P.S, hs = P.hs, o = at / (uint32_t)sizeof(T);
+    const size_t step = (size_t)hs * sizeof(T);
+    uint8_t *out = P.out + at;
+    const uint8_t *s = P.src + at;
+    uint4 p1 = make_uint4(0, 0, 0, 0), p2 = p1, p3 = p1, A;
+    if (!subpel) {
+        uint32_t nx;
+        if (s + 24 <= read_end) A = load_chunk(s, nx);
+        else if (((uintptr_t)s & 15) == 0) A = __ldg(reinterpret_cast<const uint4 *>(s));
+        else goto scalar;
+    } else {
+        const uint8_t *t = s + (size_t)S * sizeof(T);
+        uint32_t nx, nb;
+        if (o + n + S + 1 <= hs && t + 24 <= read_end) {
+            A = load_chunk(s, nx);
+            const uint4 B = load_chunk(t, nb), An = next_chunk<T>(A, nx), Bn = next_chunk<T>(B, nb);
+            p1 = avg_chunk<T>(A, An);
+            p2 = avg_chunk<T>(A, B);
+            p3 = avg_chunk<T>(A, Bn);
+            if (o < S) {  // the first row's samples of the v and hv planes are copies
+                const uint32_t *a = &A.x, *an = &An.x;
+                uint32_t *q2 = &p2.x, *q3 = &p3.x;
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const int k = (int)(S - o) - i * (int)(n / 4);  // samples of the word in the first row
+                    const uint32_t m = k <= 0 ? 0u : k >= (int)(n / 4) ? 0xFFFFFFFFu : (1u << (8 * (int)sizeof(T) * k)) - 1u;
+                    q2[i] = (a[i] & m) | (q2[i] & ~m);
+                    q3[i] = (an[i] & m) | (q3[i] & ~m);
+                }
+            }
+        } else if (o >= hs - S && o >= S && P.src + at + 24 <= read_end) {
+            // the last row: below it stands the h plane's first row (its first sample also after the last one)
+            const uint8_t *c = P.src + (size_t)(o - (hs - S)) * sizeof(T);
+            A = load_chunk(s, nx);
+            uint32_t nc, nd;
+            const uint4 C = load_chunk(c, nc), Cn = load_chunk(c + sizeof(T), nd);
+            if (o + n == hs) nx = avg8(reinterpret_cast<const T *>(P.src)[0], reinterpret_cast<const T *>(P.src)[1]);
+            p1 = avg_chunk<T>(A, next_chunk<T>(A, nx));
+            p2 = avg_chunk<T>(A, avg_chunk<T>(C, Cn));
+            p3 = avg_chunk<T>(A, avg_chunk<T>(Cn, next_chunk<T>(Cn, nd)));
+        } else {
+            goto scalar;
+        }
+    }
+    *reinterpret_cast<uint4 *>(out) = A;
+    if (nsub > 1) {
+        *reinterpret_cast<uint4 *>(out + step) = p1;
+        *reinterpret_cast<uint4 *>(out + 2 * step) = p2;
+        *reinterpret_cast<uint4 *>(out + 3 * step) = p3;
+        for (uint32_t p = 4; p < nsub; p++) *reinterpret_cast<uint4 *>(out + p * step) = make_uint4(0, 0, 0, 0);
+    }
+    return;
+scalar:  // a chunk across the last two rows, or at the end of the source buffer
+    for (uint32_t p = 0; p < nsub; p++)
+#pragma unroll 4
+        for (uint32_t k = 0; k < n; k++)
+            reinterpret_cast<T *>(out + p * step)[k] = (T)flat_value<T>(P, subpel, p, o + k);
+}
+
+// One pyramid level of one plane of one frame (reduce_6tap + horizontal_6tap_inplace,
+// super_build.rs:254-357), as reduce_band states it. A warp takes kStripe output samples of a band of
+// rows and walks down: each lane keeps the six source rows of its 8 samples, loads two more per output
+// row, makes the row's vertical 6-tap in registers, takes its neighbours' samples by shuffles and makes
+// 4 outputs. Lanes 0 and 31 only feed their neighbours.
+constexpr int kStripe = 120;
+struct LevelPlane {
+    const uint8_t *src;  // first row of the level (super frame, or the source frame at level 0)
+    uint8_t *out;        // first row of the next level in the super frame
+    int S;               // row pitch, samples
+    int src_w, src_h, dst_w, dst_h;
+    int src_rows, out_rows;  // rows that exist from src / out on
+    int stripes;             // of kStripe outputs, over all source columns
+};
+__device__ __forceinline__ LevelPlane level_plane(const SuperDev &D, const uint8_t *src, uint8_t *dst, int plane, int64_t f, int lv,
+                                                  bool from_src) {
+    const PlaneGeo g = plane_geo(D, plane);
+    const bool c = plane > 0;
+    const int px = D.px_bytes;
+    LevelPlane p;
+    p.S = (int)g.stride;
+    p.src_w = c ? D.lw[lv] / 2 : D.lw[lv]; p.src_h = c ? D.lh[lv] / 2 : D.lh[lv];
+    p.dst_w = c ? D.lw[lv + 1] / 2 : D.lw[lv + 1]; p.dst_h = c ? D.lh[lv + 1] / 2 : D.lh[lv + 1];
+    const int64_t srow = c ? D.row_c[lv] : D.row_y[lv], drow = c ? D.row_c[lv + 1] : D.row_y[lv + 1];
+    uint8_t *base = dst + f * D.frame_bytes + g.out_off * px;
+    p.src = from_src ? src + f * D.src_frame_bytes + g.src_off * px : base + srow * g.stride * px;
+    p.src_rows = from_src ? p.src_h : (int)(g.rows - srow);
+    p.out = base + drow * g.stride * px;
+    p.out_rows = (int)(g.rows - drow);
+    const int span = p.src_w > 2 * p.dst_w ? (p.src_w + 1) / 2 : p.dst_w;
+    p.stripes = (span + kStripe - 1) / kStripe;
+    return p;
+}
+
+// A lane's 8 samples of a row, as the vertical filter takes them: bytes in halfword lanes (even and odd
+// ones apart), or 16-bit samples one per register.
+template <typename T>
+struct Row8;
+template <>
+struct Row8<uint8_t> {
+    uint32_t v[4];  // even / odd bytes of words 0 and 1
+    __device__ __forceinline__ void set(const uint32_t (&w)[2]) {
+#pragma unroll
+        for (int i = 0; i < 2; i++) { v[2 * i] = w[i] & 0x00FF00FFu; v[2 * i + 1] = (w[i] >> 8) & 0x00FF00FFu; }
+    }
+};
+template <>
+struct Row8<uint16_t> {
+    uint32_t v[8];
+    __device__ __forceinline__ void set(const uint32_t (&w)[4]) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) { v[2 * i] = w[i] & 0xFFFFu; v[2 * i + 1] = w[i] >> 16; }
+    }
+};
+// The packed words of a lane's 8 samples of a row that starts at `row`, from column x on; samples outside the
+// level's columns are zeros. A row that does not exist has row == nullptr.
+template <typename T, bool CG>
+__device__ __forceinline__ void load_row8(const uint8_t *row, int x, int src_w, uint32_t (&w)[2 * sizeof(T)]) {
+    constexpr int N = 2 * (int)sizeof(T);
+#pragma unroll
+    for (int i = 0; i < N; i++) w[i] = 0;
+    if (row && x >= 0 && x < src_w) {
+        const uint8_t *q = row + (size_t)x * sizeof(T);
+        if (x + 8 <= src_w) {
+            load_words<N, CG>(q, w);
+        } else {  // the row's end: whole words only while they hold samples of it
+            const int left = (src_w - x) * (int)sizeof(T);
+            const uintptr_t a = (uintptr_t)q;
+            const uint32_t *p = reinterpret_cast<const uint32_t *>(a & ~(uintptr_t)3);
+            const int mis = (int)(a & 3);
+            uint32_t v[N + 1];
+#pragma unroll
+            for (int i = 0; i <= N; i++) v[i] = 4 * i < left + mis ? ld_word<CG>(p + i) : 0u;
+#pragma unroll
+            for (int i = 0; i < N; i++) {
+                const int k = left - 4 * i;  // bytes of the word that are samples
+                const uint32_t m = k <= 0 ? 0u : k >= 4 ? 0xFFFFFFFFu : (1u << (8 * k)) - 1u;
+                w[i] = __funnelshift_r(v[i], v[i + 1], (unsigned)mis * 8u) & m;
+            }
+        }
+    }
+}
+// the packed words of 8 samples
+template <typename T>
+__device__ __forceinline__ void pack_row8(const Row8<T> &r, uint32_t (&w)[2 * sizeof(T)]) {
+#pragma unroll
+    for (int i = 0; i < 2 * (int)sizeof(T); i++) w[i] = r.v[2 * i] | (r.v[2 * i + 1] << (sizeof(T) == 1 ? 8 : 16));
+}
+// four samples at out[x ..] clipped to n of them, as wide as the address allows
+template <typename T>
+__device__ __forceinline__ void store_samples(T *out, const uint32_t *w, int n) {
+    if (n >= 4 && ((uintptr_t)out & (4 * sizeof(T) - 1)) == 0) {
+        if (sizeof(T) == 1) *reinterpret_cast<uint32_t *>(out) = w[0];
+        else *reinterpret_cast<uint2 *>(out) = make_uint2(w[0], w[sizeof(T) - 1]);
+        return;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        if (k < n) out[k] = (T)(sizeof(T) == 1 ? w[0] >> (8 * k) : w[(k >> 1) & (int)(sizeof(T) - 1)] >> (16 * (k & 1)));
+}
+
+// The ends of a row: the first and last outputs (and all of a row of two) are averages, and the second
+// takes the first one as its left sample. w: the lane's 8 vertical samples, o: its 4 outputs from x0 on.
+template <typename T>
+__device__ __forceinline__ void row_ends(const LevelPlane &p, int x0, const uint32_t (&w)[2 * sizeof(T)], uint32_t (&o)[sizeof(T)],
+                                         unsigned pmax) {
+    constexpr int N = 2 * (int)sizeof(T);
+    auto in = [&](int k) -> unsigned {  // sample k of the lane's 8
+        return sizeof(T) == 1 ? (w[(k >> 2) & (N - 1)] >> (8 * (k & 3))) & 0xFFu : (w[(k >> 1) & (N - 1)] >> (16 * (k & 1))) & 0xFFFFu;
+    };
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const int i = x0 + k;
+        unsigned v;
+        if (i == 0 || i == p.dst_w - 1 || p.dst_w <= 2) v = avg8(in(2 * k), in(2 * k + 1));
+        else if (i == 1 && k == 1)
+            v = min((avg8(in(0), in(1)) + in(5) + 10u * (in(2) + in(3)) + 5u * (in(1) + in(4)) + 16u) >> 5, pmax);
+        else continue;
+        if (sizeof(T) == 1) o[0] = (o[0] & ~(0xFFu << (8 * k))) | (v << (8 * k));
+        else o[(k >> 1) & (int)(sizeof(T) - 1)] = (o[(k >> 1) & (int)(sizeof(T) - 1)] & ~(0xFFFFu << (16 * (k & 1)))) | (v << (16 * (k & 1)));
+    }
+}
+// The lane's vertical samples from dst_w on, one by one (a lane that straddles dst_w).
+template <typename T>
+__device__ __forceinline__ void tail_samples(const LevelPlane &p, int sx, const uint32_t (&w)[2 * sizeof(T)], T *out) {
+    constexpr int N = 2 * (int)sizeof(T);
+    for (int k = p.dst_w - sx; k < 8 && sx + k < p.src_w; k++) {
+        uint32_t v = 0;
+#pragma unroll
+        for (int i = 0; i < N; i++)
+            if (i == k / (int)(4 / sizeof(T))) v = w[i] >> (8 * sizeof(T) * (k % (4 / sizeof(T))));
+        out[sx + k] = (T)v;
+    }
+}
+// The vertical 6-tap of six rows' samples.
+template <typename T>
+__device__ __forceinline__ Row8<T> vertical6(const Row8<T> (&a)[6], unsigned pmax) {
+    constexpr int V = sizeof(T) == 1 ? 4 : 8;
+    Row8<T> m;
+#pragma unroll
+    for (int i = 0; i < V; i++) {
+        if (sizeof(T) == 1) {  // each halfword lane <= 255: the weights sum to 32
+            const uint32_t s = (a[0].v[i] + a[5].v[i] + 0x00100010u) + 5u * (a[1].v[i] + a[4].v[i]) + 10u * (a[2].v[i] + a[3].v[i]);
+            m.v[i] = (s >> 5) & 0x00FF00FFu;
+        } else {
+            const uint32_t s = (a[0].v[i] + a[5].v[i] + 16u) + 5u * (a[1].v[i] + a[4].v[i]) + 10u * (a[2].v[i] + a[3].v[i]);
+            m.v[i] = min(s >> 5, pmax);
+        }
+    }
+    return m;
+}
+// The horizontal 6-tap's interior formula for the lane's 4 outputs, from its own 8 samples (packed in w) and
+// its neighbours'.
+template <typename T>
+__device__ __forceinline__ void horizontal6(const Row8<T> &m, const uint32_t (&w)[2 * sizeof(T)], unsigned pmax, uint32_t (&o)[sizeof(T)]) {
+    constexpr int N = 2 * (int)sizeof(T), V = sizeof(T) == 1 ? 4 : 8;
+    if (sizeof(T) == 1) {
+        const uint32_t W[4] = {__shfl_up_sync(0xFFFFFFFFu, w[1], 1), w[0], w[1], __shfl_down_sync(0xFFFFFFFFu, w[0], 1)};
+        o[0] = __byte_perm(h6tap_pair<0>(W), h6tap_pair<1>(W), 0x6420);
+    } else {
+        uint32_t s[12];  // samples -2 .. 9 around the lane's 8
+        const uint32_t pv = __shfl_up_sync(0xFFFFFFFFu, w[N - 1], 1), nv = __shfl_down_sync(0xFFFFFFFFu, w[0], 1);
+        s[0] = pv & 0xFFFFu; s[1] = pv >> 16; s[10] = nv & 0xFFFFu; s[11] = nv >> 16;
+#pragma unroll
+        for (int i = 0; i < 8; i++) s[2 + i] = m.v[i & (V - 1)];
+        uint32_t q[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            q[k] = min((s[2 * k] + s[2 * k + 5] + 10u * (s[2 * k + 2] + s[2 * k + 3]) + 5u * (s[2 * k + 1] + s[2 * k + 4]) + 16u) >> 5, pmax);
+        o[0] = q[0] | (q[1] << 16);
+        o[sizeof(T) - 1] = q[2] | (q[3] << 16);
+    }
+}
+// Rows of a band whose vertical filter is the 6-tap everywhere, in a stripe whose lanes lie inside the
+// level's columns or wholly outside them, all rows word-aligned: no test is left in the loop but the
+// stores'. The lanes outside read the row's end, unused. About 120 warp instructions per row of 120
+// outputs, against 343 with every test in place.
+template <typename T, bool CG>
+__device__ __forceinline__ void reduce_rows(const LevelPlane &p, int x0, bool own, int dy0, int n, unsigned pmax) {
+    constexpr int N = 2 * (int)sizeof(T);
+    const int sx = 2 * x0, rx = min(max(sx, 0), p.src_w - 8);
+    const size_t pitch = (size_t)p.S * sizeof(T);
+    const uint8_t *row = p.src + (size_t)(2 * dy0 - 2) * pitch + (size_t)rx * sizeof(T);
+    T *out = reinterpret_cast<T *>(p.out) + (int64_t)dy0 * p.S;
+    const bool lo = own && x0 + 4 <= p.dst_w, edge = own && x0 < p.dst_w && (x0 == 0 || x0 + 4 >= p.dst_w);
+    // vertical samples kept past the outputs: whole words of the lane's 8
+    const bool hi0 = own && sx >= p.dst_w && sx < p.src_w;
+    const bool part = own && sx < p.dst_w && sx + 8 > p.dst_w;
+    auto load = [&](const uint8_t *q, uint32_t (&w)[N]) {
+#pragma unroll
+        for (int i = 0; i < N; i++) w[i] = ld_word<CG>(q + 4 * i);
+    };
+    Row8<T> a[6];
+    {
+        uint32_t t[4][N];
+#pragma unroll
+        for (int i = 0; i < 4; i++) load(row + i * pitch, t[i]);
+#pragma unroll
+        for (int i = 0; i < 4; i++) a[i].set(t[i]);
+    }
+    row += 4 * pitch;
+    uint32_t n0[N], n1[N];
+    load(row, n0);
+    load(row + pitch, n1);
+#pragma unroll 3
+    for (int r = 0; r < n; r++) {
+        a[4].set(n0);
+        a[5].set(n1);
+        if (r + 1 < n) {  // the next row's two new source rows, in flight during this one
+            row += 2 * pitch;
+            load(row, n0);
+            load(row + pitch, n1);
+        }
+        const Row8<T> m = vertical6<T>(a, pmax);
+        uint32_t w[N], o[sizeof(T)];
+        pack_row8<T>(m, w);
+        horizontal6<T>(m, w, pmax, o);
+        if (edge) row_ends<T>(p, x0, w, o, pmax);
+        if (lo) {
+            if (sizeof(T) == 1) *reinterpret_cast<uint32_t *>(out + x0) = o[0];
+            else {
+                reinterpret_cast<uint32_t *>(out + x0)[0] = o[0];
+                reinterpret_cast<uint32_t *>(out + x0)[1] = o[sizeof(T) - 1];
+            }
+        } else if (own && x0 < p.dst_w) {
+            store_samples<T>(out + x0, o, p.dst_w - x0);
+        }
+        if (hi0) {
+#pragma unroll
+            for (int i = 0; i < N; i++) reinterpret_cast<uint32_t *>(out + sx)[i] = w[i];
+        } else if (part) {
+            tail_samples<T>(p, sx, w, out);
+        }
+        out += p.S;
+#pragma unroll
+        for (int i = 0; i < 4; i++) a[i] = a[i + 2];
+    }
+}
+
+// The rows [r0, r1) of a stripe with every test in place: the first and last rows, rows and columns that
+// end inside a lane's samples, unaligned rows.
+template <typename T, bool CG>
+__device__ __noinline__ void reduce_general(const LevelPlane p, int stripe, int r0, int r1, unsigned pmax) {
+    constexpr int N = 2 * (int)sizeof(T), V = sizeof(T) == 1 ? 4 : 8;
+    const int lane = (int)(threadIdx.x & 31), nr = r1 - r0;
+    const int x0 = stripe * kStripe + (lane - 1) * 4, sx = 2 * x0;
+    const bool own = lane > 0 && lane < 31;
+    const size_t pitch = (size_t)p.S * sizeof(T);
+    auto row_at = [&](int y) -> const uint8_t * { return y < p.src_rows ? p.src + (size_t)y * pitch : nullptr; };
+    Row8<T> a[6];
+    int have = -1;  // first source row held in a
+    uint32_t n0[N], n1[N];  // the next output row's two new source rows, loaded ahead
+    bool ahead = false;
+    T *out = reinterpret_cast<T *>(p.out) + (int64_t)r0 * p.S;
+    for (int r = 0; r < nr; r++, out += p.S) {
+        const int dy = r0 + r, sy = 2 * dy;
+        if (dy >= p.out_rows) break;
+        Row8<T> m;
+        if (dy == 0 || dy + 1 == p.dst_h || sy - 2 < 0 || sy + 3 >= p.src_h) {
+            uint32_t uw[N], vw[N];
+            load_row8<T, CG>(row_at(min(sy, p.src_h - 1)), sx, p.src_w, uw);
+            load_row8<T, CG>(row_at(min(sy + 1, p.src_h - 1)), sx, p.src_w, vw);
+            Row8<T> u, v;
+            u.set(uw);
+            v.set(vw);
+#pragma unroll
+            for (int i = 0; i < V; i++)
+                m.v[i] = sizeof(T) == 1 ? avg_word<T>(u.v[i], v.v[i]) : (u.v[i] + v.v[i] + 1u) >> 1;
+            ahead = false;
+        } else {
+            if (have == sy - 4) {
+#pragma unroll
+                for (int i = 0; i < 4; i++) a[i] = a[i + 2];
+            } else {
+                uint32_t t[4][N];
+#pragma unroll
+                for (int i = 0; i < 4; i++) load_row8<T, CG>(row_at(sy - 2 + i), sx, p.src_w, t[i]);
+#pragma unroll
+                for (int i = 0; i < 4; i++) a[i].set(t[i]);
+            }
+            if (!ahead) {
+                load_row8<T, CG>(row_at(sy + 2), sx, p.src_w, n0);
+                load_row8<T, CG>(row_at(sy + 3), sx, p.src_w, n1);
+            }
+            a[4].set(n0);
+            a[5].set(n1);
+            have = sy - 2;
+            ahead = r + 1 < nr && sy + 5 < p.src_h;
+            if (ahead) {
+                load_row8<T, CG>(row_at(sy + 4), sx, p.src_w, n0);
+                load_row8<T, CG>(row_at(sy + 5), sx, p.src_w, n1);
+            }
+            m = vertical6<T>(a, pmax);
+        }
+        uint32_t w[N];
+        pack_row8<T>(m, w);
+        uint32_t o[sizeof(T)];
+        horizontal6<T>(m, w, pmax, o);
+        if (own && x0 < p.dst_w && (x0 == 0 || x0 + 4 >= p.dst_w)) row_ends<T>(p, x0, w, o, pmax);
+        if (own) {
+            if (x0 < p.dst_w) store_samples<T>(out + x0, o, p.dst_w - x0);
+            // the columns past the outputs keep the vertical filter's samples (:302-306)
+            if (sx + 8 > p.dst_w && sx < p.src_w) {
+                if (sx >= p.dst_w) {
+                    store_samples<T>(out + sx, w, p.src_w - sx);
+                    if (sx + 4 < p.src_w) store_samples<T>(out + sx + 4, w + N / 2, p.src_w - sx - 4);
+                } else {
+                    tail_samples<T>(p, sx, w, out);
+                }
+            }
+        }
+    }
+}
+
+template <typename T, bool CG>
+__device__ __forceinline__ void reduce_stripe(const LevelPlane &p, int stripe, int r0, int nr, unsigned pmax) {
+    const int lane = (int)(threadIdx.x & 31);
+    const int x0 = stripe * kStripe + (lane - 1) * 4;
+    const bool own = lane > 0 && lane < 31;
+    // the stripe's part of the zeros up to the pitch, cut at multiples of four samples
+    auto cut = [&](int k) { return k == 0 ? p.src_w : k == p.stripes ? p.S : max(p.src_w, (p.src_w + (p.S - p.src_w) * k / p.stripes) & ~3); };
+    const int z0 = cut(stripe), z1 = cut(stripe + 1);
+    const size_t pitch = (size_t)p.S * sizeof(T);
+    // rows of the band that the loop without tests may take
+    int f0 = max(r0, 1), f1 = min(min(r0 + nr, p.dst_h - 1), p.out_rows);
+    f1 = min(f1, (p.src_h - 4) / 2 + 1);                 // 2 dy + 3 < src_h
+    f1 = min(f1, (p.src_rows - 4) / 2 + 1);
+    const bool fast = f1 > f0 && p.src_w >= 8 && (p.src_w % 8 == 0 || (stripe + 1) * 2 * kStripe + 8 <= p.src_w) &&
+                      ((((uintptr_t)p.src | (uintptr_t)p.out) & 3) | (pitch & 3)) == 0;
+    if (!fast) f0 = f1 = r0;
+    reduce_general<T, CG>(p, stripe, r0, fast ? f0 : r0 + nr, pmax);
+    if (fast) {
+        reduce_rows<T, CG>(p, x0, own, f0, f1 - f0, pmax);
+        if (f1 < r0 + nr) reduce_general<T, CG>(p, stripe, f1, r0 + nr, pmax);
+    }
+    // zeros up to the pitch
+    if (z0 < z1) {
+        const uint32_t zero[2] = {0u, 0u};
+        T *out = reinterpret_cast<T *>(p.out) + (int64_t)r0 * p.S;
+        for (int r = 0; r < nr && r0 + r < p.out_rows; r++, out += p.S)
+            for (int z = z0 + 4 * lane; z < z1; z += 128) store_samples<T>(out + z, zero, min(4, z1 - z));
+    }
+}
+// Work items of one level over frames: per frame luma's (stripes x bands), then both chroma planes'.
+struct LevelItems {
+    int lv, band, sy, by, sc, bc;  // stripes and bands of luma and of a chroma plane
+    uint32_t per, total;
+};
+template <typename T, bool CG>
+__device__ __forceinline__ void level_item(const SuperDev &D, const uint8_t *src, uint8_t *dst, const LevelItems &I, uint32_t it,
+                                           bool from_src) {
+    const uint32_t f = it / I.per;
+    uint32_t e = it - f * I.per;
+    int plane = 0, sn = I.sy;
+    if (e >= (uint32_t)(I.sy * I.by)) {
+        e -= (uint32_t)(I.sy * I.by);
+        plane = 1 + (int)(e / (uint32_t)(I.sc * I.bc));
+        e %= (uint32_t)(I.sc * I.bc);
+        sn = I.sc;
+    }
+    const LevelPlane p = level_plane(D, src, dst, plane, f, I.lv, from_src);
+    const int b = (int)(e / (uint32_t)sn), s = (int)(e % (uint32_t)sn), r0 = b * I.band;
+    reduce_stripe<T, CG>(p, s, r0, min(I.band, p.dst_h - r0), (unsigned)D.px_max);
+}
+
+// Level 0 of every plane and frame, and the level 0 -> 1 reduction (from the source frames, whose rows
+// are level 0's full-pel rows), in one launch: a CTA does its share of both, every second one the
+// reduction first, so that the two kinds of work, the one bound by memory, the other by instruction
+// issue, are on every SM at the same time. Level 0 goes in tiles of kTile chunks of one plane, whose
+// place is computed once per CTA.
+constexpr uint32_t kTile = 1024;
+struct FlatItems {
+    uint32_t ty, tc;    // tiles of luma and of a chroma plane
+    uint32_t per, total;
+    int all_y, all_c;   // the plane's sub-planes are chunked together (flat_chunk_all)
+};
+template <typename T>
+__global__ void __launch_bounds__(256, sizeof(T) == 1 ? 3 : 2) super_flat_kernel(SuperDev D, const uint8_t *__restrict__ src, uint8_t *__restrict__ dst,
+                                                         const uint8_t *src_end, LevelItems I, FlatItems F) {
+    const uint32_t nsub = D.full ? (uint32_t)(D.pel * D.pel) : 1u;
+    const bool subpel = D.pel >= 2 && D.gpu <= 1 && D.full && D.scale_up == 0;
+    auto level0 = [&] {
+        for (uint32_t it = blockIdx.x; it < F.total; it += gridDim.x) {
+            const uint32_t f = it / F.per;
+            uint32_t e = it - f * F.per;
+            const int plane = e < F.ty ? 0 : e < F.ty + F.tc ? 1 : 2;
+            e -= plane == 0 ? 0 : plane == 1 ? F.ty : F.ty + F.tc;
+            const PlaneGeo g = plane_geo(D, plane);
+            FlatPlane P;
+            P.src = src + (int64_t)f * D.src_frame_bytes + g.src_off * (int)sizeof(T);
+            P.out = dst + (int64_t)f * D.frame_bytes + g.out_off * (int)sizeof(T);
+            P.S = (uint32_t)g.stride;
+            P.hs = (uint32_t)g.stride * (uint32_t)g.h;
+            const uint32_t sub = P.hs * (uint32_t)sizeof(T);
+            const int64_t region = (int64_t)nsub * sub;
+            const uint32_t mis = (uint32_t)((uintptr_t)P.out & 15);
+            const bool all = plane ? F.all_c : F.all_y;
+            if (all && mis == 0) {
+                for (uint32_t c = e * kTile + threadIdx.x; c < (e + 1) * kTile; c += blockDim.x)
+                    if (c * 16u < sub) flat_chunk_all<T>(P, subpel, nsub, c * 16u, src_end);
+            } else {
+                const uint32_t parts = all ? nsub : 1u;  // tiles were counted per sub-plane
+                for (uint32_t c = e * kTile * parts + threadIdx.x; c < (e + 1) * kTile * parts; c += blockDim.x) {
+                    const int64_t at = (int64_t)c * 16 - mis;
+                    if (at < region) flat_chunk<T>(P, subpel, nsub, at, region, src_end);
+                }
+            }
+        }
+    };
+    auto reduce = [&] {
+        const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+        for (uint32_t it = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); it < I.total; it += warps)
+            level_item<T, false>(D, src, dst, I, it, true);
+    };
+    if (blockIdx.x & 1) { reduce(); level0(); }
+    else { level0(); reduce(); }
+}
+template <typename T>
+__global__ void __launch_bounds__(256, sizeof(T) == 1 ? 3 : 2) super_level_kernel(SuperDev D, uint8_t *__restrict__ dst, LevelItems I) {
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    for (uint32_t it = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); it < I.total; it += warps)
+        level_item<T, false>(D, nullptr, dst, I, it, false);
+}
+// The levels from lv0 on, small ones, of one plane of one frame by a cluster of kTailCtas CTAs, one level
+// after another with a cluster barrier between them; a level's rows come from other SMs, so they are read
+// from L2.
+constexpr int kTailCtas = 8;
+template <typename T>
+__global__ void __cluster_dims__(kTailCtas, 1, 1) __launch_bounds__(256) super_tail_kernel(SuperDev D, uint8_t *__restrict__ dst, int lv0) {
+    const uint32_t cl = blockIdx.x / kTailCtas, rank = blockIdx.x % kTailCtas;
+    const int plane = (int)(cl % 3);
+    const int64_t f = cl / 3;
+    const int warps = kTailCtas * 8, warp = (int)(rank * 8 + (threadIdx.x >> 5));
+    for (int lv = lv0; lv + 1 < D.levels; lv++) {
+        const LevelPlane p = level_plane(D, nullptr, dst, plane, f, lv, false);
+        if (p.dst_h > 0) {
+            const int band = min(max((p.dst_h * p.stripes + warps - 1) / warps, 1), 8);
+            const int n = p.stripes * ((p.dst_h + band - 1) / band);
+            for (int i = warp; i < n; i += warps) {
+                const int r0 = i / p.stripes * band;
+                reduce_stripe<T, true>(p, i % p.stripes, r0, min(band, p.dst_h - r0), (unsigned)D.px_max);
+            }
+        }
+        __threadfence();
+        asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory");
+    }
+}
+
 // Every row start of the source and super frames on a 16-byte boundary, 8-bit samples, and
 // no bicubic planes: the fast paths apply.
 bool vec_ok(const SuperDev &D, const void *src, const void *dst, int nframes) {
@@ -644,6 +1297,76 @@ int launch_super_vec(const SuperDev &D, const uint8_t *src, uint8_t *dst, int nf
     return n;
 }
 
+// Packed frames that hold every level-0 row, with bilinear sub-planes or none: the flat path applies.
+bool flat_ok(const SuperDev &D, int nframes) {
+    const int nsub = D.pel * D.pel;
+    return D.full && D.scale_up != 2 && D.scale_down == 4 && D.width >= 4 && D.height >= 4 && D.y_stride == D.width &&
+           D.c_stride == D.width / 2 && D.src_y_stride == D.width && D.src_c_stride == D.width / 2 &&
+           (int64_t)nsub * D.height <= D.y_rows && (int64_t)nsub * (D.height / 2) <= D.c_rows &&
+           D.y_len * D.px_bytes < (1ll << 31) && (int64_t)nframes * (D.frame_bytes / 16 + 8) < (1ll << 31);
+}
+// Work items of level lv over the frames: bands of 16 rows, or fewer where that leaves warps idle.
+LevelItems level_items(const SuperDev &D, int lv, int nframes, int sms) {
+    LevelItems I{};
+    I.lv = lv;
+    auto stripes = [&](bool c) {
+        const int sw = c ? D.lw[lv] / 2 : D.lw[lv], dw = c ? D.lw[lv + 1] / 2 : D.lw[lv + 1];
+        const int span = sw > 2 * dw ? (sw + 1) / 2 : dw;
+        return (span + kStripe - 1) / kStripe;
+    };
+    I.sy = stripes(false);
+    I.sc = stripes(true);
+    for (I.band = 16;; I.band /= 2) {
+        I.by = (D.lh[lv + 1] + I.band - 1) / I.band;
+        I.bc = (D.lh[lv + 1] / 2 + I.band - 1) / I.band;
+        I.per = (uint32_t)(I.sy * I.by + 2 * I.sc * I.bc);
+        I.total = I.per * (uint32_t)nframes;
+        if (I.band == 2 || I.total >= (uint32_t)sms * 32) return I;
+    }
+}
+// Levels whose result has at most this many luma samples go to the tail kernel, a cluster per plane and frame.
+constexpr int64_t kTailSamples = 40000;
+constexpr int kTailFrames = 6;  // more frames fill the GPU at every level
+template <typename T>
+int launch_super_flat(const SuperDev &D, const uint8_t *src, uint8_t *dst, int nframes, int sms, cudaStream_t stream) {
+    const int per_sm = sizeof(T) == 1 ? 3 : 2;
+    const int nsub = D.pel * D.pel;
+    LevelItems I{};
+    if (D.levels > 1) I = level_items(D, 0, nframes, sms);
+    else I.per = 1;
+    FlatItems F{};
+    auto tiles = [&](int64_t hs, int &all) {  // + 1: a plane that does not start on 16 bytes has one chunk more
+        const int64_t sub = hs * (int)sizeof(T);
+        all = (sub & 15) == 0;
+        const int64_t bytes = all ? sub : sub * nsub;
+        return (uint32_t)((bytes / 16 + 1 + kTile) / kTile);
+    };
+    F.ty = tiles((int64_t)D.width * D.height, F.all_y);
+    F.tc = tiles((int64_t)(D.width / 2) * (D.height / 2), F.all_c);
+    F.per = F.ty + 2 * F.tc;
+    F.total = F.per * (uint32_t)nframes;
+    const int64_t want = std::max<int64_t>(F.total, (I.total + 7) / 8);
+    super_flat_kernel<T><<<(int)std::min<int64_t>(want, (int64_t)sms * per_sm), 256, 0, stream>>>(
+        D, src, dst, src + D.src_frame_bytes * nframes, I, F);
+    int n = 1, lv = 1;
+    for (; lv + 1 < D.levels && (int64_t)D.lw[lv + 1] * D.lh[lv + 1] > kTailSamples; lv++) {
+        const LevelItems L = level_items(D, lv, nframes, sms);
+        super_level_kernel<T><<<(int)std::min<int64_t>((L.total + 7) / 8, (int64_t)sms * per_sm), 256, 0, stream>>>(D, dst, L);
+        n++;
+    }
+    if (nframes > kTailFrames)  // enough work for a launch per level
+        for (; lv + 1 < D.levels; lv++) {
+            const LevelItems L = level_items(D, lv, nframes, sms);
+            super_level_kernel<T><<<(int)std::min<int64_t>((L.total + 7) / 8, (int64_t)sms * per_sm), 256, 0, stream>>>(D, dst, L);
+            n++;
+        }
+    if (lv + 1 < D.levels) {
+        super_tail_kernel<T><<<nframes * 3 * kTailCtas, 256, 0, stream>>>(D, dst, lv);
+        n++;
+    }
+    return n;
+}
+
 cudaError_t launch_super(const SuperDev &D, const uint8_t *src, uint8_t *dst, int nframes, cudaStream_t stream,
                          int *launches) {
     if (nframes <= 0) return cudaSuccess;
@@ -653,6 +1376,12 @@ cudaError_t launch_super(const SuperDev &D, const uint8_t *src, uint8_t *dst, in
             return 148;
         return v;
     }();
+    if (flat_ok(D, nframes)) {
+        const int n = D.px_bytes == 2 ? launch_super_flat<uint16_t>(D, src, dst, nframes, sms, stream)
+                                      : launch_super_flat<uint8_t>(D, src, dst, nframes, sms, stream);
+        if (launches) *launches += n;
+        return cudaGetLastError();
+    }
     if (vec_ok(D, src, dst, nframes)) {
         static const cudaError_t attr = [] {
             cudaError_t e = cudaFuncSetAttribute(super_reduce_band_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
