@@ -759,6 +759,29 @@ scalar:  // a chunk across the last two rows, or at the end of the source buffer
             reinterpret_cast<T *>(out + p * step)[k] = (T)flat_value<T>(P, subpel, p, o + k);
 }
 
+// Two chunks among the middle rows (neither the first nor the last), all sub-planes.
+template <typename T>
+__device__ __forceinline__ void flat_middle2(const FlatPlane &P, uint32_t nsub, uint32_t a0, uint32_t a1) {
+    const size_t step = (size_t)P.hs * sizeof(T), below = (size_t)P.S * sizeof(T);
+    const uint32_t at[2] = {a0, a1};
+    uint4 A[2], B[2];
+    uint32_t na[2], nb[2];
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        A[i] = load_chunk(P.src + at[i], na[i]);
+        B[i] = load_chunk(P.src + at[i] + below, nb[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        uint8_t *out = P.out + at[i];
+        *reinterpret_cast<uint4 *>(out) = A[i];
+        *reinterpret_cast<uint4 *>(out + step) = avg_chunk<T>(A[i], next_chunk<T>(A[i], na[i]));
+        *reinterpret_cast<uint4 *>(out + 2 * step) = avg_chunk<T>(A[i], B[i]);
+        *reinterpret_cast<uint4 *>(out + 3 * step) = avg_chunk<T>(A[i], next_chunk<T>(B[i], nb[i]));
+        for (uint32_t p = 4; p < nsub; p++) *reinterpret_cast<uint4 *>(out + p * step) = make_uint4(0, 0, 0, 0);
+    }
+}
+
 // One pyramid level of one plane of one frame (reduce_6tap + horizontal_6tap_inplace,
 // super_build.rs:254-357), as reduce_band states it. A warp takes kStripe output samples of a band of
 // rows and walks down: each lane keeps the six source rows of its 8 samples, loads two more per output
@@ -894,17 +917,18 @@ __device__ __forceinline__ void tail_samples(const LevelPlane &p, int sx, const 
     }
 }
 // The vertical 6-tap of six rows' samples.
-template <typename T>
+template <typename T, int K = 0>  // the oldest row is a[K], the others follow cyclically
 __device__ __forceinline__ Row8<T> vertical6(const Row8<T> (&a)[6], unsigned pmax) {
+    constexpr int k0 = K, k1 = (K + 1) % 6, k2 = (K + 2) % 6, k3 = (K + 3) % 6, k4 = (K + 4) % 6, k5 = (K + 5) % 6;
     constexpr int V = sizeof(T) == 1 ? 4 : 8;
     Row8<T> m;
 #pragma unroll
     for (int i = 0; i < V; i++) {
         if (sizeof(T) == 1) {  // each halfword lane <= 255: the weights sum to 32
-            const uint32_t s = (a[0].v[i] + a[5].v[i] + 0x00100010u) + 5u * (a[1].v[i] + a[4].v[i]) + 10u * (a[2].v[i] + a[3].v[i]);
+            const uint32_t s = (a[k0].v[i] + a[k5].v[i] + 0x00100010u) + 5u * (a[k1].v[i] + a[k4].v[i]) + 10u * (a[k2].v[i] + a[k3].v[i]);
             m.v[i] = (s >> 5) & 0x00FF00FFu;
         } else {
-            const uint32_t s = (a[0].v[i] + a[5].v[i] + 16u) + 5u * (a[1].v[i] + a[4].v[i]) + 10u * (a[2].v[i] + a[3].v[i]);
+            const uint32_t s = (a[k0].v[i] + a[k5].v[i] + 16u) + 5u * (a[k1].v[i] + a[k4].v[i]) + 10u * (a[k2].v[i] + a[k3].v[i]);
             m.v[i] = min(s >> 5, pmax);
         }
     }
@@ -936,6 +960,10 @@ __device__ __forceinline__ void horizontal6(const Row8<T> &m, const uint32_t (&w
 // level's columns or wholly outside them, all rows word-aligned: no test is left in the loop but the
 // stores'. The lanes outside read the row's end, unused. About 120 warp instructions per row of 120
 // outputs, against 343 with every test in place.
+template <int K>
+struct Phase {
+    static constexpr int value = K;
+};
 template <typename T, bool CG>
 __device__ __forceinline__ void reduce_rows(const LevelPlane &p, int x0, bool own, int dy0, int n, unsigned pmax) {
     constexpr int N = 2 * (int)sizeof(T);
@@ -963,16 +991,18 @@ __device__ __forceinline__ void reduce_rows(const LevelPlane &p, int x0, bool ow
     uint32_t n0[N], n1[N];
     load(row, n0);
     load(row + pitch, n1);
-#pragma unroll 3
-    for (int r = 0; r < n; r++) {
-        a[4].set(n0);
-        a[5].set(n1);
+    int r = 0;
+    // one row; the oldest of the six source rows is a[K], so three rows bring the ring round without a move
+    auto one = [&](auto phase) {
+        constexpr int K = decltype(phase)::value;
+        a[(K + 4) % 6].set(n0);
+        a[(K + 5) % 6].set(n1);
         if (r + 1 < n) {  // the next row's two new source rows, in flight during this one
             row += 2 * pitch;
             load(row, n0);
             load(row + pitch, n1);
         }
-        const Row8<T> m = vertical6<T>(a, pmax);
+        const Row8<T> m = vertical6<T, K>(a, pmax);
         uint32_t w[N], o[sizeof(T)];
         pack_row8<T>(m, w);
         horizontal6<T>(m, w, pmax, o);
@@ -993,8 +1023,12 @@ __device__ __forceinline__ void reduce_rows(const LevelPlane &p, int x0, bool ow
             tail_samples<T>(p, sx, w, out);
         }
         out += p.S;
-#pragma unroll
-        for (int i = 0; i < 4; i++) a[i] = a[i + 2];
+        r++;
+    };
+    while (r < n) {
+        one(Phase<0>());
+        if (r < n) one(Phase<2>());
+        if (r < n) one(Phase<4>());
     }
 }
 
@@ -1078,8 +1112,8 @@ __device__ __forceinline__ void reduce_stripe(const LevelPlane &p, int stripe, i
     const int lane = (int)(threadIdx.x & 31);
     const int x0 = stripe * kStripe + (lane - 1) * 4;
     const bool own = lane > 0 && lane < 31;
-    // the stripe's part of the zeros up to the pitch, cut at multiples of four samples
-    auto cut = [&](int k) { return k == 0 ? p.src_w : k == p.stripes ? p.S : max(p.src_w, (p.src_w + (p.S - p.src_w) * k / p.stripes) & ~3); };
+    // the stripe's part of the zeros up to the pitch, cut at multiples of 16 samples
+    auto cut = [&](int k) { return k == 0 ? p.src_w : k == p.stripes ? p.S : max(p.src_w, (p.src_w + (p.S - p.src_w) * k / p.stripes) & ~15); };
     const int z0 = cut(stripe), z1 = cut(stripe + 1);
     const size_t pitch = (size_t)p.S * sizeof(T);
     // rows of the band that the loop without tests may take
@@ -1096,10 +1130,18 @@ __device__ __forceinline__ void reduce_stripe(const LevelPlane &p, int stripe, i
     }
     // zeros up to the pitch
     if (z0 < z1) {
-        const uint32_t zero[2] = {0u, 0u};
+        // 16 bytes a lane where the range starts and ends on 16 bytes, else by four samples
         T *out = reinterpret_cast<T *>(p.out) + (int64_t)r0 * p.S;
-        for (int r = 0; r < nr && r0 + r < p.out_rows; r++, out += p.S)
-            for (int z = z0 + 4 * lane; z < z1; z += 128) store_samples<T>(out + z, zero, min(4, z1 - z));
+        const bool wide = ((((uintptr_t)(out + z0) | ((uintptr_t)(z1 - z0) * sizeof(T)) | pitch) & 15) == 0);
+        for (int r = 0; r < nr && r0 + r < p.out_rows; r++, out += p.S) {
+            if (wide) {
+                for (int z = z0 + (int)(16 / sizeof(T)) * lane; z < z1; z += (int)(512 / sizeof(T)))
+                    *reinterpret_cast<uint4 *>(out + z) = make_uint4(0, 0, 0, 0);
+            } else {
+                const uint32_t zero[2] = {0u, 0u};
+                for (int z = z0 + 4 * lane; z < z1; z += 128) store_samples<T>(out + z, zero, min(4, z1 - z));
+            }
+        }
     }
 }
 // Work items of one level over frames: per frame luma's (stripes x bands), then both chroma planes'.
@@ -1127,20 +1169,19 @@ __device__ __forceinline__ void level_item(const SuperDev &D, const uint8_t *src
 // Level 0 of every plane and frame, and the level 0 -> 1 reduction (from the source frames, whose rows
 // are level 0's full-pel rows), in one launch: a CTA does its share of both, every second one the
 // reduction first, so that the two kinds of work, the one bound by memory, the other by instruction
-// issue, are on every SM at the same time. Level 0 goes in tiles of kTile chunks of one plane, whose
+// issue, are on every SM at the same time. Level 0 goes in tiles of chunks of one plane, whose
 // place is computed once per CTA.
-constexpr uint32_t kTile = 1024;
 struct FlatItems {
+    uint32_t tile;      // chunks per tile: 1024, or 256 where that leaves SMs idle
     uint32_t ty, tc;    // tiles of luma and of a chroma plane
     uint32_t per, total;
     int all_y, all_c;   // the plane's sub-planes are chunked together (flat_chunk_all)
 };
 template <typename T>
-__global__ void __launch_bounds__(256, sizeof(T) == 1 ? 3 : 2) super_flat_kernel(SuperDev D, const uint8_t *__restrict__ src, uint8_t *__restrict__ dst,
-                                                         const uint8_t *src_end, LevelItems I, FlatItems F) {
+__device__ __forceinline__ void flat_level0(const SuperDev &D, const uint8_t *__restrict__ src, uint8_t *__restrict__ dst,
+                                            const uint8_t *src_end, const FlatItems &F) {
     const uint32_t nsub = D.full ? (uint32_t)(D.pel * D.pel) : 1u;
     const bool subpel = D.pel >= 2 && D.gpu <= 1 && D.full && D.scale_up == 0;
-    auto level0 = [&] {
         for (uint32_t it = blockIdx.x; it < F.total; it += gridDim.x) {
             const uint32_t f = it / F.per;
             uint32_t e = it - f * F.per;
@@ -1157,41 +1198,60 @@ __global__ void __launch_bounds__(256, sizeof(T) == 1 ? 3 : 2) super_flat_kernel
             const uint32_t mis = (uint32_t)((uintptr_t)P.out & 15);
             const bool all = plane ? F.all_c : F.all_y;
             if (all && mis == 0) {
-                for (uint32_t c = e * kTile + threadIdx.x; c < (e + 1) * kTile; c += blockDim.x)
-                    if (c * 16u < sub) flat_chunk_all<T>(P, subpel, nsub, c * 16u, src_end);
+                // two chunks of a thread at a time where both lie among the plane's middle rows: their loads overlap
+                for (uint32_t c = e * F.tile + threadIdx.x; c < (e + 1) * F.tile; c += 2 * blockDim.x) {
+                    const uint32_t a0 = c * 16u, a1 = (c + blockDim.x) * 16u;
+                    const uint32_t rowb = P.S * (uint32_t)sizeof(T);
+                    if (subpel && a0 >= rowb && a1 + rowb + 32u <= sub && P.src + a1 + rowb + 24 <= src_end) {
+                        flat_middle2<T>(P, nsub, a0, a1);
+                        continue;
+                    }
+                    if (a0 < sub) flat_chunk_all<T>(P, subpel, nsub, a0, src_end);
+                    if (a1 < sub) flat_chunk_all<T>(P, subpel, nsub, a1, src_end);
+                }
             } else {
                 const uint32_t parts = all ? nsub : 1u;  // tiles were counted per sub-plane
-                for (uint32_t c = e * kTile * parts + threadIdx.x; c < (e + 1) * kTile * parts; c += blockDim.x) {
+                for (uint32_t c = e * F.tile * parts + threadIdx.x; c < (e + 1) * F.tile * parts; c += blockDim.x) {
                     const int64_t at = (int64_t)c * 16 - mis;
                     if (at < region) flat_chunk<T>(P, subpel, nsub, at, region, src_end);
                 }
             }
         }
-    };
+}
+template <typename T>
+__global__ void __launch_bounds__(256, sizeof(T) == 1 ? 3 : 2) super_flat_kernel(SuperDev D, const uint8_t *__restrict__ src, uint8_t *__restrict__ dst,
+                                                         const uint8_t *src_end, LevelItems I, FlatItems F) {
     auto reduce = [&] {
         const uint32_t warps = gridDim.x * (blockDim.x >> 5);
         for (uint32_t it = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); it < I.total; it += warps)
             level_item<T, false>(D, src, dst, I, it, true);
     };
-    if (blockIdx.x & 1) { reduce(); level0(); }
-    else { level0(); reduce(); }
+    if (blockIdx.x & 1) { reduce(); flat_level0<T>(D, src, dst, src_end, F); }
+    else { flat_level0<T>(D, src, dst, src_end, F); reduce(); }
+}
+// Level 0 alone, for calls large enough to pay a launch of its own: with a third of the registers, its loads
+// and stores have twice the warps in flight.
+template <typename T>
+__global__ void __launch_bounds__(256, 6) super_level0_flat_kernel(SuperDev D, const uint8_t *__restrict__ src, uint8_t *__restrict__ dst,
+                                                                   const uint8_t *src_end, FlatItems F) {
+    flat_level0<T>(D, src, dst, src_end, F);
 }
 template <typename T>
-__global__ void __launch_bounds__(256, sizeof(T) == 1 ? 3 : 2) super_level_kernel(SuperDev D, uint8_t *__restrict__ dst, LevelItems I) {
+__global__ void __launch_bounds__(256, sizeof(T) == 1 ? 3 : 2) super_level_kernel(SuperDev D, const uint8_t *__restrict__ src, uint8_t *__restrict__ dst, LevelItems I) {
     const uint32_t warps = gridDim.x * (blockDim.x >> 5);
     for (uint32_t it = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); it < I.total; it += warps)
-        level_item<T, false>(D, nullptr, dst, I, it, false);
+        level_item<T, false>(D, src, dst, I, it, src != nullptr);
 }
 // The levels from lv0 on, small ones, of one plane of one frame by a cluster of kTailCtas CTAs, one level
 // after another with a cluster barrier between them; a level's rows come from other SMs, so they are read
 // from L2.
 constexpr int kTailCtas = 8;
 template <typename T>
-__global__ void __cluster_dims__(kTailCtas, 1, 1) __launch_bounds__(256) super_tail_kernel(SuperDev D, uint8_t *__restrict__ dst, int lv0) {
+__global__ void __cluster_dims__(kTailCtas, 1, 1) __launch_bounds__(512) super_tail_kernel(SuperDev D, uint8_t *__restrict__ dst, int lv0) {
     const uint32_t cl = blockIdx.x / kTailCtas, rank = blockIdx.x % kTailCtas;
     const int plane = (int)(cl % 3);
     const int64_t f = cl / 3;
-    const int warps = kTailCtas * 8, warp = (int)(rank * 8 + (threadIdx.x >> 5));
+    const int warps = kTailCtas * 16, warp = (int)(rank * 16 + (threadIdx.x >> 5));
     for (int lv = lv0; lv + 1 < D.levels; lv++) {
         const LevelPlane p = level_plane(D, nullptr, dst, plane, f, lv, false);
         if (p.dst_h > 0) {
@@ -1339,29 +1399,39 @@ int launch_super_flat(const SuperDev &D, const uint8_t *src, uint8_t *dst, int n
         const int64_t sub = hs * (int)sizeof(T);
         all = (sub & 15) == 0;
         const int64_t bytes = all ? sub : sub * nsub;
-        return (uint32_t)((bytes / 16 + 1 + kTile) / kTile);
+        return (uint32_t)((bytes / 16 + 1 + F.tile) / F.tile);
     };
+    F.tile = (int64_t)nframes * D.frame_bytes >= (int64_t)sms * 6 * 1024 * 16 ? 1024 : 256;
     F.ty = tiles((int64_t)D.width * D.height, F.all_y);
     F.tc = tiles((int64_t)(D.width / 2) * (D.height / 2), F.all_c);
     F.per = F.ty + 2 * F.tc;
     F.total = F.per * (uint32_t)nframes;
-    const int64_t want = std::max<int64_t>(F.total, (I.total + 7) / 8);
-    super_flat_kernel<T><<<(int)std::min<int64_t>(want, (int64_t)sms * per_sm), 256, 0, stream>>>(
-        D, src, dst, src + D.src_frame_bytes * nframes, I, F);
-    int n = 1, lv = 1;
+    int n = 1;
+    const uint8_t *src_end = src + D.src_frame_bytes * nframes;
+    if (F.tile == 1024) {
+        super_level0_flat_kernel<T><<<sms * 6, 256, 0, stream>>>(D, src, dst, src_end, F);
+        if (I.total) {
+            super_level_kernel<T><<<(int)std::min<int64_t>((I.total + 7) / 8, (int64_t)sms * per_sm), 256, 0, stream>>>(D, src, dst, I);
+            n++;
+        }
+    } else {
+        const int64_t want = std::max<int64_t>(F.total, (I.total + 7) / 8);
+        super_flat_kernel<T><<<(int)std::min<int64_t>(want, (int64_t)sms * per_sm), 256, 0, stream>>>(D, src, dst, src_end, I, F);
+    }
+    int lv = 1;
     for (; lv + 1 < D.levels && (int64_t)D.lw[lv + 1] * D.lh[lv + 1] > kTailSamples; lv++) {
         const LevelItems L = level_items(D, lv, nframes, sms);
-        super_level_kernel<T><<<(int)std::min<int64_t>((L.total + 7) / 8, (int64_t)sms * per_sm), 256, 0, stream>>>(D, dst, L);
+        super_level_kernel<T><<<(int)std::min<int64_t>((L.total + 7) / 8, (int64_t)sms * per_sm), 256, 0, stream>>>(D, nullptr, dst, L);
         n++;
     }
     if (nframes > kTailFrames)  // enough work for a launch per level
         for (; lv + 1 < D.levels; lv++) {
             const LevelItems L = level_items(D, lv, nframes, sms);
-            super_level_kernel<T><<<(int)std::min<int64_t>((L.total + 7) / 8, (int64_t)sms * per_sm), 256, 0, stream>>>(D, dst, L);
+            super_level_kernel<T><<<(int)std::min<int64_t>((L.total + 7) / 8, (int64_t)sms * per_sm), 256, 0, stream>>>(D, nullptr, dst, L);
             n++;
         }
     if (lv + 1 < D.levels) {
-        super_tail_kernel<T><<<nframes * 3 * kTailCtas, 256, 0, stream>>>(D, dst, lv);
+        super_tail_kernel<T><<<nframes * 3 * kTailCtas, 512, 0, stream>>>(D, dst, lv);
         n++;
     }
     return n;
