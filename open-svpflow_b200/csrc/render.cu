@@ -265,6 +265,31 @@ __device__ __forceinline__ int32_t alpha_at(const RenderJob &J, const RenderPlan
     return clamp_byte(interp_pair(m0, m1, p.block_w, p.x_shift, sxw[min(px - bx, kMaxBlock - 1)]));
 }
 
+// One output sample from its displaced samples v (set by set), the alphas of masks a and b, the last
+// alpha (the mode's mask, or the final one) and the undisplaced samples. See render_kernel.
+template <int KIND, bool MASK>
+__device__ __forceinline__ int32_t combine(const RenderJob &J, const int32_t (&v)[4], const int32_t (&alpha)[3], int32_t last,
+                                           int32_t c0, int32_t c1) {
+    if (KIND == 3) {  // mode23_pixel: base0, base1, next0, prev1 samples
+        const int32_t lo = min(v[0], v[1]), hi = max(v[0], v[1]);
+        const int32_t i0 = blend255(v[0], min(max(v[3], lo), hi), alpha[0]);
+        const int32_t i1 = blend255(v[1], min(max(v[2], lo), hi), alpha[1]);
+        const int32_t o = blend256(i0, i1, J.threshold);
+        return MASK ? blend255(o, blend256(c0, c1, J.threshold), last) : o;
+    }
+    if (KIND == 2) {  // mode21_or_22_pixel
+        const int32_t ea = blend255(v[0], v[1], alpha[0]), eb = blend255(v[1], v[0], alpha[1]);
+        const int32_t o = J.mode22 ? min(max(blend256(c0, c1, J.threshold), min(ea, eb)), max(ea, eb)) : blend256(ea, eb, J.threshold);
+        return MASK ? blend255(o, blend256(c0, c1, J.threshold_limit), last) : o;
+    }
+    if (KIND == 1) {  // mode11_or_13_pixel
+        const int32_t bl = blend256(c0, c1, J.threshold);
+        const int32_t o = J.mode13 ? min(max(bl, min(v[0], v[1])), max(v[0], v[1])) : blend256(v[0], v[1], J.threshold);
+        return MASK ? blend255(o, bl, last) : o;
+    }
+    return MASK ? blend255(v[0], c0, last) : v[0];  // mode1_pixel
+}
+
 // KIND 0: the single warp (source 0, set 0; mode1_pixel with the mask when MASK). KIND 1: the
 // two-source blend of algorithms 11 / 13 (set 0 reads source 0, set 1 source 1; mode11_or_13_pixel,
 // max_mask when MASK). KIND 2: algorithms 21 / 22 (the same reads; mode21_or_22_pixel with alphas from
@@ -373,29 +398,12 @@ __global__ void __launch_bounds__(256, KIND == 0 ? (MASK ? 4 : 5) : (KIND == 1 ?
     int32_t out[kPx];
 #pragma unroll
     for (int k = 0; k < kPx; k++) {
-        int32_t o;
-        if (KIND == 3) {  // mode23_pixel: a, b, c, d = base0, base1, next0, prev1 samples
-            const int32_t a = v[0][k], b = v[1 % NS][k], c = v[2 % NS][k], d = v[3 % NS][k];
-            const int32_t lo = min(a, b), hi = max(a, b);
-            const int32_t i0 = blend255(a, min(max(d, lo), hi), alpha[0][k]);
-            const int32_t i1 = blend255(b, min(max(c, lo), hi), alpha[1 % NA][k]);
-            o = blend256(i0, i1, J.threshold);
-            if (MASK) o = blend255(o, blend256(c0[k], c1[k], J.threshold), alpha[NA - 1][k]);
-        } else if (KIND == 2) {  // mode21_or_22_pixel
-            const int32_t v0 = v[0][k], v1 = v[1 % NS][k];
-            const int32_t ea = blend255(v0, v1, alpha[0][k]), eb = blend255(v1, v0, alpha[1 % NA][k]);
-            if (J.mode22) o = min(max(blend256(c0[k], c1[k], J.threshold), min(ea, eb)), max(ea, eb));
-            else o = blend256(ea, eb, J.threshold);
-            if (MASK) o = blend255(o, blend256(c0[k], c1[k], J.threshold_limit), alpha[NA - 1][k]);
-        } else if (KIND == 1) {  // mode11_or_13_pixel
-            const int32_t v0 = v[0][k], v1 = v[1 % NS][k];
-            const int32_t bl = blend256(c0[k], c1[k], J.threshold);
-            if (J.mode13) o = min(max(bl, min(v0, v1)), max(v0, v1));  // mode13_pixel
-            else o = blend256(v0, v1, J.threshold);                     // mode11_pixel
-            if (MASK) o = blend255(o, bl, alpha[0][k]);
-        } else {
-            o = MASK ? blend255(v[0][k], c0[k], alpha[0][k]) : v[0][k];  // mode1_pixel
-        }
+        int32_t vk[4], ak[3];
+#pragma unroll
+        for (int q = 0; q < 4; q++) vk[q] = v[q % NS][k];
+#pragma unroll
+        for (int a = 0; a < 3; a++) ak[a] = NA > 0 ? alpha[a % (NA > 0 ? NA : 1)][k] : 0;
+        const int32_t o = combine<KIND, MASK>(J, vk, ak, NA > 0 ? alpha[NA > 0 ? NA - 1 : 0][k] : 0, c0[k], c1[k]);
         out[k] = o;
     }
     uint8_t *dst = p.dst + (int64_t)py * p.dst_stride + px0;
@@ -403,6 +411,153 @@ __global__ void __launch_bounds__(256, KIND == 0 ? (MASK ? 4 : 5) : (KIND == 1 ?
     for (int k = 0; k < kPx; k++)
         if (px0 + k <= pxl) dst[k] = (uint8_t)out[k];
     }
+}
+
+// The same frame where motion is interpolated over power-of-two shifts, the grid starts at the blocks'
+// own origin and the planes cover every clamped position (tiled_ok): SmoothFps's usual render. A CTA renders
+// kTileW x kTileH samples. The motion samples around them are scaled once, x and y biased to 0 .. 2047 and
+// packed into one word (and the masks' bytes two to a word), in shared memory; a thread owns one column of
+// kTileH / 2 samples, so its horizontal weights and motion words stay in registers from row to row, and
+// each interpolation is two multiply-adds for both components: with the bias the fields stay in 0 .. 65504,
+// so nothing carries from one into the other. Positions are always clamped: where the reference reads
+// directly they lie inside. All offsets fit 32 bits.
+// Bound: instruction issue and the latency of a row's gathers, about 150 instructions per sample with two
+// sources (24 us per 1080p frame of algorithm 13) against 280 (49 us) with a thread that finds its tile,
+// scales its motion and computes 64-bit offsets for eight samples of one row. 32 rows per CTA (26 us), 8
+// rows (26 us) and rows taken two or four at a time (28 us) measured slower.
+constexpr int kTileW = 128, kTileH = 16;
+template <int KIND, bool MASK, int SHIFT>
+__global__ void __launch_bounds__(2 * kTileW) render_tile_kernel(const __grid_constant__ RenderJob J) {
+    constexpr bool DUAL = KIND > 0;
+    constexpr int NS = KIND == 0 ? 1 : (KIND == 3 ? 4 : 2);          // motion sets
+    constexpr int NA = KIND >= 2 ? (MASK ? 3 : 2) : (MASK ? 1 : 0);  // alphas per sample
+    constexpr int NM = (NA + 1) / 2;                                 // mask words
+    extern __shared__ uint32_t tab[];  // [NS + NM][rows][columns] of the motion grid around the CTA's samples
+    __shared__ int2 sxw[kMaxBlock], syw[kMaxBlock];
+    const RenderPlane &p = J.pl[blockIdx.z];
+    const int32_t X0 = blockIdx.x * kTileW, Y0 = blockIdx.y * kTileH;
+    if (X0 >= p.width || Y0 >= p.height) return;
+    const int tid = threadIdx.x;
+    if (tid < kMaxBlock) {
+        sxw[tid] = make_int2(p.xw[tid][0], p.xw[tid][1]);
+        syw[tid] = make_int2(p.yw[tid][0], p.yw[tid][1]);
+    }
+    int32_t g, base, len, cl, cr, rl, rr;
+    tile_of(X0, p.origin_x, p.block_w, p.bw_log2, p.width, J.grid_w, g, base, len);
+    cl = max(g, 0);
+    tile_of(min(X0 + kTileW, p.width) - 1, p.origin_x, p.block_w, p.bw_log2, p.width, J.grid_w, g, base, len);
+    cr = g < 0 ? 0 : min(g + 1, J.grid_w - 1);
+    tile_of(Y0, p.origin_y, p.block_h, p.bh_log2, p.height, J.grid_h, g, base, len);
+    rl = max(g, 0);
+    tile_of(min(Y0 + kTileH, p.height) - 1, p.origin_y, p.block_h, p.bh_log2, p.height, J.grid_h, g, base, len);
+    rr = g < 0 ? 0 : min(g + 1, J.grid_h - 1);
+    const int nc = cr - cl + 1, n = nc * (rr - rl + 1);
+    const bool chroma = p.x_div == 2;
+    for (int t = tid; t < n; t += 2 * kTileW) {
+        const int64_t i = (int64_t)(rl + t / nc) * J.grid_w + cl + t % nc;
+#pragma unroll
+        for (int k = 0; k < NS; k++) {
+            int32_t mx = motion(J, J.mx[k], i, J.lut_t[k]), my = motion(J, J.my[k], i, J.lut_t[k]);
+            if (chroma) { mx /= 2; my /= 2; }
+            tab[k * n + t] = (uint32_t)(mx + 1024) | ((uint32_t)(my + 1024) << 16);
+        }
+        if (NA == 1) tab[NS * n + t] = (uint32_t)mask_at(J, KIND >= 2 ? 0 : -1, i);
+        if (NA >= 2) tab[NS * n + t] = (uint32_t)mask_at(J, 0, i) | ((uint32_t)mask_at(J, 1, i) << 16);
+        if (NA == 3) tab[(NS + 1) * n + t] = (uint32_t)mask_at(J, 2, i);
+    }
+    __syncthreads();
+    const int32_t px = X0 + (tid & (kTileW - 1));
+    if (px >= p.width) return;
+    int32_t gx, bx, tw;
+    tile_of(px, p.origin_x, p.block_w, p.bw_log2, p.width, J.grid_w, gx, bx, tw);
+    const int c0 = max(gx, 0) - cl, c1 = c0 + (gx >= 0 && gx != J.grid_w - 1);
+    const int2 wx = sxw[min(px - bx, kMaxBlock - 1)];
+    const int shx = p.x_shift, shy = p.y_shift;
+    // weights whose sum falls short of the shift's scale: what brings the bias back to 1024
+    const uint32_t kx = 1024u * (uint32_t)((1 << shx) - wx.x - wx.y) * 0x10001u;
+    const int32_t xs0 = px * p.step - 1024;
+    const uint32_t mask = (1u << SHIFT) - 1u;
+    uint32_t w[NS + NM > 0 ? NS + NM : 1][4];
+    int32_t gy = 0, by = 0, th = 0;
+    const int32_t py0 = Y0 + (tid / kTileW) * (kTileH / 2), py1 = min(py0 + kTileH / 2, p.height);
+    uint8_t *dst = p.dst + (int64_t)py0 * p.dst_stride + px;
+    const bool bases = KIND == 0 ? MASK : (KIND == 1 ? (MASK || J.mode13) : (KIND == 2 ? (MASK || J.mode22) : MASK));
+    const uint32_t st0 = (uint32_t)p.src[0].stride, st1 = (uint32_t)p.src[1].stride;
+    const uint32_t sp0 = (uint32_t)p.src[0].span, sp1 = (uint32_t)p.src[1].span;
+    const uint32_t bx0 = SHIFT ? (uint32_t)px : (uint32_t)(px * p.step), bst = SHIFT ? 1u : (uint32_t)p.step;
+    uint32_t b0 = (uint32_t)py0 * bst * st0 + bx0, b1 = (uint32_t)py0 * bst * st1 + bx0;  // the undisplaced samples
+    int32_t ysb = py0 * p.step - 1024;
+#pragma unroll 1
+    for (int32_t py = py0; py < py1; py++, dst += p.dst_stride, b0 += bst * st0, b1 += bst * st1, ysb += p.step) {
+        if (py == py0 || (gy < 0 ? py >= p.origin_y : (py - by >= p.block_h && gy < J.grid_h - 1))) {
+            tile_of(py, p.origin_y, p.block_h, p.bh_log2, p.height, J.grid_h, gy, by, th);
+            const int r0 = (max(gy, 0) - rl) * nc, r1 = r0 + (gy >= 0 && gy != J.grid_h - 1 ? nc : 0);
+#pragma unroll
+            for (int k = 0; k < NS + NM; k++) {
+                const uint32_t *t = tab + k * n;
+                w[k][0] = t[r0 + c0]; w[k][1] = t[r0 + c1]; w[k][2] = t[r1 + c0]; w[k][3] = t[r1 + c1];
+            }
+        }
+        const int2 wy = syw[min(py - by, kMaxBlock - 1)];
+        const uint32_t ky = 1024u * (uint32_t)((1 << shy) - wy.x - wy.y) * 0x10001u;
+        uint32_t idx[4];
+#pragma unroll
+        for (int k = 0; k < NS; k++) {
+            const uint32_t a = (((uint32_t)wy.x * w[k][0] + (uint32_t)wy.y * w[k][2] + ky) >> shy) & 0x07FF07FFu;
+            const uint32_t b = (((uint32_t)wy.x * w[k][1] + (uint32_t)wy.y * w[k][3] + ky) >> shy) & 0x07FF07FFu;
+            const uint32_t d = ((uint32_t)wx.x * a + (uint32_t)wx.y * b + kx) >> shx;
+            const int32_t xs = min(max(xs0 + (int32_t)(d & 0x7FFu), 0), p.max_x);
+            const int32_t ys = min(max(ysb + (int32_t)(d >> 16), 0), p.max_y);
+            idx[k] = (uint32_t)(ys >> SHIFT) * ((k & 1) ? st1 : st0) + (uint32_t)(xs >> SHIFT);
+            if (SHIFT) idx[k] += ((((uint32_t)ys & mask) << SHIFT) | ((uint32_t)xs & mask)) * ((k & 1) ? sp1 : sp0);
+        }
+        int32_t v[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int k = 0; k < NS; k++) v[k] = __ldg(p.src[k & 1].p + idx[k]);
+        int32_t u0 = 0, u1 = 0;
+        if (bases) {  // the undisplaced samples
+            u0 = __ldg(p.src[0].p + b0);
+            if (DUAL) u1 = __ldg(p.src[1].p + b1);
+        }
+        int32_t alpha[3] = {0, 0, 0}, last = 0;
+#pragma unroll
+        for (int j = 0; j < NM; j++) {
+            const uint32_t a = (((uint32_t)wy.x * w[NS + j][0] + (uint32_t)wy.y * w[NS + j][2]) >> shy) & 0x00FF00FFu;
+            const uint32_t b = (((uint32_t)wy.x * w[NS + j][1] + (uint32_t)wy.y * w[NS + j][3]) >> shy) & 0x00FF00FFu;
+            const uint32_t d = ((uint32_t)wx.x * a + (uint32_t)wx.y * b) >> shx;
+            alpha[j == 0 ? 0 : 2] = (int32_t)(d & 0xFFu);
+            if (j == 0) alpha[1] = (int32_t)((d >> 16) & 0xFFu);
+        }
+        if (NA > 0) last = alpha[NA - 1];
+        *dst = (uint8_t)combine<KIND, MASK>(J, v, alpha, last, u0, u1);
+    }
+}
+// May the frame go through render_tile_kernel? If so, the shared memory its largest table takes.
+bool tiled_ok(const RenderJob &J, int kind, bool mask, size_t &smem) {
+    if (!J.interp || J.zero_origin) return false;
+    const int ns = kind == 0 ? 1 : (kind == 3 ? 4 : 2), na = kind >= 2 ? (mask ? 3 : 2) : (mask ? 1 : 0);
+    smem = 0;
+    for (int pl = 0; pl < 3; pl++) {
+        const RenderPlane &p = J.pl[pl];
+        if (p.width <= 0 || p.height <= 0 || p.block_w <= 0 || p.block_h <= 0) continue;  // the plane is not drawn
+        if (p.x_shift < 0 || p.y_shift < 0 || p.step <= 0 || p.origin_x < 0 || p.origin_y < 0) return false;
+        for (int i = 0; i < kMaxBlock; i++)
+            if (p.xw[i][0] < 0 || p.xw[i][1] < 0 || p.yw[i][0] < 0 || p.yw[i][1] < 0 ||
+                p.xw[i][0] + p.xw[i][1] > (1 << p.x_shift) || p.yw[i][0] + p.yw[i][1] > (1 << p.y_shift))
+                return false;
+        for (int s = 0; s < (kind > 0 ? 2 : 1); s++)
+            if (!p.src[s].covers || p.src[s].len >= (1ll << 31)) return false;  // every offset read is below len
+        const int64_t n = ((int64_t)kTileW / p.block_w + 4) * ((int64_t)kTileH / p.block_h + 4);
+        const size_t bytes = (size_t)n * 4 * (size_t)(ns + (na + 1) / 2);
+        if (bytes > smem) smem = bytes;
+    }
+    return smem <= (40u << 10);
+}
+template <int KIND, bool MASK>
+void launch_tiled(const RenderJob &J, dim3 grid, size_t smem, cudaStream_t st) {
+    if (J.shift == 0) render_tile_kernel<KIND, MASK, 0><<<grid, 2 * kTileW, smem, st>>>(J);
+    else if (J.shift == 1) render_tile_kernel<KIND, MASK, 1><<<grid, 2 * kTileW, smem, st>>>(J);
+    else render_tile_kernel<KIND, MASK, 2><<<grid, 2 * kTileW, smem, st>>>(J);
 }
 
 // Per-plane constants of one frame (plane_params for chroma = plane > 0), the sources' layouts and
@@ -435,8 +590,13 @@ int setup(RenderJob &J, const svpf_render_config *cfg, int nsrc, const uint8_t *
         p.step = cfg->source_step;
         p.max_x = sat_step_max(p.width, p.step);
         p.max_y = sat_step_max(p.height, p.step);
-        weights(p.block_w, p.x_shift, p.xw);
-        weights(p.block_h, p.y_shift, p.yw);
+        if (pl == 2) {  // the same blocks as the first chroma plane
+            memcpy(p.xw, J.pl[1].xw, sizeof(p.xw));
+            memcpy(p.yw, J.pl[1].yw, sizeof(p.yw));
+        } else {
+            weights(p.block_w, p.x_shift, p.xw);
+            weights(p.block_h, p.y_shift, p.yw);
+        }
         p.bw_log2 = p.block_w > 0 && (p.block_w & (p.block_w - 1)) == 0 ? 31 - __builtin_clz((unsigned)p.block_w) : -1;
         p.bh_log2 = p.block_h > 0 && (p.block_h & (p.block_h - 1)) == 0 ? 31 - __builtin_clz((unsigned)p.block_h) : -1;
         if (!p.dst || p.dst_stride < p.width) return SVPF_EINVAL;
@@ -487,7 +647,14 @@ int launch(const RenderJob &J, int kind, bool mask, int32_t most_w, int32_t most
     if (most_w > 0 && most_h > 0) {
         dim3 grid((unsigned)((most_w + 256 * kPx * kBatch - 1) / (256 * kPx * kBatch)), (unsigned)most_h, 3);
         cudaStream_t st = (cudaStream_t)stream;
-        if (kind == 3) {
+        size_t smem = 0;
+        if (tiled_ok(J, kind, mask, smem)) {
+            const dim3 tg((unsigned)((most_w + kTileW - 1) / kTileW), (unsigned)((most_h + kTileH - 1) / kTileH), 3);
+            if (kind == 3) mask ? launch_tiled<3, true>(J, tg, smem, st) : launch_tiled<3, false>(J, tg, smem, st);
+            else if (kind == 2) mask ? launch_tiled<2, true>(J, tg, smem, st) : launch_tiled<2, false>(J, tg, smem, st);
+            else if (kind == 1) mask ? launch_tiled<1, true>(J, tg, smem, st) : launch_tiled<1, false>(J, tg, smem, st);
+            else mask ? launch_tiled<0, true>(J, tg, smem, st) : launch_tiled<0, false>(J, tg, smem, st);
+        } else if (kind == 3) {
             if (mask) render_kernel<3, true><<<grid, 256, 0, st>>>(J);
             else render_kernel<3, false><<<grid, 256, 0, st>>>(J);
         } else if (kind == 2) {
