@@ -114,6 +114,9 @@ struct Search {
     int hbx, hby, hdir, hi, hrad, hret, bad_r, bad_max;
     unsigned found;
     int sets_mv;
+    int rx, ry;                             // a walk: the outcome before a bad-SAD expansion made ahead of the test
+    unsigned rsad;
+    long long rcost;
 };
 
 // Shared state of one search direction. A block is searched by a group of warps: the whole
@@ -1633,11 +1636,14 @@ __device__ __forceinline__ void search_level(const Ctx &x, DirSh &s, DirScratch 
 // blocks repeat it (noisy fields), waiting for each in turn was the larger part of the walk.
 //
 // The bad-SAD test needs the number of bad blocks before this one. Its threshold only grows with
-// that number, so a block at or below the first threshold is not bad whatever the number; any other
+// that number, so a block that is not bad by the number known so far is not bad; any other
 // waits until every earlier block has passed its test (each warp publishes the next block it has not
 // tested, in the histogram's words, which are free while a level is searched) and then reads the
-// number. The lowest block that is not finished waits for nothing, and every warp takes its blocks in
-// order, so the warps, all resident, always make progress; the waits are bounded all the same.
+// number. The expansion of a block that looks bad runs before that, while its seeds may still change
+// (it is what such a block mostly does: at 640x360 the coarser levels took 2.5 to 3 times as long with
+// the expansions one after another). The lowest block that is not finished waits for nothing, and every
+// warp takes its blocks in order, so the warps, all resident, always make progress; the waits are
+// bounded all the same.
 // A level with an input on which the reference would panic takes search_level instead.
 // stats (nullable): [0] blocks, [1] blocks that started before all their processed neighbours were
 // final, [2] seeds evaluated after the start (the others had the vector of a candidate already
@@ -1778,7 +1784,8 @@ __device__ __forceinline__ void walk_level(const Ctx &x, SH &s, const DirScratch
         int base = 0, win = -1;
         bool stepping = false;
         int bad_count = 0;
-        bool final = false;
+        bool final = false, expanded = false;
+        const bool may_be_bad = level > 0 && P.coarse_bad_sad > 0;
         // Each turn evaluates up to 32 candidates, one per lane: special ones that are new, else the next
         // of the search step in work (one call site of the evaluation, which is inlined). While a search
         // runs, seeds that have become final are looked at between its turns; tentative ones only when
@@ -1788,6 +1795,19 @@ __device__ __forceinline__ void walk_level(const Ctx &x, SH &s, const DirScratch
                 if (search_next(q, x, b, idx, bad_count, g_)) { stepping = true; base = 0; win = -1; }
                 else {
                     if (final) break;
+                    // ---- the refinement is done. The bad-SAD expansion depends on its outcome and on the
+                    // test alone, so it runs at once where the count of bad blocks known by now makes the
+                    // block bad, and the outcome before it is kept in case the exact count says otherwise.
+                    if (may_be_bad && !expanded && idx > 1 && (int)q.bsad > P.coarse_bad_sad) {
+                        const int known = ld_word(ctl + CTL_BAD);
+                        if ((int)q.bsad > bad_limit(P, known)) {
+                            q.rx = q.bmx; q.ry = q.bmy; q.rsad = q.bsad; q.rcost = q.bcost;
+                            expanded = true;
+                            bad_count = known;
+                            search_begin(q, RS_BAD_ONLY);
+                            continue;
+                        }
+                    }
                     if (openm) {  // publish, then wait for news
                         if (!published && lane == 0) st_tag(ds.keys + idx, tag_word(TAG_TENTATIVE, q.bmx, q.bmy));
                         published = true;
@@ -1810,9 +1830,12 @@ __device__ __forceinline__ void walk_level(const Ctx &x, SH &s, const DirScratch
                         continue;
                     }
                     final = true;  // every seed is final and is the one used
-                    if (!(level == 0 && P.distance == 0) && level > 0 && P.coarse_bad_sad > 0) {
-                        bool bad = false;
-                        if (idx > 1 && (int)q.bsad > P.coarse_bad_sad) {  // above the threshold of a count of 0
+                    if (may_be_bad) {
+                        // The exact test. The count only grows, so a block that is not bad by what is known of it
+                        // is not bad; the others wait for every earlier block's test.
+                        const unsigned sad = expanded ? q.rsad : q.bsad;
+                        bool bad = idx > 1 && (int)sad > P.coarse_bad_sad && (int)sad > bad_limit(P, ld_word(ctl + CTL_BAD));
+                        if (bad) {
                             if (!spin([&] {
                                     bool ok = true;
                                     for (int h = lane; h < D; h += 32) ok = ok && (h == g || ld_word(progress + h) >= k);
@@ -1821,12 +1844,13 @@ __device__ __forceinline__ void walk_level(const Ctx &x, SH &s, const DirScratch
                                 late = true;
                             __threadfence();
                             bad_count = ld_word(ctl + CTL_BAD);
-                            bad = (int)q.bsad > bad_limit(P, bad_count);
+                            bad = (int)sad > bad_limit(P, bad_count);
                             if (bad && lane == 0) { st_word(ctl + CTL_BAD, bad_count + 1); __threadfence(); }
                             __syncwarp();
                         }
                         if (lane == 0) st_word(progress + g, k + D);
-                        if (bad) { search_begin(q, RS_BAD_ONLY); continue; }
+                        if (bad && !expanded) { search_begin(q, RS_BAD_ONLY); continue; }
+                        if (!bad && expanded) { q.bmx = q.rx; q.bmy = q.ry; q.bsad = q.rsad; q.bcost = q.rcost; }
                     }
                     break;
                 }
@@ -1892,7 +1916,7 @@ __device__ __forceinline__ void walk_level(const Ctx &x, SH &s, const DirScratch
                     q.bmx = nx; q.bmy = ny; q.bsad = nsad; q.bcost = (long long)nsad;
                     search_begin(q, search ? RS_REFINE_ONLY : RS_NONE);
                     stepping = false;
-                    published = false;
+                    published = expanded = false;
                 }
                 started = true;
             } else {
@@ -2640,7 +2664,7 @@ __global__ void __launch_bounds__(kPackThreads)
 }
 
 // Levels of fewer blocks than this are searched by the pair's CTA, without a launch of their own.
-constexpr int kWalkCells = 160;
+constexpr int kWalkCells = 30;
 
 // Persistent form: a grid sized to the resident CTAs drains the item list in order (the
 // host sorts it largest-first); each CTA pulls the next item with one atomic, copies the
