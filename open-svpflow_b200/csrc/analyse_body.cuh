@@ -1809,8 +1809,11 @@ __device__ __forceinline__ void walk_level(const Ctx &x, SH &s, const DirScratch
                         }
                     }
                     if (openm) {  // publish, then wait for news
-                        if (!published && lane == 0) st_tag(ds.keys + idx, tag_word(TAG_TENTATIVE, q.bmx, q.bmy));
+                        const unsigned long long word = tag_word(TAG_TENTATIVE, q.bmx, q.bmy);
+                        if (!published && lane == 0) st_tag(ds.keys + idx, word);
                         published = true;
+                        // not subject to the bad-SAD test: final as soon as its seeds are
+                        const bool sure = !expanded && (!may_be_bad || idx <= 1 || (int)q.bsad <= P.coarse_bad_sad);
                         const bool open = (openm >> lane) & 1u, act = (actm >> lane) & 1u;
                         const int mx = s.lmx[wi][lane], my = s.lmy[wi][lane];
                         unsigned long long v = 0;
@@ -1822,6 +1825,8 @@ __device__ __forceinline__ void walk_level(const Ctx &x, SH &s, const DirScratch
                             }, ctl + CTL_LATE)) {
                             late = true;
                             openm = 0;
+                        } else if (!freshm && sure) {  // the next block in the chain waits for this store
+                            if (lane == 0) st_tag(ds.keys + idx, word ^ ((unsigned long long)(TAG_TENTATIVE ^ TAG_FINAL) << 32));
                         }
                         openm &= ~__ballot_sync(kFull, (int)(v >> 32) == TAG_FINAL);
                         actm |= freshm;
