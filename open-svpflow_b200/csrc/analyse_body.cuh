@@ -1306,7 +1306,6 @@ struct DirScratch {
     int *pos;
     unsigned long long *keys;
     unsigned *hist;
-    uint8_t *seen;
 };
 __device__ __forceinline__ int2 vmv(uint2 v) { return make_int2((int)(short)(v.x & 0xFFFF), (int)(short)(v.x >> 16)); }
 __device__ __forceinline__ uint2 mkvec(int dx, int dy, unsigned score) {
@@ -2201,45 +2200,115 @@ __device__ void global_doubled(const Ctx &x, DirSh &s, const uint2 *field, int64
 }
 
 // reorder_search_order (:404-419): stable sort of the interior cells by score >> shift
-__device__ void reorder(const Ctx &x, DirSh &s, const uint2 *field, int gw, int gh, DirScratch &ds, int *status) {
-    const int64_t count = (int64_t)(gw - 1) * (gh - 1);
-    if (count > s.order_len) {
+// (`sorted`: the next level takes its order from this one's, as all but level 0 do)
+__device__ void reorder(const Ctx &x, DirSh &s, const uint2 *field, int gw, int gh, DirScratch &ds, int *status, bool sorted) {
+    const unsigned count = (unsigned)(gw - 1) * (unsigned)(gh - 1);
+    if ((int64_t)count > s.order_len) {
         if (x.tid == 0) { atomicOr(status, ST_PANIC); s.abort_ = 1; }
         dbar(x.d);
         return;
     }
+    if (!sorted) return;
     unsigned v = (unsigned)imax(x.P->block_w * x.P->block_h / 8, 1), lg = 0;
     while (v >>= 1) lg++;
     const unsigned shift = lg + 1;
-    int64_t np = 1;
-    while (np < count) np <<= 1;
+    int lgn = 5;
+    while ((1u << lgn) < count) lgn++;
+    const unsigned np = 1u << lgn;
     unsigned long long *keys = ds.keys;
-    for (int64_t i = x.tid; i < np; i += NT) {
+    for (unsigned i = (unsigned)x.tid; i < np; i += NT) {
         if (i < count) {
-            const int xx = (int)(i % (gw - 1)), yy = (int)(i / (gw - 1));
-            keys[i] = ((unsigned long long)(field[(int64_t)yy * gw + xx].y >> shift) << 32) | (unsigned long long)i;
+            const unsigned xx = i % (unsigned)(gw - 1), yy = i / (unsigned)(gw - 1);
+            keys[i] = ((unsigned long long)(field[yy * (unsigned)gw + xx].y >> shift) << 32) | (unsigned long long)i;
         } else {
             keys[i] = ~0ull;
         }
     }
     dbar(x.d);
-    for (int64_t kk = 2; kk <= np; kk <<= 1)
-        for (int64_t j = kk >> 1; j > 0; j >>= 1) {
-            for (int64_t i = x.tid; i < np; i += NT) {
-                const int64_t l = i ^ j;
-                if (l > i) {
-                    const unsigned long long a = keys[i], b = keys[l];
-                    const bool up = (i & kk) == 0;
-                    if ((a > b) == up) { keys[i] = b; keys[l] = a; }
-                }
+    // Bitonic sort: the steps between keys 32 and more apart in memory, those within 32 in a warp's
+    // registers, one pass for a stage's five (2048 keys: 27 passes with barriers between in place of 66).
+    const int lane = x.tid & 31;
+    for (int stage = 5; stage <= lgn; stage++) {  // the first sorts runs of 32 outright
+        for (int lj = stage - 1; lj >= 5; lj--) {
+            const unsigned j = 1u << lj;
+            for (unsigned i = (unsigned)x.tid; i < np / 2; i += NT) {
+                const unsigned lo = ((i >> lj) << (lj + 1)) | (i & (j - 1)), hi = lo + j;
+                const unsigned long long a = keys[lo], b = keys[hi];
+                if ((a > b) == (((lo >> stage) & 1u) == 0)) { keys[lo] = b; keys[hi] = a; }
             }
             dbar(x.d);
         }
-    for (int64_t i = x.tid; i < count; i += NT) {
+        for (unsigned i = (unsigned)x.tid; i < np; i += NT) {
+            unsigned long long k = keys[i];
+            for (int st = stage == 5 ? 1 : stage; st <= stage; st++)
+                for (int lj = imin(st, 5) - 1; lj >= 0; lj--) {
+                    const unsigned long long o = __shfl_xor_sync(kFull, k, 1 << lj);
+                    const bool up = ((i >> st) & 1u) == 0, low = ((lane >> lj) & 1) == 0;
+                    if ((up == low) == (o < k)) k = o;
+                }
+            keys[i] = k;
+        }
+        dbar(x.d);
+    }
+    for (unsigned i = (unsigned)x.tid; i < count; i += NT) {
         const unsigned r = (unsigned)(keys[i] & 0xFFFFFFFFull);
         ds.order[i] = pack_xy((int)(r % (unsigned)(gw - 1)), (int)(r / (unsigned)(gw - 1)));
     }
     dbar(x.d);
+}
+
+// refine_search_order (:338-402): the children of the coarser level's sw x sh interior cells, in the order of
+// those (a permutation of them after reorder), inner cells of the grid first, then the cells on its inner
+// border, then its last row and column. Every cell of the dw x dh interior is the child of exactly one
+// coarse cell (those past twice the coarse grid, of the last column or row), so the places are two sums
+// over the coarse cells: each thread counts and then writes a run of them. What ran before the search of
+// a 1080p pair's second level was bound by one thread's chain through a mask of the cells seen, 0.55 ms;
+// it takes 0.10 so, with the sort above in fewer passes.
+__device__ void refine_order(const Ctx &x, DirSh &s, DirScratch &ds, int sw, int sh, int gw, int gh) {
+    const int dw = gw - 1, dh = gh - 1;
+    const int ex = imax(dw - 2 * sw, 0), ey = imax(dh - 2 * sh, 0);
+    const int n = sw > 0 && sh > 0 ? sw * sh : 0, run = (n + NT - 1) / NT;
+    const int first = imin(x.tid * run, n), last = imin(first + run, n);
+    const int lane = x.tid & 31;
+    uint32_t *to = ds.order2;
+    auto children = [&](int2 c, auto add) {
+        const int left = 2 * c.x, top = 2 * c.y;
+        auto one = [&](int cx, int cy) {
+            if (cx < dw && cy < dh) add(cx, cy, cx > 0 && cy > 0 && cx < dw - 1 && cy < dh - 1);
+        };
+        one(left, top); one(left + 1, top); one(left + 1, top + 1); one(left, top + 1);
+        if (c.x == sw - 1)
+            for (int dx = 2; dx < 2 + ex; dx++)
+                for (int dy = 0; dy < 2 + (c.y == sh - 1) * ey; dy++) one(left + dx, top + dy);
+        if (c.y == sh - 1)
+            for (int dy = 2; dy < 2 + ey; dy++)
+                for (int dx = 0; dx < 2; dx++) one(left + dx, top + dy);
+    };
+    int inner = 0, border = 0;
+    for (int k = first; k < last; k++) children(unpack_xy(ds.order[k]), [&](int, int, bool in) { inner += in; border += !in; });
+    long long mine = ((long long)border << 32) | inner, sum = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const long long v = __shfl_up_sync(kFull, sum, o);
+        if (lane >= o) sum += v;
+    }
+    if (lane == 31) s.r64[x.tid >> 5][0] = sum;
+    dbar(x.d);
+    long long before = sum - mine, total = 0;
+    for (int w = 0; w < NW; w++) {
+        if (w < (x.tid >> 5)) before += s.r64[w][0];
+        total += s.r64[w][0];
+    }
+    const int ninner = (int)total, nborder = (int)(total >> 32);
+    int pi = (int)before, pb = ninner + (int)(before >> 32);
+    for (int k = first; k < last; k++)
+        children(unpack_xy(ds.order[k]), [&](int cx, int cy, bool in) { to[in ? pi++ : pb++] = pack_xy(cx, cy); });
+    const int base = ninner + nborder;
+    for (int k = x.tid; k <= dw + dh; k += NT) to[base + k] = k <= dw ? pack_xy(k, dh) : pack_xy(dw, k - dw - 1);
+    const int len = base + dw + 1 + dh;
+    dbar(x.d);
+    if (x.tid == 0) s.order_len = len;
+    for (int k = x.tid; k < len; k += NT) ds.order[k] = to[k];
 }
 
 __device__ __forceinline__ DirScratch dir_scratch(const AnalyseParams &P, uint8_t *scr, int d) {
@@ -2255,7 +2324,6 @@ __device__ __forceinline__ DirScratch dir_scratch(const AnalyseParams &P, uint8_
     ds.pos = (int *)(scr + P.off_pos[d]);
     ds.keys = (unsigned long long *)(scr + P.off_keys[d]);
     ds.hist = (unsigned *)(scr + P.off_hist[d]);
-    ds.seen = scr + P.off_seen[d];
     return ds;
 }
 
@@ -2336,7 +2404,7 @@ __device__ __forceinline__ void analyse_pair_dev(const AnalyseParams &P, const P
         const LevelInfo &L = P.lv[level];
         const uint2 *f = ds.vec[level & 1];
         global_doubled(x, s, f, (int64_t)L.gw * L.gh, ds.hist);
-        reorder(x, s, f, L.gw, L.gh, ds, status);
+        reorder(x, s, f, L.gw, L.gh, ds, status, level > 1);
     };
     if (resume) {
         pgw = P.lv[hi + 1].gw; pgh = P.lv[hi + 1].gh;
@@ -2359,41 +2427,8 @@ __device__ __forceinline__ void analyse_pair_dev(const AnalyseParams &P, const P
                     ds.order[k] = pack_xy(b.x, b.y);
                 }
                 if (tid == 0) s.order_len = (int)n0;
-            } else {  // refine_search_order (:338-402), serial
-                for (int64_t i = tid; i < ncell; i += NT) ds.seen[i] = 0;
-                dbar(half);
-                if (tid == 0) {
-                    const int sw = pgw - 1, sh = pgh - 1, dw = gw - 1, dh = gh - 1;
-                    const int ex = imax(dw - 2 * sw, 0), ey = imax(dh - 2 * sh, 0);
-                    int64_t ni = 0, nb = 0;
-                    uint32_t *bnd = (uint32_t *)ds.keys;  // boundary list
-                    auto add = [&](int cx, int cy) {
-                        if (cx < 0 || cy < 0 || cx >= dw || cy >= dh) return;
-                        const int64_t ix = (int64_t)cy * gw + cx;
-                        if (ds.seen[ix]) return;
-                        ds.seen[ix] = 1;
-                        if (cx > 0 && cy > 0 && cx < dw - 1 && cy < dh - 1) ds.order2[ni++] = pack_xy(cx, cy);
-                        else bnd[nb++] = pack_xy(cx, cy);
-                    };
-                    for (int64_t k = 0; k < s.order_len; k++) {
-                        const int2 c = unpack_xy(ds.order[k]);
-                        if (c.x >= sw || c.y >= sh) continue;
-                        const int left = 2 * c.x, top = 2 * c.y;
-                        add(left, top); add(left + 1, top); add(left + 1, top + 1); add(left, top + 1);
-                        if (c.x == sw - 1)
-                            for (int dx = 2; dx < 2 + ex; dx++)
-                                for (int dy = 0; dy < 2 + (c.y == sh - 1) * ey; dy++) add(left + dx, top + dy);
-                        if (c.y == sh - 1)
-                            for (int dy = 2; dy < 2 + ey; dy++)
-                                for (int dx = 0; dx < 2; dx++) add(left + dx, top + dy);
-                    }
-                    for (int64_t i = 0; i < nb; i++) ds.order2[ni++] = bnd[i];
-                    for (int xx = 0; xx <= dw; xx++) ds.order2[ni++] = pack_xy(xx, dh);
-                    for (int yy = 0; yy < dh; yy++) ds.order2[ni++] = pack_xy(dw, yy);
-                    s.order_len = (int)ni;
-                }
-                dbar(half);
-                for (int64_t k = tid; k < s.order_len; k += NT) ds.order[k] = ds.order2[k];
+            } else {
+                refine_order(x, s, ds, pgw - 1, pgh - 1, gw, gh);
             }
             dbar(half);
             if (level > 0) {  // first position of every cell in the order ("processed" test)
@@ -2409,13 +2444,13 @@ __device__ __forceinline__ void analyse_pair_dev(const AnalyseParams &P, const P
             uint8_t *nl = ds.luma[level & 1];
             uint2 *pj = ds.proj[level & 1];
             if (first) {
-                for (int64_t i = tid; i < ncell; i += NT) { nf[i] = make_uint2(0, 0); nl[i] = 0; }
+                for (unsigned i = (unsigned)tid; i < (unsigned)ncell; i += NT) { nf[i] = make_uint2(0, 0); nl[i] = 0; }
             } else {
                 const uint2 *cf = ds.vec[(level + 1) & 1];
                 const uint8_t *cl = ds.luma[(level + 1) & 1];
                 const int cw = pgw - 1, ch = pgh - 1, pel = L.pel;
-                for (int64_t i = tid; i < ncell; i += NT) {
-                    const int xx = (int)(i % gw), yy = (int)(i / gw);
+                for (unsigned i = (unsigned)tid; i < (unsigned)ncell; i += NT) {
+                    const int xx = (int)(i % (unsigned)gw), yy = (int)(i / (unsigned)gw);
                     uint2 out = make_uint2(0, 0);
                     uint8_t ol = 0;
                     if (xx < gw - 1 && yy < gh - 1) {
@@ -2435,8 +2470,8 @@ __device__ __forceinline__ void analyse_pair_dev(const AnalyseParams &P, const P
                     ds.keys[i] = ~0ull;
                 }
                 dbar(half);
-                for (int64_t i = tid; i < ncell; i += NT) {
-                    const int xx = (int)(i % gw), yy = (int)(i / gw);
+                for (unsigned i = (unsigned)tid; i < (unsigned)ncell; i += NT) {
+                    const int xx = (int)(i % (unsigned)gw), yy = (int)(i / (unsigned)gw);
                     if (xx >= gw - 1 || yy >= gh - 1 || xx >= 2 * cw || yy >= 2 * ch) continue;
                     const uint2 p = cf[(int64_t)(yy >> 1) * pgw + (xx >> 1)];
                     if (p.y == 0xFFFFFFFFu) continue;  // `score < target.score` never holds
@@ -2448,7 +2483,7 @@ __device__ __forceinline__ void analyse_pair_dev(const AnalyseParams &P, const P
                     atomicMin(&ds.keys[(int64_t)ty * gw + tx], ((unsigned long long)p.y << 32) | (unsigned long long)i);
                 }
                 dbar(half);
-                for (int64_t i = tid; i < ncell; i += NT) {
+                for (unsigned i = (unsigned)tid; i < (unsigned)ncell; i += NT) {
                     const unsigned long long kk = ds.keys[i];
                     if (kk == ~0ull) pj[i] = make_uint2(0, 0xFFFFFFFFu);
                     else {

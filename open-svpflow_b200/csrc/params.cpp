@@ -151,7 +151,7 @@ bool build_analyse_params(const AnalyseOpts &o, const SuperLayout &Lay, AnalyseP
         return false;
     }
     // scratch layout per pair
-    int64_t np2 = 1;
+    int64_t np2 = 32;  // what the sort of the search order pads to
     while (np2 < max_cells) np2 <<= 1;
     P.max_cells = max_cells;
     P.max_order = max_order;
@@ -165,9 +165,8 @@ bool build_analyse_params(const AnalyseOpts &o, const SuperLayout &Lay, AnalyseP
         P.off_order[dd] = take(max_order * 4);
         P.off_order2[dd] = take(max_order * 4);
         P.off_pos[dd] = take(max_cells * 4);
-        P.off_keys[dd] = take(np2 * 8 > max_order * 4 ? np2 * 8 : max_order * 4);
+        P.off_keys[dd] = take(np2 * 8);
         P.off_hist[dd] = take(65536 * 4);
-        P.off_seen[dd] = take(max_cells);
         P.off_out[dd] = take(max_cells * 2);
         P.off_ctl[dd] = take(64);
     }

@@ -118,7 +118,7 @@ struct alignas(16) AnalyseParams {
     // per-pair scratch layout (bytes)
     int64_t max_cells, max_order;
     int64_t off_field[2], off_next[2], off_proj[2][2], off_order[2], off_order2[2], off_pos[2];
-    int64_t off_keys[2], off_hist[2], off_seen[2], off_out[2];
+    int64_t off_keys[2], off_hist[2], off_out[2];
     int64_t off_ctl[2];       // per direction: the words that go from launch to launch (CTL_*)
     int64_t scratch_per_pair;
 };
