@@ -27,6 +27,7 @@
 #include <cuda_runtime.h>
 #include <string.h>
 
+#include <algorithm>
 #include <atomic>
 #include <chrono>
 #include <condition_variable>
@@ -84,6 +85,7 @@ struct Request {
 struct svpf_server {
     int device = 0;
     int64_t budget = 0, used = 0, peak_used = 0;
+    int64_t grown = 0;                          // bytes the pool was grown by ahead of need (scheduler-owned)
     int max_active = 0, active = 0, peak_active = 0;
     int32_t chunk_pairs = 32;
     std::vector<cudaStream_t> streams;          // kLanes per slot
@@ -114,6 +116,8 @@ int sfail(int code, const std::string &msg) {
     set_last_error(msg);
     return code;
 }
+
+constexpr int64_t kGrowBytes = 1ll << 30;
 
 int64_t lanes_of(const Request &r) { return r.chunks.size() < (size_t)kLanes ? (int64_t)r.chunks.size() : kLanes; }
 
@@ -163,6 +167,16 @@ int enqueue(svpf_server *s, Request *r) {
     cudaStream_t st = lane[0];
     const int64_t fb = r->D.frame_bytes, sb = r->D.src_frame_bytes;
     const int64_t cmax = r->chunks.empty() ? 1 : r->chunks[0].count;
+    // Memory new to the pool takes the driver 3 to 60 ms to map, in which no other clip is queued: as long
+    // as four small clips take together (25 ms). So the pool grows by every slot's share at once, the first
+    // time a clip of a size comes, up to the budget and kGrowBytes; larger clips map what they need.
+    const int64_t share = std::min(std::min(s->budget, kGrowBytes), r->need * s->max_active);
+    if (share > s->grown && share >= r->need) {
+        void *p = nullptr;
+        if (cudaMallocAsync(&p, (size_t)share, st) == cudaSuccess) cudaFreeAsync(p, st);
+        else cudaGetLastError();  // the clip's own allocation decides
+        s->grown = share;
+    }
     cudaError_t e = cudaMallocAsync((void **)&r->dev, (size_t)r->need, st);
     if (e != cudaSuccess) {
         r->dev = nullptr;
