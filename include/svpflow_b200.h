@@ -121,8 +121,8 @@ int svpf_device_status(const void *scratch_dev, void *stream);
  * a bit set: 1 level 0, 2 the coarser levels, 4 (with 1) every level but the smallest ones
  * spread over the GPU in launches of their own, one CTA per warp, so every SM carries the same
  * share of the warps and a single pair still fills many of them. 0 turns it off; the default
- * is 5. Only the plain path and the server run it; batches always keep the serial order within
- * a pair. Affects launches made after the call. */
+ * is 5. Batches do not ask it: their shape "walk" always spreads the levels, the others never do.
+ * Affects launches made after the call. */
 int svpf_analyser_set_lookahead(svpf_analyser *a, int32_t levels);
 /* The look-ahead counters of the last device launch on `scratch_dev` (synchronises `stream`):
  * out[0] level-0 blocks, out[1] blocks that started before all their neighbour seeds were final,
@@ -296,8 +296,9 @@ int svpf_batch_run(svpf_batch *b, const uint8_t *const *frames, uint8_t *const *
  * synchronises that stream and reports. */
 int svpf_batch_launch(svpf_batch *b, void *stream);
 int svpf_batch_status(svpf_batch *b, void *stream);
-/* Launch shape: compiled variant (threads per search direction, see
- * svpf_analyse_variant_name) and 4x4 tiles per lane (2, 4 or 8). Results do not depend
+/* Launch shape: compiled variant ("walk", the default, or the threads per search direction of
+ * the form with a pair per CTA, see svpf_analyse_variant_name) and 4x4 tiles per lane (2, 4 or 8; kept
+ * and reported, without effect on the launch). Results do not depend
  * on it. svpf_batch_autotune times the shapes on the batch's largest pairs (frames must be
  * in place), keeps the fastest and remembers it per device and clip mix (and in the file
  * named by the SVPF_TUNE_CACHE environment variable, when set). */

@@ -2613,6 +2613,7 @@ __global__ void __launch_bounds__(2 * NT, SVPF_MINB)
     if (!split && !cta_abort) finish_pair(&P, pr, payloads + pair * P.payload_len, scr, P.stage_groups);
 }
 
+#if SVPF_LOOKAHEAD
 // One level spread over the GPU: a CTA per warp, D of them per search direction of the pairs first ..
 // of the launch. The warps of a direction wait on one another, so the launch is cooperative: all its
 // CTAs are resident at once, or it does not start.
@@ -2706,6 +2707,14 @@ __global__ void __launch_bounds__(kPackThreads)
 // Levels of fewer blocks than this are searched by the pair's CTA, without a launch of their own.
 constexpr int kWalkCells = 30;
 
+// The coarsest level of P that a walk takes; the levels above it are the pair kernel's.
+__host__ __device__ inline int first_walk(const AnalyseParams &P) {
+    int lo = P.nlevels - 1;
+    while (lo > 0 && P.lv[lo].gw * P.lv[lo].gh < kWalkCells) lo--;
+    return lo;
+}
+#endif
+
 // Persistent form: a grid sized to the resident CTAs drains the item list in order (the
 // host sorts it largest-first); each CTA pulls the next item with one atomic, copies the
 // item's clip parameters into shared memory and runs the pair on its own scratch slot.
@@ -2734,13 +2743,6 @@ __global__ void __launch_bounds__(2 * NT, SVPF_MINB)
         if (!cta_abort) finish_pair(&P, bi.pair, bi.payload, scr, groups);
         __syncthreads();  // P, item_sh and the shared search state are reused by the next item
     }
-}
-
-// The coarsest level of P that a walk takes; the levels above it are the pair kernel's.
-__host__ __device__ inline int first_walk(const AnalyseParams &P) {
-    int lo = P.nlevels - 1;
-    while (lo > 0 && P.lv[lo].gw * P.lv[lo].gh < kWalkCells) lo--;
-    return lo;
 }
 
 #if SVPF_LOOKAHEAD && !defined(SVPF_PX16)
@@ -2816,6 +2818,7 @@ cudaError_t prepare() {
     return once;
 }
 
+#if SVPF_LOOKAHEAD
 namespace {
 constexpr int kMinWalkers = 4;  // warps per direction of a walk, at least
 // The build and the resident CTAs of a walk over `ndirs` search directions.
@@ -2853,19 +2856,21 @@ cudaError_t launch_walk(void (*kernel)(P...), int64_t ctas, size_t smem, cudaStr
     return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 }  // namespace
+#endif
 
 cudaError_t launch_plain(const AnalyseParams &P, const PairSrc &psrc, int npairs, uint8_t *payloads, uint8_t *scratch,
                          int *status_dev, cudaStream_t stream, int *launches) {
     if (npairs <= 0) return cudaSuccess;
     if (cudaError_t e = prepare()) return e;
     const int ndir = P.vectors == 3 ? 2 : 1;
-    const bool split = SVPF_LOOKAHEAD && NW > 1 && (P.lookahead & 5) == 5;
+    const bool split = SVPF_LOOKAHEAD && (P.lookahead & 5) == 5;
     const size_t pair_smem = pair_shared(ndir, P.stage_groups);
     auto count = [&] { if (launches) *launches += 1; return cudaGetLastError(); };
     if (!split) {
         analyse_kernel<<<npairs, NT * ndir, pair_smem, stream>>>(P, psrc, payloads, scratch, status_dev, 0, P.nlevels - 1, 0);
         return count();
     }
+#if SVPF_LOOKAHEAD
     // D warps per direction, as many as are resident at once (at least kMinWalkers, with the pairs in
     // several launches when they would not be)
     WalkShape w;
@@ -2903,6 +2908,7 @@ cudaError_t launch_plain(const AnalyseParams &P, const PairSrc &psrc, int npairs
             P, payloads + (int64_t)f * P.payload_len, scratch + (int64_t)f * P.scratch_per_pair);
         if (cudaError_t e = count()) return e;
     }
+#endif
     return cudaSuccess;
 }
 

@@ -1,15 +1,14 @@
-// batch.cpp -- the batched form: many clips of uneven size and length analysed by one
-// persistent launch.
+// batch.cpp -- the batched form: many clips of uneven size and length analysed together.
 //
 // The reference analyses one clip at a time, one output frame per getFrame call
 // (crates/svpflow1/src/analyse_filter.rs:229-334); every frame pair is independent of
 // every other (analyse_search.rs:68-92 reads only its two super frames). A batch therefore
 // flattens the frame pairs of all its clips into one item list, sorted largest-first, and runs
 // it in one of two ways. The shape "walk" (the default) takes groups of items of about the same
-// size, as many as give every search direction four warps or more on the whole GPU, level by
+// size, as many as still give every search direction four warps or more on the whole GPU, level by
 // level, the clips' finest levels aligned (batch_ground_kernel, batch_walk_kernel). The other
 // shapes let a grid of resident CTAs drain the list through a device-side counter, a pair per
-// CTA (analyse_batch_kernel): 12 clips of 320x240 to 854x480 take 134 ms walked and 320 ms
+// CTA (analyse_batch_kernel): 12 clips of 320x240 to 854x480 take 128 ms walked and 320 ms
 // drained by the fastest of them, since a drained pair runs at one CTA's speed.
 //
 // Device memory of a batch is one allocation made at creation: every clip's source
@@ -286,7 +285,7 @@ int svpf_batch_create(int32_t nclips, const svpf_super *const *supers, const svp
         b->items.swap(it2);
         b->item_cost.swap(c2);
     }
-    // the variant with the most resident CTAs bounds the scratch slots
+    // the shape with the most pairs in work at a time bounds the scratch slots
     int most = 0;
     for (int v = 0; v < analyse_variant_count(); v++) {
         int per_sm = 0;
@@ -401,8 +400,8 @@ int svpf_batch_run(svpf_batch *b, const uint8_t *const *frames, uint8_t *const *
     return read_statuses(b, b->stream);
 }
 
-// Times each launch shape on the batch's largest items (one item per resident CTA of the
-// shape, so a trial lasts about one pair's latency) and keeps the one with the most pairs
+// Times each launch shape on the batch's largest items (as many as the shape has in work at a time,
+// so a trial lasts about one pair's latency) and keeps the one with the most pairs
 // per second. The source frames must be in place (svpf_batch_frames_device or a run).
 int svpf_batch_autotune(svpf_batch *b, int32_t *variant, int32_t *tiles_per_lane, double *pairs_per_s) {
     std::lock_guard<std::mutex> lk(b->mu);
@@ -415,7 +414,7 @@ int svpf_batch_autotune(svpf_batch *b, int32_t *variant, int32_t *tiles_per_lane
         if (int rc = upload_params(b)) return rc;
         int grid = 0;
         if (int rc = grid_for(b, v, (int)b->items.size(), &grid)) return rc;
-        const int n = grid;  // one item per resident CTA
+        const int n = grid;  // the items in work at a time
         int nl = 0;
         for (auto &c : b->clips) {  // Super once (untimed), then the timed Analyse
             cudaError_t e = launch_super(c.D, b->arena + c.frames_off, b->arena + c.supers_off, c.nframes, b->stream, &nl);

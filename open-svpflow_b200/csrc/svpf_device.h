@@ -39,7 +39,7 @@ struct PairSrc {
     const uint8_t *clip;
     int64_t frame_bytes;
     int32_t first, nframes, delta;
-    unsigned long long *stats;  // nullable: level-0 look-ahead counters (see search_level0_spec)
+    unsigned long long *stats;  // nullable: level-0 counters of the walk (see walk_level)
 };
 
 // One work item of a batch launch: a frame pair of some clip and where its payload goes.
@@ -108,8 +108,7 @@ cudaError_t launch_analyse(const AnalyseParams &P, const PairSrc &src, int npair
 cudaError_t launch_analyse_shape(int variant, const AnalyseParams &P, const PairSrc &src, int npairs, uint8_t *payloads,
                                  uint8_t *scratch, int *status_dev, cudaStream_t stream, int *launches);
 // The shape of the server's chunk launches, which share the GPU with other clips' chunks: nt128,
-// whose level 0 spreads over the SMs (measured at 5 clips/s against nt128_b3: 83.0 against 60.4
-// pairs/s, p50 7.9 against 13.1 s, p99 25.7 against 36.5 s).
+// whose walks take the warps that are free on every SM, however few pairs a chunk has.
 constexpr int kShapeShared = 0;
 
 }  // namespace svpf

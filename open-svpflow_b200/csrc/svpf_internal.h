@@ -105,7 +105,7 @@ struct alignas(16) AnalyseParams {
     int32_t has_refine, refine_thsad, refine_search_type, refine_distance, refine_satd, lambda;
     LevelInfo rlv[2];         // refine pass block shapes: output block, half of it (border blocks)
     int32_t rescale_denom;
-    int32_t tiles_per_lane;   // accepted (2, 4 or 8) and kept; the evaluation no longer splits a candidate over lanes
+    int32_t tiles_per_lane;   // accepted (2, 4 or 8) and kept; a candidate is evaluated by a whole warp, whatever it says
     int32_t px_bytes;         // 1: 8-bit samples; 2: uint16 samples (the 10-bit extension)
     int32_t lookahead;        // look-ahead (one block per warp in flight, exact either way): bit 0 level 0,
                               // bit 1 the coarser levels, both in the pair's CTA; bits 0 and 2: every level

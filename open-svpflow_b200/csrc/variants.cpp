@@ -19,7 +19,7 @@ const AnalyseVariant &analyse_variant(int i) {
     return kVariants[(i >= 0 && i < analyse_variant_count()) ? i : 0];
 }
 
-// The 128-register shape, whose level 0 spreads over the GPU by default; with that off, more
+// The 128-register shape, whose levels are walked over the whole GPU by default; with that off, more
 // pairs than two per SM take the 80-register shape (three pairs per SM resident). uint16
 // samples have one compiled shape.
 cudaError_t launch_analyse(const AnalyseParams &P, const PairSrc &src, int npairs, uint8_t *payloads,
@@ -31,8 +31,8 @@ cudaError_t launch_analyse(const AnalyseParams &P, const PairSrc &src, int npair
             return 0;
         return n;
     }();
-    // more pairs than two per SM: the 3-CTA shape, unless level 0 is spread over the GPU, which
-    // balances the SMs at any pair count (900 pairs at 960x540: 581.9 -> 754.1 pairs/s)
+    // more pairs than two per SM: the 3-CTA shape, unless the levels are walked over the GPU, which
+    // balances the SMs at any pair count
     if (sms > 0 && npairs > 2 * sms && (P.lookahead & 5) != 5)
         return nt128b3::launch_plain(P, src, npairs, payloads, scratch, status_dev, stream, launches);
     return nt128::launch_plain(P, src, npairs, payloads, scratch, status_dev, stream, launches);

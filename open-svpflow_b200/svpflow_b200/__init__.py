@@ -340,8 +340,8 @@ class Analyser:
         _check(lib().svpf_analyse_pairs_device(self._h, c, r, n, payloads_ptr, scratch_ptr, stream))
 
     def set_lookahead(self, levels):
-        """Look-ahead bits: 1 level 0, 2 the coarser levels, 4 level 0 spread over the GPU in a
-        launch of its own (with 1). True is the default (5), False / 0 off; results are identical
+        """Look-ahead bits: 1 level 0, 2 the coarser levels, 4 (with 1) every level but the smallest
+        spread over the GPU in launches of their own. True is the default (5), False / 0 off; results are identical
         either way."""
         _check(lib().svpf_analyser_set_lookahead(self._h, 5 if levels is True else int(levels)))
 
@@ -378,7 +378,7 @@ def reset_kernel_launches():
 
 
 class Batch:
-    """Many clips analysed by one persistent launch (no counterpart in the reference).
+    """Many clips analysed together, a CUDA graph per run (no counterpart in the reference).
 
     clips: sequence of (SuperBuilder, Analyser, nframes). Payloads equal each clip's
     Analyser.analyse_clip output byte for byte."""
