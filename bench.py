@@ -20,7 +20,7 @@ threads over a bounded sample of the same workload.
 Other workloads (one JSON line each, same keys):
   --workload batched   64 clips of uneven size and length (resolution from 360p..1440p,
                        16-240 frames log-uniform, block 8 or 16, else the 1080p options)
-                       analysed by one persistent launch replayed from a CUDA graph, with the
+                       analysed together, one CUDA graph replayed, with the
                        autotuned launch shape; `plain_per_clip` times the same clips through
                        the per-clip path one after another, and every payload is compared.
   --workload 2160p10   a 3840x2160 10-bit clip (uint16 samples) of 120 frames, Super {pel:4},
@@ -67,10 +67,9 @@ DESC = {
 }
 UNIT = "frame-pairs/s"
 # DRAM bytes per frame pair of the Analyse launch at 1080p: ncu's dram__bytes_read.sum +
-# dram__bytes_write.sum of the three kernels of the 240-pair launch (one-pass counters):
-# analyse_kernel 5.55 + 0.77 GB, analyse_level0_kernel 16.17 + 0.40 GB, analyse_finish_kernel
-# 0.14 + 0.08 GB (profiles/analyse_1080p_240_counters.md)
-TRAFFIC_PER_PAIR = 23.11e9 / 240
+# dram__bytes_write.sum of the kernels of the 240-pair launch (one-pass counters, 25.08 + 2.10 GB:
+# profiles/analyse_walk_kernels.md)
+TRAFFIC_PER_PAIR = 27.18e9 / 240
 # DRAM bytes of one 1080p render launch with the 8 x 8 effective block (ncu capture: 4.13 MB read,
 # the written frame stays in L2)
 RENDER_TRAFFIC_PER_FRAME = 4.14e6
@@ -83,13 +82,14 @@ INT32_LANES_PER_SM = 128
 # integer ops per frame pair (oracle counts of the workloads' compares), when the CPU leg is skipped
 OPS_PER_PAIR = {"1080p": 19.38e9}
 # why the Analyse launch reaches the fraction it does, from the ncu counters of the 240-pair launch
-# in profiles/analyse_1080p_240_counters.md: issue utilisation (warp instructions / (4 schedulers x
+# in profiles/analyse_walk_kernels.md: issue utilisation (warp instructions / (4 schedulers x
 # SMs x the launch's SM cycles)) x useful lane fraction (algorithmic ops / executed lane slots)
-ROOF_DECOMPOSITION = {"issue_active": 0.341, "useful_lane_fraction": 0.332,
-                      "source": "ncu counters of the 240-pair 1080p launch (analyse_kernel 142.9 G + "
-                                "analyse_level0_kernel 295.0 G + analyse_finish_kernel 0.03 G warp instructions "
-                                "in 1105.5 ms): 1.82 G warp instructions = 58.4 G lane slots per pair for 19.4 G "
-                                "algorithmic ops (profiles/analyse_1080p_240_counters.md)"}
+ROOF_DECOMPOSITION = {"issue_active": 0.322, "useful_lane_fraction": 0.530,
+                      "source": "ncu counters of the 240-pair 1080p launch (five analyse_walk_kernel launches 273.6 G, "
+                                "analyse_kernel and analyse_pack_kernel 0.7 G warp instructions in 731.6 ms): 1.14 G "
+                                "warp instructions = 36.6 G lane slots per pair for 19.4 G algorithmic ops, the SATD "
+                                "transforms among them, which run on the tensor cores "
+                                "(profiles/analyse_walk_kernels.md)"}
 # the CPU legs time this many frame pairs per host thread, so that their figure is a throughput
 # (dynamic scheduling over many pairs) rather than the latency of the slowest pair
 CPU_PAIRS_PER_THREAD = 4
@@ -870,7 +870,7 @@ def _batch_oracle_sample(torch, dev, b, clips, mix) -> dict:
 
 
 def run_batched(args, world: int, rank: int, local: int):
-    """Config 4: many clips of uneven size in one persistent launch, against per-clip launches."""
+    """Config 4: many clips of uneven size in one graph replay, against per-clip launches."""
     torch, dist = _init_dist(world, local)
     import svpflow_b200 as sv
 
@@ -978,7 +978,7 @@ def run_batched(args, world: int, rank: int, local: int):
             k = f"{w}x{h}/b{blk}"
             res[k] = res.get(k, 0) + n
         line = {
-            "metric": "Analyse frame-pairs/s, batched (64 mixed clips, one persistent launch; bit-exact MVs)",
+            "metric": "Analyse frame-pairs/s, batched (64 mixed clips, one graph replay; bit-exact MVs)",
             "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
             "ms_per_step": ms / args.steps, "higher_is_better": True, "scaling": "strong", "vs_baseline": None,
             "dtype": "u8", "data": "synthetic",
@@ -1317,17 +1317,16 @@ def main():
             ops_pair = orc.integer_ops(cnt) / pairs
             ops_src = (f"compares the oracle executed on output frames 0..{pairs - 1} (2 ops per SAD sample, 111 "
                        f"per SATD 4x4 tile)")
-        # the Analyse kernel's primary bound: the int32 pipes (no dense contraction, little HBM traffic)
+        # the Analyse kernel's primary bound: the int32 pipes (the SATD products leave the tensor cores idle, little HBM traffic)
         roof = {
-            "kernel": ("Analyse: analyse_kernel (one CTA per frame pair, fwd/bwd halves: the coarser levels), "
-                       "analyse_level0_kernel (one CTA per warp: level 0 with look-ahead), analyse_finish_kernel; "
-                       "timed together"),
+            "kernel": ("Analyse: analyse_walk_kernel per level (one-warp CTAs over the GPU), analyse_kernel between "
+                       "them (one CTA per frame pair), analyse_pack_kernel; timed together"),
             "bound": "int32 pipe", "unit": "Tops/s", "peak": int_peak / 1e12,
             "achieved": ops_pair * a_count / (a_ms / 1000) / 1e12 if ops_pair else None,
             "frac": ops_pair * a_count / (a_ms / 1000) / int_peak if ops_pair else None,
             "traffic": TRAFFIC_PER_PAIR * a_count if WORKLOAD == "1080p" and not args.size else None,
             "traffic_unit": "bytes per launch",
-            "traffic_source": ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the three kernels of the "
+            "traffic_source": ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the kernels of the "
                                "240-pair launch, per pair x pairs"),
             "ops_per_pair": ops_pair, "ops_source": ops_src, "avg_launch_ms": a_ms,
             "peak_source": f"nominal: {_sm_count()} SMs x {INT32_LANES_PER_SM} int32 lanes (64 on the ALU pipe + 64 "
@@ -1370,7 +1369,7 @@ def main():
             "lookahead": {**la, "mode": 0 if args.no_lookahead else args.lookahead,
                           "rerun_fraction": la["reruns"] / la["blocks"] if la["blocks"] else None,
                           "note": "one block per warp in flight; each block re-checks the neighbour seeds "
-                                  "committed after it started and re-runs its refinement when one wins "
+                                  "published after it started and re-runs its refinement when one wins "
                                   "(level-0 counters of the last timed step)"},
             "super_ms_per_step": statistics.mean(super_ms), "analyse_ms_per_step": statistics.mean(analyse_ms),
         }
@@ -1404,7 +1403,7 @@ def _sub_line(extra, timeout_s: int) -> dict:
 
 
 def _sub_batched(args) -> dict:
-    """Config 4 in the default line: the 64-clip mix in one persistent launch (CUDA-graph replay)
+    """Config 4 in the default line: the 64-clip mix in one CUDA-graph replay
     against the same clips through the plain per-clip path, with oracle parity on a sample."""
     extra = ["--workload", "batched", "--steps", "1", "--warmup", "1", "--e2e-steps", "0", "--shape", BATCH_SHAPE]
     if args.no_cpu:

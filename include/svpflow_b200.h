@@ -271,8 +271,8 @@ int svpf_render_mode23_device(const svpf_render_config *cfg, int32_t threshold, 
 /* No counterpart in the reference, which analyses one clip at a time, one output frame
  * per getFrame call (crates/svpflow1/src/analyse_filter.rs:229-334). A batch holds many
  * clips of any size and length (each with its own Super and Analyse handles, as for
- * svpf_clip_analyse) and analyses every output frame of every clip in one persistent
- * launch replayed from a CUDA graph; each payload is byte-identical to the per-clip
+ * svpf_clip_analyse) and analyses every output frame of every clip together, a run
+ * replayed from a CUDA graph; each payload is byte-identical to the per-clip
  * call's. Creation allocates all device memory of the batch (svpf_batch_device_bytes):
  * the clips' source frames, super frames and payloads plus the work list and scratch.
  * A batch serialises its own calls. */
