@@ -1074,8 +1074,8 @@ __device__ __noinline__ uint2 clamped_cands(const AnalyseParams *Pp, const Level
 // it. The lanes set their candidates up side by side, then the warp evaluates one after another.
 // Bound: the latency of the loads, which the candidates evaluated together overlap, then instruction
 // issue. Per 16x16 candidate with chroma this is about 120 warp instructions with all that surrounds
-// it, against 167 when groups of lanes each transformed whole tiles in f16x2 (13.7 k against 19.2 k
-// per level-0 block of the 1080p configuration).
+// it, against 167 when groups of lanes each transformed whole tiles in f16x2 (14.2 k against 19.2 k
+// per level-0 block of the 1080p configuration, its repeats included).
 __device__ __forceinline__ void eval_cands(const Ctx &x, const BlkC &b, bool ok, int mvx, int mvy, unsigned &L, unsigned &C) {
     const int lane = x.tid & 31;
     unsigned lref = 0, cref = 0;
@@ -1643,6 +1643,10 @@ __device__ __forceinline__ void search_level(const Ctx &x, DirSh &s, DirScratch 
 // the expansions one after another). The lowest block that is not finished waits for nothing, and every
 // warp takes its blocks in order, so the warps, all resident, always make progress; the waits are
 // bounded all the same.
+// Bound: at few pairs the chain (a link is the wait's L2 round trip where nothing changed, a refinement where
+// something did), at many the latency of the candidates' loads (issue 32 %). With four warps per direction
+// that handed over in order, and the coarser levels in the pair's CTA: one 1080p pair 287 ms, 23 ms now; 32
+// frames of 640x360 13.4 and 4.3 ms; 240 frames of 1080p 1087 and 729 ms.
 // A level with an input on which the reference would panic takes search_level instead.
 // stats (nullable): [0] blocks, [1] blocks that started before all their processed neighbours were
 // final, [2] seeds evaluated after the start (the others had the vector of a candidate already
@@ -2618,10 +2622,10 @@ __global__ void __launch_bounds__(2 * NT, SVPF_MINB)
 // of the launch. The warps of a direction wait on one another, so the launch is cooperative: all its
 // CTAs are resident at once, or it does not start.
 // PER_SM: CTAs per SM the registers are cut for, 16 (128 per thread) or 20 (96; more spills, but a quarter
-// more warps). Few pairs leave the chain of blocks as the bound, where the first is faster (one 1080p pair
-// 35.7 against 37.9 ms, 16 frames 640x360 10-bit 190 against 212), many pairs the latency of the loads, which
-// more warps hide (240 frames 1080p 786 against 742 ms; 24 CTAs, 80 registers: 762): the line is where the
-// first could give a direction kDenseWalkers warps.
+// more warps). Few pairs leave the chain of blocks as the bound, where the first is faster (32 frames of
+// 640x360 3.69 against 3.96 ms, 16 of them at 10 bits 134 against 158, one 1080p pair 23.4 against 24.2), many
+// pairs the latency of the loads, which more warps hide (240 frames of 1080p 800 against 731 ms; 24 CTAs with 80
+// registers were slower than 20): the line is where the first could give a direction kDenseWalkers warps.
 constexpr int kWalkPerSM = 16, kDensePerSM = 20, kDenseWalkers = 8;
 __device__ __forceinline__ void walk_cta(const AnalyseParams &P, const PairRef pr, uint8_t *scr, int dir, int g, int D, int level,
                                          int groups, int *status, unsigned long long *stats) {
@@ -2704,8 +2708,10 @@ __global__ void __launch_bounds__(kPackThreads)
     pack_cells(P, ds, d, payloads + pair * P.payload_len, i, (int64_t)gridDim.x * kPackThreads, i == 0);
 }
 
-// Levels of fewer blocks than this are searched by the pair's CTA, without a launch of their own.
-constexpr int kWalkCells = 30;
+// Levels of fewer blocks than this are searched by the pair's CTA, without a launch of their own: the least
+// that a walk takes, 3 x 3. (32 frames of 640x360, lines at 9, 30 and 120 blocks: 3.50, 3.69 and 4.45 ms; one
+// 1080p pair 23.2, 23.4 and 25.0.)
+constexpr int kWalkCells = 9;
 
 // The coarsest level of P that a walk takes; the levels above it are the pair kernel's.
 __host__ __device__ inline int first_walk(const AnalyseParams &P) {

@@ -558,6 +558,10 @@ __global__ void __launch_bounds__(256, 4) super_level01_kernel(SuperDev D, const
 // layout): any width, any alignment, both sample types. Level 0 is then one flat stream per plane
 // (its sub-planes follow one another without a gap), and the pyramid is reduced by warps that walk
 // down the rows.
+// Bound: level 0 by its stores (240 frames of 1080p: 3.8 GB in 755 us, 5.05 TB/s), the pyramid by the filters'
+// instruction issue (65 % on its first levels, 416 and 141 us). With rows staged in shared memory, or a CTA per
+// row where rows are not on 16 bytes: 1.81 and 1.45 ms for that call, 938 and 196 us for 48 frames of 854x480,
+// 2.31 and 0.69 ms for 6 frames of 2160p at 10 bits, 94 and 35 us for one of 640x360 (9 launches, 2 now).
 
 // Sample arithmetic in 32-bit words: 4 bytes or 2 halfwords.
 template <typename T>
@@ -1385,8 +1389,11 @@ LevelItems level_items(const SuperDev &D, int lv, int nframes, int sms) {
     }
 }
 // Levels whose result has at most this many luma samples go to the tail kernel, a cluster per plane and frame.
+// (One frame of 640x360: 34.9 us; with the tail from 10000 or 3000 samples on 38.6 and 41.1. The last levels of
+// 48 frames of 854x480 through the tail 441 us, by a launch each 195: more frames than kTailFrames fill the GPU at
+// every level.)
 constexpr int64_t kTailSamples = 40000;
-constexpr int kTailFrames = 6;  // more frames fill the GPU at every level
+constexpr int kTailFrames = 6;
 template <typename T>
 int launch_super_flat(const SuperDev &D, const uint8_t *src, uint8_t *dst, int nframes, int sms, cudaStream_t stream) {
     const int per_sm = sizeof(T) == 1 ? 3 : 2;
@@ -1401,6 +1408,9 @@ int launch_super_flat(const SuperDev &D, const uint8_t *src, uint8_t *dst, int n
         const int64_t bytes = all ? sub : sub * nsub;
         return (uint32_t)((bytes / 16 + 1 + F.tile) / F.tile);
     };
+    // Level 0 in a launch of its own where every resident CTA has a large tile: 240 frames of 1080p 1440 us against
+    // 2209 together with the first reduction, 6 of 2160p at 10 bits 691 against 1143, 48 of 854x480 195 against 211;
+    // one frame of 640x360 39.0 against 34.9.
     F.tile = (int64_t)nframes * D.frame_bytes >= (int64_t)sms * 6 * 1024 * 16 ? 1024 : 256;
     F.ty = tiles((int64_t)D.width * D.height, F.all_y);
     F.tc = tiles((int64_t)(D.width / 2) * (D.height / 2), F.all_c);
