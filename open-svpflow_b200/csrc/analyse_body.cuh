@@ -1646,7 +1646,7 @@ __device__ __forceinline__ void search_level(const Ctx &x, DirSh &s, DirScratch 
 // Bound: at few pairs the chain (a link is the wait's L2 round trip where nothing changed, a refinement where
 // something did), at many the latency of the candidates' loads (issue 32 %). With four warps per direction
 // that handed over in order, and the coarser levels in the pair's CTA: one 1080p pair 287 ms, 23 ms now; 32
-// frames of 640x360 13.4 and 4.3 ms; 240 frames of 1080p 1087 and 729 ms.
+// frames of 640x360 12.6 and 3.5 ms; 240 frames of 1080p 1087 and 729 ms.
 // A level with an input on which the reference would panic takes search_level instead.
 // stats (nullable): [0] blocks, [1] blocks that started before all their processed neighbours were
 // final, [2] seeds evaluated after the start (the others had the vector of a candidate already
