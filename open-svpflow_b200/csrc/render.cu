@@ -436,7 +436,8 @@ __global__ void __launch_bounds__(2 * kTileW) render_tile_kernel(const __grid_co
     __shared__ int2 sxw[kMaxBlock], syw[kMaxBlock];
     const RenderPlane &p = J.pl[blockIdx.z];
     const int32_t X0 = blockIdx.x * kTileW, Y0 = blockIdx.y * kTileH;
-    if (X0 >= p.width || Y0 >= p.height) return;
+    // outside the plane, or a plane without blocks (chroma under blocks of 1), which is not drawn
+    if (X0 >= p.width || Y0 >= p.height || p.block_w <= 0 || p.block_h <= 0) return;
     const int tid = threadIdx.x;
     if (tid < kMaxBlock) {
         sxw[tid] = make_int2(p.xw[tid][0], p.xw[tid][1]);
@@ -539,7 +540,7 @@ bool tiled_ok(const RenderJob &J, int kind, bool mask, size_t &smem) {
     smem = 0;
     for (int pl = 0; pl < 3; pl++) {
         const RenderPlane &p = J.pl[pl];
-        if (p.width <= 0 || p.height <= 0 || p.block_w <= 0 || p.block_h <= 0) continue;  // the plane is not drawn
+        if (p.width <= 0 || p.height <= 0 || p.block_w <= 0 || p.block_h <= 0) continue;  // the kernel does not draw the plane
         if (p.x_shift < 0 || p.y_shift < 0 || p.step <= 0 || p.origin_x < 0 || p.origin_y < 0) return false;
         for (int i = 0; i < kMaxBlock; i++)
             if (p.xw[i][0] < 0 || p.xw[i][1] < 0 || p.yw[i][0] < 0 || p.yw[i][1] < 0 ||
