@@ -73,7 +73,6 @@ constexpr int NW = NT / 32;
 
 enum : uint8_t { LM_DIRECT = 1, LM_SATD_MASK = 2, LM_SAD_BREAK = 3, LM_EDGE = 4, LM_DC = 5 };
 enum : uint8_t { CM_NONE = 0, CM_DIRECT = 1, CM_SAD_BREAK = 3, CM_EDGE = 4 };
-enum : int { BK_EXH = 1, BK_UMH, BK_HEX6, BK_HEX3, BK_RING };
 
 constexpr int ST_PANIC = 1;    // status bit: the reference indexes out of range here (it would panic)
 constexpr int ST_TIMEOUT = 4;  // status bit: a bounded wait inside the kernel ran out (internal error)
@@ -81,6 +80,8 @@ constexpr int ST_TIMEOUT = 4;  // status bit: a bounded wait inside the kernel r
 // a level-0 block takes well under a millisecond). After one wait of a direction has given
 // up, its other waits return at once, so a failure costs one bound, not one per block.
 constexpr long long kWaitCycles = 1000000000LL;
+
+#include "search_steps.cuh"
 
 struct Cand {
     int64_t l_sbase, l_rbase, c_sbase, c_rbase;  // flat bases of the direct read paths
@@ -93,6 +94,7 @@ struct Cand {
 
 // Per-block constants, identical in every thread of a direction. In shared memory, one copy per warp, like
 // Search: they are read once per 32 candidates, and registers are what bounds the warps in flight.
+// Changed as Search is, between two meetings of the lanes.
 struct BlkC {
     int px, py, bw, bh, px2, py2;
     int bnd0, bnd1, bnd2, bnd3;            // mv_bounds
@@ -101,22 +103,6 @@ struct BlkC {
     int lbase, llim, cbase, clim;          // ... and have lref <= llim, cref <= clim; the offsets (from the frame's
                                            // first sample) of the reference blocks at vector 0
     int64_t lsrc, csrc;                    // offset of the source block (luma, U)
-};
-
-// What a block's search keeps from turn to turn, identical in every lane of the warp (see Search_next).
-struct Search {
-    int state, stage, stype, radius;
-    int predx, predy;                       // predictor of the motion penalty
-    int lambda, own_x, own_y, ppx, ppy;     // the block's penalty factor, its own predictor and the refinement's
-    int bmx, bmy;                           // the best so far
-    unsigned bsad;
-    long long bcost;
-    int hbx, hby, hdir, hi, hrad, hret, bad_r, bad_max;
-    unsigned found;
-    int sets_mv;
-    int rx, ry;                             // a walk: the outcome before a bad-SAD expansion made ahead of the test
-    unsigned rsad;
-    long long rcost;
 };
 
 // Shared state of one search direction. A block is searched by a group of warps: the whole
@@ -166,16 +152,10 @@ __device__ __forceinline__ void dbar(int d) {
     if (d) asm volatile("bar.sync 2, %0;" ::"n"(NT) : "memory");
     else asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory");
 }
-__device__ __forceinline__ int imin(int a, int b) { return a < b ? a : b; }
-__device__ __forceinline__ int imax(int a, int b) { return a > b ? a : b; }
-__device__ __forceinline__ int iclamp(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
 __device__ __forceinline__ unsigned sat_add(unsigned a, unsigned b) { unsigned r = a + b; return r < a ? 0xFFFFFFFFu : r; }
 __device__ __forceinline__ unsigned sat_mul(unsigned a, unsigned b) {
     unsigned long long r = (unsigned long long)a * b;
     return r > 0xFFFFFFFFull ? 0xFFFFFFFFu : (unsigned)r;
-}
-__device__ __forceinline__ int sat_i32(long long r) {
-    return r > 2147483647LL ? 2147483647 : (r < -2147483648LL ? (int)0x80000000 : (int)r);
 }
 __device__ __forceinline__ bool is_blk(int n) { return n == 4 || n == 8 || n == 16 || n == 32; }
 // reads of a slice: an index past the end (or a wrapped, i.e. negative, one) is None
@@ -569,60 +549,6 @@ __device__ __forceinline__ float4 mma_hadamard(const uint4 &h, uint32_t lo, uint
 }
 
 // -------------------------------------------------------------------------------------------
-// candidate generators (the reference's loop orders)
-__constant__ int2 c_hex2[8] = {{-1, -2}, {-2, 0}, {-1, 2}, {1, 2}, {2, 0}, {1, -2}, {-1, -2}, {-2, 0}};  // :889-898
-__constant__ int c_mod6m1[8] = {5, 0, 1, 2, 3, 4, 5, 0};
-__constant__ int2 c_hex4[16] = {{-4, 2}, {-4, 1}, {-4, 0}, {-4, -1}, {-4, -2}, {4, -2}, {4, -1}, {4, 0},
-                                {4, 1},  {4, 2},  {2, 3},  {0, 4},   {-2, 3},  {-2, -3}, {0, -4}, {2, -3}};  // :1075-1092
-
-struct Gen {
-    int kind, cx, cy, r, step, odir, n;
-};
-__device__ __forceinline__ int ring_m(int r, int step) { return 2 * r > step ? (2 * r - 1) / step : 0; }
-__device__ __forceinline__ Gen make_gen(int kind, int cx, int cy, int r, int step, int odir) {
-    Gen g{kind, cx, cy, r, step, odir, 0};
-    switch (kind) {
-    case BK_EXH: g.n = (2 * r + 1) * (2 * r + 1); break;
-    case BK_UMH: g.n = 4 * (r / 2 > 0 ? r / 2 : 0) + 16 * imax(r / 4, 1); break;
-    case BK_HEX6: g.n = 6; break;
-    case BK_HEX3: g.n = 3; break;
-    case BK_RING: g.n = 4 * ring_m(r, step) + 4; break;
-    }
-    return g;
-}
-__device__ int2 gen_mv(const Gen &g, int i) {
-    const int cx = g.cx, cy = g.cy, r = g.r;
-    switch (g.kind) {
-    case BK_EXH: {  // exact_refine_search type 4, :799-823 (raster over the square)
-        const int w = 2 * r + 1;
-        return make_int2(cx - r + i % w, cy - r + i / w);
-    }
-    case BK_UMH: {  // exact_umh, :1055-1114
-        const int nd = r / 2;
-        if (i < 2 * nd) { int dd = 1 + 2 * (i >> 1); return make_int2(cx + ((i & 1) ? dd : -dd), cy); }
-        i -= 2 * nd;
-        if (i < 2 * nd) { int dd = 1 + 2 * (i >> 1); return make_int2(cx, cy + ((i & 1) ? dd : -dd)); }
-        i -= 2 * nd;
-        const int scale = 1 + i / 16;
-        const int2 h = c_hex4[i % 16];
-        return make_int2(cx + h.x * scale, cy + h.y * scale);
-    }
-    case BK_HEX6: { int2 h = c_hex2[i + 1]; return make_int2(cx + h.x, cy + h.y); }
-    case BK_HEX3: { int2 h = c_hex2[g.odir + i]; return make_int2(cx + h.x, cy + h.y); }
-    case BK_RING: {  // exact_expanding, :849-885
-        const int step = g.step, m = ring_m(r, step);
-        if (i < 2 * m) { int off = -r + step + (i >> 1) * step; return make_int2(cx + off, (i & 1) ? cy + r : cy - r); }
-        i -= 2 * m;
-        if (i < 2 * m) { int off = -r + step + (i >> 1) * step; return make_int2((i & 1) ? cx + r : cx - r, cy + off); }
-        i -= 2 * m;
-        const int sx = (i < 2) ? -r : r, sy = (i & 1) ? r : -r;
-        return make_int2(cx + sx, cy + sy);
-    }
-    }
-    return make_int2(0, 0);
-}
-
-// -------------------------------------------------------------------------------------------
 struct Ctx {
     const AnalyseParams *P;
     const LevelInfo *L;
@@ -698,7 +624,9 @@ __device__ __forceinline__ void set_stage(Ctx &x, unsigned char *area, int group
     x.off = reinterpret_cast<unsigned *>(area + (size_t)warp * groups * kGroupBytes + (size_t)groups * 512);
 }
 
-__device__ __forceinline__ void make_blk(const Ctx &x, int px, int py, bool chroma, BlkC &b) {
+// Every lane has done with the block before; on return all may read this one's.
+__device__ __forceinline__ void make_blk(const Ctx &x, int px, int py, bool chroma, BlkC &out) {
+    BlkC b;
     const LevelInfo &L = *x.L;
     const Geo &G = x.G;
     const int bw = L.bw, bh = L.bh, pel = imax(x.pel, 1);
@@ -740,6 +668,8 @@ __device__ __forceinline__ void make_blk(const Ctx &x, int px, int py, bool chro
     b.llim = (int)G.ylen - (bh - 1) * G.ys32 - bw - 8;
     b.cbase = (int)G.ylen + ((int)L.c_off + cpy) * G.cs32 + cpx;
     b.clim = (int)(G.ylen + G.clen) - (crows - 1) * G.cs32 - cw - 8;
+    out = b;
+    __syncwarp();
 }
 
 // Does (block, mv) take the fast path? If so, the byte offsets of its reference blocks (see Frame).
@@ -1319,113 +1249,6 @@ __device__ __forceinline__ uint2 mkvec(int dx, int dy, unsigned score) {
 // word says why), its payload stays unwritten.
 enum { CTL_GO, CTL_LATE, CTL_BAD, CTL_GX, CTL_GY, CTL_ORDER, CTL_PREV, CTL_ABORT };
 
-// The bad-SAD threshold after `count` bad blocks (:605-616).
-__device__ __forceinline__ int bad_limit(const AnalyseParams &P, int count) {
-    return sat_i32((long long)P.coarse_bad_sad + (long long)(sat_i32((long long)P.coarse_bad_sad * count) / 16));
-}
-
-// search states of one block (exact_search_block :684-768, exact_refine_search :771-826,
-// exact_hex2 :942-1033, exact_umh :1036-1119, bad-SAD expansion :611-672)
-enum { S_REFINE, S_HEX_START, S_HEX_ITER, S_HEX_EXIT, S_BAD, S_BAD_RING, S_FINAL_RING, S_STORE };
-
-// The refinement and bad-SAD expansion of one block (exact_refine_search :771-826,
-// exact_hex2 :942-1033, exact_umh :1036-1119, the expansion :611-672): a state machine
-// replicated in every thread of the direction, issuing one evaluation step at a time.
-// (ppx, ppy): predictor of the motion penalty; (own_x, own_y): the block's own predictor,
-// which the bad-SAD expansion switches to. `stage`: RS_ALL runs the refinement and the
-// expansion, RS_REFINE_ONLY stops where the expansion's test begins, RS_BAD_ONLY starts
-// there (a walk runs the two apart: the test reads the bad count of the blocks before),
-// RS_NONE runs nothing.
-enum { RS_NONE, RS_ALL, RS_REFINE_ONLY, RS_BAD_ONLY };
-__device__ __forceinline__ void search_begin(Search &q, int stage) {
-    q.stage = stage;
-    q.predx = q.ppx; q.predy = q.ppy;
-    q.state = stage == RS_NONE ? S_STORE : (stage == RS_BAD_ONLY ? S_BAD : S_REFINE);
-    q.hdir = -2; q.hi = q.hrad = q.hret = 0;
-}
-// The next step's candidates; false when there is none.
-__device__ __forceinline__ bool search_next(Search &q, const Ctx &x, const BlkC &b, int64_t idx, int &bad_count, Gen &g) {
-    const AnalyseParams &P = *x.P;
-    const LevelInfo &L = *x.L;
-    q.sets_mv = 1;
-    while (q.state != S_STORE) {
-        if (q.state == S_BAD && q.stage == RS_REFINE_ONLY) {
-            q.state = S_STORE;
-            break;
-        }
-        if (q.state == S_REFINE) {
-            if (q.stype == 4) { q.state = S_BAD; g = make_gen(BK_EXH, q.bmx, q.bmy, q.radius, 0, 0); return true; }
-            if (q.stype == 3) {
-                q.state = S_HEX_START; q.hrad = q.radius; q.hret = 0;
-                g = make_gen(BK_UMH, q.bmx, q.bmy, q.radius, 0, 0);
-                return true;
-            }
-            if (q.stype == 2) { q.state = S_HEX_START; q.hrad = q.radius; q.hret = 0; }
-            else q.state = S_BAD;
-        } else if (q.state == S_HEX_START) {
-            q.hbx = q.bmx; q.hby = q.bmy;
-            if (q.hrad > 1) { q.sets_mv = 0; q.state = S_HEX_ITER; g = make_gen(BK_HEX6, q.hbx, q.hby, 0, 0, 0); return true; }
-            q.state = q.hret ? S_FINAL_RING : S_BAD;
-            g = make_gen(BK_RING, q.hbx, q.hby, 1, 1, 0);
-            return true;
-        } else if (q.state == S_HEX_ITER) {
-            if (q.hi < q.hrad / 2 && q.hbx >= b.bnd0 && q.hby >= b.bnd1 && q.hbx < b.bnd2 && q.hby < b.bnd3) {
-                q.sets_mv = 0;
-                g = make_gen(BK_HEX3, q.hbx, q.hby, 0, 0, c_mod6m1[q.hdir + 1]);
-                return true;
-            }
-            q.state = S_HEX_EXIT;
-        } else if (q.state == S_HEX_EXIT) {
-            q.bmx = q.hbx; q.bmy = q.hby;
-            q.state = q.hret ? S_FINAL_RING : S_BAD;
-            g = make_gen(BK_RING, q.hbx, q.hby, 1, 1, 0);
-            return true;
-        } else if (q.state == S_BAD) {
-            q.found = q.bsad;
-            if (x.level > 0 && idx > 1 && P.coarse_bad_sad > 0 && (int)q.bsad > bad_limit(P, bad_count)) {
-                bad_count++;
-                q.predx = q.own_x; q.predy = q.own_y;  // the block's own predictor
-                if (P.coarse_bad_range < 0) {
-                    q.bad_max = -P.coarse_bad_range * L.pel; q.bad_r = L.pel;
-                    if (q.bad_r < q.bad_max) { q.state = S_BAD_RING; g = make_gen(BK_RING, 0, 0, q.bad_r, L.pel, 0); return true; }
-                    q.state = S_FINAL_RING;
-                } else if (P.coarse_bad_range > 0) {
-                    q.hrad = P.coarse_bad_range * L.pel; q.hret = 1;
-                    q.state = S_HEX_START;
-                    g = make_gen(BK_UMH, 0, 0, q.hrad, 0, 0);
-                    return true;
-                } else q.state = S_FINAL_RING;
-            } else q.state = S_STORE;
-        } else if (q.state == S_BAD_RING) {
-            if (q.bsad < q.found / 4) q.state = S_FINAL_RING;
-            else {
-                q.bad_r += L.pel;
-                if (q.bad_r < q.bad_max) { g = make_gen(BK_RING, 0, 0, q.bad_r, L.pel, 0); return true; }
-                q.state = S_FINAL_RING;
-            }
-        } else {  // S_FINAL_RING
-            q.state = S_STORE;
-            g = make_gen(BK_RING, q.bmx, q.bmy, 1, 1, 0);
-            return true;
-        }
-    }
-    return false;
-}
-// The step's outcome: candidate w of g was accepted (its cost and sad are in bcost, q.bsad), or none (-1).
-__device__ __forceinline__ void search_took(Search &q, const Gen &g, int w) {
-    if (g.kind == BK_HEX6 || g.kind == BK_HEX3) {  // exact_check_dir: a label, best.mv set at exit
-        if (w >= 0) {
-            q.hdir = g.kind == BK_HEX6 ? w : g.odir + w - 1;
-            q.hbx += c_hex2[q.hdir + 1].x; q.hby += c_hex2[q.hdir + 1].y;
-            q.hi = g.kind == BK_HEX6 ? 1 : q.hi + 1;
-            q.state = S_HEX_ITER;
-        } else q.state = S_HEX_EXIT;
-    } else if (w >= 0 && q.sets_mv) {
-        const int2 m = gen_mv(g, w);
-        q.bmx = m.x; q.bmy = m.y;
-    }
-}
-
 // Runs q (begun) to its end, one step after another.
 template <class SH>
 __device__ __forceinline__ void run_search(const Ctx &x, const BlkC &b, SH &s, int &ph, Search &q, int64_t idx, int &bad_count) {
@@ -1435,6 +1258,7 @@ __device__ __forceinline__ void run_search(const Ctx &x, const BlkC &b, SH &s, i
         long long cost = q.bcost;
         unsigned sad = q.bsad;
         eval_step(x, b, s, ph, g, q.lambda, q.predx, q.predy, cost, sad, w);
+        __syncwarp();
         q.bcost = cost;
         q.bsad = sad;
         search_took(q, g, w);
@@ -1517,6 +1341,7 @@ __device__ __forceinline__ void search_level(const Ctx &x, DirSh &s, DirScratch 
         const int2 imv = vmv(interp);
         BlkC &b = s.blk[warp];
         Search &q = s.q[warp];
+        __syncwarp();  // the block before is stored
         make_blk(x, px, py, !smallest, b);
         const int phb = ph;  // this block's entries of dc and score; the specials' barrier below publishes them
         {
@@ -1757,9 +1582,8 @@ __device__ __forceinline__ void walk_level(const Ctx &x, SH &s, const DirScratch
             }
             const int2 imv = vmv(interp);
             if (lane == kField) { mx = imv.x; my = imv.y; }
-            make_blk(x, px, py, !smallest, b);
             q.own_x = q.ppx = imv.x; q.own_y = q.ppy = imv.y;
-            __syncwarp();
+            make_blk(x, px, py, !smallest, b);
             unsigned dcsum = 0;
             if (b.fast_src) dcsum = stage_source(x, b);
             if (!(b.fast_src && b.px2 == px && b.py2 == py))  // block_luma_dc on the reference's read path
@@ -1782,7 +1606,6 @@ __device__ __forceinline__ void walk_level(const Ctx &x, SH &s, const DirScratch
         unsigned freshm = actm;  // lanes whose candidate is to be evaluated
         bool started = false, reran = false, published = false;
         int selx = 0, sely = 0;
-        q.state = S_STORE;
         Gen g_{0, 0, 0, 0, 0, 0, 0};  // the step in work, its next 32 candidates, and the one accepted so far
         int base = 0, win = -1;
         bool stepping = false;
@@ -1833,6 +1656,7 @@ __device__ __forceinline__ void walk_level(const Ctx &x, SH &s, const DirScratch
                         }
                         openm &= ~__ballot_sync(kFull, (int)(v >> 32) == TAG_FINAL);
                         actm |= freshm;
+                        __syncwarp();
                         if ((freshm >> lane) & 1u) { const int2 m = vmv(make_uint2((unsigned)v, 0)); s.lmx[wi][lane] = m.x; s.lmy[wi][lane] = m.y; }
                         __syncwarp();
                         continue;
@@ -1858,6 +1682,7 @@ __device__ __forceinline__ void walk_level(const Ctx &x, SH &s, const DirScratch
                         }
                         if (lane == 0) st_word(progress + g, k + D);
                         if (bad && !expanded) { search_begin(q, RS_BAD_ONLY); continue; }
+                        __syncwarp();
                         if (!bad && expanded) { q.bmx = q.rx; q.bmy = q.ry; q.bsad = q.rsad; q.bcost = q.rcost; }
                     }
                     break;
@@ -1931,21 +1756,25 @@ __device__ __forceinline__ void walk_level(const Ctx &x, SH &s, const DirScratch
                 const long long K = motion + pen(x.pnew, l) + (b.chroma ? pen(x.pnew, c) : 0LL);  // :1158-1221
                 const unsigned sad = sat_add(l, c);
                 long long best = q.bcost;
+                unsigned best_sad = q.bsad;
                 if (x.pnew < -256) {  // exact sequential semantics for penalties that can be negative
                     for (unsigned m = __ballot_sync(kFull, eval); m; m &= m - 1) {
                         const int j = __ffs(m) - 1;
                         const long long mj = __shfl_sync(kFull, motion, j), kj = __shfl_sync(kFull, K, j);
                         const unsigned sj = __shfl_sync(kFull, sad, j);
-                        if (mj < best && kj < best) { best = kj; q.bcost = kj; q.bsad = sj; win = base + j; }
+                        if (mj < best && kj < best) { best = kj; best_sad = sj; win = base + j; }
                     }
                 } else {
                     const int j = first_min(eval && K < best, K, lane);
                     if (j >= 0) {
-                        q.bcost = __shfl_sync(kFull, K, j);
-                        q.bsad = __shfl_sync(kFull, sad, j);
+                        best = __shfl_sync(kFull, K, j);
+                        best_sad = __shfl_sync(kFull, sad, j);
                         win = base + j;
                     }
                 }
+                __syncwarp();
+                q.bcost = best; q.bsad = best_sad;
+                __syncwarp();
                 base += 32;
                 if (base >= g_.n) { search_took(q, g_, win); stepping = false; }
             }
@@ -1956,6 +1785,7 @@ __device__ __forceinline__ void walk_level(const Ctx &x, SH &s, const DirScratch
                     const int2 m = vmv(make_uint2((unsigned)news, 0));
                     const bool fresh = fin && (!((actm >> lane) & 1u) || m.x != s.lmx[wi][lane] || m.y != s.lmy[wi][lane]);
                     freshm = __ballot_sync(kFull, fresh);
+                    __syncwarp();
                     if (fresh) { s.lmx[wi][lane] = m.x; s.lmy[wi][lane] = m.y; }
                     actm |= finm;
                     openm &= ~finm;
@@ -2107,16 +1937,16 @@ __device__ __forceinline__ void refine_block(Ctx &x, SH &s, DirScratch &ds, int 
     if (!b.fast_src) {
         dcsum = eval_slow(x, b.px, b.py, 0, 0, SLOW_DC).x;
     }
-    q.bmx = pmx; q.bmy = pmy;
-    q.bsad = parent < 0 ? 0u : (parent > 0xFFFFFFFFLL ? 0xFFFFFFFFu : (unsigned)parent);
-    q.bcost = parent < 0 ? 0 : parent;
+    unsigned best_sad = parent < 0 ? 0u : (parent > 0xFFFFFFFFLL ? 0xFFFFFFFFu : (unsigned)parent);
+    long long best = parent < 0 ? 0 : parent;
     if (search) {
         unsigned l, c;
         eval_cands(x, b, (x.tid & 31) == 0, pmx, pmy, l, c);
-        const unsigned sad = __shfl_sync(kFull, sat_add(l, c), 0);  // exact_sad at the clipped predictor
-        q.bsad = sad;
-        q.bcost = (long long)sad;
+        best_sad = __shfl_sync(kFull, sat_add(l, c), 0);  // exact_sad at the clipped predictor
+        best = (long long)best_sad;
     }
+    q.bmx = pmx; q.bmy = pmy;
+    q.bsad = best_sad; q.bcost = best;
     const int lambda = by == 0 ? 0 : (P.lambda >> 2) / factor;
     int bad = 0;
     q.stype = P.refine_search_type; q.radius = abs(P.refine_distance); q.lambda = lambda;
