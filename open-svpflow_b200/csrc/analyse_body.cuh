@@ -1493,6 +1493,10 @@ __device__ __forceinline__ void st_word(int *p, int v) {
     asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
+// A word that other warps change, as one value for the whole warp: what the lanes decide by it has to be the
+// same in all of them, and each lane's own load may find another.
+__device__ __forceinline__ int ld_warp_word(const int *p) { return __shfl_sync(kFull, ld_word(p), 0); }
+
 // The warp waits until done() holds in every lane. Bounded: false once kWaitCycles have passed or
 // another warp of the direction has given up (the caller flags ST_TIMEOUT and carries on).
 template <class F>
@@ -1625,7 +1629,7 @@ __device__ __forceinline__ void walk_level(const Ctx &x, SH &s, const DirScratch
                     // test alone, so it runs at once where the count of bad blocks known by now makes the
                     // block bad, and the outcome before it is kept in case the exact count says otherwise.
                     if (may_be_bad && !expanded && idx > 1 && (int)q.bsad > P.coarse_bad_sad) {
-                        const int known = ld_word(ctl + CTL_BAD);
+                        const int known = ld_warp_word(ctl + CTL_BAD);
                         if ((int)q.bsad > bad_limit(P, known)) {
                             q.rx = q.bmx; q.ry = q.bmy; q.rsad = q.bsad; q.rcost = q.bcost;
                             expanded = true;
@@ -1666,7 +1670,8 @@ __device__ __forceinline__ void walk_level(const Ctx &x, SH &s, const DirScratch
                         // The exact test. The count only grows, so a block that is not bad by what is known of it
                         // is not bad; the others wait for every earlier block's test.
                         const unsigned sad = expanded ? q.rsad : q.bsad;
-                        bool bad = idx > 1 && (int)sad > P.coarse_bad_sad && (int)sad > bad_limit(P, ld_word(ctl + CTL_BAD));
+                        bool bad = idx > 1 && (int)sad > P.coarse_bad_sad;
+                        if (bad) bad = (int)sad > bad_limit(P, ld_warp_word(ctl + CTL_BAD));
                         if (bad) {
                             if (!spin([&] {
                                     bool ok = true;
@@ -1675,7 +1680,7 @@ __device__ __forceinline__ void walk_level(const Ctx &x, SH &s, const DirScratch
                                 }, ctl + CTL_LATE))
                                 late = true;
                             __threadfence();
-                            bad_count = ld_word(ctl + CTL_BAD);
+                            bad_count = ld_warp_word(ctl + CTL_BAD);
                             bad = (int)sad > bad_limit(P, bad_count);
                             if (bad && lane == 0) { st_word(ctl + CTL_BAD, bad_count + 1); __threadfence(); }
                             __syncwarp();

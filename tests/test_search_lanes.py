@@ -24,3 +24,12 @@ def test_lanes_out_of_step_take_the_steps_of_one(program, seed):
     assert one.returncode == 0 and one.stdout.count("=") == 6 and len(one.stdout.splitlines()) > 60
     assert warp.returncode == 0, warp.stdout[-200:]
     assert warp.stdout == one.stdout
+
+
+def test_words_of_other_warps_decide_for_the_whole_warp():
+    # a direction's words (CTL_*) change under a walk: a branch into votes and shuffles takes one load of them,
+    # broadcast (ld_warp_word), never each lane's own
+    with open(os.path.join(CSRC, "analyse_body.cuh")) as f:
+        src = f.read()
+    assert "ld_word(ctl" not in src
+    assert src.count("ld_warp_word(ctl + CTL_BAD)") == 3
