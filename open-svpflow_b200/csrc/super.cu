@@ -1170,6 +1170,8 @@ __device__ __forceinline__ void level_item(const SuperDev &D, const uint8_t *src
     reduce_stripe<T, CG>(p, s, r0, min(I.band, p.dst_h - r0), (unsigned)D.px_max);
 }
 
+#include "flat_tiles.cuh"
+
 // Level 0 of every plane and frame, and the level 0 -> 1 reduction (from the source frames, whose rows
 // are level 0's full-pel rows), in one launch: a CTA does its share of both, every second one the
 // reduction first, so that the two kinds of work, the one bound by memory, the other by instruction
@@ -1203,16 +1205,18 @@ __device__ __forceinline__ void flat_level0(const SuperDev &D, const uint8_t *__
             const bool all = plane ? F.all_c : F.all_y;
             if (all && mis == 0) {
                 // two chunks of a thread at a time where both lie among the plane's middle rows: their loads overlap
-                for (uint32_t c = e * F.tile + threadIdx.x; c < (e + 1) * F.tile; c += 2 * blockDim.x) {
-                    const uint32_t a0 = c * 16u, a1 = (c + blockDim.x) * 16u;
-                    const uint32_t rowb = P.S * (uint32_t)sizeof(T);
-                    if (subpel && a0 >= rowb && a1 + rowb + 32u <= sub && P.src + a1 + rowb + 24 <= src_end) {
+                const uint32_t rowb = P.S * (uint32_t)sizeof(T);
+                tile_chunks(
+                    e, F.tile, threadIdx.x, blockDim.x,
+                    [&](uint32_t c0, uint32_t c1) {
+                        const uint32_t a0 = c0 * 16u, a1 = c1 * 16u;
+                        if (!(subpel && a0 >= rowb && a1 + rowb + 32u <= sub && P.src + a1 + rowb + 24 <= src_end)) return false;
                         flat_middle2<T>(P, nsub, a0, a1);
-                        continue;
-                    }
-                    if (a0 < sub) flat_chunk_all<T>(P, subpel, nsub, a0, src_end);
-                    if (a1 < sub) flat_chunk_all<T>(P, subpel, nsub, a1, src_end);
-                }
+                        return true;
+                    },
+                    [&](uint32_t c) {
+                        if (c * 16u < sub) flat_chunk_all<T>(P, subpel, nsub, c * 16u, src_end);
+                    });
             } else {
                 const uint32_t parts = all ? nsub : 1u;  // tiles were counted per sub-plane
                 for (uint32_t c = e * F.tile * parts + threadIdx.x; c < (e + 1) * F.tile * parts; c += blockDim.x) {
