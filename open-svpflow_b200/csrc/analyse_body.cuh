@@ -76,10 +76,6 @@ enum : uint8_t { CM_NONE = 0, CM_DIRECT = 1, CM_SAD_BREAK = 3, CM_EDGE = 4 };
 
 constexpr int ST_PANIC = 1;    // status bit: the reference indexes out of range here (it would panic)
 constexpr int ST_TIMEOUT = 4;  // status bit: a bounded wait inside the kernel ran out (internal error)
-// A wait on another warp's commit gives up after this many SM cycles (about 0.5 s at 1.9 GHz;
-// a level-0 block takes well under a millisecond). After one wait of a direction has given
-// up, its other waits return at once, so a failure costs one bound, not one per block.
-constexpr long long kWaitCycles = 1000000000LL;
 
 #include "search_steps.cuh"
 
@@ -1467,7 +1463,7 @@ __device__ __forceinline__ void search_level(const Ctx &x, DirSh &s, DirScratch 
 // (it is what such a block mostly does: at 640x360 the coarser levels took 2.5 to 3 times as long with
 // the expansions one after another). The lowest block that is not finished waits for nothing, and every
 // warp takes its blocks in order, so the warps, all resident, always make progress; the waits are
-// bounded all the same.
+// bounded all the same (walk_wait.h).
 // Bound: at few pairs the chain (a link is the wait's L2 round trip where nothing changed, a refinement where
 // something did), at many the latency of the candidates' loads (issue 32 %). With four warps per direction
 // that handed over in order, and the coarser levels in the pair's CTA: one 1080p pair 287 ms, 23 ms now; 32
@@ -1497,15 +1493,16 @@ __device__ __forceinline__ void st_word(int *p, int v) {
 // same in all of them, and each lane's own load may find another.
 __device__ __forceinline__ int ld_warp_word(const int *p) { return __shfl_sync(kFull, ld_word(p), 0); }
 
-// The warp waits until done() holds in every lane. Bounded: false once kWaitCycles have passed or
-// another warp of the direction has given up (the caller flags ST_TIMEOUT and carries on).
+// The warp waits until done() holds in every lane. Bounded: false once `cycles` have passed (LevelInfo::wait_cycles)
+// or another warp of the direction has given up (the caller flags ST_TIMEOUT and carries on). After one wait of a
+// direction has given up its others return at once, so a failure costs one bound, not one per block.
 template <class F>
-__device__ __forceinline__ bool spin(F done, int *late) {
+__device__ __forceinline__ bool spin(F done, int *late, int64_t cycles) {
     const long long t0 = clock64();
     for (int it = 1;; it++) {
         if (__all_sync(kFull, done())) return true;
         if ((it & 127) == 0) {
-            const int give_up = ld_word(late) || clock64() - t0 > kWaitCycles;
+            const int give_up = ld_word(late) || clock64() - t0 > cycles;
             if (__shfl_sync(kFull, give_up, 0)) {
                 if ((threadIdx.x & 31) == 0) st_word(late, 1);
                 return false;
@@ -1519,7 +1516,6 @@ __device__ __forceinline__ unsigned long long tag_word(int tag, int mx, int my) 
     return ((unsigned long long)tag << 32) | mkvec(mx, my, 0).x;
 }
 
-constexpr int kMaxWalkers = 64;  // warps of a direction that may walk a level
 template <class SH>
 __device__ __forceinline__ void walk_level(const Ctx &x, SH &s, const DirScratch &ds, const uint2 *prevp, int g, int D,
                                            int order_len, int gxv, int gyv, int *ctl, int *status, unsigned long long *stats) {
@@ -1579,7 +1575,7 @@ __device__ __forceinline__ void walk_level(const Ctx &x, SH &s, const DirScratch
             uint2 interp;
             if (edge) {  // its inner cell comes earlier in the order (level_spec_ok): that cell's final vector
                 unsigned long long v = 0;
-                if (!spin([&] { v = ld_tag(ds.keys + syi * gw + sxi); return (int)(v >> 32) == TAG_FINAL; }, ctl + CTL_LATE)) late = true;
+                if (!spin([&] { v = ld_tag(ds.keys + syi * gw + sxi); return (int)(v >> 32) == TAG_FINAL; }, ctl + CTL_LATE, L.wait_cycles)) late = true;
                 interp = make_uint2((unsigned)v, 0);  // the score is taken anew below
             } else {
                 interp = field[idx];
@@ -1652,7 +1648,7 @@ __device__ __forceinline__ void walk_level(const Ctx &x, SH &s, const DirScratch
                                 const int2 m = vmv(make_uint2((unsigned)v, 0));
                                 freshm = __ballot_sync(kFull, open && (int)(v >> 32) != TAG_NONE && (!act || m.x != mx || m.y != my));
                                 return freshm || !(open && (int)(v >> 32) != TAG_FINAL);
-                            }, ctl + CTL_LATE)) {
+                            }, ctl + CTL_LATE, L.wait_cycles)) {
                             late = true;
                             openm = 0;
                         } else if (!freshm && sure) {  // the next block in the chain waits for this store
@@ -1677,7 +1673,7 @@ __device__ __forceinline__ void walk_level(const Ctx &x, SH &s, const DirScratch
                                     bool ok = true;
                                     for (int h = lane; h < D; h += 32) ok = ok && (h == g || ld_word(progress + h) >= k);
                                     return ok;
-                                }, ctl + CTL_LATE))
+                                }, ctl + CTL_LATE, L.wait_cycles))
                                 late = true;
                             __threadfence();
                             bad_count = ld_warp_word(ctl + CTL_BAD);

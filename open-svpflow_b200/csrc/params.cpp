@@ -85,6 +85,7 @@ bool build_analyse_params(const AnalyseOpts &o, const SuperLayout &Lay, AnalyseP
             const int nl = o.levels > 1 ? o.levels : 1;
             L.base_radius = dd == 0 ? ((lv == 0 && nl > 1) ? 0 : 10) : (dd < 0 ? -dd : dd);
         }
+        L.wait_cycles = wait_cycles(most_candidates(L.search_type, L.base_radius, lv > 0 && o.coarse_bad_sad > 0, o.coarse_bad_range));
         if (L.smallest) {
             L.bw = o.block_w >> 1; L.bh = o.block_h >> 1; L.pxoff = o.block_w >> 2; L.pyoff = o.block_h >> 2;
         } else {

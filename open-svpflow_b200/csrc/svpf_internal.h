@@ -10,6 +10,8 @@
 
 #include <string>
 
+#include "walk_wait.h"
+
 namespace svpf {
 
 constexpr int kMaxLevels = 16;
@@ -90,6 +92,7 @@ struct LevelInfo {
     int32_t satd, search_type, base_radius, smallest;
     int32_t bw, bh, pxoff, pyoff;  // searched block (halved and centred at the smallest level)
     int32_t tl, tc;           // 4x4 luma tiles, 4x4 chroma tiles per plane of one candidate
+    int64_t wait_cycles;      // a walk of the level: SM cycles without a finished block after which a wait gives up
 };
 
 struct alignas(16) AnalyseParams {
