@@ -2658,39 +2658,44 @@ cudaError_t prepare() {
 #if SVPF_LOOKAHEAD
 namespace {
 constexpr int kMinWalkers = 4;  // warps per direction of a walk, at least
-// The build and the resident CTAs of a walk over `ndirs` search directions.
+// The build of a walk over `ndirs` search directions, its shared memory and how many CTAs of that very kernel are
+// resident at once: the plain and the batch's kernels need not have the same registers.
+template <class KERNEL>
 struct WalkShape {
+    KERNEL kernel;
     bool dense;
     size_t smem;
     int64_t resident;
 };
-cudaError_t walk_shape(int groups, int64_t ndirs, WalkShape &w) {
+template <class KERNEL>
+cudaError_t walk_shape(KERNEL sparse, KERNEL dense, int groups, int64_t ndirs, WalkShape<KERNEL> &w) {
     w.smem = (size_t)groups * kGroupBytes;
     int dev = 0, sms = 0, per_sm = 0;
     if (cudaError_t e = cudaGetDevice(&dev)) return e;
     if (cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) return e;
-    if (cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, analyse_walk_kernel<kWalkPerSM>, 32, w.smem)) return e;
+    if (cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sparse, 32, w.smem)) return e;
     w.dense = (int64_t)sms * per_sm < ndirs * kDenseWalkers;
+    w.kernel = w.dense ? dense : sparse;
     if (w.dense)
-        if (cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, analyse_walk_kernel<kDensePerSM>, 32, w.smem)) return e;
+        if (cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dense, 32, w.smem)) return e;
     w.resident = (int64_t)sms * per_sm;
     return cudaSuccess;
 }
 // The CTAs of a walk wait on one another, so the launch is cooperative and takes the directions whose
 // CTAs are all resident at once.
-template <class... P, class... A>
-cudaError_t launch_walk(void (*kernel)(P...), int64_t ctas, size_t smem, cudaStream_t stream, A... args) {
+template <class KERNEL, class... A>
+cudaError_t launch_walk(const WalkShape<KERNEL> &w, int64_t ctas, cudaStream_t stream, A... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)ctas);
     cfg.blockDim = dim3(32);
-    cfg.dynamicSmemBytes = smem;
+    cfg.dynamicSmemBytes = w.smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
+    return cudaLaunchKernelEx(&cfg, w.kernel, args...);
 }
 }  // namespace
 #endif
@@ -2710,8 +2715,10 @@ cudaError_t launch_plain(const AnalyseParams &P, const PairSrc &psrc, int npairs
 #if SVPF_LOOKAHEAD
     // D warps per direction, as many as are resident at once (at least kMinWalkers, with the pairs in
     // several launches when they would not be)
-    WalkShape w;
-    if (cudaError_t e = walk_shape(P.stage_groups, (int64_t)npairs * ndir, w)) return e;
+    WalkShape<decltype(&analyse_walk_kernel<kWalkPerSM>)> w;
+    if (cudaError_t e = walk_shape(analyse_walk_kernel<kWalkPerSM>, analyse_walk_kernel<kDensePerSM>, P.stage_groups,
+                                   (int64_t)npairs * ndir, w))
+        return e;
     const size_t stage = w.smem;
     const int64_t resident = w.resident;
     const int64_t most = resident / (ndir * kMinWalkers);
@@ -2726,9 +2733,7 @@ cudaError_t launch_plain(const AnalyseParams &P, const PairSrc &psrc, int npairs
         if (cudaError_t e = count()) return e;
         for (int64_t f = 0; f < npairs; f += group) {
             const int64_t n = npairs - f < group ? npairs - f : group;
-            if (cudaError_t e = launch_walk(w.dense ? analyse_walk_kernel<kDensePerSM> : analyse_walk_kernel<kWalkPerSM>,
-                                            n * ndir * D, stage, stream, P, psrc, f, lo, (int)D, scratch, status_dev))
-                return e;
+            if (cudaError_t e = launch_walk(w, n * ndir * D, stream, P, psrc, f, lo, (int)D, scratch, status_dev)) return e;
             if (launches) *launches += 1;
         }
     }
@@ -2770,11 +2775,16 @@ cudaError_t launch_batch(const AnalyseParams *clips_dev, const BatchItem *items_
 // The batch walked level by level (batch_ground_kernel): `grid` pairs at a time.
 int first_walk_level(const AnalyseParams &P) { return first_walk(P); }
 
+using BatchWalkShape = WalkShape<decltype(&batch_walk_kernel<kWalkPerSM>)>;
+cudaError_t batch_walk_shape(int groups, int64_t ndirs, BatchWalkShape &w) {
+    return walk_shape(batch_walk_kernel<kWalkPerSM>, batch_walk_kernel<kDensePerSM>, groups, ndirs, w);
+}
+
 // Pairs of a group per SM: enough to fill the SMs with at least kMinWalkers warps per direction.
 cudaError_t batch_walk_pairs_per_sm(const BatchInfo &info, int *pairs) {
-    WalkShape w;
+    BatchWalkShape w;
     if (cudaError_t e = prepare()) return e;
-    if (cudaError_t e = walk_shape(info.groups, (int64_t)1 << 30, w)) return e;
+    if (cudaError_t e = batch_walk_shape(info.groups, (int64_t)1 << 30, w)) return e;
     int dev = 0, sms = 0;
     if (cudaError_t e = cudaGetDevice(&dev)) return e;
     if (cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) return e;
@@ -2792,8 +2802,8 @@ cudaError_t launch_batch_walk(const AnalyseParams *clips_dev, const BatchItem *i
     if (ground != cudaSuccess) return ground;
     auto count = [&] { if (launches) *launches += 1; return cudaGetLastError(); };
     const int ngroups = (nitems + grid - 1) / grid, group = (nitems + ngroups - 1) / ngroups;  // even groups
-    WalkShape w;
-    if (cudaError_t e = walk_shape(info.groups, (int64_t)group * 2, w)) return e;
+    BatchWalkShape w;
+    if (cudaError_t e = batch_walk_shape(info.groups, (int64_t)group * 2, w)) return e;
     int64_t D = w.resident / (group * 2);
     if (D < 1) return cudaErrorCooperativeLaunchTooLarge;
     if (D > kMaxWalkers) D = kMaxWalkers;
@@ -2804,8 +2814,7 @@ cudaError_t launch_batch_walk(const AnalyseParams *clips_dev, const BatchItem *i
             batch_ground_kernel<<<n, 2 * NT, pair_shared(2, info.groups), stream>>>(clips_dev, it, lo, scratch, scratch_per_slot,
                                                                                     clip_status_dev, info.groups);
             if (cudaError_t e = count()) return e;
-            if (cudaError_t e = launch_walk(w.dense ? batch_walk_kernel<kDensePerSM> : batch_walk_kernel<kWalkPerSM>, n * 2 * D,
-                                            w.smem, stream, clips_dev, it, lo, (int)D, scratch, scratch_per_slot,
+            if (cudaError_t e = launch_walk(w, n * 2 * D, stream, clips_dev, it, lo, (int)D, scratch, scratch_per_slot,
                                             clip_status_dev, info.groups))
                 return e;
             if (launches) *launches += 1;

@@ -41,3 +41,14 @@ def test_waits_outlast_the_chain_they_wait_for(tmp_path):
     subprocess.run(["g++", "-std=c++17", "-I", CSRC, str(src), "-o", exe], check=True)
     r = subprocess.run([exe], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stdout
+
+
+def test_residency_is_asked_of_the_kernel_that_is_launched():
+    # a walk's CTAs wait on one another, so its grid is sized by the occupancy of the very kernel it launches: the shape
+    # that holds the answer holds the kernel too, and the plain and the batch's walks each make their own
+    with open(os.path.join(CSRC, "analyse_body.cuh")) as f:
+        src = f.read()
+    assert src.count("cudaLaunchKernelEx(&cfg, w.kernel, args...)") == src.count("cudaLaunchKernelEx(") == 1
+    for name in ("analyse", "batch"):
+        assert f"walk_shape({name}_walk_kernel<kWalkPerSM>, {name}_walk_kernel<kDensePerSM>" in src
+        assert f"cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, {name}_walk_kernel" not in src
