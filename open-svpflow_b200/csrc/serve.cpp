@@ -73,6 +73,7 @@ struct Request {
     int64_t need = 0;
     int slot = -1;
     uint8_t *dev = nullptr;
+    int64_t room = 0;            // what the clips active at its admission left of the budget
     bool pinned_out = false;     // payloads are page-locked host memory
     int status = 0;
     bool done = false;
@@ -156,6 +157,18 @@ void CUDART_CB request_done(void *arg) {
     s->done_cv.notify_all();
 }
 
+// Device memory that the pool the server's clips come from holds, in use or not.
+int64_t pool_bytes(const svpf_server *s) {
+    cudaMemPool_t pool;
+    uint64_t held = 0;
+    if (cudaDeviceGetDefaultMemPool(&pool, s->device) != cudaSuccess ||
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess) {
+        cudaGetLastError();
+        return s->budget;  // no growth
+    }
+    return (int64_t)held;
+}
+
 // Queues the whole of one admitted request on its slot's lanes: lane 0 allocates, copies the
 // frames in and builds the super frames; every lane then analyses its chunks (own scratch,
 // own staging) and copies their payloads out; lane 0 joins the lanes, copies the status word
@@ -169,12 +182,17 @@ int enqueue(svpf_server *s, Request *r) {
     const int64_t cmax = r->chunks.empty() ? 1 : r->chunks[0].count;
     // Memory new to the pool takes the driver 3 to 60 ms to map, in which no other clip is queued: as long
     // as four small clips take together (25 ms). So the pool grows by every slot's share at once, the first
-    // time a clip of a size comes, up to the budget and kGrowBytes; larger clips map what they need.
-    const int64_t share = std::min(std::min(s->budget, kGrowBytes), r->need * s->max_active);
+    // time a clip of a size comes, up to kGrowBytes and as far as what the pool holds and what the other clips
+    // take leave room in the budget; larger clips map what they need.
+    const int64_t share = std::min(std::min(std::min(r->room, s->budget - pool_bytes(s)), kGrowBytes), r->need * s->max_active);
     if (share > s->grown && share >= r->need) {
         void *p = nullptr;
-        if (cudaMallocAsync(&p, (size_t)share, st) == cudaSuccess) cudaFreeAsync(p, st);
-        else cudaGetLastError();  // the clip's own allocation decides
+        if (cudaMallocAsync(&p, (size_t)share, st) == cudaSuccess) {
+            cudaFreeAsync(p, st);
+            cudaStreamSynchronize(st);  // free for every stream; else the next clip's would map memory of its own
+        } else {
+            cudaGetLastError();  // the clip's own allocation decides
+        }
         s->grown = share;
     }
     cudaError_t e = cudaMallocAsync((void **)&r->dev, (size_t)r->need, st);
@@ -267,6 +285,7 @@ void scheduler(svpf_server *s) {
         while (s->slot_busy[(size_t)slot]) slot++;
         s->slot_busy[(size_t)slot] = true;
         r->slot = slot;
+        r->room = s->budget - s->used;
         s->used += r->need;
         s->peak_used = s->used > s->peak_used ? s->used : s->peak_used;
         s->active++;
@@ -440,6 +459,10 @@ void svpf_server_destroy(svpf_server *s) {
     for (auto &st : s->streams) {
         cudaStreamSynchronize(st);
         cudaStreamDestroy(st);
+    }
+    {  // what its clips no longer use goes back to the device
+        cudaMemPool_t pool;
+        if (cudaDeviceGetDefaultMemPool(&pool, s->device) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
     }
     for (auto &ev : s->events)
         if (ev) cudaEventDestroy(ev);
