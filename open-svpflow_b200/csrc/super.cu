@@ -1392,12 +1392,35 @@ LevelItems level_items(const SuperDev &D, int lv, int nframes, int sms) {
         if (I.band == 2 || I.total >= (uint32_t)sms * 32) return I;
     }
 }
-// Levels whose result has at most this many luma samples go to the tail kernel, a cluster per plane and frame.
-// (One frame of 640x360: 34.9 us; with the tail from 10000 or 3000 samples on 38.6 and 41.1. The last levels of
-// 48 frames of 854x480 through the tail 441 us, by a launch each 195: more frames than kTailFrames fill the GPU at
-// every level.)
+// Levels whose result has at most this many luma samples go to the tail kernel, a cluster per plane and frame. (From
+// 20000, 40000, 80000 and 160000 samples on, us: one frame of 640x360 34.9, 34.9, 34.9, 34.9, 10000 37.7; of 1080p
+// 61.2, 59.5, 59.9, 64.9; of 2160p at 10 bits 163, 164, 165, 176.)
 constexpr int64_t kTailSamples = 40000;
-constexpr int kTailFrames = 6;
+// It takes as many frames as have all their clusters resident at once: 15 clusters, so 5 frames. With a second wave
+// of clusters, a launch per level is faster. (The tail against a launch per level, us, 5 and 6 frames: 640x360 37.0 to
+// 53.6 and 55.4 to 55.4; 854x480 69.7 to 84.1 and 98.5 to 84.2; 1080p 79.4 to 101.2 and 108.9 to 105.9; 2160p at 10
+// bits 558 to 574 and 692 to 676.)
+template <typename T>
+int tail_frames() {
+    static const int most = [] {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(kTailCtas);
+        cfg.blockDim = dim3(512);
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = kTailCtas;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, super_tail_kernel<T>, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            return 0;
+        }
+        return clusters / 3;
+    }();
+    return most;
+}
 template <typename T>
 int launch_super_flat(const SuperDev &D, const uint8_t *src, uint8_t *dst, int nframes, int sms, cudaStream_t stream) {
     const int per_sm = sizeof(T) == 1 ? 3 : 2;
@@ -1438,7 +1461,7 @@ int launch_super_flat(const SuperDev &D, const uint8_t *src, uint8_t *dst, int n
         super_level_kernel<T><<<(int)std::min<int64_t>((L.total + 7) / 8, (int64_t)sms * per_sm), 256, 0, stream>>>(D, nullptr, dst, L);
         n++;
     }
-    if (nframes > kTailFrames)  // enough work for a launch per level
+    if (nframes > tail_frames<T>())  // a launch per level
         for (; lv + 1 < D.levels; lv++) {
             const LevelItems L = level_items(D, lv, nframes, sms);
             super_level_kernel<T><<<(int)std::min<int64_t>((L.total + 7) / 8, (int64_t)sms * per_sm), 256, 0, stream>>>(D, nullptr, dst, L);

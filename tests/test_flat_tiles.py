@@ -1,7 +1,14 @@
-"""A tile of Super's level-0 chunks (csrc/flat_tiles.cuh, the loop the kernel runs, compiled for the host): every
-chunk of a plane is done once, whatever the tile's size and whichever pairs can be taken together."""
+"""Super's path for packed frames: a tile of level-0 chunks (csrc/flat_tiles.cuh, the loop the kernel runs, compiled
+for the host) does every chunk of a plane once, whatever the tile's size and whichever pairs can be taken together;
+frame counts around the line between its two ways to the last levels, against the oracle."""
 import os
 import subprocess
+
+import numpy as np
+import pytest
+
+from oracle import oracle as orc
+from test_px16 import clip10
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "open-svpflow_b200", "csrc")
 PROGRAM = r"""
@@ -36,3 +43,22 @@ def test_every_chunk_is_done_once(tmp_path):
     subprocess.run(["g++", "-std=c++17", "-I", CSRC, str(src), "-o", exe], check=True)
     r = subprocess.run([exe], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stdout
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bits", [8, 10])
+@pytest.mark.parametrize("frames", [4, 5, 6])
+def test_super_around_the_most_frames_of_the_tail(frames, bits):
+    # the last levels go to clusters that are all resident at once (5 frames on 148 SMs), else to a launch each
+    import svpflow_b200 as sv
+
+    w, h, opt = 326, 182, "{pel:2}"
+    if bits > 8:
+        clip = clip10(w, h, frames, 60 + frames)
+    else:
+        from svpflow_b200.synth import make_clip
+
+        clip = make_clip(w, h, frames, seed=60 + frames)
+    so = orc.super_opts(w, h, opt)
+    want = orc.build_super_many16(so, clip) if bits > 8 else orc.build_super_many(so, clip, os.cpu_count() or 1)
+    assert np.array_equal(sv.Super(w, h, opt, bits=bits).build_many(clip), want)
