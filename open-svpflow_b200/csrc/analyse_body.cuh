@@ -1419,7 +1419,8 @@ __device__ __forceinline__ void search_level(const Ctx &x, DirSh &s, DirScratch 
         const bool search = !(level == 0 && P.distance == 0);
         if (!search) act = lane == (field_valid ? kField : kZero);
         const unsigned sd = special_sads(x, b, s, ph, act, mx, my);
-        const int pp = lane < 9 ? P.pnbour : lane == kPrev ? P.prev : lane == kGlobal ? P.pglobal : lane == kZero ? P.pzero : 0;
+        // the penalty of the lane's special candidate; read here, since a meeting of the lanes makes the loop read it anew
+    const int pp = lane < 9 ? P.pnbour : lane == kPrev ? P.prev : lane == kGlobal ? P.pglobal : lane == kZero ? P.pzero : 0;
         const int place = lane < 9 ? 4 + __popc(seeds & ((1u << lane) - 1u)) : lane - kField;
         const long long cost = (long long)sd + (((long long)pp * sd) >> 8);
         const int wl = first_min(act, cost, place);
@@ -1560,6 +1561,8 @@ __device__ __forceinline__ void walk_level(const Ctx &x, SH &s, const DirScratch
     Search &q = s.q[wi];
     int n_blk = 0, n_def = 0, n_eval = 0, n_rerun = 0;
     bool late = false;
+    // the penalty of the lane's special candidate; read here, since a meeting of the lanes makes the loop read it anew
+    const int pp = lane < 9 ? P.pnbour : lane == kPrev ? P.prev : lane == kGlobal ? P.pglobal : lane == kZero ? P.pzero : 0;
     for (int k = g; k < order_len; k += D) {
         const int2 bxy = level == 0 ? initial_order_at(gw, gh, k) : unpack_xy(ds.order[k]);
         const int bx = bxy.x, by = bxy.y;
@@ -1751,7 +1754,6 @@ __device__ __forceinline__ void walk_level(const Ctx &x, SH &s, const DirScratch
                 __syncwarp();
                 s.lsd[wi][lane] = sd;
                 freshm = 0;
-                const int pp = lane < 9 ? P.pnbour : lane == kPrev ? P.prev : lane == kGlobal ? P.pglobal : lane == kZero ? P.pzero : 0;
                 const int place = lane < 9 ? 4 + __popc(seeds & ((1u << lane) - 1u)) : lane - kField;
                 const long long cost = (long long)sd + (((long long)pp * sd) >> 8);
                 const int wl = first_min((actm >> lane) & 1u, cost, place);
