@@ -67,38 +67,45 @@ DESC = {
 }
 UNIT = "frame-pairs/s"
 # DRAM bytes per frame pair of the Analyse launch at 1080p: ncu's dram__bytes_read.sum +
-# dram__bytes_write.sum of the kernels of the 240-pair launch (one-pass counters, 25.08 + 2.10 GB:
-# profiles/analyse_walk_kernels.md)
-TRAFFIC_PER_PAIR = 27.18e9 / 240
-# DRAM bytes of one 1080p render launch with the 8 x 8 effective block (ncu capture: 4.13 MB read,
+# dram__bytes_write.sum of the kernels of the 240-pair launch (one-pass counters, 25.02 + 2.13 GB)
+TRAFFIC_PER_PAIR = 27.15e9 / 240
+# DRAM bytes of one 1080p render launch with the 8 x 8 effective block (ncu capture: 4.2 MB read,
 # the written frame stays in L2)
-RENDER_TRAFFIC_PER_FRAME = 4.14e6
+RENDER_TRAFFIC_PER_FRAME = 4.2e6
 # graph replays per timed render step (about 40 ms, so the clock sampler sees the step)
 RENDER_REPLAYS = 48
 # int32 lanes per SM on sm_100 (64 on the ALU pipe, 64 IMAD on the FMA-heavy pipe; ncu's pipe counters
 # of the Analyse kernel put the ALU pipe's peak at 2 warp instructions per SM cycle) and the SM clock
 # ceiling, for the nominal integer peak
 INT32_LANES_PER_SM = 128
-# integer ops per frame pair (oracle counts of the workloads' compares), when the CPU leg is skipped
-OPS_PER_PAIR = {"1080p": 19.38e9}
-# why the Analyse launch reaches the fraction it does, from the ncu counters of the 240-pair launch
-# in profiles/analyse_walk_kernels.md: issue utilisation (warp instructions / (4 schedulers x
-# SMs x the launch's SM cycles)) x useful lane fraction (algorithmic ops / executed lane slots)
-ROOF_DECOMPOSITION = {"issue_active": 0.322, "useful_lane_fraction": 0.530,
-                      "source": "ncu counters of the 240-pair 1080p launch (five analyse_walk_kernel launches 273.6 G, "
-                                "analyse_kernel and analyse_pack_kernel 0.7 G warp instructions in 731.6 ms): 1.14 G "
-                                "warp instructions = 36.6 G lane slots per pair for 19.4 G algorithmic ops, the SATD "
-                                "transforms among them, which run on the tensor cores "
-                                "(profiles/analyse_walk_kernels.md)"}
+# SATD 4x4 tiles per frame pair (oracle counts; every compare of the workload is SATD), when the CPU leg is skipped
+TILES_PER_PAIR = {"1080p": 174.9e6}
+# A tile's transform is a 16 x 16 product on the tensor cores; its absolute values and sums are left to the lanes.
+TILE_TENSOR_FLOPS, TILE_LANE_OPS = 512, 32
+# why the Analyse launch reaches the fraction it does, from the ncu counters of the 240-pair launch:
+# issue utilisation (warp instructions / (4 schedulers x SMs x the launch's SM cycles)) x useful lane
+# fraction (lane ops / executed lane slots)
+ROOF_DECOMPOSITION = {"issue_active": 0.327, "useful_lane_fraction": 0.152,
+                      "source": "ncu counters of the 240-pair 1080p launch (the analyse_walk_kernel launches 276.3 G, "
+                                "analyse_kernel and analyse_pack_kernel 0.5 G warp instructions in 728 ms): 1.15 G "
+                                "warp instructions = 36.9 G lane slots per pair for 5.6 G lane ops; the rest is loads, "
+                                "funnel shifts, operand set-up and reductions"}
 # the CPU legs time this many frame pairs per host thread, so that their figure is a throughput
 # (dynamic scheduling over many pairs) rather than the latency of the slowest pair
 CPU_PAIRS_PER_THREAD = 4
-# the batched object of the default line runs this launch shape (the fastest for the 64-clip mix: 174.2
-# pairs/s against 154.7 walked), so the default run spends no time on autotune trials
+# the batched object of the default line runs this launch shape (the fastest for the 64-clip mix: 168.7
+# pairs/s against 150.7 walked), so the default run spends no time on autotune trials
 BATCH_SHAPE = "nt32_b8:8"
 # the served object's arrival rates, clips/s: below the server's capacity, and the configuration's lowest
 SERVED_RATES = "0.25,5"
 SM_MAX_MHZ = 1965.0
+
+
+def _work(cnt, pairs):
+    """SATD 4x4 tiles and lane operations per frame pair of the compares counted in `cnt`."""
+    satd = cnt[3] + cnt[4]
+    tiles = satd / 16 / pairs
+    return tiles, 2.0 * (cnt[1] + cnt[2] - satd) / pairs + TILE_LANE_OPS * tiles
 
 
 def _sm_count() -> int:
@@ -117,17 +124,18 @@ def _peaks():
 
 
 def _chain(an, nf: int, a_ms: float) -> dict:
-    """The non-roofline bound: every pair of a launch runs concurrently (one CTA each), so the launch
-    lasts about one pair's serial block chain; per level-0 block of one direction."""
+    """The non-roofline bound: every pair of a walk runs concurrently (at least four one-warp CTAs per
+    direction, 20 per SM), so the launch lasts about one pair's chain of blocks; per level-0 block of one
+    direction."""
     vd = an.vector_header()
-    sms = _sm_count()
-    waves = -(-nf // (3 * sms)) if nf > 2 * sms else 1  # 3-CTA shape above 2 pairs per SM, else one wave
+    most = 20 * _sm_count() // (2 * 4)  # pairs whose warps are resident at once
+    waves = -(-nf // most)
     l0 = vd[11] * vd[12]
-    return {"pairs_in_flight": min(nf, 3 * sms if nf > 2 * sms else nf), "waves": waves,
+    return {"pairs_in_flight": -(-nf // waves), "waves": waves,
             "pair_latency_ms": a_ms / waves, "level0_blocks_per_direction": l0,
             "us_per_level0_block": a_ms / waves * 1000.0 / max(l0, 1),
-            "note": "blocks of a level run in the reference's serial order (each reads its processed "
-                    "neighbours); the time per block, not issue or memory throughput, bounds one pair"}
+            "note": "blocks of a level depend on their processed neighbours in the reference's serial order; with "
+                    "few pairs that chain bounds the launch, with many the latency of the candidates' loads"}
 
 
 def _config(nframes: int, world: int, shard_frames: bool = False) -> dict:
@@ -657,17 +665,17 @@ def run_render(args, world: int, rank: int, local: int):
                     "d2h_bytes_per_step": int(nf * w * h * 3 // 2), "api": "svpf_render_warp_device with host copies",
                     "matches_device_path": same},
             "gpu_launches": int(launches),
-            "roofline": {"kernel": "render_kernel<0, 0> (single warp)", "bound": "hbm",
+            "roofline": {"kernel": "render_tile_kernel<0, 0, 1> (single warp)", "bound": "hbm",
                          "achieved": per_frame * nf * reps / (ms / args.steps / 1000) / 1e9, "peak": peak,
                          "unit": "GB/s", "frac": per_frame * nf * reps / (ms / args.steps / 1000) / 1e9 / peak,
                          "traffic": RENDER_TRAFFIC_PER_FRAME * nf * reps,
                          "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch (1080p "
                                            "frame; the output stays in L2), x frames per step",
                          "peak_source": peak_kind, "algorithmic_bytes_per_frame": per_frame,
-                         "note": "issue-bound, not HBM-bound: per sample a tile lookup, motion interpolation and "
-                                 "an index computation (67 % issue active in the ncu capture)"},
+                         "note": "issue-bound, not HBM-bound: per sample the motion interpolation and an index "
+                                 "computation (53 % issue active in the ncu capture, and the gathers' latency)"},
             "cpu_baseline": cpu, "parity_vs_oracle": parity,
-            "blend_mode13": {"value": blend_value, "unit": "frames/s", "kernel": "render_kernel<dual>",
+            "blend_mode13": {"value": blend_value, "unit": "frames/s", "kernel": "render_tile_kernel<1, 0, 1>",
                              "how": "svpf_render_blend_device (algorithm 13: frames f and f+1, the two vector sets "
                                     "of frame f's payload), same frames and timing", "parity_vs_oracle": blend_check},
             "masked_mode21": {"value": masked_value, "unit": "frames/s",
@@ -777,7 +785,7 @@ def run_2160p10(args, world: int, rank: int, local: int):
         alg_analyse = nf * (2 * fb + pl)
         alg_super = nf * (sb.source_len() + fb)
         roof = {
-            "kernel": "analyse_kernel, uint16 build (one CTA per frame pair, fwd/bwd halves)",
+            "kernel": "Analyse, uint16 build: analyse_walk_kernel per level, analyse_kernel between them, analyse_pack_kernel",
             "bound": "hbm", "achieved": alg_analyse / (a_ms / 1000) / 1e9, "peak": peak, "unit": "GB/s",
             "frac": alg_analyse / (a_ms / 1000) / 1e9 / peak, "traffic": None, "peak_source": peak_kind,
             "algorithmic_bytes_per_launch": alg_analyse, "avg_launch_ms": a_ms,
@@ -802,12 +810,13 @@ def run_2160p10(args, world: int, rank: int, local: int):
                              f"threads, the oracle's uint16 build (scalar SAD/SATD)",
                    "cpu_model": _cpu_model()}
             parity = {"pairs_checked": pairs, "bit_exact": bool(np.array_equal(pay_cpu, pay_host[:pairs]))}
-            ops_pair = orc.integer_ops(cnt) / pairs
+            tiles_pair, ops_pair = _work(cnt, pairs)
             int_peak = INT32_LANES_PER_SM * _sm_count() * SM_MAX_MHZ * 1e6
             hbm = {k: roof.pop(k) for k in ("bound", "achieved", "peak", "unit", "frac", "peak_source")}
             roof.update({
                 "bound": "int32 pipe", "achieved": ops_pair * nf / (a_ms / 1000) / 1e12, "peak": int_peak / 1e12,
                 "unit": "Tops/s", "frac": ops_pair * nf / (a_ms / 1000) / int_peak, "ops_per_pair": ops_pair,
+                "tensor_flops_per_pair": TILE_TENSOR_FLOPS * tiles_pair,
                 "evaluations_per_pair": cnt[0] / pairs, "samples_compared_per_pair": (cnt[1] + cnt[2]) / pairs,
                 "satd_share": (cnt[3] + cnt[4]) / max(cnt[1] + cnt[2], 1),
                 "peak_source": f"nominal: {_sm_count()} SMs x {INT32_LANES_PER_SM} int32 lanes (64 ALU + 64 IMAD on "
@@ -1301,7 +1310,8 @@ def main():
         alg_analyse = a_count * (2 * fb + pl)  # algorithmic bytes of one Analyse launch: 2 super frames + payload per pair
         alg_super = n_src * (sb.source_len() + fb)  # one Super launch sequence: source read + super frame write
         int_peak = INT32_LANES_PER_SM * _sm_count() * SM_MAX_MHZ * 1e6
-        ops_pair = None if args.size else OPS_PER_PAIR.get(WORKLOAD)  # the constants hold at the workload's size
+        tiles_pair = None if args.size else TILES_PER_PAIR.get(WORKLOAD)  # the constants hold at the workload's size
+        ops_pair = tiles_pair * TILE_LANE_OPS if tiles_pair else None
         ops_src = ("no count at this frame size (CPU leg not run)" if args.size else
                    "constant from an earlier oracle count of the same workload (CPU leg not run)")
         cpu = None
@@ -1314,10 +1324,10 @@ def main():
             from oracle import oracle as orc
 
             cnt = cpu_reference.counters
-            ops_pair = orc.integer_ops(cnt) / pairs
-            ops_src = (f"compares the oracle executed on output frames 0..{pairs - 1} (2 ops per SAD sample, 111 "
-                       f"per SATD 4x4 tile)")
-        # the Analyse kernel's primary bound: the int32 pipes (the SATD products leave the tensor cores idle, little HBM traffic)
+            tiles_pair, ops_pair = _work(cnt, pairs)
+            ops_src = (f"compares the oracle executed on output frames 0..{pairs - 1} (2 ops per SAD sample, {TILE_LANE_OPS} "
+                       f"per SATD 4x4 tile beside its transform, which runs on the tensor cores)")
+        # the Analyse kernel's primary bound of the two kinds of arithmetic: the int32 pipes (little HBM traffic)
         roof = {
             "kernel": ("Analyse: analyse_walk_kernel per level (one-warp CTAs over the GPU), analyse_kernel between "
                        "them (one CTA per frame pair), analyse_pack_kernel; timed together"),
@@ -1329,6 +1339,7 @@ def main():
             "traffic_source": ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the kernels of the "
                                "240-pair launch, per pair x pairs"),
             "ops_per_pair": ops_pair, "ops_source": ops_src, "avg_launch_ms": a_ms,
+            "tensor_flops_per_pair": TILE_TENSOR_FLOPS * tiles_pair if tiles_pair is not None else None,
             "peak_source": f"nominal: {_sm_count()} SMs x {INT32_LANES_PER_SM} int32 lanes (64 on the ALU pipe + 64 "
                            f"IMAD on the FMA-heavy pipe) x {SM_MAX_MHZ:.0f} MHz; no measured integer peak exists",
             "decomposition": ROOF_DECOMPOSITION,

@@ -102,10 +102,10 @@ struct BlkC {
 };
 
 // Shared state of one search direction. A block is searched by a group of warps: the whole
-// direction (coarser levels), or one warp (level 0 with look-ahead, one block per warp in
+// direction (search_level), or one warp (a walk, the refine pass: a block per warp in
 // flight). Per-warp entries are indexed by the warp's place in the direction; a group's
 // entries are those of its first warp (Ctx::wbase). W: the warps it holds state for (the
-// direction's, or one for a CTA of the level-0 kernel).
+// direction's, or one for a CTA of a walk).
 template <int W>
 struct alignas(16) DirShT {
     Search q[W];                          // per warp: its block's search ...
@@ -130,7 +130,7 @@ struct alignas(16) DirShT {
 // eight tiles) and the group's offsets (128 bytes), AnalyseParams::stage_groups of each.
 constexpr int kGroupBytes = 640;
 using DirSh = DirShT<NW>;  // a search direction of the pair kernels
-using WarpSh = DirShT<1>;  // a CTA (one warp) of the level-0 kernel
+using WarpSh = DirShT<1>;  // a CTA (one warp) of a walk or the refine pass
 
 struct Planes {
     const px_t *y, *u, *v;
@@ -397,8 +397,6 @@ __device__ unsigned luma_tile(const Cand &c, const Planes &S, const Planes &R, c
     for (int i = 0; i < 16; i++) s += (unsigned)abs(d[i]);
     return s;
 }
-
-// One 4x4 tile of both chroma planes of a candidate.
 
 // One 4x4 tile of one chroma plane of a candidate on the general path.
 __device__ unsigned chroma_tile1(const Cand &c, const px_t *sp, const px_t *rp, const Geo &G, int cw, int tile) {
@@ -1495,9 +1493,9 @@ __device__ __forceinline__ void search_level(const Ctx &x, DirSh &s, DirScratch 
 // warp takes its blocks in order, so the warps, all resident, always make progress; the waits are
 // bounded all the same (walk_wait.h).
 // Bound: at few pairs the chain (a link is the wait's L2 round trip where nothing changed, a refinement where
-// something did), at many the latency of the candidates' loads (issue 32 %). With four warps per direction
+// something did), at many the latency of the candidates' loads (issue 33 %). With four warps per direction
 // that handed over in order, and the coarser levels in the pair's CTA: one 1080p pair 287 ms, 23 ms now; 32
-// frames of 640x360 12.6 and 3.5 ms; 240 frames of 1080p 1087 and 729 ms.
+// frames of 640x360 12.6 and 3.5 ms; 240 frames of 1080p 1087 and 730 ms.
 // A level with an input on which the reference would panic takes search_level instead.
 // stats (nullable): [0] blocks, [1] blocks that started before all their processed neighbours were
 // final, [2] seeds evaluated after the start (the others had the vector of a candidate already
@@ -1916,7 +1914,7 @@ __device__ __forceinline__ long long floor_div(long long a, long long b) {  // i
 // interpolated onto the half-size output blocks and each block whose interpolated score is
 // above the threshold is searched again. Blocks do not read each other's results, so the
 // visiting order does not matter: one warp takes one block, with the same evaluation machinery as
-// the hierarchy. x: a one-warp group; `border`: the block shape x is set to, -1 before the first
+// the hierarchy. x: a one-warp group; `shape`: the block shape x is set to, -1 before the first
 // block. Output: ds.vec[1] / ds.luma[1].
 template <class SH>
 __device__ __forceinline__ void refine_block(Ctx &x, SH &s, DirScratch &ds, int bx, int by, int &shape) {

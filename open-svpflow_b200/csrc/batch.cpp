@@ -8,7 +8,7 @@
 // size, as many as still give every search direction four warps or more on the whole GPU, level by
 // level, the clips' finest levels aligned (batch_ground_kernel, batch_walk_kernel). The other
 // shapes let a grid of resident CTAs drain the list through a device-side counter, a pair per
-// CTA (analyse_batch_kernel): 12 clips of 320x240 to 854x480 take 128 ms walked and 320 ms
+// CTA (analyse_batch_kernel): 12 clips of 320x240 to 854x480 take 130 ms walked and 320 ms
 // drained by the fastest of them, since a drained pair runs at one CTA's speed.
 //
 // Device memory of a batch is one allocation made at creation: every clip's source

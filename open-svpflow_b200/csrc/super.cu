@@ -558,10 +558,10 @@ __global__ void __launch_bounds__(256, 4) super_level01_kernel(SuperDev D, const
 // layout): any width, any alignment, both sample types. Level 0 is then one flat stream per plane
 // (its sub-planes follow one another without a gap), and the pyramid is reduced by warps that walk
 // down the rows.
-// Bound: level 0 by its stores (240 frames of 1080p: 3.8 GB in 755 us, 5.05 TB/s), the pyramid by the filters'
-// instruction issue (65 % on its first levels, 416 and 141 us). With rows staged in shared memory, or a CTA per
+// Bound: level 0 by its stores (240 frames of 1080p: 3.8 GB in 745 us, 5.1 TB/s), the pyramid by the filters'
+// instruction issue (65 % on its first levels, 419 and 140 us). With rows staged in shared memory, or a CTA per
 // row where rows are not on 16 bytes: 1.81 and 1.45 ms for that call, 938 and 196 us for 48 frames of 854x480,
-// 2.31 and 0.69 ms for 6 frames of 2160p at 10 bits, 94 and 35 us for one of 640x360 (9 launches, 2 now).
+// 2.31 and 0.68 ms for 6 frames of 2160p at 10 bits, 94 and 35 us for one of 640x360 (9 launches, 2 now).
 
 // Sample arithmetic in 32-bit words: 4 bytes or 2 halfwords.
 template <typename T>
@@ -1435,9 +1435,9 @@ int launch_super_flat(const SuperDev &D, const uint8_t *src, uint8_t *dst, int n
         const int64_t bytes = all ? sub : sub * nsub;
         return (uint32_t)((bytes / 16 + 1 + F.tile) / F.tile);
     };
-    // Level 0 in a launch of its own where every resident CTA has a large tile: 240 frames of 1080p 1440 us against
-    // 2209 together with the first reduction, 6 of 2160p at 10 bits 691 against 1143, 48 of 854x480 195 against 211;
-    // one frame of 640x360 39.0 against 34.9.
+    // Level 0 in a launch of its own where every resident CTA has a large tile. Against it together with the first
+    // reduction, us: 48 frames of 1080p 340 and 384, 8 of them 119 and 124, 1 of them 59.8 and 57.3; 48 of 854x480 194
+    // and 206, 6 of them 85.2 and 82.0; one of 640x360 39.0 and 34.9; 48 of 2160p at 10 bits 4760 and 4826.
     F.tile = (int64_t)nframes * D.frame_bytes >= (int64_t)sms * 6 * 1024 * 16 ? 1024 : 256;
     F.ty = tiles((int64_t)D.width * D.height, F.all_y);
     F.tc = tiles((int64_t)(D.width / 2) * (D.height / 2), F.all_c);
