@@ -32,7 +32,7 @@ def test_the_pool_stays_within_the_budget_and_is_given_back():
     import svpflow_b200 as sv
     from svpflow_b200.synth import make_clip
 
-    opt = "{block:{w:8,overlap:3},main:{search:{type:4,distance:8,satd:true}}}"  # searches that outlast the queueing
+    opt = "{block:{w:8,overlap:3},main:{search:{type:4,distance:24,satd:true}}}"  # searches that outlast the queueing by far
     chunk = 4
     clips = []
     for k, n in enumerate((8, 8, 24)):
