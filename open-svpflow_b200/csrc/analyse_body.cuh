@@ -508,8 +508,7 @@ __device__ __forceinline__ unsigned sad4(const Smp &s, const Smp &r, unsigned m,
     return __dp4a(__vabsdiffu4(s.a, r.a), m & 0x01010101u, acc);
 }
 __device__ __forceinline__ unsigned sum4(const Smp &s) { return __dp4a(s.a, 0x01010101u, 0u); }
-__device__ __forceinline__ unsigned high_bits(const Smp &) { return 0u; }
-constexpr bool kMayExceed = false;
+constexpr unsigned kHighBits = 0u;
 #else
 // four 16-bit samples (2-byte aligned): three aligned words funnel-shifted into two pairs
 __device__ __forceinline__ Smp ld4(const Frame &f, unsigned o) {
@@ -518,10 +517,9 @@ __device__ __forceinline__ Smp ld4(const Frame &f, unsigned o) {
     return Smp{__funnelshift_r(w0, w1, o * 8u), __funnelshift_r(w1, w2, o * 8u)};
 }
 // Samples 0..1023 fit the mantissa of 1024 + s too. Larger ones are outside the extension's range but not refused: the
-// callers look at high_bits of what they turn into halves, and take the general path, which is right for every
-// uint16, where any is set.
-__device__ __forceinline__ unsigned high_bits(const Smp &w) { return (w.a | w.b) & 0xFC00FC00u; }
-constexpr bool kMayExceed = true;
+// callers gather the bits of what they turn into halves, and take the general path, which is right for every
+// uint16, where any of kHighBits is set.
+constexpr unsigned kHighBits = 0xFC00FC00u;
 __device__ __forceinline__ void halves(const Smp &w, uint32_t &lo, uint32_t &hi) {
     lo = w.a | 0x64006400u;
     hi = w.b | 0x64006400u;
@@ -775,7 +773,7 @@ __device__ __forceinline__ void eval_groups(const Ctx &x, int g0, const unsigned
             for (int q = 0; q < NB; q++) {
                 uint32_t lo, hi;
                 halves(w[u][q], lo, hi);
-                high |= high_bits(w[u][q]);
+                if (kHighBits) high |= w[u][q].a | w[u][q].b;
                 const float4 d = mma_hadamard(x.h, lo, hi, c[u]);
                 const float v = (fabsf(d.x) + fabsf(d.y)) + (fabsf(d.z) + fabsf(d.w));
                 fl[q] = fmaf(v, wl, fl[q]);
@@ -796,15 +794,14 @@ __device__ __forceinline__ void eval_groups(const Ctx &x, int g0, const unsigned
 // NB candidates on the fast path by the whole warp. lref, cref: the lanes' set-ups; m: the lanes
 // still to take, of which the lowest NB go (fewer left: the last one again, unused). Three groups,
 // all SATD (16x16 blocks with chroma, TRI): in one go; else group by group. A 4x4 tile's SATD is even
-// (its coefficients share their parity), so halving the sum of tiles is halving each plane's. Lanes whose
-// candidate may hold samples too large for it are added to `redo`.
+// (its coefficients share their parity), so halving the sum of tiles is halving each plane's. `high` gathers the bits of
+// the samples turned into halves.
 template <int NB, bool TRI>
 __device__ __forceinline__ void eval_fast(const Ctx &x, unsigned lref, unsigned cref, unsigned &m, unsigned &L, unsigned &C,
-                                          unsigned &redo) {
+                                          unsigned &high) {
     const int lane = x.tid & 31;
     unsigned lr[NB], cr[NB], il[NB], ic[NB];
     float fl[NB], fc[NB];
-    unsigned high = 0;
     int who[NB];
 #pragma unroll
     for (int q = 0; q < NB; q++) {
@@ -833,10 +830,6 @@ __device__ __forceinline__ void eval_fast(const Ctx &x, unsigned lref, unsigned 
             C = x.satd ? (sc >> 1) * 4u : sc * 4u;
         }
     }
-    if (kMayExceed && __any_sync(kFull, high != 0)) {
-#pragma unroll
-        for (int q = 0; q < NB; q++) redo |= 1u << who[q];
-    }
 }
 
 // The block's source for the fast path (Ctx::src) and the sum of its luma samples, each warp of
@@ -847,11 +840,11 @@ __device__ __forceinline__ unsigned stage_source(const Ctx &x, BlkC &b) {
     const int lane = x.tid & 31;
     const unsigned lo_ = (unsigned)b.lsrc * (unsigned)sizeof(px_t) + x.fs.mis, co = (unsigned)b.csrc * (unsigned)sizeof(px_t) + x.fs.mis;
 #pragma unroll 1
-    for (int g = kMayExceed ? 0 : x.tid >> 5; g < x.ng; g += kMayExceed ? 1 : x.nw) {
+    for (int g = kHighBits ? 0 : x.tid >> 5; g < x.ng; g += kHighBits ? 1 : x.nw) {
         const bool chroma = (x.cmask >> g) & 1u;
         const Smp w = ld4(x.fs, (chroma ? co : lo_) + x.off[g * 32 + lane]);
-        if ((x.smask >> g) & 1u) high |= high_bits(w);
-        if (kMayExceed && x.nw > 1 && g % x.nw != (x.tid >> 5)) continue;
+        if (kHighBits && ((x.smask >> g) & 1u)) high |= w.a | w.b;
+        if (kHighBits && x.nw > 1 && g % x.nw != (x.tid >> 5)) continue;
         if (((x.lmask >> g) & 1u) && !(x.lshift == 2 && lane >= 4)) s += sum4(w);
         float4 c = make_float4(__uint_as_float(w.a), __uint_as_float(w.b), 0.f, 0.f);
         if ((x.smask >> g) & 1u) {
@@ -862,7 +855,7 @@ __device__ __forceinline__ unsigned stage_source(const Ctx &x, BlkC &b) {
         }
         x.src[g * 32 + lane] = c;
     }
-    if (kMayExceed && __any_sync(kFull, high != 0)) {
+    if (kHighBits && __any_sync(kFull, (high & kHighBits) != 0)) {
         __syncwarp();
         b.fast_src = 0;
         b.fx1 = b.fx0 - 1;  // an empty box
@@ -983,7 +976,7 @@ __device__ __noinline__ uint2 clamped_cands(const AnalyseParams *Pp, const Level
                     for (int q = 0; q < NB; q++) {
                         uint32_t lo, hi;
                         halves(w[q], lo, hi);
-                        high |= high_bits(w[q]);
+                        if (kHighBits) high |= w[q].a | w[q].b;
                         const float4 d = mma_hadamard(h, lo, hi, c);
                         const float v = (fabsf(d.x) + fabsf(d.y)) + (fabsf(d.z) + fabsf(d.w));
                         fl[q] = fmaf(v, wl, fl[q]);
@@ -1007,7 +1000,7 @@ __device__ __noinline__ uint2 clamped_cands(const AnalyseParams *Pp, const Level
                 if (lane == who[q])
                     out = make_uint2(sl >> lshift, L.satd && ((cdm >> who[q]) & 1u) ? (st_ >> 1) * 4u : sa * 4u);
             }
-            if (kMayExceed && __any_sync(kFull, high != 0)) {
+            if (kHighBits && __any_sync(kFull, (high & kHighBits) != 0)) {
 #pragma unroll
                 for (int q = 0; q < NB; q++) ms |= 1u << who[q];
             }
@@ -1035,12 +1028,15 @@ __device__ __forceinline__ void eval_cands(const Ctx &x, const BlkC &b, bool ok,
     const bool fast = ok && fast_setup(x, b, mvx, mvy, lref, cref);
     unsigned mf = __ballot_sync(kFull, fast), ms = __ballot_sync(kFull, ok && !fast);
     L = C = 0;
+    unsigned high = 0;
+    const unsigned all = mf;
 #pragma unroll 1
     while (mf) {
-        if (x.ng == 3 && x.smask == 7u) eval_fast<4, true>(x, lref, cref, mf, L, C, ms);
-        else if (__popc(mf) > 4) eval_fast<8, false>(x, lref, cref, mf, L, C, ms);
-        else eval_fast<4, false>(x, lref, cref, mf, L, C, ms);
+        if (x.ng == 3 && x.smask == 7u) eval_fast<4, true>(x, lref, cref, mf, L, C, high);
+        else if (__popc(mf) > 4) eval_fast<8, false>(x, lref, cref, mf, L, C, high);
+        else eval_fast<4, false>(x, lref, cref, mf, L, C, high);
     }
+    if (kHighBits && __any_sync(kFull, (high & kHighBits) != 0)) ms |= all;  // samples too large for the fast path
     if (ms) {
         const uint2 r = clamped_cands(x.P, x.L, x.S.y, x.R.y, x.src, x.level, b.px, b.py, ms, mvx, mvy,
                                       (b.chroma ? SLOW_CHROMA : 0) | (b.fast_src ? SLOW_STAGED : 0));
